@@ -576,7 +576,7 @@ int run_plan(ket_state* s, const Plan& plan, const ket_exec_opts& o, bool wait, 
       for (int gi : p.gates) devops.push_back(encode_devop(plan.gates[gi], p, prune));
     } else {
       const Gate& g = plan.gates[p.gates[0]];
-      if (g.type == G_MATK) {
+      if (matk_on_device(g)) {
         matk_off[i] = matk_bytes;
         matk_bytes += 64 + 16 * g.mk.size();
         matk_bytes = (matk_bytes + 255) & ~size_t(255);
@@ -597,7 +597,7 @@ int run_plan(ket_state* s, const Plan& plan, const ket_exec_opts& o, bool wait, 
       const Pass& p = plan.passes[first + i];
       if (p.fused) continue;
       const Gate& g = plan.gates[p.gates[0]];
-      if (g.type != G_MATK) continue;
+      if (!matk_on_device(g)) continue;
       unsigned char* dst = host.data() + f_bytes + d_bytes + matk_off[i];
       int* q = reinterpret_cast<int*>(dst);
       for (size_t j = 0; j < g.tk.size(); j++) q[j] = g.tk[j];
@@ -639,7 +639,7 @@ int run_plan(ket_state* s, const Plan& plan, const ket_exec_opts& o, bool wait, 
     } else {
       const Gate& g = plan.gates[p.gates[0]];
       const void* mk =
-          g.type == G_MATK ? (const void*)((const char*)dev + f_bytes + d_bytes + matk_off[i]) : nullptr;
+          matk_on_device(g) ? (const void*)((const char*)dev + f_bytes + d_bytes + matk_off[i]) : nullptr;
       e = launch_gate(g, s->precision, s->amp, s->n, mk, c->stream);
     }
     prof_end(c, kind);

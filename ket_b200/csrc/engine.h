@@ -57,6 +57,10 @@ struct Plan {
   int anc = -1;               // adjoint sweep: qubit that selects psi / lambda, kept in every tile
 };
 
+// A dense unitary whose matrix the kernel reads from device memory (smaller
+// ones are kernel parameters).
+inline bool matk_on_device(const Gate& g) { return g.type == G_MATK && g.tk.size() > 4; }
+
 inline bool is_grad(const Gate& g) { return g.type == G_GRADM || g.type == G_GRADD || g.type == G_GRADM2; }
 
 // Lower and validate an op list (mirrors #checkOp, circuit.ts:1113-1146).

@@ -138,48 +138,151 @@ __global__ void k_mat2(typename Vec2<R>::T* a, uint64_t nq, int ta, int tb, uint
   }
 }
 
-// Dense k-qubit unitary: one CTA per group of 2^k amplitudes, staged in smem
-// (inputs xs, outputs ys, global indices idx).
-template <typename R>
-__global__ void k_matk(typename Vec2<R>::T* a, uint64_t ngroups, int k, const int* tq, const double* mat, int prune,
-                       double thr, double qthr) {
-  extern __shared__ unsigned char smraw[];
-  const uint32_t D = 1u << k;
-  cpx<R>* xs = reinterpret_cast<cpx<R>*>(smraw);
-  cpx<R>* ys = xs + D;
-  uint64_t* idx = reinterpret_cast<uint64_t*>(ys + D);
-  int sorted[KET_MAX_OP_QUBITS];
-  for (int j = 0; j < k; j++) sorted[j] = tq[j];
-  for (int x = 1; x < k; x++)
-    for (int y = x; y > 0 && sorted[y - 1] > sorted[y]; y--) { int t = sorted[y]; sorted[y] = sorted[y - 1]; sorted[y - 1] = t; }
-  for (uint64_t g = blockIdx.x; g < ngroups; g += gridDim.x) {
-    uint64_t ctx = g;
-    for (int j = 0; j < k; j++) ctx = insert0(ctx, sorted[j]);
-    for (uint32_t i = threadIdx.x; i < D; i += blockDim.x) {
-      uint64_t b = ctx;
-      for (int bit = 0; bit < k; bit++)
-        if ((i >> (k - 1 - bit)) & 1) b |= uint64_t(1) << tq[bit];
-      idx[i] = b;
-      xs[i] = ld_amp<R>(a + b);
-    }
-    __syncthreads();
-    for (uint32_t r = threadIdx.x; r < D; r += blockDim.x) {
-      double sr = 0, si = 0;
-      const double* row = mat + 2 * (size_t)r * D;
-      for (uint32_t c = 0; c < D; c++) {
-        double mr = row[2 * c], mi = row[2 * c + 1];
-        double xr = xs[c].re, xi = xs[c].im;
-        sr = fma(mr, xr, fma(-mi, xi, sr));
-        si = fma(mr, xi, fma(mi, xr, si));
-      }
-      cpx<R> o{(R)sr, (R)si};
-      if (prune) prune_amp(o, thr, qthr);
-      ys[r] = o;
-    }
-    __syncthreads();
-    for (uint32_t r = threadIdx.x; r < D; r += blockDim.x) st_amp<R>(a + idx[r], ys[r]);
-    __syncthreads();
+// Dense k-qubit unitaries.  Row r of a group of D = 2^k amplitudes is
+// sum_c m[r][c] x[c], the terms added in ascending c in FP64 whatever the state's
+// precision (the order of applyUnitary, statevector.ts:240-270).
+
+// k = 3, 4: a thread holds the whole group in registers and the matrix is a
+// kernel parameter, so every product reads its entry from the constant bank
+// and nothing is staged or synchronised.  Bound: HBM at k = 3 (32 FP64 FMAs an
+// amplitude), about even with the FP64 pipe at k = 4 (64).  In place of one CTA
+// per group: 3 qubits on 2^25 c64 amplitudes 5.9 -> 0.08 ms, 4 qubits on 2^22
+// c128 amplitudes 0.91 -> 0.05 ms.
+template <int K>
+struct MatKArgs {
+  uint64_t off[1 << K];   // amplitude offset of local index i
+  int sorted[K];          // target qubits, ascending
+  double m[2 << (2 * K)];
+};
+
+template <typename R, int K>
+__global__ void __launch_bounds__(128) k_matk_reg(typename Vec2<R>::T* a, uint64_t ngroups,
+                                                  const __grid_constant__ MatKArgs<K> g, int prune, double thr,
+                                                  double qthr) {
+  constexpr int D = 1 << K;
+  const uint64_t id = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+  if (id >= ngroups) return;
+  uint64_t base = id;
+#pragma unroll
+  for (int j = 0; j < K; j++) base = insert0(base, g.sorted[j]);
+  typename Vec2<R>::T* p = a + base;
+  double xr[D], xi[D];
+#pragma unroll
+  for (int c = 0; c < D; c++) {
+    const cpx<R> v = ld_amp<R>(p + g.off[c]);
+    xr[c] = v.re;
+    xi[c] = v.im;
   }
+#pragma unroll
+  for (int r = 0; r < D; r++) {
+    double sr = 0, si = 0;
+#pragma unroll
+    for (int c = 0; c < D; c++) {
+      const double mr = g.m[2 * (r * D + c)], mi = g.m[2 * (r * D + c) + 1];
+      sr = fma(mr, xr[c], fma(-mi, xi[c], sr));
+      si = fma(mr, xi[c], fma(mi, xr[c], si));
+    }
+    cpx<R> o{(R)sr, (R)si};
+    if (prune) prune_amp(o, thr, qthr);
+    st_amp<R>(p + g.off[r], o);
+  }
+}
+
+// k >= 5: a CTA multiplies the matrix by the 2^12 amplitudes of GB = 2^(12-k)
+// groups, held in shared memory as FP64; each thread accumulates 4 rows x 4
+// groups in registers, so 8 shared-memory reads feed 64 FMAs, and the matrix
+// passes through shared memory 2^10 entries at a time.  Bound: the FP64 pipe.
+// From 5 qubits on a group no longer fits a thread's registers.
+constexpr int kMatkThreads = 256;
+constexpr size_t kMatkSmem = sizeof(double2) * ((1 << 12) + (1 << 10));
+
+template <typename R>
+__global__ void __launch_bounds__(kMatkThreads) k_matk(typename Vec2<R>::T* a, uint64_t ngroups, int k, const int* tq,
+                                                       const double2* mat, int prune, double thr, double qthr) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  double2* xs = reinterpret_cast<double2*>(smraw);  // [c][group]
+  double2* ms = xs + (1 << 12);                     // [column of the chunk][row]
+  __shared__ int sorted[KET_MAX_OP_QUBITS];
+  const int tid = threadIdx.x;
+  const uint32_t D = 1u << k, lgb = 12 - k, GB = 1u << lgb, cols = 1u << (10 - k);
+  const uint32_t R4 = D >> 2, G4 = GB >> 2, tr = tid & (R4 - 1), tg = tid >> (k - 2);
+  if (tid == 0) {
+    for (int j = 0; j < k; j++) {
+      int x = tq[j], y = j;
+      for (; y > 0 && sorted[y - 1] > x; y--) sorted[y] = sorted[y - 1];
+      sorted[y] = x;
+    }
+  }
+  __syncthreads();
+  auto at = [&](uint64_t group, uint32_t i) -> uint64_t {  // index of local index i of a group
+    for (int j = 0; j < k; j++) group = insert0(group, sorted[j]);
+    for (int b = 0; b < k; b++)
+      if ((i >> (k - 1 - b)) & 1) group |= uint64_t(1) << tq[b];
+    return group;
+  };
+  for (uint64_t g0 = (uint64_t)blockIdx.x << lgb; g0 < ngroups; g0 += (uint64_t)gridDim.x << lgb) {
+    for (uint32_t e = tid; e < (1u << 12); e += kMatkThreads) {
+      const uint64_t g = g0 + (e & (GB - 1));
+      double2 v = make_double2(0.0, 0.0);
+      if (g < ngroups) {
+        const cpx<R> x = ld_amp<R>(a + at(g, e >> lgb));
+        v = make_double2(x.re, x.im);
+      }
+      xs[e] = v;
+    }
+    double sr[4][4], si[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+      for (int j = 0; j < 4; j++) sr[i][j] = si[i][j] = 0.0;
+    for (uint32_t c0 = 0; c0 < D; c0 += cols) {
+      __syncthreads();
+      for (uint32_t e = tid; e < (1u << 10); e += kMatkThreads) {
+        const uint32_t r = e >> (10 - k), c = e & (cols - 1);
+        ms[c * D + r] = __ldg(mat + (size_t)r * D + c0 + c);
+      }
+      __syncthreads();
+      for (uint32_t c = 0; c < cols; c++) {
+        double2 m[4], x[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) m[i] = ms[c * D + tr + i * R4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) x[j] = xs[((c0 + c) << lgb) + tg + j * G4];
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+#pragma unroll
+          for (int j = 0; j < 4; j++) {
+            sr[i][j] = fma(m[i].x, x[j].x, fma(-m[i].y, x[j].y, sr[i][j]));
+            si[i][j] = fma(m[i].x, x[j].y, fma(m[i].y, x[j].x, si[i][j]));
+          }
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        const uint64_t g = g0 + tg + j * G4;
+        cpx<R> o{(R)sr[i][j], (R)si[i][j]};
+        if (prune) prune_amp(o, thr, qthr);
+        if (g < ngroups) st_amp<R>(a + at(g, tr + i * R4), o);
+      }
+    __syncthreads();  // xs is refilled for the next groups
+  }
+}
+
+template <typename R, int K>
+void launch_matk_reg(typename Vec2<R>::T* a, uint64_t ngroups, const Gate& g, int pr, double thr, double qthr,
+                     cudaStream_t s) {
+  MatKArgs<K> m;
+  for (int i = 0; i < (1 << K); i++) {
+    m.off[i] = 0;
+    for (int b = 0; b < K; b++)
+      if ((i >> (K - 1 - b)) & 1) m.off[i] |= uint64_t(1) << g.tk[b];
+  }
+  for (int j = 0; j < K; j++) m.sorted[j] = g.tk[j];
+  std::sort(m.sorted, m.sorted + K);
+  for (int e = 0; e < (1 << (2 * K)); e++) { m.m[2 * e] = g.mk[e].re; m.m[2 * e + 1] = g.mk[e].im; }
+  k_matk_reg<R, K><<<(unsigned)((ngroups + 127) / 128), 128, 0, s>>>(a, ngroups, m, pr, thr, qthr);
 }
 
 // ------------------------------------------------------------------ fused tile pass
@@ -342,14 +445,16 @@ cudaError_t launch_gate_t(const Gate& g, void* ampv, int n, const void* dev_matk
       break;
     }
     case G_MATK: {
-      int k = (int)g.tk.size();
+      const int k = (int)g.tk.size();
+      const uint64_t ngroups = N >> k;
+      if (k == 3) { launch_matk_reg<R, 3>(a, ngroups, g, pr, thr, qthr, s); break; }
+      if (k == 4) { launch_matk_reg<R, 4>(a, ngroups, g, pr, thr, qthr, s); break; }
       const int* dq = reinterpret_cast<const int*>(dev_matk);
-      const double* dm = reinterpret_cast<const double*>(reinterpret_cast<const char*>(dev_matk) + 64);
-      size_t smem = (2 * sizeof(cpx<R>) + sizeof(uint64_t)) * (size_t(1) << k);
-      if (smem > 48 * 1024) cudaFuncSetAttribute(k_matk<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      uint64_t ngroups = N >> k;
-      unsigned blocks = (unsigned)std::min<uint64_t>(ngroups, (uint64_t)num_sms() * 8);
-      k_matk<R><<<blocks, NT, smem, s>>>(a, ngroups, k, dq, dm, pr, thr, qthr);
+      const double2* dm = reinterpret_cast<const double2*>(reinterpret_cast<const char*>(dev_matk) + 64);
+      cudaFuncSetAttribute(k_matk<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMatkSmem);
+      const uint64_t ctas = (ngroups + (uint64_t(1) << (12 - k)) - 1) >> (12 - k);
+      k_matk<R><<<(unsigned)std::min<uint64_t>(ctas, (uint64_t)num_sms() * 2), kMatkThreads, kMatkSmem, s>>>(
+          a, ngroups, k, dq, dm, pr, thr, qthr);
       break;
     }
   }
