@@ -3,6 +3,7 @@
 // per-block partial sums in a fixed tree order, then a fixed-order combine,
 // all in FP64 whatever the state precision.
 #include <algorithm>
+#include <type_traits>
 
 #include "common.cuh"
 #include "read.h"
@@ -737,6 +738,164 @@ __global__ void __launch_bounds__(NT) k_pauli_group(const typename Vec2<R>::T* a
   if (threadIdx.x == 0) partial[blockIdx.x] = t;
 }
 
+// Sums of Pauli terms over tiles of 2^12 amplitudes held in shared memory: every
+// term whose flips lie inside the tile is evaluated on one read of the state,
+// where k_pauli_group reads it once per flip mask.
+//
+// Thread t of 512 holds amplitudes t + 512 j, so tile bits 9-11 are register bits
+// (8 amplitudes in 64 registers let 32 warps cover each other's loads; 16
+// amplitudes in 128 registers were several times slower).  A group's products are
+// |psi_y|^2 (8 a thread) or, with flips, Re or Im of conj(psi_x) psi_y, one per
+// pair, so 4 a thread: the pairs of a register flip by the member with its top
+// flip bit clear, those of a thread flip half by either thread; the other member
+// comes from shared memory.  A term's sign is a tile part, folded into its
+// coefficient once a tile, a thread part, and a parity of the products' index:
+// a group of several terms takes one Walsh transform over that index, after
+// which a term costs one addition.
+// Bound: HBM for few groups; for many, issue and the latency of the partners'
+// shared-memory reads (half a tile a group).  25 qubits, 24 Z Z and 25 X terms:
+// 26 passes of 136 us before, 3 passes of 374, 225 and 178 us now (12, 8 and 5
+// flips; one read of the state is 82 us).  Below 12 qubits a tile is not full and
+// a group a pass costs a launch each.
+constexpr int kPauliThreads = 512;
+
+// One sum over a group's products b: its terms are entries [first, first + nterms)
+// of sc (signed coefficients) and zm (thread mask | index mask << 16), sorted by
+// index mask.
+template <int NB>
+__device__ __forceinline__ double pauli_terms(double (&b)[NB], const double* sc, const uint32_t* zm, int first,
+                                              int nterms, int t) {
+  auto coeff = [&](int i, uint32_t z) {
+    const uint32_t odd = (uint32_t)__popc(t & z & 0xffffu) << 31;
+    const double c = sc[i];
+    return __hiloint2double(__double2hiint(c) ^ (int)odd, __double2loint(c));
+  };
+  if (nterms == 1) {
+    const uint32_t z = zm[first], zi = z >> 16;
+    if (zi) {
+#pragma unroll
+      for (int j = 1; j < NB; j++) {
+        const uint32_t sg = (0x96u >> (j & zi)) << 31;
+        b[j] = __hiloint2double(__double2hiint(b[j]) ^ (int)sg, __double2loint(b[j]));
+      }
+    }
+#pragma unroll
+    for (int st = NB / 2; st > 0; st >>= 1)
+#pragma unroll
+      for (int j = 0; j < st; j++) b[j] += b[j + st];
+    return coeff(first, z) * b[0];
+  }
+#pragma unroll
+  for (int st = 1; st < NB; st <<= 1)
+#pragma unroll
+    for (int j = 0; j < NB; j++)
+      if (!(j & st)) {
+        const double x = b[j], y = b[j | st];
+        b[j] = x + y;
+        b[j | st] = x - y;
+      }
+  double acc = 0.0;
+  int i = first;
+#pragma unroll
+  for (int w = 0; w < NB; w++) {
+    double c = 0.0;
+    for (; i < first + nterms; i++) {
+      const uint32_t z = zm[i];
+      if ((z >> 16) != w) break;
+      c += coeff(i, z);
+    }
+    acc += c * b[w];
+  }
+  return acc;
+}
+
+template <typename R>
+__global__ void __launch_bounds__(kPauliThreads, 2) k_pauli_tile(const typename Vec2<R>::T* a, PauliTileArgs g,
+                                                                 const PauliTileGroup* groups,
+                                                                 const PauliTileTerm* terms, double* partial) {
+  typedef typename Vec2<R>::T V;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  V* s = reinterpret_cast<V*>(smraw);
+  __shared__ double red[32];
+  __shared__ double sc[KET_PAULI_TILE_TERMS];
+  __shared__ uint32_t zm[KET_PAULI_TILE_TERMS];
+  __shared__ PauliTileGroup gs[KET_PAULI_TILE_TERMS];
+  const int t = threadIdx.x;
+  static_assert(kPauliThreads == KET_PAULI_TILE_TERMS, "one term and one group a thread");
+  if (t < g.ngroups) gs[t] = groups[t];
+  double coeff = 0.0;
+  uint64_t zctx = 0;
+  if (t < g.nterms) {
+    coeff = terms[t].coeff;
+    zctx = terms[t].zctx;
+    zm[t] = terms[t].zm;
+  }
+  const int lane = t & 31, ctxq = lane < g.nctx ? g.ctxbits[lane] : 63;
+  uint64_t toff = 0;
+#pragma unroll
+  for (int b = 0; b < 9; b++)
+    if ((t >> b) & 1) toff |= uint64_t(1) << g.bits[b];
+  double acc = 0.0;
+  for (uint64_t tile = blockIdx.x; tile < g.ntiles; tile += gridDim.x) {
+    // lane b places tile bit b (at most 28 qubits lie outside the tile)
+    const uint64_t mine = ((tile >> lane) & 1) << ctxq;
+    const uint64_t ctx = ((uint64_t)__reduce_or_sync(0xffffffffu, (uint32_t)(mine >> 32)) << 32) |
+                         __reduce_or_sync(0xffffffffu, (uint32_t)mine);
+    V v[8];
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+      uint64_t o = ctx | toff;
+#pragma unroll
+      for (int b = 0; b < 3; b++)
+        if ((j >> b) & 1) o |= uint64_t(1) << g.bits[9 + b];
+      v[j] = a[o];
+    }
+    __syncthreads();  // the last tile's reads of s and sc are done
+    if (t < g.nterms) sc[t] = (__popcll(ctx & zctx) & 1) ? -coeff : coeff;
+    if (g.flips) {
+#pragma unroll
+      for (int j = 0; j < 8; j++) s[t + 512 * j] = v[j];
+    }
+    __syncthreads();
+    for (int k = 0; k < g.ngroups; k++) {
+      const PauliTileGroup G = gs[k];
+      if (G.flip == 0) {
+        double b[8];
+#pragma unroll
+        for (int j = 0; j < 8; j++) b[j] = norm2_ref(v[j].x, v[j].y);
+        acc += pauli_terms<8>(b, sc, zm, G.first, G.nterms, t);
+        continue;
+      }
+      double b[4];
+      // this thread's pairs: register index u with a bit inserted at P, clear for a
+      // register flip, the thread's top flip bit (`set`) for a thread flip
+      auto products = [&](auto PP, auto ODD, bool set) {
+        constexpr int P = decltype(PP)::value;
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+          const int j0 = ((u >> P) << (P + 1)) | (u & ((1 << P) - 1)), j1 = j0 | (1 << P);
+          const V w = s[(t + 512 * (set ? j1 : j0)) ^ G.flip];
+          const double vr = set ? v[j1].x : v[j0].x, vi = set ? v[j1].y : v[j0].y, wr = w.x, wi = w.y;
+          b[u] = decltype(ODD)::value ? vi * wr - vr * wi : vr * wr + vi * wi;
+        }
+      };
+      auto by_top = [&](auto ODD) {
+        switch (G.top) {
+          case 9: products(std::integral_constant<int, 0>(), ODD, false); break;
+          case 10: products(std::integral_constant<int, 1>(), ODD, false); break;
+          case 11: products(std::integral_constant<int, 2>(), ODD, false); break;
+          default: products(std::integral_constant<int, 2>(), ODD, (t >> G.top) & 1); break;
+        }
+      };
+      if (G.odd) by_top(std::true_type());
+      else by_top(std::false_type());
+      acc += pauli_terms<4>(b, sc, zm, G.first, G.nterms, t);
+    }
+  }
+  const double sum = block_sum<kPauliThreads>(acc, red);
+  if (t == 0) partial[blockIdx.x] = sum;
+}
+
 inline unsigned gridn(uint64_t work, int nt, int cap_per_sm = 16) {
   uint64_t b = (work + nt - 1) / nt;
   uint64_t cap = (uint64_t)num_sms() * cap_per_sm;
@@ -911,6 +1070,28 @@ cudaError_t launch_pauli_group(const void* amp, int n, int prec, const PauliGrou
   return prec == KET_C64 ? pauli_t<float>(amp, n, g, partial, out, s) : pauli_t<double>(amp, n, g, partial, out, s);
 }
 size_t pauli_scratch(int n) { return 8 * 4096 + 64; }
+
+unsigned pauli_tile_grid(int n) {
+  return (unsigned)std::min<uint64_t>(uint64_t(1) << (n - KET_PAULI_TILE_BITS), (uint64_t)num_sms() * 2);
+}
+template <typename R>
+static cudaError_t pauli_tile_t(const void* amp, const PauliTileArgs& g, const PauliTileGroup* groups,
+                                const PauliTileTerm* terms, double* partial, unsigned grid, cudaStream_t s) {
+  const int smem = (int)(sizeof(typename Vec2<R>::T) << KET_PAULI_TILE_BITS);
+  cudaError_t e = cudaFuncSetAttribute(k_pauli_tile<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) return e;
+  k_pauli_tile<R><<<grid, kPauliThreads, smem, s>>>((const typename Vec2<R>::T*)amp, g, groups, terms, partial);
+  return cudaGetLastError();
+}
+cudaError_t launch_pauli_tile(const void* amp, int n, int prec, const PauliTileArgs& g, const PauliTileGroup* groups,
+                              const PauliTileTerm* terms, double* partial, cudaStream_t s) {
+  return prec == KET_C64 ? pauli_tile_t<float>(amp, g, groups, terms, partial, pauli_tile_grid(n), s)
+                         : pauli_tile_t<double>(amp, g, groups, terms, partial, pauli_tile_grid(n), s);
+}
+cudaError_t launch_sum(const double* partial, uint64_t count, double* out, cudaStream_t s) {
+  k_sum<256><<<1, 256, 0, s>>>(partial, count, out);
+  return cudaGetLastError();
+}
 
 template <typename RA, typename RB>
 static cudaError_t compare_t(const void* a, const void* b, int n, double* scratch, double* out, cudaStream_t s) {

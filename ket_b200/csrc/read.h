@@ -25,6 +25,30 @@ struct PauliGroup {
   double coeff[KET_PAULI_GROUP_TERMS];
 };
 
+// Tiled Pauli sums: a tile is 2^12 amplitudes, tile bit b = qubit bits[b].
+#define KET_PAULI_TILE_BITS 12
+#define KET_PAULI_TILE_LOW 4     // qubits 0-3 stay tile bits 0-3: 256 contiguous bytes at c128, 128 at c64
+#define KET_PAULI_TILE_TERMS 512 // terms (so groups) of one pass
+struct PauliTileArgs {
+  uint64_t ntiles;
+  int ngroups, nterms, flips;    // flips: whether any group flips a qubit
+  int nctx;
+  int bits[KET_PAULI_TILE_BITS];
+  int ctxbits[KET_MAX_QUBITS];   // qubits outside the tile, ascending
+};
+struct PauliTileGroup {          // terms sharing a flip mask and i^ny
+  uint32_t flip;                 // tile bits
+  uint8_t top, odd;              // highest flipped tile bit; whether the imaginary part counts
+  uint16_t nterms;
+  int32_t first;
+};
+struct PauliTileTerm {
+  double coeff;                  // with the sign of i^ny folded in, and 2 for a pair
+  uint64_t zctx;                 // Z|Y qubits outside the tile
+  uint32_t zm;                   // thread mask | mask over the products' index << 16
+  uint32_t pad;
+};
+
 int num_sms();
 
 cudaError_t launch_norm2(const void* amp, int n, int prec, double* scratch, double* out, cudaStream_t s);
@@ -51,6 +75,12 @@ cudaError_t launch_gather(const void* amp, int prec, const uint64_t* idx, uint64
 cudaError_t launch_pauli_group(const void* amp, int n, int prec, const PauliGroup& g, double* partial, double* out,
                                cudaStream_t s);
 size_t pauli_scratch(int n);
+// One pass of tiled Pauli sums: pauli_tile_grid(n) partials.
+unsigned pauli_tile_grid(int n);
+cudaError_t launch_pauli_tile(const void* amp, int n, int prec, const PauliTileArgs& g, const PauliTileGroup* groups,
+                              const PauliTileTerm* terms, double* partial, cudaStream_t s);
+// Fixed-order sum of `count` partials.
+cudaError_t launch_sum(const double* partial, uint64_t count, double* out, cudaStream_t s);
 
 // <a|b> (re, im) and max |a_i - b_i| of two states of the same size, any precisions.
 cudaError_t launch_compare(const void* a, int pa, const void* b, int pb, int n, double* scratch, double* out,
