@@ -168,11 +168,9 @@ int ket_marginal_dist(const ket_state* s, const int* qubits, int m, double* out)
     spec.q[k] = qubits[k];
     spec.mask |= uint64_t(1) << qubits[k];
   }
-  int c = mdist_chunk_bits(s->n, m);
-  uint64_t nb = uint64_t(1) << (s->n - c);
   uint64_t width = uint64_t(1) << m;
   void* scr;
-  TRY(ctx_scratch(s->ctx, 8 * (nb * width + width) + 512, &scr));
+  TRY(ctx_scratch(s->ctx, 8 * (mdist_partials(s->n, spec.mask) + width) + 512, &scr));
   double* res = (double*)scr;
   double* partial = (double*)align_up((char*)(res + width), 256);
   TRY(LAUNCH_READ2(s->ctx, launch_marginal_dist(s->amp, s->n, s->precision, spec, partial, res, s->ctx->stream)));

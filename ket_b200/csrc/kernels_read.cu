@@ -41,13 +41,31 @@ __global__ void __launch_bounds__(NT) k_sum(const double* partial, uint64_t n, d
   if (threadIdx.x == 0) *out = t;
 }
 
-// out[j] = sum over blocks b of partial[b*stride + j], in block order.
-__global__ void k_sum_columns(const double* partial, uint64_t nblocks, int width, double* out) {
-  int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= width) return;
+// out[j] = sum over rows b of partial[b*width + j], in a fixed order: 32 threads
+// a column, each a strided run of rows (64 of the 2048 partials marginals makes,
+// several loads in flight), then their sums in order.  One thread a column took
+// 179 us for those 2048 rows, this takes 12.
+constexpr int kColRows = 32;
+__device__ __forceinline__ void column_combine(double acc, int j, int width, double* out) {
+  __shared__ double red[kColRows][33];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  red[ty][tx] = acc;
+  __syncthreads();
+  if (ty == 0 && j < width) {
+    double t = red[0][tx];
+    for (int r = 1; r < kColRows; r++) t += red[r][tx];
+    out[j] = t;
+  }
+}
+__global__ void __launch_bounds__(32 * kColRows) k_sum_columns(const double* partial, uint64_t rows, int width,
+                                                               double* out) {
+  const int j = blockIdx.x * 32 + (threadIdx.x & 31);
   double acc = 0.0;
-  for (uint64_t b = 0; b < nblocks; b++) acc += partial[b * width + j];
-  out[j] = acc;
+  if (j < width) {
+#pragma unroll 8
+    for (uint64_t b = threadIdx.x >> 5; b < rows; b += kColRows) acc += partial[b * width + j];
+  }
+  column_combine(acc, j, width, out);
 }
 
 // ------------------------------------------------------------------ state comparison
@@ -155,69 +173,176 @@ __global__ void __launch_bounds__(NT) k_compact_kept(const typename Vec2<R>::T* 
 }
 
 // ------------------------------------------------------------------ marginals
-// P(q = 1) for every qubit: per-block partials [block][n].
-template <typename R, int NT>
-__global__ void __launch_bounds__(NT) k_marginals(const typename Vec2<R>::T* a, int n, uint64_t chunk, double* partial) {
-  __shared__ double red[32];
-  uint64_t N = uint64_t(1) << n;
-  uint64_t lo = blockIdx.x * chunk, hi = min(N, lo + chunk);
-  double acc[KET_MAX_QUBITS];
+// P(q = 1) for every qubit: per-block partials [block][n].  A block covers 2^c
+// indices; index bits 0-7 are thread bits, 8-11 register bits (16 amplitudes in
+// flight a thread), 12..c-1 loop bits, the rest the block's.  The 16
+// probabilities are added pairwise, level by level, and each level's odd halves are
+// its bit's marginal: about 3 additions an amplitude in place of one for every
+// qubit, which made the pass FP64-bound (27 qubits: 2.03 -> 0.36 ms; one read of
+// the state is 0.33).
+constexpr int kMargLoopBits = KET_MAX_QUBITS - 11 - 12;  // marg_chunk() leaves at most 2^11 blocks
+
+template <typename R>
+__global__ void __launch_bounds__(256) k_marginals(const typename Vec2<R>::T* a, int n, int c, double* partial) {
+  constexpr int NV = 1 + 4 + 5 + kMargLoopBits;  // total, register bits, lane bits, loop bits
+  __shared__ double ws[8][NV];
+  const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+  const uint64_t N = uint64_t(1) << n, base = (uint64_t)blockIdx.x << c;
+  double tot = 0.0, mj[4] = {0.0, 0.0, 0.0, 0.0}, mo[kMargLoopBits];
 #pragma unroll
-  for (int q = 0; q < KET_MAX_QUBITS; q++) acc[q] = 0.0;
-  for (uint64_t i = lo + threadIdx.x; i < hi; i += NT) {
-    double p = pref<R>(a, i);
+  for (int b = 0; b < kMargLoopBits; b++) mo[b] = 0.0;
+  for (uint64_t o = 0; o < uint64_t(1) << (c - 12); o++) {
+    double p[16];
 #pragma unroll
-    for (int q = 0; q < KET_MAX_QUBITS; q++)
-      if (q < n && ((i >> q) & 1)) acc[q] += p;
-  }
-#pragma unroll
-  for (int q = 0; q < KET_MAX_QUBITS; q++) {
-    if (q < n) {  // uniform across the block
-      double t = block_sum<NT>(acc[q], red);
-      if (threadIdx.x == 0) partial[blockIdx.x * (uint64_t)n + q] = t;
+    for (int j = 0; j < 16; j++) {
+      const uint64_t i = base | (o << 12) | (uint64_t)(j << 8) | t;
+      p[j] = i < N ? pref<R>(a, i) : 0.0;
     }
+#pragma unroll
+    for (int b = 0; b < 4; b++) {
+      double odd = 0.0;
+#pragma unroll
+      for (int j = 0; j < (8 >> b); j++) {
+        odd += p[2 * j + 1];
+        p[j] = p[2 * j] + p[2 * j + 1];
+      }
+      mj[b] += odd;
+    }
+    tot += p[0];
+#pragma unroll
+    for (int b = 0; b < kMargLoopBits; b++)
+      if ((o >> b) & 1) mo[b] += p[0];
+  }
+  auto put = [&](int k, double v) {
+    v = warp_sum(v);
+    if (lane == 0) ws[w][k] = v;
+  };
+  put(0, tot);
+#pragma unroll
+  for (int b = 0; b < 4; b++) put(1 + b, mj[b]);
+#pragma unroll
+  for (int b = 0; b < 5; b++) put(5 + b, ((lane >> b) & 1) ? tot : 0.0);
+#pragma unroll
+  for (int b = 0; b < kMargLoopBits; b++)
+    if (b < c - 12) put(10 + b, mo[b]);
+  __syncthreads();
+  if (t < n) {
+    const int q = t;
+    const int k = q < 5 ? 5 + q : q < 8 ? 0 : q < 12 ? 1 + (q - 8) : q < c ? 10 + (q - 12) : 0;
+    double sum = 0.0;
+    for (int x = 0; x < 8; x++)
+      if (q < 5 || q >= 8 || ((x >> (q - 5)) & 1)) sum += ws[x][k];
+    if (q >= c && !((base >> q) & 1)) sum = 0.0;
+    partial[blockIdx.x * (uint64_t)n + q] = sum;
   }
 }
 
-// Joint distribution of m qubits.  Block b covers indices [b*2^c, (b+1)*2^c).
-// Thread u walks the in-chunk bin combination u over the other in-chunk bits
-// in ascending order; the out-of-chunk bin bits are fixed by the block.
+// Joint distribution of the qubits in `mask`: per-block sums over the in-block
+// bins (bin bits in ascending qubit order).  A block covers 2^c indices, split as
+// in k_marginals.  Register sums v[j] run over the loop bits outside the mask;
+// for each setting of the masked loop bits the register bits, then the lane bits
+// outside the mask are folded, and the warps' sums added in shared memory.  Every
+// load is of consecutive amplitudes and every block runs 16 of them a thread, where
+// a thread a bin over 2^20 indices left most of the chip idle (20 qubits, 10 low
+// qubits: one block, 489 -> 8 us; 27 qubits: 2.86 -> 0.30 ms).
 template <typename R>
-__global__ void k_marginal_dist(const typename Vec2<R>::T* a, int c, MarginalSpec spec, double* partial) {
-  uint64_t base = (uint64_t)blockIdx.x << c;
-  uint64_t chunkmask = (c >= 64) ? ~uint64_t(0) : ((uint64_t(1) << c) - 1);
-  uint64_t inmask = spec.mask & chunkmask;
-  uint64_t other = chunkmask & ~inmask;
-  int nin = __popcll(inmask);
-  uint32_t width = 1u << spec.m;
-  // out-of-chunk bin bits from the block base
-  uint32_t outbin = 0;
-  for (int k = 0; k < spec.m; k++)
-    if (spec.q[k] >= c && ((base >> spec.q[k]) & 1)) outbin |= 1u << k;
-  for (uint32_t u = threadIdx.x; u < (1u << nin); u += blockDim.x) {
-    // scatter u over inmask
-    uint64_t ubits = 0;
-    {
-      uint64_t msk = inmask;
-      uint32_t uu = u;
-      while (msk) {
-        uint64_t low = msk & (~msk + 1);
-        if (uu & 1) ubits |= low;
-        uu >>= 1;
-        msk ^= low;
-      }
-    }
-    double acc = 0.0;
+__global__ void __launch_bounds__(256) k_marginal_dist(const typename Vec2<R>::T* a, int n, int c, uint64_t mask,
+                                                       double* partial) {
+  __shared__ double red[8][16][32];
+  const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+  const uint64_t N = uint64_t(1) << n, base = (uint64_t)blockIdx.x << c, inmask = mask & ((uint64_t(1) << c) - 1);
+  const uint32_t tmask = (uint32_t)inmask & 0xffu, jmask = (uint32_t)(inmask >> 8) & 15u;
+  const uint64_t omask = inmask >> 12, oother = ((uint64_t(1) << (c - 12)) - 1) & ~omask;
+  const uint32_t tj = tmask | jmask << 8, wother = 7u & ~(tmask >> 5);
+  const uint32_t nout = 1u << __popc(tj);
+  double* dst = partial + ((uint64_t)blockIdx.x << __popcll(inmask));
+  uint64_t uo = 0;
+  do {
+    double v[16];
+#pragma unroll
+    for (int j = 0; j < 16; j++) v[j] = 0.0;
     uint64_t x = 0;
     do {
-      acc += pref<R>(a, base | ubits | x);
-      x = (x - other) & other;
+      const uint64_t i0 = base | ((uo | x) << 12) | t;
+#pragma unroll
+      for (int j = 0; j < 16; j++) {
+        const uint64_t i = i0 | (uint64_t)(j << 8);
+        if (i < N) v[j] += pref<R>(a, i);
+      }
+      x = (x - oother) & oother;
     } while (x != 0);
-    uint32_t bin = outbin;
-    for (int k = 0; k < spec.m; k++)
-      if (spec.q[k] < c && ((ubits >> spec.q[k]) & 1)) bin |= 1u << k;
-    partial[(uint64_t)blockIdx.x * width + bin] = acc;
+#pragma unroll
+    for (int b = 0; b < 4; b++)
+      if (!((jmask >> b) & 1)) {
+#pragma unroll
+        for (int j = 0; j < 16; j++)
+          if (!((j >> b) & 1)) v[j] += v[j | 1 << b];
+      }
+#pragma unroll
+    for (int j = 0; j < 16; j++) {
+      if (j & ~jmask) continue;
+#pragma unroll
+      for (int b = 0; b < 5; b++)
+        if (!((tmask >> b) & 1)) v[j] += __shfl_xor_sync(0xffffffffu, v[j], 1 << b);
+    }
+    __syncthreads();  // the last round's sums are read
+    if (!(lane & ~tmask)) {
+#pragma unroll
+      for (int j = 0; j < 16; j++)
+        if (!(j & ~jmask)) red[w][j][lane] = v[j];
+    }
+    __syncthreads();
+    for (uint32_t e = t; e < nout; e += 256) {
+      uint32_t at = 0, m = tj;  // e scattered over the masked thread and register bits
+      for (uint32_t y = e; y; y >>= 1, m &= m - 1)
+        if (y & 1) at |= m & (0u - m);
+      double sum = 0.0;
+      uint32_t z = 0;
+      do {
+        sum += red[((at >> 5) & 7u) | z][at >> 8][at & 31];
+        z = (z - wother) & wother;
+      } while (z != 0);
+      dst[e] = sum;
+    }
+    dst += nout;
+    uo = (uo - omask) & omask;
+  } while (uo != 0);
+}
+
+// out[bin] = sum of the blocks' sums whose out-of-block bits match the bin, in
+// ascending block order within each of 32 strided runs, the runs in order.
+__global__ void __launch_bounds__(32 * kColRows) k_marginal_dist_combine(const double* partial, int n, int c,
+                                                                         MarginalSpec spec, double* out) {
+  const uint32_t bin = blockIdx.x * 32 + (threadIdx.x & 31), width = 1u << spec.m;
+  const uint64_t inmask = spec.mask & ((uint64_t(1) << c) - 1);
+  const int nin = __popcll(inmask);
+  double acc = 0.0;
+  if (bin < width) {
+    uint64_t at = 0, ob = 0;  // the bin's place in a block, and its block bits
+    for (int k = 0; k < spec.m; k++) {
+      if (!((bin >> k) & 1)) continue;
+      if (spec.q[k] < c) at |= uint64_t(1) << __popcll(inmask & ((uint64_t(1) << spec.q[k]) - 1));
+      else ob |= uint64_t(1) << (spec.q[k] - c);
+    }
+    const uint64_t other = n > c ? ((uint64_t(1) << (n - c)) - 1) & ~(spec.mask >> c) : 0;
+    const uint64_t rows = uint64_t(1) << __popcll(other);
+    auto scatter = [&](uint64_t r) {
+      uint64_t o = 0, m = other;
+      for (; r; r >>= 1, m &= m - 1)
+        if (r & 1) o |= m & (0ull - m);
+      return o;
+    };
+    const uint64_t r0 = threadIdx.x >> 5;
+    if (r0 < rows) {
+      uint64_t b = scatter(r0);
+      const uint64_t step = rows > kColRows ? scatter(kColRows) : 0;
+      for (uint64_t r = r0; r < rows; r += kColRows) {
+        acc += partial[((ob | b) << nin) + at];
+        b = (b + ~other + step) & other;  // + step, carrying over the bits not in `other`
+      }
+    }
   }
+  column_combine(acc, (int)bin, (int)width, out);
 }
 
 // ------------------------------------------------------------------ sampling
@@ -957,31 +1082,35 @@ cudaError_t launch_compact_kept(const void* amp, int n, int prec, double thr, co
                          : compact_t<double>(amp, n, thr, offs, cap, oidx, op, s);
 }
 
-uint64_t marg_chunk(int n) {
-  uint64_t N = uint64_t(1) << n;
-  return std::max<uint64_t>(N / 2048, 256);
-}
+// At most 2048 blocks, of at least 2^12 indices (16 a thread).
+static int marg_chunk_bits(int n) { return std::max(12, n - 11); }
+uint64_t marg_chunk(int n) { return uint64_t(1) << marg_chunk_bits(n); }
 template <typename R>
 static cudaError_t marginals_t(const void* amp, int n, double* partial, double* out, cudaStream_t s) {
-  uint64_t N = uint64_t(1) << n, chunk = marg_chunk(n), nb = (N + chunk - 1) / chunk;
-  k_marginals<R, 256><<<(unsigned)nb, 256, 0, s>>>((const typename Vec2<R>::T*)amp, n, chunk, partial);
-  k_sum_columns<<<1, 64, 0, s>>>(partial, nb, n, out);
+  const int c = marg_chunk_bits(n);
+  const uint64_t nb = n > c ? uint64_t(1) << (n - c) : 1;
+  k_marginals<R><<<(unsigned)nb, 256, 0, s>>>((const typename Vec2<R>::T*)amp, n, c, partial);
+  k_sum_columns<<<(n + 31) / 32, 32 * kColRows, 0, s>>>(partial, nb, n, out);
   return cudaGetLastError();
 }
 cudaError_t launch_marginals(const void* amp, int n, int prec, double* partial, double* out, cudaStream_t s) {
   return prec == KET_C64 ? marginals_t<float>(amp, n, partial, out, s) : marginals_t<double>(amp, n, partial, out, s);
 }
 
-int mdist_chunk_bits(int n, int m) { return std::min(n, std::max(20, m)); }
+// At most 1024 blocks of at least 2^12 indices: the blocks' sums (2^12 bins at
+// most) stay below a thirtieth of a large state's bytes.
+static int mdist_chunk_bits(int n) { return std::max(12, n - 10); }
+size_t mdist_partials(int n, uint64_t mask) {
+  const int c = mdist_chunk_bits(n);
+  return (size_t)(n > c ? uint64_t(1) << (n - c) : 1) << __builtin_popcountll(mask & ((uint64_t(1) << c) - 1));
+}
 template <typename R>
 static cudaError_t mdist_t(const void* amp, int n, const MarginalSpec& spec, double* partial, double* out,
                            cudaStream_t s) {
-  int c = mdist_chunk_bits(n, spec.m);
-  uint64_t nb = uint64_t(1) << (n - c);
-  uint32_t width = 1u << spec.m;
-  cudaMemsetAsync(partial, 0, sizeof(double) * nb * width, s);
-  k_marginal_dist<R><<<(unsigned)nb, 1024, 0, s>>>((const typename Vec2<R>::T*)amp, c, spec, partial);
-  k_sum_columns<<<(width + 255) / 256, 256, 0, s>>>(partial, nb, (int)width, out);
+  const int c = mdist_chunk_bits(n);
+  const uint64_t nb = n > c ? uint64_t(1) << (n - c) : 1;
+  k_marginal_dist<R><<<(unsigned)nb, 256, 0, s>>>((const typename Vec2<R>::T*)amp, n, c, spec.mask, partial);
+  k_marginal_dist_combine<<<((1u << spec.m) + 31) / 32, 32 * kColRows, 0, s>>>(partial, n, c, spec, out);
   return cudaGetLastError();
 }
 cudaError_t launch_marginal_dist(const void* amp, int n, int prec, const MarginalSpec& spec, double* partial,

@@ -61,7 +61,7 @@ cudaError_t launch_compact_kept(const void* amp, int n, int prec, double thr, co
                                 uint64_t* oidx, double* op, cudaStream_t s);
 uint64_t marg_chunk(int n);
 cudaError_t launch_marginals(const void* amp, int n, int prec, double* partial, double* out, cudaStream_t s);
-int mdist_chunk_bits(int n, int m);
+size_t mdist_partials(int n, uint64_t mask);  // doubles of scratch
 cudaError_t launch_marginal_dist(const void* amp, int n, int prec, const MarginalSpec& spec, double* partial,
                                  double* out, cudaStream_t s);
 // Sampling: the reference's running FP64 sum over kept entries in ascending
