@@ -424,14 +424,17 @@ __global__ void __launch_bounds__(32 << (7 - NR), NR == 5 ? 2 : 1) k_fused2(Pass
   }
 }
 
-// out[s] = sum over CTAs c and warps w of gpart[c][s][w], in a fixed order.
-__global__ void k_grad_reduce(const double* gpart, int nctas, int nslots, double* out) {
-  int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= nslots) return;
+// out[s] = sum over CTAs c and warps w of gpart[c][s][w], in a fixed order: a
+// CTA a slot, whose threads add strided runs.  (One thread a slot took 127 us for
+// the 2368 partials of a full grid, as long as a quarter of the pass before it;
+// this takes 7 us.)
+__global__ void __launch_bounds__(256) k_grad_reduce(const double* gpart, int nctas, int nslots, double* out) {
+  __shared__ double red[32];
+  const int s = blockIdx.x;
   double acc = 0.0;
-  for (int c = 0; c < nctas; c++)
-    for (int w = 0; w < 8; w++) acc += gpart[((size_t)c * nslots + s) * 8 + w];
-  out[s] = acc;
+  for (int i = threadIdx.x; i < 8 * nctas; i += 256) acc += gpart[((size_t)(i >> 3) * nslots + s) * 8 + (i & 7)];
+  acc = block_sum<256>(acc, red);
+  if (threadIdx.x == 0) out[s] = acc;
 }
 
 // Resident CTAs per SM for a register-bit count: 5 -> two CTAs of 128 threads
@@ -511,7 +514,7 @@ cudaError_t launch_fused2(const Pass2Args& a, int precision, cudaStream_t s) {
 }
 
 cudaError_t launch_grad_reduce(const double* gpart, int nctas, int nslots, double* out, cudaStream_t s) {
-  k_grad_reduce<<<(nslots + 127) / 128, 128, 0, s>>>(gpart, nctas, nslots, out);
+  k_grad_reduce<<<nslots, 256, 0, s>>>(gpart, nctas, nslots, out);
   return cudaGetLastError();
 }
 
