@@ -108,13 +108,7 @@ int expected_kind(int pg) {
 }
 
 // ---------------------------------------------------------------- H psi
-struct Term {
-  uint64_t flip, zm;
-  int ny;
-  double coeff;
-};
-
-int parse_terms(int n, int nterms, const double* coeffs, const char* ops, std::vector<Term>& out, double& ident) {
+int parse_terms(int n, int nterms, const double* coeffs, const char* ops, std::vector<PauliTerm>& out, double& ident) {
   ident = 0;
   out.clear();
   for (int t = 0; t < nterms; t++) {
@@ -122,7 +116,7 @@ int parse_terms(int n, int nterms, const double* coeffs, const char* ops, std::v
     for (int j = 0; j < n; j++)
       if (o[j] == 0) return fail(KET_ERR_TYPE, "ops length must equal ansatz.qubits (" + std::to_string(n) + ")");
     if (std::fabs(coeffs[t]) < 1e-15) continue;
-    Term tm{0, 0, 0, coeffs[t]};
+    PauliTerm tm{coeffs[t], 0, 0, 0};
     bool any = false;
     for (int q = 0; q < n; q++) {
       char ch = (char)toupper((unsigned char)o[n - 1 - q]);
@@ -144,6 +138,7 @@ struct DevTerm {
   double cre, cim;  // coeff * i^ny
 };
 
+// The terms that flip too many qubits for a tile of k_hpsi_tile:
 // lambda_y = sum_t coeff_t i^ny_t (-1)^popc((y^f_t) & zm_t) psi_{y^f_t}  (+ ident * psi_y),
 // and per-block partials of Re <psi|lambda>.
 __global__ void k_hpsi(const double2* psi, double2* lam, uint64_t N, const DevTerm* terms, int nt, double ident,
@@ -166,13 +161,6 @@ __global__ void k_hpsi(const double2* psi, double2* lam, uint64_t N, const DevTe
   }
   double t = block_sum<256>(e, red);
   if (threadIdx.x == 0) partial[blockIdx.x] = t;
-}
-
-__global__ void k_sum_fixed(const double* partial, int n, double* out) {
-  if (blockIdx.x != 0 || threadIdx.x != 0) return;
-  double a = 0.0;
-  for (int i = 0; i < n; i++) a += partial[i];
-  *out = a;
 }
 
 // ---------------------------------------------------------------- helpers
@@ -352,7 +340,8 @@ struct AdjWork {
   double* slot_out = nullptr;  // [batch][nbinds] probe sums
   double* gpart = nullptr;
   size_t gpart_cap = 0;
-  DevTerm* terms = nullptr;
+  DevTerm* terms = nullptr;    // terms for k_hpsi
+  char* tiles = nullptr;       // groups and terms for k_hpsi_tile
   double* epart = nullptr;     // Hpsi partials, then [batch] energies
 };
 
@@ -376,7 +365,7 @@ int ket_adjoint_gradient(ket_ctx* ctx, int n, uint64_t init, const ket_op* ops, 
   if (batch < 0 || nparams < 0) return fail(KET_ERR_TYPE, "negative batch or parameter count");
   if ((init >> n) != 0) return fail(KET_ERR_RANGE, "initial basis index out of range");
   cudaSetDevice(ctx->device);
-  std::vector<Term> terms;
+  std::vector<PauliTerm> terms;
   double ident = 0;
   int rc = parse_terms(n, nterms, coeffs, pauli_ops, terms, ident);
   if (rc) return rc;
@@ -422,6 +411,7 @@ int ket_adjoint_gradient(ket_ctx* ctx, int n, uint64_t init, const ket_op* ops, 
     if (w.slot_out) cudaFree(w.slot_out);
     if (w.gpart) cudaFree(w.gpart);
     if (w.terms) cudaFree(w.terms);
+    if (w.tiles) cudaFree(w.tiles);
     if (w.epart) cudaFree(w.epart);
     cudaFree(buf);
   };
@@ -463,10 +453,20 @@ int ket_adjoint_gradient(ket_ctx* ctx, int n, uint64_t init, const ket_op* ops, 
     const Ckpt& k = w.ckpt[sg - 1];
     return cudaMemcpyAsync(buf, k.p, half, k.host ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice, ctx->stream);
   };
+  // lambda = H psi by tiles; the terms that do not fit a tile go first
+  PauliGroups wide;
+  const std::vector<PauliTilePass> tiled = plan_pauli_tiles(n, terms, false, wide);
   std::vector<DevTerm> dterms;
-  for (const Term& t : terms) {
-    zc ph = std::pow(zc(0, 1), t.ny & 3) * t.coeff;
-    dterms.push_back(DevTerm{t.flip, t.zm, ph.real(), ph.imag()});
+  for (const auto& kv : wide)
+    for (const PauliTerm* t : kv.second) {
+      zc ph = std::pow(zc(0, 1), t->ny & 3) * t->coeff;
+      dterms.push_back(DevTerm{t->flip, t->zm, ph.real(), ph.imag()});
+    }
+  std::vector<PauliTileGroup> tgroups;
+  std::vector<PauliTileTerm> tterms;
+  for (const PauliTilePass& P : tiled) {
+    tgroups.insert(tgroups.end(), P.groups.begin(), P.groups.end());
+    tterms.insert(tterms.end(), P.terms.begin(), P.terms.end());
   }
   const int hblocks = 1024;
   const size_t nslot = std::max<size_t>(nbinds, 1);
@@ -476,10 +476,17 @@ int ket_adjoint_gradient(ket_ctx* ctx, int n, uint64_t init, const ket_op* ops, 
     rc = dev_alloc((void**)&w.gpart, sizeof(double) * w.gpart_cap);
   }
   if (!rc) rc = dev_alloc((void**)&w.terms, sizeof(DevTerm) * std::max<size_t>(dterms.size(), 1));
+  const size_t tt_off = (sizeof(PauliTileGroup) * tgroups.size() + 255) & ~size_t(255);
+  if (!rc && !tiled.empty()) rc = dev_alloc((void**)&w.tiles, tt_off + sizeof(PauliTileTerm) * tterms.size());
   if (!rc) rc = dev_alloc((void**)&w.epart, sizeof(double) * (hblocks + 8 + std::max(batch, 1)));
   if (rc) { cleanup(); return rc; }
   if (!dterms.empty())
     cudaMemcpyAsync(w.terms, dterms.data(), sizeof(DevTerm) * dterms.size(), cudaMemcpyHostToDevice, ctx->stream);
+  if (!tiled.empty()) {
+    cudaMemcpyAsync(w.tiles, tgroups.data(), sizeof(PauliTileGroup) * tgroups.size(), cudaMemcpyHostToDevice, ctx->stream);
+    cudaMemcpyAsync(w.tiles + tt_off, tterms.data(), sizeof(PauliTileTerm) * tterms.size(), cudaMemcpyHostToDevice,
+                    ctx->stream);
+  }
   if (batch > 0) cudaMemsetAsync(w.slot_out, 0, sizeof(double) * nslot * batch, ctx->stream);
   // Batches run their passes on kernels compiled for each pass's program
   // (compiled once, on the first vector, and reused by the rest); a single
@@ -536,11 +543,24 @@ int ket_adjoint_gradient(ket_ctx* ctx, int n, uint64_t init, const ket_op* ops, 
     }
     // ---- lambda = H psi, energy
     prof_begin(ctx);
-    k_hpsi<<<hblocks, 256, 0, ctx->stream>>>((const double2*)buf, (double2*)((char*)buf + half), uint64_t(1) << n,
-                                             w.terms, (int)dterms.size(), ident, w.epart);
-    k_sum_fixed<<<1, 32, 0, ctx->stream>>>(w.epart, hblocks, d_energy + b);
+    void* lam = (char*)buf + half;
+    if (tiled.empty() || !dterms.empty()) {
+      k_hpsi<<<hblocks, 256, 0, ctx->stream>>>((const double2*)buf, (double2*)lam, uint64_t(1) << n, w.terms,
+                                               (int)dterms.size(), ident, w.epart);
+      ctx->launches++;
+    }
+    const PauliTileGroup* tg = (const PauliTileGroup*)w.tiles;
+    const PauliTileTerm* tt = (const PauliTileTerm*)(w.tiles + tt_off);
+    for (size_t i = 0; i < tiled.size(); i++) {
+      cudaError_t e = launch_hpsi_tile(buf, lam, n, tiled[i].args, tg, tt, ident, i == 0 && dterms.empty(),
+                                       i + 1 == tiled.size(), w.epart, ctx->stream);
+      if (e != cudaSuccess) { cleanup(); return cuda_fail(e, "H psi launch"); }
+      ctx->launches++;
+      tg += tiled[i].groups.size();
+      tt += tiled[i].terms.size();
+    }
+    launch_sum(w.epart, tiled.empty() ? hblocks : pauli_tile_grid(n), d_energy + b, ctx->stream);
     prof_end(ctx, PK_ADJOINT);
-    ctx->launches += 1;
     tick(3);
     // ---- reverse sweep
     double* slots_b = w.slot_out + (size_t)b * nslot;

@@ -3,7 +3,6 @@
 #include <cctype>
 #include <cmath>
 #include <cstring>
-#include <map>
 #include <vector>
 
 #include "ctx.h"
@@ -209,104 +208,18 @@ int sample_indices(const ket_state* s, const double* r, size_t shots, double thr
 
 namespace {
 
-struct Term {
-  double coeff;
-  uint64_t flip, zm;
-  int ny;
-};
-
-// One pass of k_pauli_tile: its tile, and its groups and terms in tile bits.
-struct TilePass {
-  PauliTileArgs args;
-  std::vector<PauliTileGroup> groups;
-  std::vector<PauliTileTerm> terms;
-};
-
-typedef std::map<std::pair<uint64_t, int>, std::vector<const Term*>> TermGroups;  // by (flip mask, ny mod 4)
-
-// Tile passes for the groups, first fit in ascending flip order, each pass with
-// as many flipped qubits (and terms) as its tile takes; groups that flip more
-// qubits above the low ones than a tile holds are left in `wide`.
-std::vector<TilePass> plan_tile_passes(int n, const TermGroups& all, TermGroups& wide) {
-  const uint64_t low = (uint64_t(1) << KET_PAULI_TILE_LOW) - 1;
-  std::vector<TilePass> passes;
-  TermGroups left;
-  for (auto& kv : all)
-    (__builtin_popcountll(kv.first.first | low) <= KET_PAULI_TILE_BITS ? left : wide).insert(kv);
-  while (!left.empty()) {
-    uint64_t S = low;
-    size_t room = KET_PAULI_TILE_TERMS;
-    TermGroups now, rest;
-    for (auto& kv : left) {
-      const size_t take = __builtin_popcountll(S | kv.first.first) <= KET_PAULI_TILE_BITS
-                              ? std::min(room, kv.second.size()) : 0;
-      const auto cut = kv.second.begin() + take;
-      if (take) now[kv.first].assign(kv.second.begin(), cut);
-      if (cut != kv.second.end()) rest[kv.first].assign(cut, kv.second.end());
-      if (take) S |= kv.first.first;
-      room -= take;
-    }
-    for (int q = 0; __builtin_popcountll(S) < KET_PAULI_TILE_BITS; q++) S |= uint64_t(1) << q;
-    TilePass P;
-    memset(&P.args, 0, sizeof(P.args));
-    int nb = 0;
-    for (int q = 0; q < n; q++) {
-      if ((S >> q) & 1) P.args.bits[nb++] = q;
-      else P.args.ctxbits[P.args.nctx++] = q;
-    }
-    P.args.ntiles = uint64_t(1) << (n - KET_PAULI_TILE_BITS);
-    auto tile_mask = [&](uint64_t m) {
-      uint32_t r = 0;
-      for (int b = 0; b < KET_PAULI_TILE_BITS; b++)
-        if ((m >> P.args.bits[b]) & 1) r |= 1u << b;
-      return r;
-    };
-    for (auto& kv : now) {
-      const int ny = kv.first.second;
-      PauliTileGroup G;
-      G.flip = tile_mask(kv.first.first);
-      G.top = G.flip ? (uint8_t)(31 - __builtin_clz(G.flip)) : 0;
-      G.odd = (uint8_t)(ny & 1);
-      G.first = (int)P.terms.size();
-      G.nterms = (uint16_t)kv.second.size();
-      // Re(i^ny z) = Re z, -Im z, -Re z, Im z with z = psi_y conj(psi_x); a pair counts twice
-      const double w = (ny == 1 || ny == 2 ? -1.0 : 1.0) * (G.flip ? 2.0 : 1.0);
-      for (const Term* t : kv.second) {
-        const uint32_t z = tile_mask(t->zm);
-        uint32_t zthr = z & 0x1ffu, zidx = z >> 9;
-        if (G.flip) {
-          // the products' index leaves out register bit p: clear in a register
-          // flip, equal to the thread's bit `top` in a thread flip
-          const int p = G.top >= 9 ? G.top - 9 : 2;
-          if (G.top < 9 && ((zidx >> p) & 1)) zthr ^= 1u << G.top;
-          zidx = ((zidx >> (p + 1)) << p) | (zidx & ((1u << p) - 1));
-        }
-        P.terms.push_back(PauliTileTerm{w * t->coeff, t->zm & ~S, zthr | zidx << 16, 0});
-      }
-      std::stable_sort(P.terms.begin() + G.first, P.terms.end(), [](const PauliTileTerm& x, const PauliTileTerm& y) {
-        return (x.zm >> 16) < (y.zm >> 16);
-      });
-      P.groups.push_back(G);
-      P.args.flips |= G.flip != 0;
-    }
-    P.args.ngroups = (int)P.groups.size();
-    P.args.nterms = (int)P.terms.size();
-    passes.push_back(std::move(P));
-    left.swap(rest);
-  }
-  return passes;
-}
-
 // Sum over groups of Pauli terms that share (flip mask, i^nY phase).  States of
 // 12 and more qubits go by tiles, where a pass over the state takes all the
 // groups that fit; smaller states, and groups too wide for a tile, take one
 // pass a group.
-int pauli_terms_expect(const ket_state* s, const std::vector<Term>& terms, double* out) {
-  TermGroups groups, wide;
-  for (const Term& t : terms) groups[{t.flip, t.ny & 3}].push_back(&t);
-  std::vector<TilePass> tiled;
-  if (s->n >= KET_PAULI_TILE_BITS) tiled = plan_tile_passes(s->n, groups, wide);
-  else wide.swap(groups);
+int pauli_terms_expect(const ket_state* s, const std::vector<PauliTerm>& terms, double* out) {
+  PauliGroups wide;
+  std::vector<PauliTilePass> tiled;
+  if (s->n >= KET_PAULI_TILE_BITS) {
+    tiled = plan_pauli_tiles(s->n, terms, true, wide);
+  } else {
+    for (const PauliTerm& t : terms) wide[{t.flip, t.ny & 3}].push_back(&t);
+  }
   std::vector<PauliGroup> gl;
   for (auto& kv : wide) {
     const auto& v = kv.second;
@@ -324,7 +237,7 @@ int pauli_terms_expect(const ket_state* s, const std::vector<Term>& terms, doubl
   if (nres == 0) { *out = 0.0; return KET_OK; }
   std::vector<PauliTileGroup> hg;
   std::vector<PauliTileTerm> ht;
-  for (const TilePass& P : tiled) {
+  for (const PauliTilePass& P : tiled) {
     hg.insert(hg.end(), P.groups.begin(), P.groups.end());
     ht.insert(ht.end(), P.terms.begin(), P.terms.end());
   }
@@ -369,7 +282,7 @@ int ket_expect_pauli(const ket_state* s, const char* pauli, double* out) {
   if (!pauli || !out) return fail(KET_ERR_TYPE, "null argument");
   if ((int)strlen(pauli) != s->n)
     return fail(KET_ERR_TYPE, "pauli length must equal qubits (" + std::to_string(s->n) + ")");
-  Term t{1.0, 0, 0, 0};
+  PauliTerm t{1.0, 0, 0, 0};
   bool any = false;
   for (int q = 0; q < s->n; q++) {
     char ch = (char)toupper((unsigned char)pauli[q]);
@@ -382,7 +295,7 @@ int ket_expect_pauli(const ket_state* s, const char* pauli, double* out) {
     if (ch == 'Y') t.ny++;
   }
   if (!any) { *out = 1.0; return KET_OK; }  // circuit.ts:3735
-  return pauli_terms_expect(s, std::vector<Term>{t}, out);
+  return pauli_terms_expect(s, std::vector<PauliTerm>{t}, out);
 }
 
 int ket_expect_pauli_sum(const ket_state* s, int nterms, const double* coeffs, const char* ops, double* out) {
@@ -390,13 +303,13 @@ int ket_expect_pauli_sum(const ket_state* s, int nterms, const double* coeffs, c
   if (!out || (nterms && (!coeffs || !ops))) return fail(KET_ERR_TYPE, "null argument");
   const int n = s->n;
   double ident = 0.0;
-  std::vector<Term> terms;
+  std::vector<PauliTerm> terms;
   for (int t = 0; t < nterms; t++) {
     const char* o = ops + (size_t)t * n;
     for (int j = 0; j < n; j++)
       if (o[j] == 0) return fail(KET_ERR_TYPE, "ops length must equal ansatz.qubits (" + std::to_string(n) + ")");
     if (std::fabs(coeffs[t]) < 1e-15) continue;      // algorithms.ts:308
-    Term tm{coeffs[t], 0, 0, 0};
+    PauliTerm tm{coeffs[t], 0, 0, 0};
     bool any = false;
     for (int q = 0; q < n; q++) {
       char ch = (char)toupper((unsigned char)o[n - 1 - q]);  // ops[n-1-q] acts on qubit q

@@ -1021,6 +1021,130 @@ __global__ void __launch_bounds__(kPauliThreads, 2) k_pauli_tile(const typename 
   if (t == 0) partial[blockIdx.x] = sum;
 }
 
+// lambda = H psi by the same tiles (c128): a pass adds the terms it holds to
+// lambda, every amplitude's partner coming from shared memory; the last pass sums
+// Re <psi|lambda>.  A group's coefficients over the register bits are one number
+// (a term without Z or Y there), or the Walsh transform of its terms'.
+// Bound: shared memory (the tile once a group) and, for few groups, HBM.  24
+// qubits, 23 Z Z and 24 X terms: 3 passes of 167 us,
+// where one kernel over all terms took 1340 (and 43 for a serial sum).
+__global__ void __launch_bounds__(kPauliThreads, 2) k_hpsi_tile(const double2* psi, double2* lam, PauliTileArgs g,
+                                                                const PauliTileGroup* groups,
+                                                                const PauliTileTerm* terms, double ident, int first,
+                                                                int last, double* partial) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  double2* s = reinterpret_cast<double2*>(smraw);
+  __shared__ double red[32];
+  __shared__ double sc[KET_PAULI_TILE_TERMS];
+  __shared__ uint32_t zm[KET_PAULI_TILE_TERMS];
+  __shared__ PauliTileGroup gs[KET_PAULI_TILE_TERMS];
+  const int t = threadIdx.x, lane = t & 31, ctxq = lane < g.nctx ? g.ctxbits[lane] : 63;
+  if (t < g.ngroups) gs[t] = groups[t];
+  double coeff = 0.0;
+  uint64_t zctx = 0;
+  if (t < g.nterms) {
+    coeff = terms[t].coeff;
+    zctx = terms[t].zctx;
+    zm[t] = terms[t].zm;
+  }
+  uint64_t toff = 0;
+#pragma unroll
+  for (int b = 0; b < 9; b++)
+    if ((t >> b) & 1) toff |= uint64_t(1) << g.bits[b];
+  auto signed_coeff = [&](int i, uint32_t z) {
+    const uint32_t odd = (uint32_t)__popc(t & z & 0xffffu) << 31;
+    const double c = sc[i];
+    return __hiloint2double(__double2hiint(c) ^ (int)odd, __double2loint(c));
+  };
+  double e = 0.0;
+  for (uint64_t tile = blockIdx.x; tile < g.ntiles; tile += gridDim.x) {
+    const uint64_t mine = ((tile >> lane) & 1) << ctxq;
+    const uint64_t ctx = ((uint64_t)__reduce_or_sync(0xffffffffu, (uint32_t)(mine >> 32)) << 32) |
+                         __reduce_or_sync(0xffffffffu, (uint32_t)mine);
+    auto at = [&](int j) {
+      uint64_t o = ctx | toff;
+#pragma unroll
+      for (int b = 0; b < 3; b++)
+        if ((j >> b) & 1) o |= uint64_t(1) << g.bits[9 + b];
+      return o;
+    };
+    __syncthreads();  // the last tile's reads of s and sc are done
+    if (t < g.nterms) sc[t] = (__popcll(ctx & zctx) & 1) ? -coeff : coeff;
+    double2 l[8];
+#pragma unroll
+    for (int j = 0; j < 8; j++) s[t + 512 * j] = psi[at(j)];
+    if (first) {
+#pragma unroll
+      for (int j = 0; j < 8; j++) {
+        const double2 v = s[t + 512 * j];
+        l[j] = make_double2(ident * v.x, ident * v.y);
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < 8; j++) l[j] = lam[at(j)];
+    }
+    __syncthreads();
+    for (int k = 0; k < g.ngroups; k++) {
+      const PauliTileGroup G = gs[k];
+      const uint32_t z0 = zm[G.first];
+      double c[8];
+      if (G.nterms == 1) {
+        const double c0 = signed_coeff(G.first, z0);
+#pragma unroll
+        for (int j = 0; j < 8; j++) c[j] = ((0x96u >> (j & (z0 >> 16))) & 1u) ? -c0 : c0;
+      } else {
+        int i = G.first;
+#pragma unroll
+        for (int w = 0; w < 8; w++) {
+          c[w] = 0.0;
+          for (; i < G.first + G.nterms; i++) {
+            const uint32_t z = zm[i];
+            if ((z >> 16) != w) break;
+            c[w] += signed_coeff(i, z);
+          }
+        }
+#pragma unroll
+        for (int st = 1; st < 8; st <<= 1)
+#pragma unroll
+          for (int j = 0; j < 8; j++)
+            if (!(j & st)) {
+              const double x = c[j], y = c[j | st];
+              c[j] = x + y;
+              c[j | st] = x - y;
+            }
+      }
+      if (G.odd) {
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+          const double2 w = s[(t + 512 * j) ^ G.flip];
+          l[j].x = fma(-c[j], w.y, l[j].x);
+          l[j].y = fma(c[j], w.x, l[j].y);
+        }
+      } else {
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+          const double2 w = s[(t + 512 * j) ^ G.flip];
+          l[j].x = fma(c[j], w.x, l[j].x);
+          l[j].y = fma(c[j], w.y, l[j].y);
+        }
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 8; j++) lam[at(j)] = l[j];
+    if (last) {
+#pragma unroll
+      for (int j = 0; j < 8; j++) {
+        const double2 v = s[t + 512 * j];
+        e += v.x * l[j].x + v.y * l[j].y;
+      }
+    }
+  }
+  if (last) {
+    const double sum = block_sum<kPauliThreads>(e, red);
+    if (t == 0) partial[blockIdx.x] = sum;
+  }
+}
+
 inline unsigned gridn(uint64_t work, int nt, int cap_per_sm = 16) {
   uint64_t b = (work + nt - 1) / nt;
   uint64_t cap = (uint64_t)num_sms() * cap_per_sm;
@@ -1216,6 +1340,16 @@ cudaError_t launch_pauli_tile(const void* amp, int n, int prec, const PauliTileA
                               const PauliTileTerm* terms, double* partial, cudaStream_t s) {
   return prec == KET_C64 ? pauli_tile_t<float>(amp, g, groups, terms, partial, pauli_tile_grid(n), s)
                          : pauli_tile_t<double>(amp, g, groups, terms, partial, pauli_tile_grid(n), s);
+}
+cudaError_t launch_hpsi_tile(const void* psi, void* lam, int n, const PauliTileArgs& g, const PauliTileGroup* groups,
+                             const PauliTileTerm* terms, double ident, bool first, bool last, double* partial,
+                             cudaStream_t s) {
+  const int smem = (int)(sizeof(double2) << KET_PAULI_TILE_BITS);
+  cudaError_t e = cudaFuncSetAttribute(k_hpsi_tile, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) return e;
+  k_hpsi_tile<<<pauli_tile_grid(n), kPauliThreads, smem, s>>>((const double2*)psi, (double2*)lam, g, groups, terms, ident,
+                                                              first, last, partial);
+  return cudaGetLastError();
 }
 cudaError_t launch_sum(const double* partial, uint64_t count, double* out, cudaStream_t s) {
   k_sum<256><<<1, 256, 0, s>>>(partial, count, out);

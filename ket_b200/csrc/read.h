@@ -4,6 +4,10 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <map>
+#include <utility>
+#include <vector>
+
 #include "ket_sv.h"
 
 namespace ket {
@@ -49,6 +53,23 @@ struct PauliTileTerm {
   uint32_t pad;
 };
 
+// A Pauli string: it flips the X|Y qubits, signs by the Z|Y qubits, times i^ny.
+struct PauliTerm {
+  double coeff;
+  uint64_t flip, zm;
+  int ny;
+};
+typedef std::map<std::pair<uint64_t, int>, std::vector<const PauliTerm*>> PauliGroups;  // by (flip, ny mod 4)
+
+// One pass of a tiled Pauli kernel: its tile, and its groups and terms in tile bits.
+struct PauliTilePass {
+  PauliTileArgs args;
+  std::vector<PauliTileGroup> groups;
+  std::vector<PauliTileTerm> terms;
+};
+std::vector<PauliTilePass> plan_pauli_tiles(int n, const std::vector<PauliTerm>& terms, bool expectation,
+                                            PauliGroups& wide);
+
 int num_sms();
 
 cudaError_t launch_norm2(const void* amp, int n, int prec, double* scratch, double* out, cudaStream_t s);
@@ -79,6 +100,11 @@ size_t pauli_scratch(int n);
 unsigned pauli_tile_grid(int n);
 cudaError_t launch_pauli_tile(const void* amp, int n, int prec, const PauliTileArgs& g, const PauliTileGroup* groups,
                               const PauliTileTerm* terms, double* partial, cudaStream_t s);
+// lam (+)= the pass's terms applied to psi (first: lam = ident * psi + ...); last:
+// pauli_tile_grid(n) partials of Re <psi|lam>.
+cudaError_t launch_hpsi_tile(const void* psi, void* lam, int n, const PauliTileArgs& g, const PauliTileGroup* groups,
+                             const PauliTileTerm* terms, double ident, bool first, bool last, double* partial,
+                             cudaStream_t s);
 // Fixed-order sum of `count` partials.
 cudaError_t launch_sum(const double* partial, uint64_t count, double* out, cudaStream_t s);
 

@@ -56,3 +56,23 @@ def test_pauli_sum_by_tiles(n, precision):
     assert abs(st.expect_pauli_sum(terms) - energy(a, terms)) <= bound
     for some in (terms[:1], terms[n - 1:n + 1], terms[-8:-4]):
         assert abs(st.expect_pauli_sum(some) - energy(a, some)) <= 1e-13 * sum(abs(c) for c, _ in some)
+
+
+@pytest.mark.parametrize("n", [12, 15, 18])
+def test_h_psi_by_tiles(n):
+    """lambda = H psi in adjoint gradients: shared flip masks, Y factors and flips wider than a tile."""
+    from ket_b200.adjoint import adjoint_gradient, shift_gradient
+    from ket_b200.workloads import hea_ladder
+    r = np.random.default_rng(50 + n)
+    terms = [(float(r.normal()), word(n, {q: "X"})) for q in range(n)]
+    terms += [(float(r.normal()), word(n, {q: "Z", q + 1: "Z"})) for q in range(n - 1)]
+    terms += [(float(r.normal()), word(n, {0: a, n - 1: b, n // 2: c})) for a in "XY" for b in "XY" for c in "IZ"]
+    terms += [(float(r.normal()), "".join(r.choice(list("IXYZ"), n))) for _ in range(6)]
+    terms += [(float(r.normal()), "X" * n), (0.3, "I" * n)]
+    ansatz = hea_ladder(n, 1)
+    params = r.uniform(0, 6.28, (2, 2 * n))
+    e, g = adjoint_gradient(ansatz, terms, params)
+    es, gs = shift_gradient(ansatz, terms, params)
+    # both are FP64 over a unit vector: a few thousand roundings at most, scaled by the terms' weights
+    bound = 1e-12 * sum(abs(c) for c, _ in terms)
+    assert np.abs(e - es).max() <= bound and np.abs(g - gs).max() <= bound
