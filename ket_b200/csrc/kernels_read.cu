@@ -6,6 +6,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "pauli_terms.cuh"
 #include "read.h"
 
 namespace ket {
@@ -884,56 +885,6 @@ __global__ void __launch_bounds__(NT) k_pauli_group(const typename Vec2<R>::T* a
 // a group a pass costs a launch each.
 constexpr int kPauliThreads = 512;
 
-// One sum over a group's products b: its terms are entries [first, first + nterms)
-// of sc (signed coefficients) and zm (thread mask | index mask << 16), sorted by
-// index mask.
-template <int NB>
-__device__ __forceinline__ double pauli_terms(double (&b)[NB], const double* sc, const uint32_t* zm, int first,
-                                              int nterms, int t) {
-  auto coeff = [&](int i, uint32_t z) {
-    const uint32_t odd = (uint32_t)__popc(t & z & 0xffffu) << 31;
-    const double c = sc[i];
-    return __hiloint2double(__double2hiint(c) ^ (int)odd, __double2loint(c));
-  };
-  if (nterms == 1) {
-    const uint32_t z = zm[first], zi = z >> 16;
-    if (zi) {
-#pragma unroll
-      for (int j = 1; j < NB; j++) {
-        const uint32_t sg = (0x96u >> (j & zi)) << 31;
-        b[j] = __hiloint2double(__double2hiint(b[j]) ^ (int)sg, __double2loint(b[j]));
-      }
-    }
-#pragma unroll
-    for (int st = NB / 2; st > 0; st >>= 1)
-#pragma unroll
-      for (int j = 0; j < st; j++) b[j] += b[j + st];
-    return coeff(first, z) * b[0];
-  }
-#pragma unroll
-  for (int st = 1; st < NB; st <<= 1)
-#pragma unroll
-    for (int j = 0; j < NB; j++)
-      if (!(j & st)) {
-        const double x = b[j], y = b[j | st];
-        b[j] = x + y;
-        b[j | st] = x - y;
-      }
-  double acc = 0.0;
-  int i = first;
-#pragma unroll
-  for (int w = 0; w < NB; w++) {
-    double c = 0.0;
-    for (; i < first + nterms; i++) {
-      const uint32_t z = zm[i];
-      if ((z >> 16) != w) break;
-      c += coeff(i, z);
-    }
-    acc += c * b[w];
-  }
-  return acc;
-}
-
 template <typename R>
 __global__ void __launch_bounds__(kPauliThreads, 2) k_pauli_tile(const typename Vec2<R>::T* a, PauliTileArgs g,
                                                                  const PauliTileGroup* groups,
@@ -956,6 +907,8 @@ __global__ void __launch_bounds__(kPauliThreads, 2) k_pauli_tile(const typename 
     zm[t] = terms[t].zm;
   }
   const int lane = t & 31, ctxq = lane < g.nctx ? g.ctxbits[lane] : 63;
+  auto coeff_of = [&](int i) { return sc[i]; };
+  auto mask_of = [&](int i) { return zm[i]; };
   uint64_t toff = 0;
 #pragma unroll
   for (int b = 0; b < 9; b++)
@@ -988,7 +941,7 @@ __global__ void __launch_bounds__(kPauliThreads, 2) k_pauli_tile(const typename 
         double b[8];
 #pragma unroll
         for (int j = 0; j < 8; j++) b[j] = norm2_ref(v[j].x, v[j].y);
-        acc += pauli_terms<8>(b, sc, zm, G.first, G.nterms, t);
+        acc += pauli_terms<8>(b, coeff_of, mask_of, G.first, G.nterms, t);
         continue;
       }
       double b[4];
@@ -1014,7 +967,7 @@ __global__ void __launch_bounds__(kPauliThreads, 2) k_pauli_tile(const typename 
       };
       if (G.odd) by_top(std::true_type());
       else by_top(std::false_type());
-      acc += pauli_terms<4>(b, sc, zm, G.first, G.nterms, t);
+      acc += pauli_terms<4>(b, coeff_of, mask_of, G.first, G.nterms, t);
     }
   }
   const double sum = block_sum<kPauliThreads>(acc, red);
@@ -1051,11 +1004,7 @@ __global__ void __launch_bounds__(kPauliThreads, 2) k_hpsi_tile(const double2* p
 #pragma unroll
   for (int b = 0; b < 9; b++)
     if ((t >> b) & 1) toff |= uint64_t(1) << g.bits[b];
-  auto signed_coeff = [&](int i, uint32_t z) {
-    const uint32_t odd = (uint32_t)__popc(t & z & 0xffffu) << 31;
-    const double c = sc[i];
-    return __hiloint2double(__double2hiint(c) ^ (int)odd, __double2loint(c));
-  };
+  auto signed_coeff = [&](int i, uint32_t z) { return flip_sign(sc[i], __popc(t & z & 0xffffu) & 1); };
   double e = 0.0;
   for (uint64_t tile = blockIdx.x; tile < g.ntiles; tile += gridDim.x) {
     const uint64_t mine = ((tile >> lane) & 1) << ctxq;

@@ -1,0 +1,180 @@
+// rounds.h -- planning of in-shared-memory simulation: gates on a state of at
+// most 13 qubits grouped into rounds, with CNOTs and swaps as relabellings.
+//
+// The state sits in shared memory at physical indices p; the logical index is
+// B p over GF(2).  A CNOT or an uncontrolled swap only changes B, so it moves
+// nothing.  A gate on logical qubit q pairs p with p ^ col[q], and p's logical bit
+// q is the parity of p & row[q].
+//
+// A round is a run of consecutive one-qubit gates whose pair masks span at most
+// four dimensions: each thread loads the 16 amplitudes of one coset of the span into
+// registers, applies every gate of the round there, in program order, and stores
+// them back -- one pass over shared memory and one barrier for the whole run.  A
+// coset is closed under the round's gates, so each amplitude sees them in program
+// order, pruning after every gate included.
+#pragma once
+
+#include <stdint.h>
+
+#include <algorithm>
+#include <utility>
+#include <vector>
+
+namespace ket {
+
+constexpr int kRoundBits = 4;        // dimension of a round's span, at most
+constexpr int kRoundGates = 16;      // gates in a round, at most
+constexpr int kRoundQubits = 13;
+
+// Shared-memory slot of amplitude i: the low three bits XORed with every higher
+// group of three, so that eight threads on any of the usual index patterns touch
+// eight 16-byte banks.  Linear over GF(2): slot(p ^ m) = slot(p) ^ slot(m).
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+inline uint32_t round_slot(uint32_t i) {
+  return i ^ (((i >> 3) ^ (i >> 6) ^ (i >> 9) ^ (i >> 12)) & 7u);
+}
+
+struct RoundGate {
+  uint8_t x;         // 1: X under its controls, 0: a 2x2 under its controls
+  uint8_t bit;       // the gate's mask = basis mask `bit` of the round
+  uint8_t nc;        // controls
+  uint8_t cj[3];     // per control: the basis masks that flip it
+  uint16_t r;        // row functional of the target
+  uint16_t m;        // pair mask of the target
+  uint16_t rc[3];    // row functionals of the controls
+  int32_t op;        // the caller's op
+};
+
+struct Round {
+  uint8_t k;                     // dimension; a two-qubit round has k = 2
+  uint8_t two;                   // 1: one 4x4, on masks (1: first qubit, 0: second)
+  uint8_t piv[kRoundBits];       // pivot bits of the span, ascending
+  uint16_t m[kRoundBits];        // basis masks
+  uint16_t slot[1 << kRoundBits];  // round_slot of the XOR of the masks in j
+  uint16_t r2[2];                // two: row functionals of (second, first) qubit
+  int32_t gate0, ngates;
+};
+
+// The relabelling and the round under construction.
+class RoundPlan {
+ public:
+  std::vector<Round> rounds;
+  std::vector<RoundGate> gates;
+  uint16_t row[kRoundQubits], col[kRoundQubits];
+
+  explicit RoundPlan(int kmax = kRoundBits) : kmax_(kmax) {
+    for (int q = 0; q < kRoundQubits; q++) row[q] = col[q] = (uint16_t)(1u << q);
+  }
+  void cnot(int c, int t) { row[t] ^= row[c]; col[c] ^= col[t]; }
+  void swap(int a, int b) { std::swap(row[a], row[b]); std::swap(col[a], col[b]); }
+
+  // A one-qubit gate (or X) on q under controls cs.
+  void gate(int q, const int* cs, int nc, bool x, int op) {
+    RoundGate g = {};
+    g.x = x;
+    g.nc = (uint8_t)nc;
+    g.r = row[q];
+    g.m = col[q];
+    for (int i = 0; i < nc; i++) g.rc[i] = row[cs[i]];
+    g.op = op;
+    if (!join(g)) {
+      close();
+      join(g);
+    }
+  }
+  // A 4x4 on (a = MSB, b) under controls cs: a round of its own.
+  void gate2(int a, int b, const int* cs, int nc, int op) {
+    close();
+    RoundGate g = {};
+    g.nc = (uint8_t)nc;
+    for (int i = 0; i < nc; i++) g.rc[i] = row[cs[i]];
+    g.op = op;
+    cur_ = {g};
+    basis_ = {col[b], col[a]};
+    r2_[0] = row[b];
+    r2_[1] = row[a];
+    two_ = true;
+    close();
+  }
+  // End the round under construction (before anything that is not a gate).
+  void close() {
+    if (!cur_.empty()) {
+      Round R = {};
+      R.k = (uint8_t)basis_.size();
+      R.two = two_;
+      std::vector<uint16_t> e = basis_;
+      for (size_t i = 0; i < e.size(); i++) {  // echelon form: pivot = highest set bit
+        const int h = 31 - __builtin_clz((unsigned)e[i]);
+        R.piv[i] = (uint8_t)h;
+        for (size_t j = i + 1; j < e.size(); j++)
+          if ((e[j] >> h) & 1) e[j] ^= e[i];
+      }
+      std::sort(R.piv, R.piv + R.k);
+      for (int i = 0; i < R.k; i++) R.m[i] = basis_[i];
+      for (int j = 0; j < (1 << R.k); j++) {
+        uint32_t x = 0;
+        for (int i = 0; i < R.k; i++)
+          if ((j >> i) & 1) x ^= basis_[i];
+        R.slot[j] = (uint16_t)round_slot(x);
+      }
+      R.r2[0] = r2_[0];
+      R.r2[1] = r2_[1];
+      R.gate0 = (int32_t)gates.size();
+      R.ngates = (int32_t)cur_.size();
+      for (RoundGate& g : cur_) {
+        for (int c = 0; c < g.nc; c++) {
+          g.cj[c] = 0;
+          for (int i = 0; i < R.k; i++)
+            if (odd(basis_[i] & g.rc[c])) g.cj[c] |= (uint8_t)(1u << i);
+        }
+        gates.push_back(g);
+      }
+      rounds.push_back(R);
+    }
+    cur_.clear();
+    basis_.clear();
+    two_ = false;
+  }
+
+ private:
+  int kmax_;
+  std::vector<RoundGate> cur_;
+  std::vector<uint16_t> basis_;
+  uint16_t r2_[2] = {0, 0};
+  bool two_ = false;
+
+  static bool odd(uint32_t x) { return __builtin_popcount(x) & 1; }
+  bool independent(uint16_t m) const {
+    uint32_t x = m;
+    std::vector<uint16_t> e = basis_;
+    for (size_t i = 0; i < e.size(); i++) {
+      const int h = 31 - __builtin_clz((unsigned)e[i]);
+      for (size_t j = i + 1; j < e.size(); j++)
+        if ((e[j] >> h) & 1) e[j] ^= e[i];
+      if ((x >> h) & 1) x ^= e[i];
+    }
+    return x != 0;
+  }
+  // Every target's logical bit is fixed by its own mask alone across a coset, so
+  // one test on the coset's base gives a thread's role for all its pairs.
+  bool join(RoundGate& g) {
+    if ((int)cur_.size() >= kRoundGates) return false;
+    size_t at = 0;
+    while (at < basis_.size() && basis_[at] != g.m) at++;
+    for (size_t i = 0; i < basis_.size(); i++)
+      if (i != at && odd(basis_[i] & g.r)) return false;
+    if (at == basis_.size()) {
+      if ((int)at >= kmax_ || !independent(g.m)) return false;
+      for (const RoundGate& o : cur_)
+        if (odd(g.m & o.r)) return false;
+      basis_.push_back(g.m);
+    }
+    g.bit = (uint8_t)at;
+    cur_.push_back(g);
+    return true;
+  }
+};
+
+}  // namespace ket
