@@ -78,7 +78,7 @@ struct BRoundGate {
   int32_t slot;
 };
 
-struct BRound {
+struct __align__(16) BRound {
   uint16_t slot[16];
   uint8_t piv[4];
   uint8_t k, two;
@@ -235,9 +235,9 @@ __device__ __forceinline__ void reg_x(cpx<double>* v, uint32_t ok) {
     if (!(j & (1 << I)) && ((ok >> j) & 1)) swap_c(v[j], v[j | 1 << I]);
 }
 
-template <int K>
 __device__ __forceinline__ void run_round(double2* s, const BRound& R, const BRoundGate* gates, const double2* mats,
                                           int n, int lgpack) {
+  constexpr int K = kRoundBits;
   const uint32_t nsub = 1u << (n + lgpack - K);
   for (uint32_t u = threadIdx.x; u < nsub; u += kVqeThreads) {
     uint32_t base = u;
@@ -245,11 +245,15 @@ __device__ __forceinline__ void run_round(double2* s, const BRound& R, const BRo
     for (int i = 0; i < K; i++) base = insert0_32(base, R.piv[i]);
     const uint32_t sb = round_slot(base), inst = base >> n;
     cpx<double> v[1 << K];
+    RoundSlots slots;
+    slots.read(R.slot);
 #pragma unroll
     for (int j = 0; j < (1 << K); j++) {
-      const double2 t = s[sb ^ R.slot[j]];
+      const double2 t = s[sb ^ slots(j)];
       v[j] = cpx<double>{t.x, t.y};
     }
+    // cosets of zeros stay zeros (most of a state in its first gates)
+    if (!__any_sync(__activemask(), !all_zero<double, 1 << K>(v))) continue;
     for (int k = 0; k < R.ngates; k++) {
       const BRoundGate& g = gates[k];
       const uint32_t ok = g.nc ? controls_ok(g, base) : 0xffffu;
@@ -257,16 +261,17 @@ __device__ __forceinline__ void run_round(double2* s, const BRound& R, const BRo
       const double2* M = mats + 4 * ((g.slot << lgpack) + inst);
       const bool ctl = g.nc != 0;
       switch (g.bit + 4 * g.form) {
-#define KET_BIT(I)                                                                     \
-  case I: if constexpr (K > I) reg_gate<K, I, 0>(v, M, role, ctl, ok); break;          \
-  case 4 + I: if constexpr (K > I) reg_gate<K, I, 1>(v, M, role, ctl, ok); break;      \
-  case 8 + I: if constexpr (K > I) reg_x<K, I>(v, ok); break;
+#define KET_BIT(I)                                             \
+  case I: reg_gate<K, I, 0>(v, M, role, ctl, ok); break;       \
+  case 4 + I: reg_gate<K, I, 1>(v, M, role, ctl, ok); break;   \
+  case 8 + I: reg_x<K, I>(v, ok); break;
         KET_BIT(0) KET_BIT(1) KET_BIT(2) KET_BIT(3)
 #undef KET_BIT
       }
     }
+    slots.read(R.slot);
 #pragma unroll
-    for (int j = 0; j < (1 << K); j++) s[sb ^ R.slot[j]] = make_double2(v[j].re, v[j].im);
+    for (int j = 0; j < (1 << K); j++) s[sb ^ slots(j)] = make_double2(v[j].re, v[j].im);
   }
 }
 
@@ -393,12 +398,7 @@ __global__ void __launch_bounds__(kVqeThreads) k_batch_vqe(BArgs a) {
         if (R.two) {
           run_two(s, R, *G, mats, n, T.lgpack);
         } else {
-          switch (R.k) {
-            case 1: run_round<1>(s, R, G, mats, n, T.lgpack); break;
-            case 2: run_round<2>(s, R, G, mats, n, T.lgpack); break;
-            case 3: run_round<3>(s, R, G, mats, n, T.lgpack); break;
-            default: run_round<4>(s, R, G, mats, n, T.lgpack); break;
-          }
+          run_round(s, R, G, mats, n, T.lgpack);
         }
       }
       __syncthreads();
@@ -480,13 +480,17 @@ struct BImage {
 // Returns the work of one instance (gates x amplitudes).
 int64_t lower_template(std::vector<HOp>& ops, const std::vector<PauliTerm>& terms, BTmpl& T, BImage& im) {
   fold_ops(ops);
-  RoundPlan rp;
+  RoundPlan rp(T.n);
   for (size_t i = 0; i < ops.size(); i++) {
     const HOp& o = ops[i];
     if (o.dead) continue;
     switch (o.kind) {
       case HOp::M1: rp.gate(o.q0, o.cs, o.nc, false, (int)i); break;
-      case HOp::M2: rp.gate2(o.q0, o.q1, o.cs, o.nc, (int)i); break;
+      case HOp::M2: {
+        const int qs[2] = {o.q0, o.q1};
+        rp.dense(qs, 2, o.cs, o.nc, (int)i);
+        break;
+      }
       case HOp::X:
         if (o.nc == 1) rp.cnot(o.cs[0], o.q0);
         else rp.gate(o.q0, o.cs, o.nc, true, (int)i);
@@ -519,15 +523,15 @@ int64_t lower_template(std::vector<HOp>& ops, const std::vector<PauliTerm>& term
   new_chunk();
   for (const Round& r : rp.rounds) {
     int need = 0;
-    for (int k = 0; k < r.ngates; k++) need += rp.gates[r.gate0 + k].x ? 0 : r.two ? 4 : 1;
+    for (int k = 0; k < r.ngates; k++) need += rp.gates[r.gate0 + k].x ? 0 : r.dense ? 4 : 1;
     if (slot + need - C.slot0 > room || C.nrounds == kVqeRounds || C.ngates + r.ngates > kVqeGates) end_chunk();
     BRound R = {};
     std::copy(r.slot, r.slot + 16, R.slot);
     std::copy(r.piv, r.piv + 4, R.piv);
     R.k = r.k;
-    R.two = r.two;
-    R.r2[0] = r.r2[0];
-    R.r2[1] = r.r2[1];
+    R.two = r.dense;
+    R.r2[0] = r.rd[0];
+    R.r2[1] = r.rd[1];
     R.ngates = (uint16_t)r.ngates;
     R.gate0 = C.ngates;
     im.rounds.push_back(R);
@@ -536,7 +540,7 @@ int64_t lower_template(std::vector<HOp>& ops, const std::vector<PauliTerm>& term
     for (int k = 0; k < r.ngates; k++) {
       const RoundGate& g = rp.gates[r.gate0 + k];
       BRoundGate G = {};
-      G.form = g.x ? 2 : !r.two && ops[g.op].real ? 1 : 0;
+      G.form = g.x ? 2 : !r.dense && ops[g.op].real ? 1 : 0;
       G.bit = g.bit;
       G.nc = g.nc;
       G.r = g.r;
@@ -545,9 +549,9 @@ int64_t lower_template(std::vector<HOp>& ops, const std::vector<PauliTerm>& term
       G.slot = slot - C.slot0;
       if (!g.x) {
         const std::vector<BFactor>& f = ops[g.op].factors;
-        im.matv.push_back(BMat{(int32_t)im.factors.size(), (int16_t)f.size(), (int16_t)r.two, slot});
+        im.matv.push_back(BMat{(int32_t)im.factors.size(), (int16_t)f.size(), (int16_t)r.dense, slot});
         im.factors.insert(im.factors.end(), f.begin(), f.end());
-        slot += r.two ? 4 : 1;
+        slot += r.dense ? 4 : 1;
         C.nmats++;
       }
       im.gates.push_back(G);

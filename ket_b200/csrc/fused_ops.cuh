@@ -142,6 +142,22 @@ __device__ __forceinline__ void prune_slots(cpx<R>* x, double thr, double qthr) 
   }
 }
 
+// Whether all NS amplitudes are (+-)0.
+template <typename R, int NS>
+__device__ __forceinline__ bool all_zero(const cpx<R>* x) {
+  uint32_t o = 0;
+#pragma unroll
+  for (int j = 0; j < NS; j++) {
+    if constexpr (sizeof(R) == 8) {
+      o |= ((uint32_t)(__double2hiint(x[j].re) | __double2hiint(x[j].im)) << 1) | (uint32_t)__double2loint(x[j].re) |
+           (uint32_t)__double2loint(x[j].im);
+    } else {
+      o |= (uint32_t)(__float_as_int(x[j].re) | __float_as_int(x[j].im)) << 1;
+    }
+  }
+  return o == 0;
+}
+
 // ---------------------------------------------------------------- register and lane ops
 template <typename R>
 __device__ __forceinline__ cpx<R> shfl_xor_c(cpx<R> v, int mask, uint32_t members) {

@@ -7,7 +7,8 @@
 // q is the parity of p & row[q].
 //
 // A round is a run of consecutive one-qubit gates whose pair masks span at most
-// four dimensions: each thread loads the 16 amplitudes of one coset of the span into
+// four dimensions (the span is filled up to four, so that one form of the code
+// serves all rounds): each thread loads the 16 amplitudes of one coset of the span into
 // registers, applies every gate of the round there, in program order, and stores
 // them back -- one pass over shared memory and one barrier for the whole run.  A
 // coset is closed under the round's gates, so each amplitude sees them in program
@@ -22,7 +23,7 @@
 
 namespace ket {
 
-constexpr int kRoundBits = 4;        // dimension of a round's span, at most
+constexpr int kRoundBits = 4;        // dimension of a round's span
 constexpr int kRoundGates = 16;      // gates in a round, at most
 constexpr int kRoundQubits = 13;
 
@@ -36,6 +37,22 @@ inline uint32_t round_slot(uint32_t i) {
   return i ^ (((i >> 3) ^ (i >> 6) ^ (i >> 9) ^ (i >> 12)) & 7u);
 }
 
+#ifdef __CUDACC__
+// A round's 16 slot offsets, two a register, from shared memory (16-byte aligned).
+// Read before the loads and again before the stores: kept across the gates, the 16
+// addresses spilled as many amplitudes.
+struct RoundSlots {
+  uint32_t w[8];
+  __device__ __forceinline__ void read(const uint16_t* p) {
+    const uint32_t a = (uint32_t)__cvta_generic_to_shared(p);
+    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]) : "r"(a));
+    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7]) : "r"(a + 16));
+  }
+  __device__ __forceinline__ uint32_t operator()(int j) const { return j & 1 ? w[j >> 1] >> 16 : w[j >> 1] & 0xffffu; }
+};
+#endif
+
 struct RoundGate {
   uint8_t x;         // 1: X under its controls, 0: a 2x2 under its controls
   uint8_t bit;       // the gate's mask = basis mask `bit` of the round
@@ -48,12 +65,12 @@ struct RoundGate {
 };
 
 struct Round {
-  uint8_t k;                     // dimension; a two-qubit round has k = 2
-  uint8_t two;                   // 1: one 4x4, on masks (1: first qubit, 0: second)
+  uint8_t k;                     // dimension: kRoundBits, or that of a dense round
+  uint8_t dense;                 // 1: one 2^k x 2^k, local index bit i on mask i
   uint8_t piv[kRoundBits];       // pivot bits of the span, ascending
   uint16_t m[kRoundBits];        // basis masks
   uint16_t slot[1 << kRoundBits];  // round_slot of the XOR of the masks in j
-  uint16_t r2[2];                // two: row functionals of (second, first) qubit
+  uint16_t rd[kRoundBits];       // dense: row functional of local index bit i
   int32_t gate0, ngates;
 };
 
@@ -64,7 +81,8 @@ class RoundPlan {
   std::vector<RoundGate> gates;
   uint16_t row[kRoundQubits], col[kRoundQubits];
 
-  explicit RoundPlan(int kmax = kRoundBits) : kmax_(kmax) {
+  // n: the state's qubits, at least kRoundBits.
+  explicit RoundPlan(int n) : n_(n) {
     for (int q = 0; q < kRoundQubits; q++) row[q] = col[q] = (uint16_t)(1u << q);
   }
   void cnot(int c, int t) { row[t] ^= row[c]; col[c] ^= col[t]; }
@@ -84,26 +102,28 @@ class RoundPlan {
       join(g);
     }
   }
-  // A 4x4 on (a = MSB, b) under controls cs: a round of its own.
-  void gate2(int a, int b, const int* cs, int nc, int op) {
+  // A 2^k x 2^k on qs (qs[0] = MSB) under controls cs: a round of its own.
+  void dense(const int* qs, int k, const int* cs, int nc, int op) {
     close();
     RoundGate g = {};
     g.nc = (uint8_t)nc;
     for (int i = 0; i < nc; i++) g.rc[i] = row[cs[i]];
     g.op = op;
     cur_ = {g};
-    basis_ = {col[b], col[a]};
-    r2_[0] = row[b];
-    r2_[1] = row[a];
-    two_ = true;
+    for (int i = 0; i < k; i++) {
+      basis_.push_back(col[qs[k - 1 - i]]);
+      rd_[i] = row[qs[k - 1 - i]];
+    }
+    dense_ = true;
     close();
   }
   // End the round under construction (before anything that is not a gate).
   void close() {
     if (!cur_.empty()) {
+      if (!dense_) fill();
       Round R = {};
       R.k = (uint8_t)basis_.size();
-      R.two = two_;
+      R.dense = dense_;
       std::vector<uint16_t> e = basis_;
       for (size_t i = 0; i < e.size(); i++) {  // echelon form: pivot = highest set bit
         const int h = 31 - __builtin_clz((unsigned)e[i]);
@@ -119,8 +139,7 @@ class RoundPlan {
           if ((j >> i) & 1) x ^= basis_[i];
         R.slot[j] = (uint16_t)round_slot(x);
       }
-      R.r2[0] = r2_[0];
-      R.r2[1] = r2_[1];
+      for (int i = 0; i < kRoundBits; i++) R.rd[i] = rd_[i];
       R.gate0 = (int32_t)gates.size();
       R.ngates = (int32_t)cur_.size();
       for (RoundGate& g : cur_) {
@@ -135,15 +154,16 @@ class RoundPlan {
     }
     cur_.clear();
     basis_.clear();
-    two_ = false;
+    brow_.clear();
+    dense_ = false;
   }
 
  private:
-  int kmax_;
+  int n_;
   std::vector<RoundGate> cur_;
-  std::vector<uint16_t> basis_;
-  uint16_t r2_[2] = {0, 0};
-  bool two_ = false;
+  std::vector<uint16_t> basis_, brow_;  // masks, and the targets' row functionals: brow_[i] . basis_[j] = (i == j)
+  uint16_t rd_[kRoundBits] = {};
+  bool dense_ = false;
 
   static bool odd(uint32_t x) { return __builtin_popcount(x) & 1; }
   bool independent(uint16_t m) const {
@@ -163,17 +183,29 @@ class RoundPlan {
     if ((int)cur_.size() >= kRoundGates) return false;
     size_t at = 0;
     while (at < basis_.size() && basis_[at] != g.m) at++;
-    for (size_t i = 0; i < basis_.size(); i++)
-      if (i != at && odd(basis_[i] & g.r)) return false;
-    if (at == basis_.size()) {
-      if ((int)at >= kmax_ || !independent(g.m)) return false;
-      for (const RoundGate& o : cur_)
-        if (odd(g.m & o.r)) return false;
+    if (at < basis_.size()) {
+      if (brow_[at] != g.r) return false;
+    } else {
+      if ((int)at >= kRoundBits || !independent(g.m)) return false;
+      for (size_t i = 0; i < at; i++)
+        if (odd(basis_[i] & g.r) || odd(g.m & brow_[i])) return false;
       basis_.push_back(g.m);
+      brow_.push_back(g.r);
     }
     g.bit = (uint8_t)at;
     cur_.push_back(g);
     return true;
+  }
+  // Masks that complete the span and flip none of the round's targets: unit
+  // vectors, each made orthogonal to the targets' functionals.
+  void fill() {
+    const size_t k = brow_.size();
+    for (int b = n_ - 1; b >= 0 && (int)basis_.size() < kRoundBits; b--) {
+      uint16_t m = (uint16_t)(1u << b);
+      for (size_t i = 0; i < k; i++)
+        if (odd(m & brow_[i])) m ^= basis_[i];
+      if (m && independent(m)) basis_.push_back(m);
+    }
   }
 };
 

@@ -28,7 +28,9 @@
 #include "common.cuh"
 #include "ctx.h"
 #include "engine.h"
+#include "fused_ops.cuh"
 #include "launch.h"
+#include "rounds.h"
 
 using namespace ket;
 
@@ -90,10 +92,22 @@ __global__ void k_collapse(typename Vec2<R>::T* a, uint64_t N, int q, int outcom
 
 // ---------------------------------------------------------------- batched trajectories
 // Small states (2^n amplitudes fit in shared memory) run one shot per CTA,
-// many shots at a time.  Every thread keeps the same copy of the xorshift32
-// state and makes the same draws, so a draw needs no communication; gate
-// arithmetic rounds exactly as the reference's complex.ts does (products and
-// sums each rounded, no fused multiply-add), pruning as accumulate() does.
+// many shots at a time.  Gate arithmetic rounds exactly as the reference's
+// complex.ts does (products and sums each rounded, no fused multiply-add; the
+// products of zero matrix entries, which add nothing, are left out), pruning as
+// accumulate() does.
+//
+// The op list is planned once for all shots (plan_shots): one-qubit gates run in
+// rounds on cosets of 16 amplitudes held in registers, and CNOTs and swaps outside
+// if-bodies are relabellings of the shared-memory state (rounds.h).  What differs
+// from shot to shot is carried beside the plan:
+//   * the Paulis the noise draws select are a frame: an X on a qubit moves the
+//     physical indices by a mask (beta), a Z signs them by a functional (zeta), and
+//     a gate reads both as of its place in the program -- the swapped rows and
+//     columns, or negated off-diagonal entries, a Pauli before it amounts to.
+//     (A Y is both, up to a phase that no probability sees.)
+//   * draw d of the shot's xorshift32 stream is the start state under a GF(2) power
+//     of the step, so the threads make the draws of a segment in parallel.
 
 enum { T_NOISE1 = 20, T_NOISE2 = 21 };
 
@@ -112,307 +126,524 @@ __device__ __forceinline__ cd cmul_rn(cd a, cd b) {  // complex.ts mul
 }
 __device__ __forceinline__ cd cadd_rn(cd a, cd b) { return {__dadd_rn(a.re, b.re), __dadd_rn(a.im, b.im)}; }
 __device__ __forceinline__ double norm2_rn(cd a) { return __dadd_rn(__dmul_rn(a.re, a.re), __dmul_rn(a.im, a.im)); }
-__device__ __forceinline__ cd pruned(cd a) { return norm2_rn(a) < 1e-14 ? cd{0.0, 0.0} : a; }
+__device__ __forceinline__ cd pruned(cd a) {
+  // (the high words rule out all but components of about 1e-7 and below)
+  if (fmaxf(hiabs(a.re), hiabs(a.im)) < tiny_screen(0.0) && norm2_rn(a) < 1e-14) return cd{0.0, 0.0};
+  return a;
+}
 
 template <typename V>
-__device__ __forceinline__ cd ldc(const V* st, uint64_t i) { const V v = st[i]; return {(double)v.x, (double)v.y}; }
+__device__ __forceinline__ cd ldc(const V* st, uint32_t i) { const V v = st[i]; return {(double)v.x, (double)v.y}; }
 template <typename V>
-__device__ __forceinline__ void stc(V* st, uint64_t i, cd a) {
+__device__ __forceinline__ void stc(V* st, uint32_t i, cd a) {
   V v;
   v.x = (decltype(v.x))a.re;
   v.y = (decltype(v.y))a.im;
   st[i] = v;
 }
-__device__ __forceinline__ cd mat_at(const double* M, int64_t off, int i) {
-  return {__ldg(M + 2 * (off + i)), __ldg(M + 2 * (off + i) + 1)};
-}
 
-// xorshift32 (circuit.ts:813-819), identical in every thread
-__device__ __forceinline__ double tdraw(uint32_t& s) {
+constexpr int kShotBits = kRoundBits;
+constexpr int kShotMinQubits = 4;  // narrower states get idle qubits, so that a coset of 16 exists
+
+struct __align__(16) SRound {
+  uint16_t slot[16], m[4], rd[4];
+  uint8_t piv[4];
+  uint8_t k, dense;
+  uint16_t ngates;
+  int32_t gate0;      // in the segment
+  int32_t pad;
+};
+enum : uint8_t { SF_GEN = 0, SF_REAL = 1, SF_RX = 2, SF_DIAG = 3, SF_X = 4 };
+struct __align__(16) SGate {
+  uint8_t form, bit, nc, pad;
+  uint16_t r, m;      // the target's functional and mask
+  int32_t slot;       // matrix, in 64-byte slots of the segment
+  uint32_t frame;     // beta | zeta << 16 as of this gate (shared memory only)
+  uint16_t rc[2];     // controls
+  uint8_t cj[2];
+  uint16_t pad2;
+  int32_t dpos;       // noise draws of the segment before this gate
+  int32_t pad3;
+};
+static_assert(sizeof(SGate) == 32, "two 16-byte reads");
+// A noise draw: the masks and functionals of its qubits at its place in the program.
+struct SNoise {
+  uint16_t ma, ra, mb, rb;
+  int32_t two;
+};
+// Gates between measurements, resets and ifs, as many as shared memory holds.
+struct SSeg {
+  int32_t round0, nrounds, gate0, ngates, slot0, nslots;
+  int32_t noise0, ndraws, per, jump0;  // draws, draws a thread, first jump row
+};
+enum { ST_SEG = 0, ST_MEASURE = 1, ST_RESET = 2, ST_IF = 3 };
+struct SStep {
+  int32_t kind;
+  int32_t a, b, c, d;  // SEG: index; MEASURE: cbit, jump row; RESET: -, jump row; IF: first, size, value, steps to skip
+  uint16_t r, m;       // MEASURE, RESET: the qubit's functional and mask (r = 0: a qubit outside the state)
+};
+
+struct SArgs {
+  const SStep* steps;
+  const SSeg* segs;
+  const SRound* rounds;
+  const SGate* gates;
+  const double2* mats;   // by 64-byte slots
+  const SNoise* noise;
+  const uint32_t* jump;  // rows of 32 columns: the step's power that makes the row's draw
+  const uint32_t* start;
+  uint64_t* out_idx;
+  uint8_t* out_bits;
+  uint64_t shots, init;
+  ket_noise nz;
+  int nsteps, n, ne, ncbits;  // ne: qubits with idle ones
+  int last_row;               // jump row of the sampling draw
+  // shared-memory layout (bytes)
+  int off_mats, off_rounds, off_gates, off_events, off_red, off_bits;
+  uint16_t acol[kRoundQubits];  // the final relabelling: physical mask of each logical bit
+};
+
+struct SEvent {
+  int32_t d;
+  uint32_t bz;  // beta | zeta << 16
+};
+
+__device__ __forceinline__ uint32_t xs_step(uint32_t s) {  // xorshift32 (circuit.ts:813-819)
   s ^= s << 13;
   s ^= s >> 17;
-  s ^= s << 5;
-  return (double)s / 4294967296.0;
+  return s ^ (s << 5);
+}
+__device__ __forceinline__ double xs_value(uint32_t s) { return (double)s / 4294967296.0; }
+__device__ __forceinline__ uint32_t xs_jump(const uint32_t* row, uint32_t s) {
+  uint32_t o = 0;
+#pragma unroll
+  for (int k = 0; k < 32; k += 4) {
+    const uint4 c = __ldg(reinterpret_cast<const uint4*>(row + k));
+    o ^= ((s >> k) & 1 ? c.x : 0u) ^ ((s >> (k + 1)) & 1 ? c.y : 0u) ^ ((s >> (k + 2)) & 1 ? c.z : 0u) ^
+         ((s >> (k + 3)) & 1 ? c.w : 0u);
+  }
+  return o;
 }
 
-// 2x2 on target t; c >= 0: controlled on c, whose 0-entries pass through
-// accumulate() and are pruned in place (applyControlled, statevector.ts:212-234)
-template <typename V, int NT>
-__device__ void t_apply2(V* st, int n, int t, int c, const double* M, int64_t off) {
-  const cd g0 = mat_at(M, off, 0), g1 = mat_at(M, off, 1), g2 = mat_at(M, off, 2), g3 = mat_at(M, off, 3);
-  const uint64_t half = uint64_t(1) << (n - 1);
-  for (uint64_t j = threadIdx.x; j < half; j += NT) {
-    const uint64_t i0 = insert0(j, t), i1 = i0 | (uint64_t(1) << t);
-    const cd a0 = ldc(st, i0), a1 = ldc(st, i1);
-    if (c >= 0 && !((i0 >> c) & 1)) {
-      stc(st, i0, pruned(a0));
-      stc(st, i1, pruned(a1));
-      continue;
+__device__ __forceinline__ double neg_if(double v, uint32_t odd) {
+  return __hiloint2double(__double2hiint(v) ^ (int)(odd << 31), __double2loint(v));
+}
+__device__ __forceinline__ uint32_t par(uint32_t x) { return (uint32_t)__popc(x) & 1u; }
+
+// The amplitudes j of a coset whose controls all hold (p: the base, moved by beta).
+__device__ __forceinline__ uint32_t shot_controls(const SGate& g, uint32_t p) {
+  uint32_t ok = 0xffffu;
+  for (int c = 0; c < g.nc; c++) {
+    const uint32_t cj = g.cj[c];
+    uint32_t x = par(p & g.rc[c]) ? 0xffffu : 0u;
+    x ^= (cj & 1 ? 0xaaaau : 0u) ^ (cj & 2 ? 0xccccu : 0u) ^ (cj & 4 ? 0xf0f0u : 0u) ^ (cj & 8 ? 0xff00u : 0u);
+    ok &= x;
+  }
+  return ok;
+}
+
+// A 2x2 on register bit I.  role: the amplitude with the bit clear holds logical 1
+// (entry e becomes e ^ 3); neg: the off-diagonal entries change sign.
+// The pair's new values, in place: inline PTX with tied operands (the cross products
+// first), so that every amplitude keeps its registers across the forms the gate loop
+// switches between.  Written as expressions, the loop re-homed the thread's 64
+// registers of amplitudes at every gate.  Each product and sum is rounded.
+template <int FORM>
+__device__ __forceinline__ void shot_pair(cd& a, cd& b, const cd* g) {
+  if (FORM == SF_REAL) {
+    asm("{\n .reg .f64 x, y, u, w;\n"
+        " mul.rn.f64 x, %5, %2;\n mul.rn.f64 y, %5, %3;\n mul.rn.f64 u, %6, %0;\n mul.rn.f64 w, %6, %1;\n"
+        " mul.rn.f64 %0, %4, %0;\n add.rn.f64 %0, %0, x;\n mul.rn.f64 %1, %4, %1;\n add.rn.f64 %1, %1, y;\n"
+        " mul.rn.f64 %2, %7, %2;\n add.rn.f64 %2, u, %2;\n mul.rn.f64 %3, %7, %3;\n add.rn.f64 %3, w, %3;\n}"
+        : "+d"(a.re), "+d"(a.im), "+d"(b.re), "+d"(b.im)
+        : "d"(g[0].re), "d"(g[1].re), "d"(g[2].re), "d"(g[3].re));
+  } else if (FORM == SF_RX) {
+    asm("{\n .reg .f64 x, y, u, w;\n"
+        " mul.rn.f64 x, %5, %3;\n mul.rn.f64 y, %5, %2;\n mul.rn.f64 u, %6, %1;\n mul.rn.f64 w, %6, %0;\n"
+        " mul.rn.f64 %0, %4, %0;\n sub.rn.f64 %0, %0, x;\n mul.rn.f64 %1, %4, %1;\n add.rn.f64 %1, %1, y;\n"
+        " mul.rn.f64 %2, %7, %2;\n sub.rn.f64 %2, %2, u;\n mul.rn.f64 %3, %7, %3;\n add.rn.f64 %3, w, %3;\n}"
+        : "+d"(a.re), "+d"(a.im), "+d"(b.re), "+d"(b.im)
+        : "d"(g[0].re), "d"(g[1].im), "d"(g[2].im), "d"(g[3].re));
+  } else if (FORM == SF_DIAG) {
+    asm("{\n .reg .f64 x, y;\n"
+        " mul.rn.f64 x, %5, %1;\n mul.rn.f64 y, %5, %0;\n mul.rn.f64 %0, %4, %0;\n sub.rn.f64 %0, %0, x;\n"
+        " mul.rn.f64 %1, %4, %1;\n add.rn.f64 %1, %1, y;\n"
+        " mul.rn.f64 x, %7, %3;\n mul.rn.f64 y, %7, %2;\n mul.rn.f64 %2, %6, %2;\n sub.rn.f64 %2, %2, x;\n"
+        " mul.rn.f64 %3, %6, %3;\n add.rn.f64 %3, %3, y;\n}"
+        : "+d"(a.re), "+d"(a.im), "+d"(b.re), "+d"(b.im)
+        : "d"(g[0].re), "d"(g[0].im), "d"(g[3].re), "d"(g[3].im));
+  } else {
+    asm("{\n .reg .f64 x, y, u, w, t, s;\n"
+        // x + i y = g1 b, u + i w = g2 a
+        " mul.rn.f64 x, %6, %2;\n mul.rn.f64 t, %7, %3;\n sub.rn.f64 x, x, t;\n"
+        " mul.rn.f64 y, %6, %3;\n mul.rn.f64 t, %7, %2;\n add.rn.f64 y, y, t;\n"
+        " mul.rn.f64 u, %8, %0;\n mul.rn.f64 t, %9, %1;\n sub.rn.f64 u, u, t;\n"
+        " mul.rn.f64 w, %8, %1;\n mul.rn.f64 t, %9, %0;\n add.rn.f64 w, w, t;\n"
+        // a = g0 a + (x + i y), b = (u + i w) + g3 b
+        " mul.rn.f64 t, %5, %1;\n mul.rn.f64 s, %5, %0;\n"
+        " mul.rn.f64 %0, %4, %0;\n sub.rn.f64 %0, %0, t;\n add.rn.f64 %0, %0, x;\n"
+        " mul.rn.f64 %1, %4, %1;\n add.rn.f64 %1, %1, s;\n add.rn.f64 %1, %1, y;\n"
+        " mul.rn.f64 t, %11, %3;\n mul.rn.f64 s, %11, %2;\n"
+        " mul.rn.f64 %2, %10, %2;\n sub.rn.f64 %2, %2, t;\n add.rn.f64 %2, u, %2;\n"
+        " mul.rn.f64 %3, %10, %3;\n add.rn.f64 %3, %3, s;\n add.rn.f64 %3, w, %3;\n}"
+        : "+d"(a.re), "+d"(a.im), "+d"(b.re), "+d"(b.im)
+        : "d"(g[0].re), "d"(g[0].im), "d"(g[1].re), "d"(g[1].im), "d"(g[2].re), "d"(g[2].im), "d"(g[3].re), "d"(g[3].im));
+  }
+}
+
+template <typename R, int K, int I, int FORM>
+__device__ __forceinline__ void shot_gate(cpx<R>* v, const double2* M, bool role, uint32_t neg, bool ctl, uint32_t ok) {
+  constexpr int NS = 1 << K;
+  cd g[4];
+#pragma unroll
+  for (int e = 0; e < 4; e++) {
+    const double2 t = M[role ? e ^ 3 : e];
+    g[e] = (e == 1 || e == 2) ? cd{neg_if(t.x, neg), neg_if(t.y, neg)} : cd{t.x, t.y};
+  }
+#pragma unroll
+  for (int j = 0; j < NS; j++) {
+    if (j & (1 << I)) continue;
+    const int j1 = j | 1 << I;
+    if (ctl && !((ok >> j) & 1)) continue;
+    cd a = {(double)v[j].re, (double)v[j].im}, b = {(double)v[j1].re, (double)v[j1].im};
+    shot_pair<FORM>(a, b, g);
+    if constexpr (sizeof(R) == 4) {  // the pruning reads the value before its rounding to FP32
+      a = pruned(a);
+      b = pruned(b);
     }
-    stc(st, i0, pruned(cadd_rn(cmul_rn(g0, a0), cmul_rn(g1, a1))));
-    stc(st, i1, pruned(cadd_rn(cmul_rn(g2, a0), cmul_rn(g3, a1))));
+    v[j] = cpx<R>{(R)a.re, (R)a.im};
+    v[j1] = cpx<R>{(R)b.re, (R)b.im};
+  }
+  if constexpr (sizeof(R) == 8) {  // one screen over the thread's amplitudes
+    // (an exact zero, of which a state has many in its first gates, need not be
+    // flushed: less one, its word is the largest)
+    uint32_t tiny = 0xffffffffu;
+#pragma unroll
+    for (int j = 0; j < NS; j++)
+      tiny = min(tiny, __float_as_uint(fmaxf(hiabs(v[j].re), hiabs(v[j].im))) - 1u);
+    if (tiny < __float_as_uint(tiny_screen(0.0)) - 1u) {
+#pragma unroll
+      for (int j = 0; j < NS; j++) {
+        const cd y = pruned(cd{v[j].re, v[j].im});
+        v[j] = cpx<R>{(R)y.re, (R)y.im};
+      }
+    }
+  }
+}
+// X under controls: the two trade places, with the sign the frame puts between them.
+template <typename R, int K, int I>
+__device__ __forceinline__ void shot_x(cpx<R>* v, uint32_t neg, uint32_t ok) {
+#pragma unroll
+  for (int j = 0; j < (1 << K); j++) {
+    if ((j & (1 << I)) || !((ok >> j) & 1)) continue;
+    const cpx<R> a = v[j], b = v[j | 1 << I];
+    v[j] = cpx<R>{neg ? -b.re : b.re, neg ? -b.im : b.im};
+    v[j | 1 << I] = cpx<R>{neg ? -a.re : a.re, neg ? -a.im : a.im};
   }
 }
 
-// X on t where all bits of cm are set (applyCNOT / applyToffoli: copies)
-template <typename V, int NT>
-__device__ void t_permx(V* st, int n, int t, uint64_t cm) {
-  const uint64_t half = uint64_t(1) << (n - 1);
-  for (uint64_t j = threadIdx.x; j < half; j += NT) {
-    const uint64_t i0 = insert0(j, t), i1 = i0 | (uint64_t(1) << t);
-    if ((i0 & cm) != cm) continue;
-    const V v0 = st[i0];
-    st[i0] = st[i1];
-    st[i1] = v0;
+#define KET_BITS KET_BIT(0) KET_BIT(1) KET_BIT(2) KET_BIT(3)
+static_assert(kShotBits == 4, "one KET_BIT a register bit");
+
+template <typename R, int NT>
+__device__ __forceinline__ void shot_round(typename Vec2<R>::T* st, const SRound& Q, const SGate* gates,
+                                           const double2* mats, int n) {
+  constexpr int K = kShotBits;
+  const uint32_t nsub = 1u << (n - K);
+  for (uint32_t u = threadIdx.x; u < nsub; u += NT) {
+    uint32_t base = u;
+#pragma unroll
+    for (int i = 0; i < K; i++) base = insert0_32(base, Q.piv[i]);
+    const uint32_t sb = round_slot(base);
+    cpx<R> v[1 << K];
+    RoundSlots slots;
+    slots.read(Q.slot);
+#pragma unroll
+    for (int j = 0; j < (1 << K); j++) v[j] = ld_amp<R>(st + (sb ^ slots(j)));
+    // cosets of zeros stay zeros (most of a state in its first gates)
+    if (!__any_sync(__activemask(), !all_zero<R, 1 << K>(v))) continue;
+    for (int k = 0; k < Q.ngates; k++) {
+      // form, bit, controls | functional, mask | matrix | frame
+      const uint4 g = *reinterpret_cast<const uint4*>(gates + k);
+      const uint32_t p = base ^ (g.w & 0xffffu), neg = par((g.y >> 16) & (g.w >> 16));
+      const bool role = par(p & g.y & 0xffffu);
+      const double2* M = mats + 4 * g.z;
+      const int form = g.x & 0xff, bit = (g.x >> 8) & 0xff;
+      if (g.x >> 16) {
+        const uint32_t ok = shot_controls(gates[k], p);
+        switch (2 * bit + (form == SF_X)) {
+#define KET_BIT(I)                                                                    \
+  case 2 * I: shot_gate<R, K, I, SF_GEN>(v, M, role, neg, true, ok); break;           \
+  case 2 * I + 1: shot_x<R, K, I>(v, neg, ok); break;
+          KET_BITS
+#undef KET_BIT
+        }
+        continue;
+      }
+      switch (4 * bit + form) {
+#define KET_BIT(I)                                                                      \
+  case 4 * I + SF_GEN: shot_gate<R, K, I, SF_GEN>(v, M, role, neg, false, 0); break;    \
+  case 4 * I + SF_REAL: shot_gate<R, K, I, SF_REAL>(v, M, role, neg, false, 0); break;  \
+  case 4 * I + SF_RX: shot_gate<R, K, I, SF_RX>(v, M, role, neg, false, 0); break;      \
+  case 4 * I + SF_DIAG: shot_gate<R, K, I, SF_DIAG>(v, M, role, neg, false, 0); break;
+        KET_BITS
+#undef KET_BIT
+      }
+    }
+    slots.read(Q.slot);
+#pragma unroll
+    for (int j = 0; j < (1 << K); j++) st_amp<R>(st + (sb ^ slots(j)), v[j]);
   }
 }
 
-// swap bits a, b where all bits of cm are set (applySWAP / applyCSwap)
-template <typename V, int NT>
-__device__ void t_swap(V* st, int n, int a, int b, uint64_t cm) {
-  const int lo = a < b ? a : b, hi = a < b ? b : a;
-  const uint64_t quarter = uint64_t(1) << (n - 2);
-  for (uint64_t j = threadIdx.x; j < quarter; j += NT) {
-    const uint64_t base = insert0(insert0(j, lo), hi);
-    if ((base & cm) != cm) continue;
-    const uint64_t x = base | (uint64_t(1) << a), y = base | (uint64_t(1) << b);
-    const V v = st[x];
-    st[x] = st[y];
-    st[y] = v;
-  }
-}
-
-// 4x4 on (a, b), a = MSB: [ctx, ctx|b, ctx|a, ctx|a|b] (applyTwo, statevector.ts:110-132)
-template <typename V, int NT>
-__device__ void t_apply4(V* st, int n, int a, int b, const double* M, int64_t off) {
-  const int lo = a < b ? a : b, hi = a < b ? b : a;
-  const uint64_t quarter = uint64_t(1) << (n - 2);
-  for (uint64_t j = threadIdx.x; j < quarter; j += NT) {
-    const uint64_t base = insert0(insert0(j, lo), hi);
-    const uint64_t idx[4] = {base, base | (uint64_t(1) << b), base | (uint64_t(1) << a),
-                             base | (uint64_t(1) << a) | (uint64_t(1) << b)};
-    cd x[4];
-    for (int c = 0; c < 4; c++) x[c] = ldc(st, idx[c]);
-    for (int r = 0; r < 4; r++) {
+// A dense 2^K x 2^K (two-qubit gates, csrswap, unitaries of up to 4 qubits):
+// applyTwo and applyUnitary add a row's products in ascending column order.
+template <typename R, int NT, int K>
+__device__ void shot_dense(typename Vec2<R>::T* st, const SRound& Q, const SGate& g, const double2* mats,
+                           int n) {
+  constexpr int D = 1 << K;
+  const uint32_t f = g.frame;
+  const uint32_t nsub = 1u << (n - K);
+  const double2* M = mats + 4 * g.slot;
+  uint32_t z = 0;  // the frame's sign of mask i
+#pragma unroll
+  for (int i = 0; i < K; i++) z |= par(Q.m[i] & (f >> 16)) << i;
+  for (uint32_t u = threadIdx.x; u < nsub; u += NT) {
+    uint32_t base = u;
+#pragma unroll
+    for (int i = 0; i < K; i++) base = insert0_32(base, Q.piv[i]);
+    const uint32_t p = base ^ (f & 0xffffu), sb = round_slot(base);
+    if (g.nc && !(shot_controls(g, p) & 1)) continue;
+    uint32_t l0 = 0;  // local index of the coset's base
+#pragma unroll
+    for (int i = 0; i < K; i++) l0 |= par(p & Q.rd[i]) << i;
+    cd x[D];
+#pragma unroll
+    for (int c = 0; c < D; c++) {
+      const cd t = ldc(st, sb ^ Q.slot[c ^ l0]);
+      const uint32_t odd = par((c ^ l0) & z);
+      x[c] = cd{neg_if(t.re, odd), neg_if(t.im, odd)};
+    }
+    for (int r = 0; r < D; r++) {
       cd out = {0.0, 0.0};
-      for (int c = 0; c < 4; c++) out = cadd_rn(out, cmul_rn(mat_at(M, off, 4 * r + c), x[c]));
-      stc(st, idx[r], pruned(out));
+#pragma unroll
+      for (int c = 0; c < D; c++) {
+        const double2 m = M[r * D + c];
+        out = cadd_rn(out, cmul_rn(cd{m.x, m.y}, x[c]));
+      }
+      out = pruned(out);
+      const uint32_t odd = par((r ^ l0) & z);
+      stc(st, sb ^ Q.slot[r ^ l0], cd{neg_if(out.re, odd), neg_if(out.im, odd)});
     }
   }
 }
 
-// applyCsrSwap (statevector.ts:177-207): sqrt(iSWAP) on (a, b) where c is set;
-// every other entry passes through accumulate()
-template <typename V, int NT>
-__device__ void t_csrswap(V* st, int n, int c, int a, int b) {
-  const double sq2 = 1.0 / 1.4142135623730951;  // 1 / Math.sqrt(2)
-  const uint64_t quarter = uint64_t(1) << (n - 2);
-  const int lo = a < b ? a : b, hi = a < b ? b : a;
-  for (uint64_t j = threadIdx.x; j < quarter; j += NT) {
-    const uint64_t base = insert0(insert0(j, lo), hi);
-    const uint64_t i00 = base, i01 = base | (uint64_t(1) << b), i10 = base | (uint64_t(1) << a),
-                   i11 = i01 | (uint64_t(1) << a);
-    const cd a00 = ldc(st, i00), a01 = ldc(st, i01), a10 = ldc(st, i10), a11 = ldc(st, i11);
-    stc(st, i00, pruned(a00));
-    stc(st, i11, pruned(a11));
-    if (!((base >> c) & 1)) {
-      stc(st, i01, pruned(a01));
-      stc(st, i10, pruned(a10));
-      continue;
-    }
-    stc(st, i01, pruned(cadd_rn(cmul_rn({sq2, 0.0}, a01), cmul_rn({0.0, sq2}, a10))));
-    stc(st, i10, pruned(cadd_rn(cmul_rn({0.0, sq2}, a01), cmul_rn({sq2, 0.0}, a10))));
-  }
-}
-
-// applyUnitary (statevector.ts:240-270): 2^k x 2^k on qs (qs[0] = MSB), k <= 4
-template <typename V, int NT>
-__device__ void t_applyk(V* st, int n, const int* qs, int k, const double* M, int64_t off) {
-  int sorted[4];
-  for (int i = 0; i < k; i++) sorted[i] = qs[i];
-  for (int i = 1; i < k; i++)
-    for (int j = i; j > 0 && sorted[j - 1] > sorted[j]; j--) { const int w = sorted[j]; sorted[j] = sorted[j - 1]; sorted[j - 1] = w; }
-  const int dim = 1 << k;
-  const uint64_t groups = uint64_t(1) << (n - k);
-  for (uint64_t j = threadIdx.x; j < groups; j += NT) {
-    uint64_t base = j;
-    for (int i = 0; i < k; i++) base = insert0(base, sorted[i]);
-    cd x[16];
-    uint64_t idx[16];
-    for (int i = 0; i < dim; i++) {
-      uint64_t v = base;
-      for (int bit = 0; bit < k; bit++)
-        if ((i >> (k - 1 - bit)) & 1) v |= uint64_t(1) << qs[bit];
-      idx[i] = v;
-      x[i] = ldc(st, v);
-    }
-    for (int r = 0; r < dim; r++) {
-      cd out = {0.0, 0.0};
-      for (int c = 0; c < dim; c++) out = cadd_rn(out, cmul_rn(mat_at(M, off, r * dim + c), x[c]));
-      stc(st, idx[r], pruned(out));
-    }
-  }
-}
-
-// block sum of v in a fixed order (per-thread partial, then a tree); all
-// threads get the result
+// block sum of v in a fixed order (warps, then their sums in order)
 template <int NT>
-__device__ double t_block_sum(double v, double* red) {
-  red[threadIdx.x] = v;
+__device__ double shot_sum(double v, double* red) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v = __dadd_rn(v, __shfl_xor_sync(0xffffffffu, v, o));
   __syncthreads();
-  for (int w = NT / 2; w > 0; w >>= 1) {
-    if ((int)threadIdx.x < w) red[threadIdx.x] = __dadd_rn(red[threadIdx.x], red[threadIdx.x + w]);
-    __syncthreads();
-  }
-  const double r = red[0];
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
   __syncthreads();
-  return r;
+  double s = red[0];
+#pragma unroll
+  for (int w = 1; w < NT / 32; w++) s = __dadd_rn(s, red[w]);
+  return s;
 }
 
 // collapseQubit (circuit.ts:55-72) on the shared-memory state
-template <typename V, int NT>
-__device__ int t_collapse(V* st, int n, int q, double rand, double* red) {
-  if (q < 0 || q >= n) return 0;  // a qubit outside the state reads 0; the state is unchanged
-  const uint64_t half = uint64_t(1) << (n - 1);
+template <typename R, int NT>
+__device__ int shot_collapse(typename Vec2<R>::T* st, int n, uint32_t r, uint32_t beta, double rand, double* red) {
+  if (r == 0) return 0;  // a qubit outside the state reads 0; the state is unchanged
+  const uint32_t N = 1u << n;
   double acc = 0.0;
-  for (uint64_t j = threadIdx.x; j < half; j += NT)
-    acc = __dadd_rn(acc, norm2_rn(ldc(st, insert0(j, q) | (uint64_t(1) << q))));
-  const double p1 = t_block_sum<NT>(acc, red);
+  for (uint32_t i = threadIdx.x; i < N; i += NT)
+    if (par((i ^ beta) & r)) acc = __dadd_rn(acc, norm2_rn(ldc(st, round_slot(i))));
+  const double p1 = shot_sum<NT>(acc, red);
   const int outcome = rand < p1 ? 1 : 0;
   const double inv = 1 / sqrt(outcome == 1 ? p1 : 1 - p1);
-  const uint64_t N = uint64_t(1) << n;
-  for (uint64_t i = threadIdx.x; i < N; i += NT) {
-    cd a = ldc(st, i);
-    if ((int)((i >> q) & 1) == outcome) a = {__dmul_rn(a.re, inv), __dmul_rn(a.im, inv)};
+  for (uint32_t i = threadIdx.x; i < N; i += NT) {
+    cd a = ldc(st, round_slot(i));
+    if ((int)par((i ^ beta) & r) == outcome) a = {__dmul_rn(a.re, inv), __dmul_rn(a.im, inv)};
     else a = {0.0, 0.0};
-    stc(st, i, a);
+    stc(st, round_slot(i), a);
   }
+  __syncthreads();
   return outcome;
 }
 
+__device__ __forceinline__ void copy_words(void* dst, const void* src, int bytes, int nt) {
+  for (int i = threadIdx.x; i < bytes / 4; i += nt)
+    static_cast<uint32_t*>(dst)[i] = __ldg(static_cast<const uint32_t*>(src) + i);
+}
+
+// Bound: the FP64 pipe (unfused products and sums).  In place of one pass over
+// shared memory and one barrier per op, every gate as a general complex one:
+// 16384 shots of 12 qubits, 120 one-qubit gates and 55 CNOTs with noise, 22.6 ->
+// 8.4 ms (FP64 pipe 28% busy, issue slots 52%: register moves between the gate
+// forms take a fifth of the instructions).  Cosets of 16 at 16 warps an SM beat
+// cosets of 8 at 32 warps (9.9 ms), which pass over shared memory more often.
 template <typename R, int NT>
-__global__ void __launch_bounds__(NT) k_shots(const TOp* ops, int nops, const double* M, int64_t pauli0, int n,
-                                              uint64_t init, const uint32_t* start, uint64_t shots, ket_noise nz,
-                                              int ncbits, uint64_t* out_idx, uint8_t* out_bits) {
+__global__ void __launch_bounds__(NT, NT <= 64 ? 8 : 512 / NT) k_shots(const __grid_constant__ SArgs a) {
   typedef typename Vec2<R>::T V;
   extern __shared__ __align__(16) unsigned char smraw[];
   V* st = reinterpret_cast<V*>(smraw);
-  const uint64_t N = uint64_t(1) << n;
-  double* red = reinterpret_cast<double*>(smraw + sizeof(V) * N);
-  uint8_t* bits = reinterpret_cast<uint8_t*>(red + NT);
-  // sampling: per-thread chunk of C entries
-  const uint64_t C = N >= (uint64_t)NT ? N / NT : 1;
-  for (uint64_t shot = blockIdx.x; shot < shots; shot += gridDim.x) {
-    uint32_t s = start[shot];
-    for (uint64_t i = threadIdx.x; i < N; i += NT) {
-      V v;
-      v.x = (R)(i == init ? 1 : 0);
-      v.y = (R)0;
-      st[i] = v;
-    }
-    for (int b = threadIdx.x; b < ncbits; b += NT) bits[b] = 0;
+  double2* mats = reinterpret_cast<double2*>(smraw + a.off_mats);
+  SRound* rounds = reinterpret_cast<SRound*>(smraw + a.off_rounds);
+  SGate* gates = reinterpret_cast<SGate*>(smraw + a.off_gates);
+  SEvent* events = reinterpret_cast<SEvent*>(smraw + a.off_events);
+  double* red = reinterpret_cast<double*>(smraw + a.off_red);
+  uint8_t* bits = smraw + a.off_bits;
+  __shared__ int nev;
+  __shared__ uint32_t pick, last;
+  const int t = threadIdx.x, n = a.ne;
+  int loaded = -1;
+  for (uint64_t shot = blockIdx.x; shot < a.shots; shot += gridDim.x) {
+    const uint32_t s0 = a.start[shot];
+    uint32_t beta = 0, zeta = 0;
+    for (uint32_t i = t; i < 1u << n; i += NT) stc(st, round_slot(i), cd{i == a.init ? 1.0 : 0.0, 0.0});
+    for (int b = t; b < a.ncbits; b += NT) bits[b] = 0;
     __syncthreads();
-    for (int pc = 0; pc < nops; pc++) {
-      const TOp o = ops[pc];
-      switch (o.kind) {
-        case KET_OP_SINGLE: t_apply2<V, NT>(st, n, o.q[0], -1, M, o.mat); break;
-        case KET_OP_CONTROLLED: t_apply2<V, NT>(st, n, o.q[1], o.q[0], M, o.mat); break;
-        case KET_OP_CNOT: t_permx<V, NT>(st, n, o.q[1], uint64_t(1) << o.q[0]); break;
-        case KET_OP_TOFFOLI: t_permx<V, NT>(st, n, o.q[2], (uint64_t(1) << o.q[0]) | (uint64_t(1) << o.q[1])); break;
-        case KET_OP_SWAP: t_swap<V, NT>(st, n, o.q[0], o.q[1], 0); break;
-        case KET_OP_CSWAP: t_swap<V, NT>(st, n, o.q[1], o.q[2], uint64_t(1) << o.q[0]); break;
-        case KET_OP_TWO: t_apply4<V, NT>(st, n, o.q[0], o.q[1], M, o.mat); break;
-        case KET_OP_CSRSWAP: t_csrswap<V, NT>(st, n, o.q[0], o.q[1], o.q[2]); break;
-        case KET_OP_UNITARY: t_applyk<V, NT>(st, n, o.q, o.k, M, o.mat); break;
-        case T_NOISE1: {  // dep1 (circuit.ts:289-295)
-          const double r = tdraw(s);
-          if (r < nz.p1) {
-            const double u = r / nz.p1;
-            const int w = u < 1.0 / 3 ? 0 : u < 2.0 / 3 ? 1 : 2;
-            t_apply2<V, NT>(st, n, o.q[0], -1, M, pauli0 + 4 * w);
+    for (int pc = 0; pc < a.nsteps; pc++) {
+      const SStep& o = a.steps[pc];
+      const int kind = o.kind;
+      if (kind == ST_SEG) {
+        const SSeg S = a.segs[o.a];
+        if (loaded != o.a) {
+          copy_words(rounds, a.rounds + S.round0, S.nrounds * sizeof(SRound), NT);
+          copy_words(gates, a.gates + S.gate0, S.ngates * sizeof(SGate), NT);
+          copy_words(mats, a.mats + 4 * S.slot0, S.nslots * 64, NT);
+          loaded = o.a;
+        }
+        if (t == 0) nev = 0;
+        __syncthreads();
+        const int d0 = t * S.per, d1 = min(d0 + S.per, S.ndraws);
+        if (d0 < d1) {
+          uint32_t x = xs_jump(a.jump + 32 * (S.jump0 + t), s0);
+          for (int d = d0; d < d1; d++) {
+            const SNoise q = a.noise[S.noise0 + d];
+            const double r = xs_value(x), p = q.two ? a.nz.p2 : a.nz.p1;
+            x = xs_step(x);
+            if (!(r < p)) continue;
+            int pa, pb = 0;  // 0 none, 1 X, 2 Y, 3 Z
+            const double u = r / p;
+            if (q.two) {  // dep2 (circuit.ts:298-304), TWO_PAULI order
+              int k = (int)floor(u * 15);
+              if (k > 14) k = 14;
+              pa = (k + 1) >> 2;  // k + 1 = 4 * pa + pb over {I, X, Y, Z}^2 \ {II}
+              pb = (k + 1) & 3;
+            } else {  // dep1 (circuit.ts:289-295)
+              pa = u < 1.0 / 3 ? 1 : u < 2.0 / 3 ? 2 : 3;
+            }
+            const uint32_t be = (pa == 1 || pa == 2 ? q.ma : 0u) ^ (pb == 1 || pb == 2 ? q.mb : 0u);
+            const uint32_t ze = (pa >= 2 ? q.ra : 0u) ^ (pb >= 2 ? q.rb : 0u);
+            events[atomicAdd(&nev, 1)] = SEvent{d, be | ze << 16};  // (their order does not matter: XORs)
           }
-          break;
         }
-        case T_NOISE2: {  // dep2 (circuit.ts:298-304), TWO_PAULI order
-          const double r = tdraw(s);
-          if (r < nz.p2) {
-            int k = (int)floor(r / nz.p2 * 15);
-            if (k > 14) k = 14;
-            const int pa = (k + 1) >> 2, pb = (k + 1) & 3;  // k + 1 = 4 * pa + pb over {I, X, Y, Z}^2 \ {II}
-            if (pa) { t_apply2<V, NT>(st, n, o.q[0], -1, M, pauli0 + 4 * (pa - 1)); __syncthreads(); }
-            if (pb) t_apply2<V, NT>(st, n, o.q[1], -1, M, pauli0 + 4 * (pb - 1));
+        __syncthreads();
+        const int ne = nev;
+        for (int g = t; g < S.ngates; g += NT) {
+          uint32_t f = beta | zeta << 16;
+          for (int e = 0; e < ne; e++)
+            if (events[e].d < gates[g].dpos) f ^= events[e].bz;
+          gates[g].frame = f;
+        }
+        for (int e = 0; e < ne; e++) {
+          beta ^= events[e].bz & 0xffffu;
+          zeta ^= events[e].bz >> 16;
+        }
+        for (int q = 0; q < S.nrounds; q++) {
+          __syncthreads();
+          const SRound& Q = rounds[q];
+          const SGate* G = gates + Q.gate0;
+          if (Q.dense) {
+            switch (Q.k) {
+              case 2: shot_dense<R, NT, 2>(st, Q, *G, mats, n); break;
+              case 3: shot_dense<R, NT, 3>(st, Q, *G, mats, n); break;
+              default: shot_dense<R, NT, 4>(st, Q, *G, mats, n); break;
+            }
+          } else {
+            shot_round<R, NT>(st, Q, G, mats, n);
           }
-          break;
         }
-        case KET_OP_MEASURE: {
-          const double r = tdraw(s);
-          const int outcome = t_collapse<V, NT>(st, n, o.q[0], r, red);
-          const int reported = (nz.pmeas != 0 && tdraw(s) < nz.pmeas) ? 1 - outcome : outcome;
-          if (threadIdx.x == 0 && o.q[1] >= 0) bits[o.q[1]] = (uint8_t)reported;
-          break;
+      } else if (kind == ST_MEASURE || kind == ST_RESET) {
+        uint32_t x = xs_jump(a.jump + 32 * o.b, s0);
+        const int outcome = shot_collapse<R, NT>(st, n, o.r, beta, xs_value(x), red);
+        if (kind == ST_RESET) {
+          if (outcome == 1) beta ^= o.m;
+        } else {
+          x = xs_step(x);
+          const int reported = (a.nz.pmeas != 0 && xs_value(x) < a.nz.pmeas) ? 1 - outcome : outcome;
+          if (t == 0 && o.a >= 0) bits[o.a] = (uint8_t)reported;
         }
-        case KET_OP_RESET: {
-          const double r = tdraw(s);
-          if (t_collapse<V, NT>(st, n, o.q[0], r, red) == 1) {
-            __syncthreads();
-            t_apply2<V, NT>(st, n, o.q[0], -1, M, pauli0);
-          }
-          break;
-        }
-        case KET_OP_IF: {
-          int v = 0;
-          for (int kk = 0; kk < o.q[1]; kk++)
-            if (bits[o.q[0] + kk]) v |= 1 << kk;
-          if (v != o.q[2]) pc += o.q[3];
-          break;
-        }
-        default: break;  // barrier
+      } else {
+        int v = 0;
+        for (int kk = 0; kk < o.b; kk++)
+          if (bits[o.a + kk]) v |= 1 << kk;
+        if (v != o.c) pc += o.d;
       }
       __syncthreads();
     }
-    // sampleSV (circuit.ts:75-83): the first index whose running sum of |a|^2
-    // reaches the draw, else the last nonzero entry.  Chunk sums, then a walk
-    // inside one chunk.
-    const double r = tdraw(s);
-    const uint64_t c0 = (uint64_t)threadIdx.x * C;
-    double csum = 0.0;
-    long long clast = -1;
-    if (c0 < N)
-      for (uint64_t i = c0; i < c0 + C; i++) {
-        const double p = norm2_rn(ldc(st, i));
-        if (p > 0) { csum = __dadd_rn(csum, p); clast = (long long)i; }
+    // sampleSV (circuit.ts:75-83): the first logical index whose running sum of
+    // |a|^2 reaches the draw, else the last nonzero entry.  Thread t holds logical
+    // indices 16 t .. 16 t + 15; a scan gives it the sum before them.
+    uint32_t x = xs_jump(a.jump + 32 * a.last_row, s0);
+    const double r = xs_value(x);
+    if (t == 0) { pick = 0xffffffffu; last = 0; }
+    const uint32_t N = 1u << a.n;
+    constexpr int NW = NT / 32;
+    double carry = 0.0;  // sums of the tiles of 16 NT indices before this one
+    for (uint32_t l0 = 0; l0 < N; l0 += 16 * NT) {
+      const uint32_t l = l0 + 16 * t;
+      uint32_t phys = beta;
+      for (int b = 4; b < n; b++)
+        if ((l >> b) & 1) phys ^= a.acol[b];
+      double pv[16], csum = 0.0;
+#pragma unroll
+      for (int j = 0; j < 16; j++) {
+        const uint32_t pj = phys ^ (j & 1 ? a.acol[0] : 0) ^ (j & 2 ? a.acol[1] : 0) ^ (j & 4 ? a.acol[2] : 0) ^
+                            (j & 8 ? a.acol[3] : 0);
+        pv[j] = l + j < N ? norm2_rn(ldc(st, round_slot(pj))) : 0.0;
+        if (pv[j] > 0) csum = __dadd_rn(csum, pv[j]);
       }
-    red[threadIdx.x] = csum;
-    long long* lastk = reinterpret_cast<long long*>(bits + ((ncbits + 7) & ~7));
-    lastk[threadIdx.x] = clast;
-    __syncthreads();
-    __shared__ long long pick;
-    if (threadIdx.x == 0) {
-      double cum = 0.0;
-      long long last = -1, res = -1;
-      for (int t = 0; t < NT && (uint64_t)t * C < N; t++) {
-        if (lastk[t] >= 0) last = lastk[t];
-        if (res < 0 && lastk[t] >= 0 && __dadd_rn(cum, red[t]) >= r) {
-          double w = cum;
-          for (uint64_t i = (uint64_t)t * C; i < (uint64_t)(t + 1) * C; i++) {
-            const double p = norm2_rn(ldc(st, i));
-            if (p > 0) {
-              w = __dadd_rn(w, p);
-              if (r <= w) { res = (long long)i; break; }
-            }
-          }
-        }
-        cum = __dadd_rn(cum, red[t]);
+      double incl = csum;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const double y = __shfl_up_sync(0xffffffffu, incl, o);
+        if ((t & 31) >= o) incl = __dadd_rn(incl, y);
       }
-      pick = res >= 0 ? res : (last >= 0 ? last : 0);
+      __syncthreads();
+      if ((t & 31) == 31) red[t >> 5] = incl;
+      __syncthreads();
+      double before = carry;
+      for (int w = 0; w < (t >> 5); w++) before = __dadd_rn(before, red[w]);
+      for (int w = 0; w < NW; w++) carry = __dadd_rn(carry, red[w]);
+      // the sum before the thread's own entries (rounded, so kept from going below 0)
+      const double y = __shfl_up_sync(0xffffffffu, incl, 1);
+      if (t & 31) before = __dadd_rn(before, y);
+      double w = before;
+      uint32_t hit = 0xffffffffu, end = 0;
+#pragma unroll
+      for (int j = 15; j >= 0; j--)
+        if (pv[j] > 0 && end == 0) end = l + j + 1;
+      for (int j = 0; j < 16; j++) {
+        if (!(pv[j] > 0)) continue;
+        w = __dadd_rn(w, pv[j]);
+        if (hit == 0xffffffffu && r <= w) hit = l + j;
+      }
+      if (hit != 0xffffffffu) atomicMin(&pick, hit);
+      if (end) atomicMax(&last, end);
     }
     __syncthreads();
-    uint64_t idx = (uint64_t)pick;
-    if (nz.pmeas != 0)
-      for (int q = 0; q < n; q++)
-        if (tdraw(s) < nz.pmeas) idx ^= uint64_t(1) << q;
-    if (threadIdx.x == 0) out_idx[shot] = idx;
-    for (int b = threadIdx.x; b < ncbits; b += NT) out_bits[shot * (uint64_t)ncbits + b] = bits[b];
+    uint64_t idx = pick != 0xffffffffu ? pick : last ? last - 1 : 0;
+    if (a.nz.pmeas != 0)
+      for (int q = 0; q < a.n; q++) {
+        x = xs_step(x);
+        if (xs_value(x) < a.nz.pmeas) idx ^= uint64_t(1) << q;
+      }
+    if (t == 0) a.out_idx[shot] = idx;
+    for (int b = t; b < a.ncbits; b += NT) a.out_bits[shot * (uint64_t)a.ncbits + b] = bits[b];
     __syncthreads();
   }
 }
@@ -420,6 +651,11 @@ __global__ void __launch_bounds__(NT) k_shots(const TOp* ops, int nops, const do
 // xorshift32 as a linear map over GF(2)^32: col[k] = image of bit k
 struct Jump {
   uint32_t col[32];
+  static uint32_t step(uint32_t s) {
+    s ^= s << 13;
+    s ^= s >> 17;
+    return s ^ (s << 5);
+  }
   uint32_t apply(uint32_t v) const {
     uint32_t o = 0;
     for (int k = 0; k < 32; k++)
@@ -430,11 +666,7 @@ struct Jump {
 Jump jump_power(uint64_t d) {
   Jump step, acc;
   for (int k = 0; k < 32; k++) {
-    uint32_t s = 1u << k;
-    s ^= s << 13;
-    s ^= s >> 17;
-    s ^= s << 5;
-    step.col[k] = s;
+    step.col[k] = Jump::step(1u << k);
     acc.col[k] = 1u << k;
   }
   while (d) {
@@ -499,30 +731,246 @@ int64_t lower_shots(const ket_op* ops, size_t b, size_t e, const ket_noise& nz, 
   return draws;
 }
 
+// What a segment may hold of shared memory beside the state.
+struct SCaps {
+  int rounds, gates, slots, draws;
+};
+SCaps shot_caps(int nt) { return nt <= 64 ? SCaps{32, 64, 64, 128} : SCaps{64, 192, 192, 1024}; }
+
+// Threads of a CTA: 16 amplitudes each.
+int shot_threads(int ne) { return std::max(32, 1 << (ne - kShotBits)); }
+
+// The plan all shots of a call share.
+struct ShotPlan {
+  int ne = 0, nt = 0;
+  std::vector<SStep> steps;
+  std::vector<SSeg> segs;
+  std::vector<SRound> rounds;
+  std::vector<SGate> gates;
+  std::vector<double> mats;    // 8 doubles a slot
+  std::vector<SNoise> noise;
+  std::vector<int64_t> rows;   // draw index (0-based) of each jump row
+  SCaps used = {0, 0, 0, 0};
+  uint16_t acol[kRoundQubits];
+};
+
+class ShotPlanner {
+ public:
+  ShotPlanner(ShotPlan& p, int n, const std::vector<TOp>& ops, const std::vector<double>& mats)
+      : P(p), n_(n), ops_(ops), mats_(mats), caps_(shot_caps(p.nt)), rp_(p.ne) {}
+
+  void run(size_t b, size_t e, bool in_if) {
+    for (size_t i = b; i < e; i++) {
+      const TOp& o = ops_[i];
+      const int* q = o.q;
+      switch (o.kind) {
+        case KET_OP_SINGLE: gate(q[0], nullptr, 0, false, (int)i); break;
+        case KET_OP_CONTROLLED: gate(q[1], q, 1, false, (int)i); break;
+        case KET_OP_CNOT:
+          if (in_if) gate(q[1], q, 1, true, (int)i);
+          else rp_.cnot(q[0], q[1]);
+          break;
+        case KET_OP_TOFFOLI: gate(q[2], q, 2, true, (int)i); break;
+        case KET_OP_SWAP:
+          if (!in_if) { rp_.swap(q[0], q[1]); break; }
+          x1(q[0], q[1], (int)i);  // an if-body runs in some shots only: its swaps move data
+          x1(q[1], q[0], (int)i);
+          x1(q[0], q[1], (int)i);
+          break;
+        case KET_OP_CSWAP: {  // cswap(c, a, b) = cnot(b, a) toffoli(c, a, b) cnot(b, a)
+          const int cs[2] = {q[0], q[1]};
+          if (in_if) x1(q[2], q[1], (int)i); else rp_.cnot(q[2], q[1]);
+          gate(q[2], cs, 2, true, (int)i);
+          if (in_if) x1(q[2], q[1], (int)i); else rp_.cnot(q[2], q[1]);
+          break;
+        }
+        case KET_OP_TWO: dense(q, 2, nullptr, 0, (int)i); break;
+        case KET_OP_CSRSWAP: dense(q + 1, 2, q, 1, (int)i); break;
+        case KET_OP_UNITARY:
+          if (o.k == 1) gate(q[0], nullptr, 0, false, (int)i);
+          else dense(q, o.k, nullptr, 0, (int)i);
+          break;
+        case T_NOISE1: case T_NOISE2: {
+          if (ndraws_ == caps_.draws) end_segment();
+          SNoise z = {rp_.col[q[0]], rp_.row[q[0]], 0, 0, o.kind == T_NOISE2};
+          if (z.two) { z.mb = rp_.col[q[1]]; z.rb = rp_.row[q[1]]; }
+          noise_.push_back(z);
+          ndraws_++;
+          break;
+        }
+        case KET_OP_MEASURE: case KET_OP_RESET: {
+          end_segment();
+          SStep s = {};
+          s.kind = o.kind == KET_OP_MEASURE ? ST_MEASURE : ST_RESET;
+          s.a = o.kind == KET_OP_MEASURE ? q[1] : -1;
+          s.b = (int)P.rows.size();
+          P.rows.push_back(draw_);
+          draw_ += o.kind == KET_OP_MEASURE && flips_ ? 2 : 1;
+          if (q[0] >= 0 && q[0] < n_) { s.r = rp_.row[q[0]]; s.m = rp_.col[q[0]]; }
+          P.steps.push_back(s);
+          break;
+        }
+        case KET_OP_IF: {
+          end_segment();
+          const size_t at = P.steps.size();
+          P.steps.push_back(SStep{ST_IF, q[0], q[1], q[2], 0, 0, 0});
+          run(i + 1, i + 1 + q[3], true);
+          end_segment();
+          P.steps[at].d = (int)(P.steps.size() - at - 1);
+          i += q[3];
+          break;
+        }
+        default: break;  // barrier
+      }
+    }
+  }
+  void finish() {
+    end_segment();
+    std::copy(rp_.col, rp_.col + kRoundQubits, P.acol);
+    P.rows.push_back(draw_);
+  }
+  void set_flips(bool f) { flips_ = f; }
+
+ private:
+  ShotPlan& P;
+  int n_;
+  const std::vector<TOp>& ops_;
+  const std::vector<double>& mats_;
+  SCaps caps_;
+  RoundPlan rp_;
+  std::vector<SNoise> noise_;          // of the segment under construction
+  std::vector<int> dpos_;              // per gate of it, in program order
+  int ndraws_ = 0;
+  int64_t draw_ = 0;                   // first draw of the segment
+  bool flips_ = false;
+
+  void x1(int c, int t, int op) { gate(t, &c, 1, true, op); }
+  static int slots_of(int k) { return k <= 1 ? 1 : 1 << (2 * k - 2); }
+  void room(int slots) {
+    // (a round under construction may hold kRoundGates gates that are not in rp_.gates yet)
+    if ((int)dpos_.size() + 1 > caps_.gates - 1 || (int)rp_.rounds.size() + 2 > caps_.rounds || slots_ + slots > caps_.slots)
+      end_segment();
+    slots_ += slots;
+  }
+  int slots_ = 0;
+  void gate(int q, const int* cs, int nc, bool x, int op) {
+    room(x ? 0 : 1);
+    rp_.gate(q, cs, nc, x, op);
+    dpos_.push_back(ndraws_);
+  }
+  void dense(const int* qs, int k, const int* cs, int nc, int op) {
+    room(slots_of(k));
+    rp_.dense(qs, k, cs, nc, op);
+    dpos_.push_back(ndraws_);
+  }
+  void end_segment() {
+    rp_.close();
+    if (rp_.rounds.empty() && ndraws_ == 0) return;
+    SSeg S = {};
+    S.round0 = (int)P.rounds.size();
+    S.nrounds = (int)rp_.rounds.size();
+    S.gate0 = (int)P.gates.size();
+    S.ngates = (int)rp_.gates.size();
+    S.slot0 = (int)(P.mats.size() / 8);
+    int slot = 0;
+    for (const Round& r : rp_.rounds) {
+      SRound Q = {};
+      std::copy(r.slot, r.slot + 16, Q.slot);
+      std::copy(r.m, r.m + 4, Q.m);
+      std::copy(r.rd, r.rd + 4, Q.rd);
+      std::copy(r.piv, r.piv + 4, Q.piv);
+      Q.k = r.k;
+      Q.dense = r.dense;
+      Q.ngates = (uint16_t)r.ngates;
+      Q.gate0 = r.gate0;
+      P.rounds.push_back(Q);
+      for (int g = r.gate0; g < r.gate0 + r.ngates; g++) {
+        const RoundGate& o = rp_.gates[g];
+        SGate G = {};
+        G.bit = o.bit;
+        G.nc = o.nc;
+        G.r = o.r;
+        G.m = o.m;
+        std::copy(o.cj, o.cj + 2, G.cj);
+        std::copy(o.rc, o.rc + 2, G.rc);
+        G.slot = slot;
+        G.dpos = dpos_[g];
+        if (o.x) {
+          G.form = SF_X;
+        } else {
+          const int ns = r.dense ? slots_of(r.k) : 1;
+          std::vector<double> m(8 * (size_t)ns, 0.0);
+          matrix(ops_[o.op], r.dense ? r.k : 1, m.data());
+          G.form = r.dense ? SF_GEN : form_of(m.data());
+          P.mats.insert(P.mats.end(), m.begin(), m.end());
+          slot += ns;
+        }
+        P.gates.push_back(G);
+      }
+    }
+    S.nslots = slot;
+    S.noise0 = (int)P.noise.size();
+    S.ndraws = ndraws_;
+    P.noise.insert(P.noise.end(), noise_.begin(), noise_.end());
+    S.per = (ndraws_ + P.nt - 1) / P.nt;
+    S.jump0 = (int)P.rows.size();
+    for (int d = 0; d < ndraws_; d += std::max(S.per, 1)) P.rows.push_back(draw_ + d);
+    draw_ += ndraws_;
+    P.used.rounds = std::max(P.used.rounds, S.nrounds);
+    P.used.gates = std::max(P.used.gates, S.ngates);
+    P.used.slots = std::max(P.used.slots, S.nslots);
+    P.used.draws = std::max(P.used.draws, S.ndraws);
+    SStep st = {};
+    st.kind = ST_SEG;
+    st.a = (int)P.segs.size();
+    P.segs.push_back(S);
+    P.steps.push_back(st);
+    rp_.rounds.clear();
+    rp_.gates.clear();
+    noise_.clear();
+    dpos_.clear();
+    ndraws_ = slots_ = 0;
+  }
+  void matrix(const TOp& o, int k, double* m) const {
+    if (o.kind == KET_OP_CSRSWAP) {  // applyCsrSwap (statevector.ts:177-207): sqrt(iSWAP)
+      const double sq2 = 1.0 / 1.4142135623730951;  // 1 / Math.sqrt(2)
+      m[0] = m[30] = 1.0;
+      m[2 * 5] = m[2 * 10] = sq2;
+      m[2 * 6 + 1] = m[2 * 9 + 1] = sq2;
+      return;
+    }
+    std::copy(mats_.begin() + 2 * (size_t)o.mat, mats_.begin() + 2 * ((size_t)o.mat + (size_t(1) << (2 * k))), m);
+  }
+  static uint8_t form_of(const double* m) {
+    if (m[2] == 0 && m[3] == 0 && m[4] == 0 && m[5] == 0) return SF_DIAG;
+    if (m[1] == 0 && m[3] == 0 && m[5] == 0 && m[7] == 0) return SF_REAL;
+    if (m[1] == 0 && m[2] == 0 && m[4] == 0 && m[7] == 0) return SF_RX;
+    return SF_GEN;
+  }
+};
+
 template <typename R, int NT>
-cudaError_t launch_shots_t(const TOp* dops, int nops, const double* dmats, int64_t pauli0, int n, uint64_t init,
-                           const uint32_t* dstart, uint64_t shots, const ket_noise& nz, int ncbits, uint64_t* dout,
-                           uint8_t* dbits, cudaStream_t s) {
-  const size_t smem = (sizeof(typename Vec2<R>::T) << n) + 8 * NT + ((ncbits + 7) & ~7) + 8 * NT;
+cudaError_t launch_shots_t(const SArgs& a, size_t smem, cudaStream_t s) {
   cudaError_t e = cudaFuncSetAttribute(k_shots<R, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   int per_sm = 0;
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_shots<R, NT>, NT, smem);
   if (e != cudaSuccess) return e;
   if (per_sm < 1) return cudaErrorInvalidConfiguration;
-  const uint64_t grid = std::min<uint64_t>(shots, (uint64_t)per_sm * num_sms());
-  k_shots<R, NT><<<(unsigned)grid, NT, smem, s>>>(dops, nops, dmats, pauli0, n, init, dstart, shots, nz, ncbits,
-                                                  dout, dbits);
+  const uint64_t grid = std::min<uint64_t>(a.shots, (uint64_t)per_sm * num_sms());
+  k_shots<R, NT><<<(unsigned)grid, NT, smem, s>>>(a);
   return cudaGetLastError();
 }
 
 template <typename R>
-cudaError_t launch_shots(const TOp* dops, int nops, const double* dmats, int64_t pauli0, int n, uint64_t init,
-                         const uint32_t* dstart, uint64_t shots, const ket_noise& nz, int ncbits, uint64_t* dout,
-                         uint8_t* dbits, cudaStream_t s) {
-  if (n <= 6) return launch_shots_t<R, 32>(dops, nops, dmats, pauli0, n, init, dstart, shots, nz, ncbits, dout, dbits, s);
-  if (n <= 9) return launch_shots_t<R, 128>(dops, nops, dmats, pauli0, n, init, dstart, shots, nz, ncbits, dout, dbits, s);
-  return launch_shots_t<R, 256>(dops, nops, dmats, pauli0, n, init, dstart, shots, nz, ncbits, dout, dbits, s);
+cudaError_t launch_shots(const SArgs& a, int nt, size_t smem, cudaStream_t s) {
+  switch (nt) {
+    case 32: return launch_shots_t<R, 32>(a, smem, s);
+    case 64: return launch_shots_t<R, 64>(a, smem, s);
+    case 128: return launch_shots_t<R, 128>(a, smem, s);
+    case 256: return launch_shots_t<R, 256>(a, smem, s);
+    default: return launch_shots_t<R, 512>(a, smem, s);
+  }
 }
 
 // Largest state the batched kernel holds in shared memory.
@@ -535,44 +983,106 @@ size_t align256(size_t b) { return (b + 255) & ~size_t(255); }
 // All shots in one launch: shot i starts from the stream state after i * D
 // draws (D = draws per shot), found by the GF(2) jump of xorshift32.
 int run_batched(ket_state* st, const std::vector<TOp>& tops, int64_t draws, const std::vector<double>& mats,
-                int64_t pauli0, uint64_t init, const ket_noise& nz, size_t shots, uint32_t* prng, int ncbits,
-                uint64_t* out_idx, uint8_t* out_bits) {
+                uint64_t init, const ket_noise& nz, size_t shots, uint32_t* prng, int ncbits, uint64_t* out_idx,
+                uint8_t* out_bits) {
   ket_ctx* c = st->ctx;
+  ShotPlan P;
+  P.ne = std::max(st->n, kShotMinQubits);
+  P.nt = shot_threads(P.ne);
+  ShotPlanner planner(P, st->n, tops, mats);
+  planner.set_flips(nz.pmeas != 0);
+  planner.run(0, tops.size(), false);
+  planner.finish();
+  // jump rows: the step's power that leads from a shot's start to the row's draw
+  std::vector<uint32_t> jump(32 * P.rows.size());
+  {
+    Jump J = jump_power(0);
+    int64_t at = 0;
+    std::vector<size_t> by(P.rows.size());
+    for (size_t i = 0; i < by.size(); i++) by[i] = i;
+    std::stable_sort(by.begin(), by.end(), [&](size_t x, size_t y) { return P.rows[x] < P.rows[y]; });
+    for (size_t i : by) {
+      for (; at < P.rows[i] + 1; at++)
+        for (int k = 0; k < 32; k++) J.col[k] = Jump::step(J.col[k]);
+      std::copy(J.col, J.col + 32, jump.begin() + 32 * i);
+    }
+  }
+  // the shots' start states, a byte of the state at a time
   const Jump J = jump_power((uint64_t)draws);
+  std::vector<uint32_t> byte_img(4 * 256);
+  for (int b = 0; b < 4; b++)
+    for (uint32_t v = 0; v < 256; v++) byte_img[256 * b + v] = J.apply(v << (8 * b));
   std::vector<uint32_t> start(shots);
   uint32_t s = *prng ? *prng : 1u;
   for (size_t i = 0; i < shots; i++) {
     start[i] = s;
-    s = J.apply(s);
+    s = byte_img[s & 255] ^ byte_img[256 + ((s >> 8) & 255)] ^ byte_img[512 + ((s >> 16) & 255)] ^ byte_img[768 + (s >> 24)];
   }
-  const size_t b_ops = align256(sizeof(TOp) * std::max<size_t>(1, tops.size()));
-  const size_t b_mat = align256(8 * mats.size());
-  const size_t b_start = align256(4 * shots), b_idx = align256(8 * shots), b_bits = align256(shots * ncbits + 1);
+  size_t total = 0;
+  struct Part { const void* src; size_t bytes, at; };
+  std::vector<Part> parts;
+  auto place = [&](size_t bytes) {
+    const size_t at = total;
+    total += align256(std::max<size_t>(bytes, 1));
+    return at;
+  };
+  auto part = [&](const auto& v) {
+    parts.push_back(Part{v.data(), v.size() * sizeof(v[0]), place(v.size() * sizeof(v[0]))});
+    return parts.back().at;
+  };
+  const size_t o_steps = part(P.steps), o_segs = part(P.segs), o_rounds = part(P.rounds), o_gates = part(P.gates),
+               o_mats = part(P.mats), o_noise = part(P.noise), o_jump = part(jump), o_start = part(start);
+  const size_t image = total, o_idx = place(8 * shots), o_bits = place(shots * ncbits);
   void* scr;
-  TRY(ctx_scratch(c, b_ops + b_mat + b_start + b_idx + b_bits, &scr));
+  TRY(ctx_scratch(c, total, &scr));
   char* base = (char*)scr;
-  TOp* dops = (TOp*)base;
-  double* dmats = (double*)(base + b_ops);
-  uint32_t* dstart = (uint32_t*)(base + b_ops + b_mat);
-  uint64_t* didx = (uint64_t*)(base + b_ops + b_mat + b_start);
-  uint8_t* dbits = (uint8_t*)(base + b_ops + b_mat + b_start + b_idx);
-  cudaError_t e = cudaSuccess;
-  if (!tops.empty()) e = cudaMemcpyAsync(dops, tops.data(), sizeof(TOp) * tops.size(), cudaMemcpyHostToDevice, c->stream);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(dmats, mats.data(), 8 * mats.size(), cudaMemcpyHostToDevice, c->stream);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(dstart, start.data(), 4 * shots, cudaMemcpyHostToDevice, c->stream);
+  std::vector<unsigned char> img(image, 0);
+  for (const Part& p : parts)
+    if (p.bytes) memcpy(img.data() + p.at, p.src, p.bytes);
+  cudaError_t e = cudaMemcpyAsync(base, img.data(), image, cudaMemcpyHostToDevice, c->stream);
   if (e != cudaSuccess) return cuda_fail(e, "cudaMemcpyAsync(trajectory inputs)");
-  c->h2d_bytes += sizeof(TOp) * tops.size() + 8 * mats.size() + 4 * shots;
+  c->h2d_bytes += image;
+  SArgs a;
+  memset(&a, 0, sizeof(a));
+  a.steps = (const SStep*)(base + o_steps);
+  a.segs = (const SSeg*)(base + o_segs);
+  a.rounds = (const SRound*)(base + o_rounds);
+  a.gates = (const SGate*)(base + o_gates);
+  a.mats = (const double2*)(base + o_mats);
+  a.noise = (const SNoise*)(base + o_noise);
+  a.jump = (const uint32_t*)(base + o_jump);
+  a.start = (const uint32_t*)(base + o_start);
+  a.out_idx = (uint64_t*)(base + o_idx);
+  a.out_bits = (uint8_t*)(base + o_bits);
+  a.shots = shots;
+  a.init = init;
+  a.nz = nz;
+  a.nsteps = (int)P.steps.size();
+  a.n = st->n;
+  a.ne = P.ne;
+  a.ncbits = ncbits;
+  a.last_row = (int)P.rows.size() - 1;
+  std::copy(P.acol, P.acol + kRoundQubits, a.acol);
+  size_t smem = (st->precision == KET_C64 ? sizeof(float2) : sizeof(double2)) << P.ne;
+  auto area = [&](size_t bytes) {
+    const size_t at = smem;
+    smem += (bytes + 15) & ~size_t(15);
+    return (int)at;
+  };
+  a.off_mats = area(64 * (size_t)P.used.slots);
+  a.off_rounds = area(sizeof(SRound) * P.used.rounds);
+  a.off_gates = area(sizeof(SGate) * P.used.gates);
+  a.off_events = area(sizeof(SEvent) * P.used.draws);
+  a.off_red = area(8 * 32);
+  a.off_bits = area(ncbits);
   prof_begin(c);
-  e = st->precision == KET_C64
-          ? launch_shots<float>(dops, (int)tops.size(), dmats, pauli0, st->n, init, dstart, shots, nz, ncbits, didx,
-                                dbits, c->stream)
-          : launch_shots<double>(dops, (int)tops.size(), dmats, pauli0, st->n, init, dstart, shots, nz, ncbits, didx,
-                                 dbits, c->stream);
+  e = st->precision == KET_C64 ? launch_shots<float>(a, P.nt, smem, c->stream)
+                               : launch_shots<double>(a, P.nt, smem, c->stream);
   prof_end(c, PK_BATCH);
   if (e != cudaSuccess) return cuda_fail(e, "trajectory launch");
-  e = cudaMemcpyAsync(out_idx, didx, 8 * shots, cudaMemcpyDeviceToHost, c->stream);
+  e = cudaMemcpyAsync(out_idx, a.out_idx, 8 * shots, cudaMemcpyDeviceToHost, c->stream);
   if (e == cudaSuccess && ncbits)
-    e = cudaMemcpyAsync(out_bits, dbits, shots * (size_t)ncbits, cudaMemcpyDeviceToHost, c->stream);
+    e = cudaMemcpyAsync(out_bits, a.out_bits, shots * (size_t)ncbits, cudaMemcpyDeviceToHost, c->stream);
   if (e != cudaSuccess) return cuda_fail(e, "cudaMemcpyAsync(trajectory outputs)");
   c->d2h_bytes += 8 * shots + shots * (size_t)ncbits;
   TRY(ctx_wait(c));
@@ -797,13 +1307,8 @@ int ket_run_shots(ket_state* st, const ket_op* ops, size_t nops, const double* m
     bool fits = draws > 0;
     for (const TOp& t : tops) fits = fits && t.mat >= -1;
     if (fits) {
-      std::vector<double> tm(mats, mats + 2 * nmat);
-      const int64_t pauli0 = (int64_t)nmat;
-      static const double P[24] = {0, 0, 1, 0, 1, 0, 0, 0,    // X (gates.ts:15-17)
-                                   0, 0, 0, -1, 0, 1, 0, 0,   // Y
-                                   1, 0, 0, 0, 0, 0, -1, 0};  // Z
-      tm.insert(tm.end(), P, P + 24);
-      return run_batched(st, tops, draws, tm, pauli0, init, nz0, shots, prng_state, ncbits, out_idx, out_bits);
+      const std::vector<double> tm(mats, mats + 2 * nmat);
+      return run_batched(st, tops, draws, tm, init, nz0, shots, prng_state, ncbits, out_idx, out_bits);
     }
   }
   if (g_pershot_path == 2) return fail(KET_ERR_UNSUPPORTED, "trajectories not batchable (state size or draws inside if)");
