@@ -8,18 +8,28 @@
 // vqe(., maxCutHamiltonian(n, E)) (algorithms.ts:231-241, 301-336).
 //
 // Work items are pulled from a global queue by a persistent grid:
-//   * an instance of n <= TILE qubits is one item, simulated entirely in
-//     shared memory (all layers and the <C> reduction);
-//   * a wider instance is split into 2p passes of tiles of 2^TILE amplitudes
-//     (pass A of a layer: the cost phase, which is diagonal, plus Rx on qubits
-//     0..TILE-1; pass B: Rx on the remaining qubits).  A tile of pass k waits
-//     (bounded spin, error flag on timeout) until every tile of pass k-1 of
-//     its instance has been written back; the queue hands items out in an
-//     order where everything a tile waits on was handed out earlier, so the
-//     fully resident grid cannot deadlock.
-// The cost phase exp(-i gamma (|E| - 2 cut(x))) takes cut(x) from the edge
-// masks and a per-layer table of |E|+1 phases.  <C> partials are written per
-// (instance, tile) and reduced in a fixed order.
+//   * an instance of n <= TILE qubits is one item, simulated on the chip (all
+//     layers and the <C> reduction);
+//   * a wider instance is split into p + 1 passes of tiles of 2^TILE amplitudes.
+//     A tile holds either the low TILE qubits (even passes) or the qubits above
+//     them with the lowest qubits (odd passes).  Rx gates commute and the cost
+//     phase is diagonal, so pass k finishes layer k - 1 on its qubits, applies
+//     layer k's phase (every other qubit's Rx of layer k - 1 was done in pass k - 1)
+//     and starts layer k on its qubits: one read and write of the state a layer.
+//     A tile of pass k waits (bounded spin, error flag on timeout) until every tile
+//     of pass k-1 of its instance has been written back; the queue hands items
+//     out in an order where everything a tile waits on was handed out earlier, so
+//     the fully resident grid cannot deadlock.
+// A tile lives in registers, 2^K consecutive values of K of its bits a thread; Rx on
+// those bits needs no exchange, and the other bits come round through shared memory.
+// Rx(2 beta) = cos(beta) (1 - i tan(beta) X) is applied without its scalar, so an
+// amplitude takes two FMAs a gate; <C> is divided by the norm that is left.  Where
+// |tan(beta)| > 1, beta - pi/2 stands in for beta: the two differ by X on every
+// qubit, which commutes with the circuit and leaves every cut as it is.
+// The cost phase exp(-i gamma (|E| - 2 cut(x))) comes from a table of |E|+1 phases
+// a layer; a thread counts cut(x) once and follows its register bits from there.
+// Partials of <C> and of the norm are written per (instance, tile) and reduced
+// in a fixed order.
 #include <algorithm>
 #include <atomic>
 #include <chrono>
@@ -30,6 +40,7 @@
 #include "common.cuh"
 #include "ctx.h"
 #include "launch.h"
+#include "rounds.h"
 
 namespace ket {
 
@@ -40,314 +51,419 @@ namespace {
 
 struct QInst {
   int n, ne, p, ntiles;     // ntiles = 2^(n - tile) for split instances, 1 otherwise
+  int multi, pad;           // an edge occurs twice: cut(x) is counted for every amplitude
   int64_t state;            // offset (amplitudes) of the instance's state in the workspace (split only)
-  int64_t cut;              // offset (bytes) of the instance's cut values in the cut area (split only)
   int64_t edge_off;         // first edge in the edge array
   int64_t part_off;         // first <C> partial of the instance
+  int64_t tab_off;          // first phase of layer 0; a layer has ne + 1
 };
 
-struct QItem {
-  int inst;
-  int pass;   // -1: whole instance in shared memory; else pass index 0..2p-1
-  int tile;
+// The queue's items in order: run r holds items [first, the next run's first), the
+// tiles of one pass of an instance (or one whole instance).
+struct QRun {
+  int first, inst;
+  int pass;   // -1: whole instance on the chip; else pass index 0..p
+  int pad;
 };
 
 struct QArgs {
   const QInst* inst;
-  const QItem* items;
-  const uint64_t* emask;    // edge masks (1<<u | 1<<v)
+  const QRun* runs;         // and an end mark
+  const uint32_t* emask;    // edge masks (1<<u | 1<<v)
   const double* gamma;      // [inst * p + l]
   const double* beta;
+  double* tan;              // [inst * p + l]: tan(beta), beta taken to [-pi/4, pi/4]
+  double2* tab;             // phases by instance, layer and cut
   double2* work;            // split-instance states
-  uint8_t* cutw;            // split-instance cut(x) per amplitude, written by pass 0
-  double* part;             // <C> partials
+  double2* part;            // (<C>, norm) partials
   unsigned int* next;       // queue head
   unsigned int* done;       // per instance: tiles finished (pass-major)
   int* status;
   uint32_t spin_limit;      // polls before a wait gives up (status KET_ERR_TIMEOUT)
   int nitems;
-  int tile;                 // tile qubits
+  int drop;                 // test hook: an item that is left out (-1: none)
 };
 
-__device__ __forceinline__ int cut_of(uint64_t x, const uint64_t* em, int ne) {
+// Layer angles to phase tables and tangents, once a call: a CTA a (instance, layer).
+__global__ void k_qaoa_tables(QArgs a, int p) {
+  const int i = blockIdx.x / p, l = blockIdx.x % p;
+  const QInst I = a.inst[i];
+  const double gamma = a.gamma[blockIdx.x];
+  for (int c = threadIdx.x; c <= I.ne; c += blockDim.x) {
+    double s, co;
+    sincos(-gamma * (double)(I.ne - 2 * c), &s, &co);
+    a.tab[I.tab_off + (int64_t)l * (I.ne + 1) + c] = make_double2(co, s);
+  }
+  if (threadIdx.x == 0) {
+    double sb, cb;
+    sincos(a.beta[blockIdx.x], &sb, &cb);
+    a.tan[blockIdx.x] = fabs(cb) < fabs(sb) ? -cb / sb : sb / cb;
+  }
+}
+
+// What a CTA keeps of an instance in shared memory beside the tile.
+struct QShared {
+  double2 tab[KQ_MAX_EDGES + 1];
+  uint32_t em[KQ_MAX_EDGES];
+  uint32_t nbr[32];          // neighbours of each qubit
+  double red[32];
+  int item[2], failed;
+  QRun run;
+  QInst inst;
+};
+
+__device__ __forceinline__ int cut_of(uint32_t x, const uint32_t* em, int ne) {
   int c = 0;
-  for (int e = 0; e < ne; e++) c += __popcll(x & em[e]) & 1;
+  for (int e = 0; e < ne; e++) c += __popc(x & em[e]) & 1;
   return c;
 }
 
-template <int NT>
-__device__ void fill_phase(double2* tab, double gamma, int ne) {
-  for (int c = threadIdx.x; c <= ne; c += NT) {
-    double s, co;
-    sincos(-gamma * (double)(ne - 2 * c), &s, &co);
-    tab[c] = make_double2(co, s);
+// The layouts of a tile of T bits on NT threads: in layout g the thread's 2^K
+// amplitudes run over the tile bits reg(g, 0..K-1), and thread bit b is tile bit
+// thr(g, b).  Every tile bit is turned in one layout.  The last layout's lanes are
+// the lowest tile bits, so loads and stores are of runs.
+//
+// In general layout g holds the bits from K g (the last reaches back when K does not
+// divide T).  A tile of 12 bits on 256 threads orders them so that layouts 1 and 2
+// keep the same warp bits (9-11): that move stays inside a warp, and a pass meets
+// two CTA barriers instead of four (19.3 -> 18.7 ms on 512 instances).  The lowest
+// three lanes of each layout fall on three different bank bits.
+template <int NT, int T>
+struct QLay {
+  static constexpr int LT = NT == 128 ? 7 : NT == 256 ? 8 : 9;
+  static constexpr int K = T - LT, NS = 1 << K, NG = (T + K - 1) / K;
+  // CTAs an SM holds: by registers (4 an amplitude and as many again), by shared memory
+  static constexpr int CTAS = T == 11 ? (NT == 512 ? 2 : 4) : 2;
+  static constexpr bool WARP = T == 12 && NT == 256;
+  static constexpr int s(int g) { return K * g < T - K ? K * g : T - K; }
+  __host__ __device__ static constexpr int reg(int g, int b) {
+    if (!WARP) return s(g) + b;
+    return g == 0 ? (b == 0 ? 0 : 8 + b) : g == 1 ? 1 + b : 5 + b;
   }
-}
-
-// Shared-memory position of local amplitude i: the three low index bits are
-// XORed with bits 3-5.  For every group of rotated bits below, the eight
-// threads of a quarter warp then touch eight distinct 16-byte slots of a
-// 128-byte row (conflict-free), whichever bits the group holds.
-__device__ __forceinline__ uint32_t sw(uint32_t i) { return i ^ ((i >> 3) & 7u); }
-
-// Rx(2 beta) = [[c, -i s], [-i s, c]] on one pair, in registers.
-__device__ __forceinline__ void rx_pair(double2& a, double2& b, double cb, double sb) {
-  const double2 x = a, y = b;
-  a = make_double2(fma(cb, x.x, sb * y.y), fma(cb, x.y, -sb * y.x));
-  b = make_double2(fma(cb, y.x, sb * x.y), fma(cb, y.y, -sb * x.x));
-}
-
-// Rx(2 beta) on the K local bits g[0] < ... < g[K-1] of a shared-memory block
-// of 2^m amplitudes: each thread loads the 2^K amplitudes of a subcube into
-// registers, rotates every bit of the group there (lowest first), and stores
-// them back -- one shared-memory round trip per group instead of one per
-// bit.  Per amplitude the rotations run in the same order as bit by bit, so
-// results are the same.
-template <int NT, int K>
-__device__ void rx_group(double2* s, int m, uint32_t gp, double cb, double sb) {
-  int g[K];  // the group's bits, packed one per byte of gp (kept in registers)
-#pragma unroll
-  for (int q = 0; q < K; q++) g[q] = (int)((gp >> (8 * q)) & 0xffu);
-  const uint32_t nsub = 1u << (m - K);
-  for (uint32_t u = threadIdx.x; u < nsub; u += NT) {
-    uint32_t b = u;
-#pragma unroll
-    for (int q = 0; q < K; q++) b = insert0_32(b, g[q]);
-    double2 v[1 << K];
-#pragma unroll
-    for (int j = 0; j < (1 << K); j++) {
-      uint32_t o = b;
-#pragma unroll
-      for (int q = 0; q < K; q++)
-        if ((j >> q) & 1) o |= 1u << g[q];
-      v[j] = s[sw(o)];
-    }
-#pragma unroll
-    for (int q = 0; q < K; q++)
-#pragma unroll
-      for (int j = 0; j < (1 << K); j++)
-        if (!((j >> q) & 1)) rx_pair(v[j], v[j | (1 << q)], cb, sb);
-#pragma unroll
-    for (int j = 0; j < (1 << K); j++) {
-      uint32_t o = b;
-#pragma unroll
-      for (int q = 0; q < K; q++)
-        if ((j >> q) & 1) o |= 1u << g[q];
-      s[sw(o)] = v[j];
-    }
+  __host__ __device__ static constexpr int thr(int g, int b) {
+    if (!WARP) return b < s(g) ? b : b + K;
+    constexpr int one[8] = {0, 5, 7, 6, 8, 9, 10, 11};
+    return g == 0 ? 1 + b : g == 1 ? one[b] : b < 5 ? b : 4 + b;
   }
+  // whether layout g turns its register bit b (the last layout reaches back)
+  __host__ __device__ static constexpr bool turns(int g, int b) { return WARP || s(g) + b >= K * g; }
+  __host__ __device__ static constexpr bool in_warp(int g, int h) { return WARP && g + h == 3; }  // 1 <-> 2
+};
+
+// Tile qubits to global qubits: pass A tiles hold qubits 0..T-1; pass B tiles the
+// low lowB qubits and qubits T..n-1.
+struct QMap {
+  uint32_t base;   // global index of tile element 0
+  int lowB, T;     // lowB = T: pass A
+  __device__ __forceinline__ int qubit(int b) const { return b < lowB ? b : T + b - lowB; }
+  __device__ __forceinline__ uint32_t index(uint32_t i) const {  // of tile element i, but for base
+    return (i & ((1u << lowB) - 1)) | (i >> lowB) << T;
+  }
+};
+
+template <int NT, int T, int G>
+__device__ __forceinline__ uint32_t tile_index(int t) {  // of the thread's register index 0
+  uint32_t i = 0;
+#pragma unroll
+  for (int b = 0; b < QLay<NT, T>::LT; b++) i |= (((uint32_t)t >> b) & 1u) << QLay<NT, T>::thr(G, b);
+  return i;
+}
+template <int NT, int T, int G>
+__host__ __device__ constexpr uint32_t reg_index(int j) {  // tile bits of register index j
+  uint32_t i = 0;
+  for (int b = 0; b < QLay<NT, T>::K; b++)
+    if ((j >> b) & 1) i |= 1u << QLay<NT, T>::reg(G, b);
+  return i;
 }
 
-// Bits per group: three at 256 threads per CTA, so that the registers of three
-// resident CTAs (the shared-memory limit) hold a group's 8 amplitudes without
-// spills; four at 128 and 512 threads.
-template <int NT>
-constexpr int rx_group_bits() { return NT == 256 ? 3 : 4; }
-template <int NT>
-constexpr int batch_min_blocks() { return NT == 512 ? 1 : 3; }
-
-// Rx(2 beta) on every local bit set in `bits`, in ascending order, a group of
-// bits per shared-memory round trip.
-template <int NT>
-__device__ void rx_bits(double2* s, int m, uint32_t bits, double cb, double sb) {
-  constexpr int KM = rx_group_bits<NT>();
-  while (bits) {
-    uint32_t gp = 0;
-    int k = 0;
-    while (bits && k < KM) {
-      gp |= (uint32_t)(__ffs(bits) - 1) << (8 * k++);
-      bits &= bits - 1;
-    }
-    __syncthreads();
-    if constexpr (KM == 4) {
-      if (k == 4) { rx_group<NT, 4>(s, m, gp, cb, sb); continue; }
-    }
-    switch (k) {
-      case 3: rx_group<NT, 3>(s, m, gp, cb, sb); break;
-      case 2: rx_group<NT, 2>(s, m, gp, cb, sb); break;
-      default: rx_group<NT, 1>(s, m, gp, cb, sb); break;
+// Rx on the layout's own bits in `rotate` (tile bits).  The others turn by zero,
+// which leaves them as they are: with a branch a bit, half of the new values moved
+// back to their old registers, as many moves as FMAs (17.5 -> 16.0 ms on 512
+// instances).
+template <int NT, int T, int G>
+__device__ __forceinline__ void rotate_regs(double2* v, uint32_t rotate, double tan) {
+  constexpr int K = QLay<NT, T>::K, NS = QLay<NT, T>::NS;
+#pragma unroll
+  for (int b = 0; b < K; b++) {
+    if (!QLay<NT, T>::turns(G, b)) continue;
+    const double r = (rotate >> QLay<NT, T>::reg(G, b)) & 1 ? tan : 0.0;
+#pragma unroll
+    for (int j = 0; j < NS; j++) {
+      if (j & (1 << b)) continue;
+      // x' = x - i r y, y' = y - i r x
+      const double2 x = v[j], y = v[j | 1 << b];
+      v[j] = make_double2(fma(r, y.y, x.x), fma(-r, y.x, x.y));
+      v[j | 1 << b] = make_double2(fma(r, x.y, y.x), fma(-r, x.x, y.y));
     }
   }
 }
 
-// 16-byte asynchronous copy global -> shared (through L2 only: the data was
-// written by other CTAs of the same launch).
-__device__ __forceinline__ void cp_async16(void* sdst, const void* gsrc) {
-  const uint32_t d = (uint32_t)__cvta_generic_to_shared(sdst);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(gsrc) : "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() {
-  asm volatile("cp.async.commit_group;\n cp.async.wait_group 0;" ::: "memory");
+// cut(x) of the thread's 2^K amplitudes: counted at register index 0, then
+// followed bit by bit -- setting a bit whose qubit has d neighbours, c of them
+// set, changes the cut by d - 2 c.
+template <int NT, int T, int G>
+__device__ __forceinline__ void cuts(int (&c)[QLay<NT, T>::NS], const QMap& m, int t, const QShared& sh, const QInst& I) {
+  typedef QLay<NT, T> L;
+  constexpr int K = L::K, NS = L::NS;
+  const uint32_t x0 = m.base | m.index(tile_index<NT, T, G>(t));
+  c[0] = cut_of(x0, sh.em, I.ne);
+  if (I.multi) {
+#pragma unroll
+    for (int j = 1; j < NS; j++) {
+      uint32_t x = x0;
+#pragma unroll
+      for (int b = 0; b < K; b++)
+        if ((j >> b) & 1) x |= 1u << m.qubit(L::reg(G, b));
+      c[j] = cut_of(x, sh.em, I.ne);
+    }
+    return;
+  }
+#pragma unroll
+  for (int b = K - 1; b >= 0; b--) {
+    const uint32_t nb = sh.nbr[m.qubit(L::reg(G, b))];
+    uint32_t adj = 0;  // the register bits above b that neighbour it
+#pragma unroll
+    for (int u = b + 1; u < K; u++) adj |= ((nb >> m.qubit(L::reg(G, u))) & 1u) << u;
+    const int d = __popc(nb) - 2 * __popc(x0 & nb);
+#pragma unroll
+    for (int j = 0; j < NS; j++)
+      if (((j >> b) & 1) && !(j & ((1 << b) - 1))) c[j] = c[j ^ (1 << b)] + d - 2 * __popc(j & adj);
+  }
 }
 
-template <int NT>
-__global__ void __launch_bounds__(NT, batch_min_blocks<NT>()) k_batch_qaoa(QArgs a) {
+template <int NT, int T, int G>
+__device__ __forceinline__ void phase_regs(double2* v, const QMap& m, int t, const QShared& sh, const QInst& I) {
+  constexpr int NS = QLay<NT, T>::NS;
+  int c[NS];
+  cuts<NT, T, G>(c, m, t, sh, I);
+#pragma unroll
+  for (int j = 0; j < NS; j++) {
+    const double2 ph = sh.tab[c[j]], x = v[j];
+    v[j] = make_double2(fma(ph.x, x.x, -ph.y * x.y), fma(ph.x, x.y, ph.y * x.x));
+  }
+}
+
+// From layout G to layout H through shared memory.  A thread writes the slots it
+// read last, which no other thread reads until the barrier: one barrier a move (of
+// the warp where it moves only between its own threads).
+template <int NT, int T, int G, int H>
+__device__ __forceinline__ void relayout(double2* v, double2* s, int t) {
+  constexpr int NS = QLay<NT, T>::NS;
+  const uint32_t g0 = round_slot(tile_index<NT, T, G>(t)), h0 = round_slot(tile_index<NT, T, H>(t));
+#pragma unroll
+  for (int j = 0; j < NS; j++) s[g0 ^ round_slot(reg_index<NT, T, G>(j))] = v[j];
+  if constexpr (QLay<NT, T>::in_warp(G, H)) __syncwarp();
+  else __syncthreads();
+#pragma unroll
+  for (int j = 0; j < NS; j++) v[j] = s[h0 ^ round_slot(reg_index<NT, T, H>(j))];
+}
+
+// Rx on every bit in `rotate`, from layout G up to the top layout / down to layout 0.
+template <int NT, int T, int G>
+__device__ __forceinline__ void rx_up(double2* v, double2* s, int t, uint32_t rotate, double r) {
+  rotate_regs<NT, T, G>(v, rotate, r);
+  if constexpr (G + 1 < QLay<NT, T>::NG) {
+    relayout<NT, T, G, G + 1>(v, s, t);
+    rx_up<NT, T, G + 1>(v, s, t, rotate, r);
+  }
+}
+template <int NT, int T, int G>
+__device__ __forceinline__ void rx_down(double2* v, double2* s, int t, uint32_t rotate, double r) {
+  rotate_regs<NT, T, G>(v, rotate, r);
+  if constexpr (G > 0) {
+    relayout<NT, T, G, G - 1>(v, s, t);
+    rx_down<NT, T, G - 1>(v, s, t, rotate, r);
+  }
+}
+
+// Sums of |a|^2 cut(x) and |a|^2 over the tile, in layout G.
+template <int NT, int T, int G>
+__device__ __forceinline__ void tile_cut(const double2* v, const QMap& m, int t, QShared& sh, const QInst& I, double2* out) {
+  constexpr int NS = QLay<NT, T>::NS;
+  int c[NS];
+  cuts<NT, T, G>(c, m, t, sh, I);
+  double acc = 0.0, nrm = 0.0;
+#pragma unroll
+  for (int j = 0; j < NS; j++) {
+    const double q = v[j].x * v[j].x + v[j].y * v[j].y;
+    nrm += q;
+    acc = fma(q, (double)c[j], acc);
+  }
+  acc = block_sum<NT>(acc, sh.red);
+  __syncthreads();
+  nrm = block_sum<NT>(nrm, sh.red);
+  if (t == 0) *out = make_double2(acc, nrm);
+}
+
+// Bound: for wide instances the state's traffic (2 p reads and writes) and shared
+// memory's (a tile moves through it four times a pass), then the FP64 pipe (two
+// FMAs an amplitude and Rx).  512 instances of 10 to 22 qubits, p = 4:
+// 35.9 ms as 2 p passes of three-bit rounds, 15.3 now (FP64 pipe 28% busy, HBM a
+// fifth; two CTAs of 8 warps wait for barriers and loads).
+template <int NT, int T>
+__global__ void __launch_bounds__(NT, QLay<NT, T>::CTAS) k_batch_qaoa(QArgs a) {
+  typedef QLay<NT, T> L;
+  constexpr int NS = L::NS, TOP = L::NG - 1;
   extern __shared__ __align__(16) unsigned char smraw[];
   double2* s = reinterpret_cast<double2*>(smraw);
-  double2* tab = s + (1u << a.tile);                             // phase table (<= 65 entries)
-  uint64_t* em = reinterpret_cast<uint64_t*>(tab + KQ_MAX_EDGES + 1);
-  double* red = reinterpret_cast<double*>(em + KQ_MAX_EDGES);     // 32 doubles
-  uint8_t* cutb = reinterpret_cast<uint8_t*>(red + 32);           // cut(x) per amplitude (whole instance / tile)
-  static_assert((16 * (KQ_MAX_EDGES + 1) + 8 * KQ_MAX_EDGES + 8 * 32) % 16 == 0, "cut bytes 16-byte aligned");
-  __shared__ int item_sh;
-  const int T = a.tile;
-  for (;;) {
-    if (threadIdx.x == 0) item_sh = (int)atomicAdd(a.next, 1u);
-    __syncthreads();
-    const int it = item_sh;
-    __syncthreads();
+  QShared& sh = *reinterpret_cast<QShared*>(smraw + (sizeof(double2) << T));
+  const int t = threadIdx.x;
+  if (t == 0) sh.item[0] = (int)atomicAdd(a.next, 1u);
+  __syncthreads();
+  // A CTA's items ascend, so its place in the runs only moves on; what a run's tiles
+  // share is read once, and its wait is over once it has been.
+  int run = 0, have = -1, end = a.runs[1].first;
+  bool ready = false;
+  const QRun& w = sh.run;
+  const QInst& I = sh.inst;
+  for (int turn = 0;; turn ^= 1) {
+    const int it = sh.item[turn];
     if (it >= a.nitems) break;
-    const QItem w = a.items[it];
-    const QInst I = a.inst[w.inst];
-    for (int e = threadIdx.x; e < I.ne; e += NT) em[e] = a.emask[I.edge_off + e];
-    const int n = I.n;
-    if (w.pass < 0) {
-      // ---- whole instance in shared memory
-      const uint32_t N = 1u << n;
-      const double amp0 = 1.0 / sqrt((double)N);
-      __syncthreads();  // edge masks in
-      // cut(x) depends on x only: computed once, read by every layer and <C>
-      for (uint32_t i = threadIdx.x; i < N; i += NT) {
-        s[sw(i)] = make_double2(amp0, 0.0);
-        cutb[i] = (uint8_t)cut_of(i, em, I.ne);
+    if (t == 0) sh.item[turn ^ 1] = (int)atomicAdd(a.next, 1u);  // the next item, while this one runs
+    while (it >= end) end = a.runs[++run + 1].first;
+    const bool fresh = run != have;
+    if (fresh) {
+      have = run;
+      if (t == 0) {
+        sh.run = a.runs[run];
+        sh.inst = a.inst[sh.run.inst];
       }
-      for (int l = 0; l < I.p; l++) {
-        __syncthreads();
-        fill_phase<NT>(tab, a.gamma[w.inst * I.p + l], I.ne);
-        __syncthreads();
-        for (uint32_t i = threadIdx.x; i < N; i += NT) {
-          const double2 ph = tab[cutb[i]];
-          const double2 v = s[sw(i)];
-          s[sw(i)] = make_double2(fma(ph.x, v.x, -ph.y * v.y), fma(ph.x, v.y, ph.y * v.x));
-        }
-        double sb, cb;
-        sincos(a.beta[w.inst * I.p + l], &sb, &cb);
-        rx_bits<NT>(s, n, (1u << n) - 1u, cb, sb);
-      }
+      if (t < 32) sh.nbr[t] = 0;
       __syncthreads();
-      double acc = 0.0;
-      for (uint32_t i = threadIdx.x; i < N; i += NT) {
-        const double2 v = s[sw(i)];
-        acc += (v.x * v.x + v.y * v.y) * (double)cutb[i];
+      ready = w.pass <= 0;
+      for (int e = t; e < I.ne; e += NT) sh.em[e] = a.emask[I.edge_off + e];
+      __syncthreads();
+      for (int e = t; e < I.ne; e += NT) {
+        const uint32_t m = sh.em[e], u = __ffs(m) - 1, q = 31 - __clz(m);
+        atomicOr(&sh.nbr[u], 1u << q);
+        atomicOr(&sh.nbr[q], 1u << u);
       }
-      acc = block_sum<NT>(acc, red);
-      if (threadIdx.x == 0) a.part[I.part_off] = acc;
+    }
+    const int tile = it - w.first;
+    if (it == a.drop) {
+      __syncthreads();
+      continue;
+    }
+    const int n = I.n;
+    auto load_table = [&](int l) {
+      for (int c = t; c <= I.ne; c += NT) sh.tab[c] = a.tab[I.tab_off + (int64_t)l * (I.ne + 1) + c];
+    };
+    double2 v[NS];
+    if (w.pass < 0) {
+      // ---- whole instance on the chip (p = 0: <C> of the uniform state, whatever n)
+      const QMap m = {0u, T, T};
+      if (I.p == 0) {
+        if (t == 0) a.part[I.part_off] = make_double2(0.5 * I.ne, 1.0);
+        __syncthreads();
+        continue;
+      }
+      const double amp0 = 1.0 / sqrt((double)(1u << n));
+#pragma unroll
+      for (int j = 0; j < NS; j++)
+        v[j] = make_double2((tile_index<NT, T, 0>(t) | reg_index<NT, T, 0>(j)) < (1u << n) ? amp0 : 0.0, 0.0);
+      const uint32_t bits = (1u << n) - 1u;
+      for (int l = 0; l < I.p; l++) {
+        __syncthreads();  // the last layer's reads of the table
+        load_table(l);
+        __syncthreads();
+        const double r = a.tan[(int64_t)w.inst * I.p + l];
+        if (l & 1) {
+          phase_regs<NT, T, TOP>(v, m, t, sh, I);
+          rx_down<NT, T, TOP>(v, s, t, bits, r);
+        } else {
+          phase_regs<NT, T, 0>(v, m, t, sh, I);
+          rx_up<NT, T, 0>(v, s, t, bits, r);
+        }
+      }
+      if (I.p & 1) tile_cut<NT, T, TOP>(v, m, t, sh, I, a.part + I.part_off);
+      else tile_cut<NT, T, 0>(v, m, t, sh, I, a.part + I.part_off);
       __syncthreads();
       continue;
     }
     // ---- one tile of one pass of a wide instance
-    const int layer = w.pass >> 1;
-    const bool passA = (w.pass & 1) == 0;
-    // tile bits: pass A = qubits 0..T-1; pass B = low (T - (n - T)) qubits + qubits T..n-1
-    const int nhigh = n - T;               // qubits >= T
-    const int lowB = T - nhigh;            // low qubits kept in pass-B tiles
-    if (w.pass > 0) {
+    if (fresh && w.pass < I.p) load_table(w.pass);
+    if (!ready) {
       // wait until every tile of the previous pass has been written back; a
       // wait that ran out anywhere (status set) ends every later wait at once
       const unsigned int need = (unsigned int)w.pass * (unsigned int)I.ntiles;
-      if (threadIdx.x == 0) {
+      if (t == 0) {
         volatile unsigned int* d = a.done + w.inst;
         volatile int* st = a.status;
         uint32_t spins = 0;
         while (*d < need) {
           if (*st != 0) break;
           if (++spins > a.spin_limit) { atomicExch(a.status, (int)KET_ERR_TIMEOUT); break; }
-          __nanosleep(200);
+          __nanosleep(100);
         }
         __threadfence();
-        item_sh = *st;
+        sh.failed = *st;
       }
-      __syncthreads();
-      const bool failed = item_sh != 0;
-      __syncthreads();
-      if (failed) {
+      __syncthreads();  // (masks and table are in, too)
+      if (sh.failed != 0) {
         // the call reports the timeout; drain the queue without the tile's work
-        if (threadIdx.x == 0) atomicAdd(a.done + w.inst, 1u);
+        __syncthreads();
+        if (t == 0) atomicAdd(a.done + w.inst, 1u);
         continue;
       }
+      ready = true;
+    } else if (fresh) {
+      __syncthreads();
     }
-    double2* g = a.work + I.state;
-    // global index of tile element i
-    auto gidx = [&](uint32_t i) -> uint64_t {
-      if (passA) return ((uint64_t)w.tile << T) | i;
-      const uint64_t lo = i & ((1u << lowB) - 1);
-      const uint64_t hi = (uint64_t)(i >> lowB) << T;                 // qubits T..n-1
-      const uint64_t mid = (uint64_t)w.tile << lowB;                  // qubits lowB..T-1 from the tile id
-      return hi | mid | lo;
+    const bool passA = (w.pass & 1) == 0;
+    const int nhigh = n - T;                          // qubits >= T
+    const QMap m = passA ? QMap{(uint32_t)tile << T, T, T}
+                         : QMap{(uint32_t)tile << (T - nhigh), T - nhigh, T};
+    const uint32_t rotate = passA ? (1u << T) - 1u : ((1u << T) - 1u) & ~((1u << m.lowB) - 1u);
+    double2* g = a.work + I.state + m.base + m.index(tile_index<NT, T, TOP>(t));
+    auto off = [&](int j) {
+      uint32_t o = 0;
+#pragma unroll
+      for (int b = 0; b < L::K; b++)
+        if ((j >> b) & 1) o |= 1u << m.qubit(L::reg(TOP, b));
+      return o;
     };
-    const uint32_t TN = 1u << T;
     if (w.pass == 0) {
-      const double amp0 = 1.0 / sqrt((double)(uint64_t(1) << n));
-      for (uint32_t i = threadIdx.x; i < TN; i += NT) s[sw(i)] = make_double2(amp0, 0.0);
+      const double amp0 = 1.0 / sqrt((double)(1u << n));
+#pragma unroll
+      for (int j = 0; j < NS; j++) v[j] = make_double2(amp0, 0.0);
     } else {
-      // the whole tile in flight at once, straight into shared memory, and
-      // for pass A of later layers its cut values (kept by layer 0; pass-A
-      // tiles are contiguous)
-      for (uint32_t i = threadIdx.x; i < TN; i += NT) cp_async16(s + sw(i), g + gidx(i));
-      if (passA && layer > 0) {
-        const uint8_t* cw = a.cutw + I.cut + ((uint64_t)w.tile << T);
-        for (uint32_t i = 16 * threadIdx.x; i < TN; i += 16 * NT) cp_async16(cutb + i, cw + i);
-      }
-      cp_async_wait_all();
+#pragma unroll
+      for (int j = 0; j < NS; j++) v[j] = __ldcg(g + off(j));
+      rx_down<NT, T, TOP>(v, s, t, rotate, a.tan[(int64_t)w.inst * I.p + w.pass - 1]);
     }
-    double sb, cb;
-    sincos(a.beta[w.inst * I.p + layer], &sb, &cb);
-    if (passA) {
-      __syncthreads();
-      fill_phase<NT>(tab, a.gamma[w.inst * I.p + layer], I.ne);
-      __syncthreads();
-      // pass A tiles are contiguous: layer 0 computes cut(x) and keeps it,
-      // later layers copied it into shared memory with the tile
-      uint8_t* cw = a.cutw + I.cut;
-      for (uint32_t i = threadIdx.x; i < TN; i += NT) {
-        const uint64_t x = gidx(i);
-        int cx;
-        if (layer == 0) {
-          cx = cut_of(x, em, I.ne);
-          cw[x] = (uint8_t)cx;
-        } else {
-          cx = cutb[i];
-        }
-        const double2 ph = tab[cx];
-        const double2 v = s[sw(i)];
-        s[sw(i)] = make_double2(fma(ph.x, v.x, -ph.y * v.y), fma(ph.x, v.y, ph.y * v.x));
-      }
-      rx_bits<NT>(s, T, (1u << T) - 1u, cb, sb);
+    if (w.pass == I.p) {
+      tile_cut<NT, T, 0>(v, m, t, sh, I, a.part + I.part_off + tile);
     } else {
-      rx_bits<NT>(s, T, ((1u << T) - 1u) & ~((1u << lowB) - 1u), cb, sb);
+      phase_regs<NT, T, 0>(v, m, t, sh, I);
+      rx_up<NT, T, 0>(v, s, t, rotate, a.tan[(int64_t)w.inst * I.p + w.pass]);
+#pragma unroll
+      for (int j = 0; j < NS; j++) g[off(j)] = v[j];
     }
     __syncthreads();
-    const bool last = w.pass == 2 * I.p - 1;
-    if (last) {
-      double acc = 0.0;
-      for (uint32_t i = threadIdx.x; i < TN; i += NT) {
-        const double2 v = s[sw(i)];
-        acc += (v.x * v.x + v.y * v.y) * (double)cut_of(gidx(i), em, I.ne);
-      }
-      acc = block_sum<NT>(acc, red);
-      if (threadIdx.x == 0) a.part[I.part_off + w.tile] = acc;
-    } else {
-      for (uint32_t i = threadIdx.x; i < TN; i += NT) g[gidx(i)] = s[sw(i)];
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
+    if (t == 0) {
       __threadfence();
       atomicAdd(a.done + w.inst, 1u);
     }
-    __syncthreads();
   }
 }
 
-__global__ void k_qaoa_reduce(const QInst* inst, int ninst, const double* part, double* out) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
+// <C> of an instance: its partials added by a warp (strided runs, then a tree).
+__global__ void k_qaoa_reduce(const QInst* inst, int ninst, const double2* part, double* out) {
+  const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (i >= ninst) return;
   const QInst I = inst[i];
-  double acc = 0.0;
-  for (int t = 0; t < I.ntiles; t++) acc += part[I.part_off + t];
-  out[i] = acc;
+  double acc = 0.0, nrm = 0.0;
+  for (int t = lane; t < I.ntiles; t += 32) {
+    const double2 p = part[I.part_off + t];
+    acc += p.x;
+    nrm += p.y;
+  }
+  acc = warp_sum(acc);
+  nrm = warp_sum(nrm);
+  if (lane == 0) out[i] = acc / nrm;
 }
 
-// Test hook (ket_debug_batch_hook): drop one work item from the queue and
+// Test hook (ket_debug_batch_hook): leave one work item out and
 // shorten the waits, so that the tiles depending on it time out.
 int g_drop_item = -1;
 uint32_t g_spin_limit = 1u << 24;
@@ -357,28 +473,29 @@ uint32_t g_spin_limit = 1u << 24;
 
 using namespace ket;
 
-// Launch the persistent batch kernel with NT threads per CTA (every CTA
-// resident at once) and its fixed-order reduction, captured in a CUDA graph
-// when use_graph is set.
-template <int NT>
-static cudaError_t run_batch(ket_ctx* c, const QArgs& a, size_t smem, int ninst, double* dout, int use_graph) {
+// Launch the tables, the persistent batch kernel (NT threads per CTA, every CTA
+// resident at once) and its fixed-order reduction, captured in a CUDA graph when
+// use_graph is set.
+template <int NT, int T>
+static cudaError_t run_batch(ket_ctx* c, const QArgs& a, int p, int ninst, double* dout, int use_graph) {
+  const size_t smem = (sizeof(double2) << T) + sizeof(QShared);
   // the shared-memory limit is a per-device attribute of the kernel
   static std::atomic<uint64_t> attr_set{0};
   const uint64_t bit = uint64_t(1) << (c->device & 63);
   if (!(attr_set.load() & bit)) {
-    const size_t smax = (17u << 12) + 16 * (KQ_MAX_EDGES + 1) + 8 * KQ_MAX_EDGES + 8 * 32;
-    cudaError_t e = cudaFuncSetAttribute(k_batch_qaoa<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smax);
+    cudaError_t e = cudaFuncSetAttribute(k_batch_qaoa<NT, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     attr_set.fetch_or(bit);
   }
   int per_sm = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch_qaoa<NT>, NT, smem);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch_qaoa<NT, T>, NT, smem);
   per_sm = std::max(1, per_sm);
   const int grid = num_sms() * per_sm;
   auto record = [&]() -> cudaError_t {
     cudaMemsetAsync(a.next, 0, 4 * ((size_t)ninst + 2), c->stream);
-    k_batch_qaoa<NT><<<grid, NT, smem, c->stream>>>(a);
-    k_qaoa_reduce<<<(ninst + 127) / 128, 128, 0, c->stream>>>(a.inst, ninst, a.part, dout);
+    if (p > 0) k_qaoa_tables<<<(unsigned)ninst * p, 64, 0, c->stream>>>(a, p);
+    k_batch_qaoa<NT, T><<<grid, NT, smem, c->stream>>>(a);
+    k_qaoa_reduce<<<(ninst + 3) / 4, 128, 0, c->stream>>>(a.inst, ninst, a.part, dout);
     return cudaGetLastError();
   };
   if (!use_graph) return record();
@@ -389,9 +506,10 @@ static cudaError_t run_batch(ket_ctx* c, const QArgs& a, size_t smem, int ninst,
   auto mix = [&](const void* p, size_t nb) {
     for (size_t i = 0; i < nb; i++) key = (key ^ ((const unsigned char*)p)[i]) * 1099511628211ull;
   };
-  const int nt = NT;
+  const int nt = NT, tile = T;
   mix(&a, sizeof(a));
-  mix(&smem, sizeof(smem));
+  mix(&tile, sizeof(tile));
+  mix(&p, sizeof(p));
   mix(&ninst, sizeof(ninst));
   mix(&dout, sizeof(dout));
   mix(&nt, sizeof(nt));
@@ -441,8 +559,8 @@ extern "C" int ket_batch_qaoa(ket_ctx* c, int ninst, const int* n, const int* ne
   cudaSetDevice(c->device);
   const int T = c->batch_tile;
   std::vector<QInst> inst(ninst);
-  std::vector<uint64_t> masks;
-  int64_t work = 0, parts = 0, nedges = 0;
+  std::vector<uint32_t> masks;
+  int64_t work = 0, parts = 0, phases = 0;
   for (int i = 0; i < ninst; i++) {
     if (n[i] < 1 || n[i] > 30) return fail(KET_ERR_RANGE, "instance qubit count out of range (1..30)");
     if (ne[i] < 0 || ne[i] > KQ_MAX_EDGES) return fail(KET_ERR_TYPE, "instance edge count out of range (0..64)");
@@ -457,43 +575,67 @@ extern "C" int ket_batch_qaoa(ket_ctx* c, int ninst, const int* n, const int* ne
       int u = edges[2 * (eoff[i] + e)], v = edges[2 * (eoff[i] + e) + 1];
       if (u < 0 || v < 0 || u >= n[i] || v >= n[i]) return fail(KET_ERR_RANGE, "edge endpoint out of range");
       if (u == v) return fail(KET_ERR_TYPE, "self-loop edge");
-      masks.push_back((uint64_t(1) << u) | (uint64_t(1) << v));
+      masks.push_back((uint32_t(1) << u) | (uint32_t(1) << v));
     }
-    nedges += ne[i];
+    std::vector<uint32_t> em(masks.begin() + I.edge_off, masks.end());
+    std::sort(em.begin(), em.end());
+    I.multi = std::adjacent_find(em.begin(), em.end()) != em.end();
+    I.tab_off = phases;
+    phases += (int64_t)p * (ne[i] + 1);
     const bool split = I.n > T && p > 0;
     I.ntiles = split ? (1 << (I.n - T)) : 1;
     I.state = split ? work : 0;
-    I.cut = split ? work : 0;  // the cut bytes sit at the same index offset in their own area
     if (split) work += int64_t(1) << I.n;
     I.part_off = parts;
     parts += I.ntiles;
   }
-  // Work order: wide instances pass by pass (largest first, interleaved so a
-  // tile rarely waits), then the shared-memory instances (largest first).
+  // Work order: wide instances (largest first), then those that fit the chip.
   std::vector<int> order(ninst);
   for (int i = 0; i < ninst; i++) order[i] = i;
   std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return inst[x].n > inst[y].n; });
-  std::vector<QItem> items;
-  for (int k = 0; k < 2 * p; k++)
-    for (int i : order) {
-      const QInst& I = inst[i];
-      if (!(I.n > T && p > 0)) continue;
-      for (int t = 0; t < I.ntiles; t++) items.push_back(QItem{i, k, t});
-    }
+  std::vector<QRun> runs;
+  int64_t nitems = 0;
+  auto add = [&](int i, int pass) {
+    runs.push_back(QRun{(int)nitems, i, pass, 0});
+    nitems += pass < 0 ? 1 : inst[i].ntiles;
+  };
+  // Wide instances go in sets whose states share the 126 MB L2, all passes of a set
+  // before the next, the set's instances in turn so that a tile rarely waits (512
+  // instances of up to 64 MB: 15.9 ms in one set, 15.3 in sets of 80 MB, 15.5 and
+  // 15.7 of 70 and 112 MB).
+  constexpr int64_t kSetBytes = int64_t(80) << 20;
+  std::vector<int> wide;
   for (int i : order)
-    if (!(inst[i].n > T && p > 0)) items.push_back(QItem{i, -1, 0});
-  if (g_drop_item >= 0 && (size_t)g_drop_item < items.size()) items.erase(items.begin() + g_drop_item);
+    if (inst[i].n > T && p > 0) wide.push_back(i);
+  while (!wide.empty()) {
+    std::vector<int> set, rest;
+    int64_t bytes = 0;
+    for (int i : wide) {
+      const int64_t b = int64_t(16) << inst[i].n;
+      if (set.empty() || bytes + b <= kSetBytes) { set.push_back(i); bytes += b; }
+      else rest.push_back(i);
+    }
+    for (int k = 0; k <= p; k++)
+      for (int i : set) add(i, k);
+    wide.swap(rest);
+  }
+  for (int i : order)
+    if (!(inst[i].n > T && p > 0)) add(i, -1);
+  if (nitems > INT32_MAX / 2) return fail(KET_ERR_UNSUPPORTED, "too many tiles in a batch");
+  runs.push_back(QRun{INT32_MAX, 0, 0, 0});  // end marks
+  runs.push_back(QRun{INT32_MAX, 0, 0, 0});
   // device buffers in the second scratch pool
   auto al = [](size_t b) { return (b + 255) & ~size_t(255); };
-  size_t off_inst = 0, off_items = al(sizeof(QInst) * ninst), off_mask = off_items + al(sizeof(QItem) * items.size());
-  size_t off_g = off_mask + al(8 * std::max<size_t>(masks.size(), 1));
+  size_t off_inst = 0, off_runs = al(sizeof(QInst) * ninst), off_mask = off_runs + al(sizeof(QRun) * runs.size());
+  size_t off_g = off_mask + al(4 * std::max<size_t>(masks.size(), 1));
   size_t off_b = off_g + al(8 * (size_t)ninst * p + 8);
-  size_t off_part = off_b + al(8 * (size_t)ninst * p + 8);
-  size_t off_out = off_part + al(8 * (size_t)parts);
+  size_t off_tan = off_b + al(8 * (size_t)ninst * p + 8);
+  size_t off_tab = off_tan + al(8 * std::max<size_t>((size_t)ninst * p, 1));
+  size_t off_part = off_tab + al(16 * std::max<size_t>((size_t)phases, 1));
+  size_t off_out = off_part + al(16 * (size_t)parts);
   size_t off_cnt = off_out + al(8 * (size_t)ninst);
   size_t off_work = off_cnt + al(4 * ((size_t)ninst + 2));
-  size_t off_cut = off_work + al(16 * (size_t)work);
-  size_t total = off_cut + (size_t)work + 256;
+  size_t total = off_work + al(16 * (size_t)work) + 256;
   if (c->scratch2_bytes < total) {
     int rc = ctx_wait(c);
     if (rc) return rc;
@@ -509,39 +651,43 @@ extern "C" int ket_batch_qaoa(ket_ctx* c, int ninst, const int* n, const int* ne
   char* base = (char*)c->scratch2;
   std::vector<double> gv(gamma, gamma + (size_t)ninst * p), bv(beta, beta + (size_t)ninst * p);
   cudaMemcpyAsync(base + off_inst, inst.data(), sizeof(QInst) * ninst, cudaMemcpyHostToDevice, c->stream);
-  cudaMemcpyAsync(base + off_items, items.data(), sizeof(QItem) * items.size(), cudaMemcpyHostToDevice, c->stream);
-  if (!masks.empty()) cudaMemcpyAsync(base + off_mask, masks.data(), 8 * masks.size(), cudaMemcpyHostToDevice, c->stream);
+  cudaMemcpyAsync(base + off_runs, runs.data(), sizeof(QRun) * runs.size(), cudaMemcpyHostToDevice, c->stream);
+  if (!masks.empty()) cudaMemcpyAsync(base + off_mask, masks.data(), 4 * masks.size(), cudaMemcpyHostToDevice, c->stream);
   if (p > 0) {
     cudaMemcpyAsync(base + off_g, gv.data(), 8 * gv.size(), cudaMemcpyHostToDevice, c->stream);
     cudaMemcpyAsync(base + off_b, bv.data(), 8 * bv.size(), cudaMemcpyHostToDevice, c->stream);
   }
-  c->h2d_bytes += sizeof(QInst) * ninst + sizeof(QItem) * items.size() + 8 * masks.size() + 16 * gv.size();
+  c->h2d_bytes += sizeof(QInst) * ninst + sizeof(QRun) * runs.size() + 4 * masks.size() + 16 * gv.size();
   QArgs a;
+  memset(&a, 0, sizeof(a));  // its bytes are the graph's key
   a.inst = (const QInst*)(base + off_inst);
-  a.items = (const QItem*)(base + off_items);
-  a.emask = (const uint64_t*)(base + off_mask);
+  a.runs = (const QRun*)(base + off_runs);
+  a.emask = (const uint32_t*)(base + off_mask);
   a.gamma = (const double*)(base + off_g);
   a.beta = (const double*)(base + off_b);
-  a.part = (double*)(base + off_part);
+  a.tan = (double*)(base + off_tan);
+  a.tab = (double2*)(base + off_tab);
+  a.part = (double2*)(base + off_part);
   a.next = (unsigned int*)(base + off_cnt);
   a.done = a.next + 2;
   a.status = c->d_status;
   a.spin_limit = g_spin_limit;
   a.work = (double2*)(base + off_work);
-  a.cutw = (uint8_t*)(base + off_cut);
-  a.nitems = (int)items.size();
-  a.tile = T;
-  const size_t smem = (17u << T) + 16 * (KQ_MAX_EDGES + 1) + 8 * KQ_MAX_EDGES + 8 * 32;  // state, table, masks, sums, cuts
+  a.nitems = (int)nitems;
+  a.drop = g_drop_item;
   double* dout = (double*)(base + off_out);
   prof_begin(c);
   cudaError_t e;
-  switch (c->batch_threads) {
-    case 128: e = run_batch<128>(c, a, smem, ninst, dout, use_graph); break;
-    case 512: e = run_batch<512>(c, a, smem, ninst, dout, use_graph); break;
-    default: e = run_batch<256>(c, a, smem, ninst, dout, use_graph); break;
+  switch (c->batch_threads + T) {
+    case 128 + 11: e = run_batch<128, 11>(c, a, p, ninst, dout, use_graph); break;
+    case 256 + 11: e = run_batch<256, 11>(c, a, p, ninst, dout, use_graph); break;
+    case 512 + 11: e = run_batch<512, 11>(c, a, p, ninst, dout, use_graph); break;
+    case 128 + 12: e = run_batch<128, 12>(c, a, p, ninst, dout, use_graph); break;
+    case 512 + 12: e = run_batch<512, 12>(c, a, p, ninst, dout, use_graph); break;
+    default: e = run_batch<256, 12>(c, a, p, ninst, dout, use_graph); break;
   }
   prof_end(c, PK_BATCH);
-  c->launches += 1;  // the reduction (prof_end counted the batch kernel)
+  c->launches += 1 + (p > 0);  // the reduction and the tables (prof_end counted the batch kernel)
   if (e != cudaSuccess) return cuda_fail(e, "batch launch");
   e = cudaMemcpyAsync(out, dout, 8 * (size_t)ninst, cudaMemcpyDeviceToHost, c->stream);
   if (e != cudaSuccess) return cuda_fail(e, "cudaMemcpyAsync(out)");
