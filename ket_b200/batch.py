@@ -16,7 +16,7 @@ from typing import Sequence, Tuple
 
 import numpy as np
 
-from ._lib import RangeError, check, default_ctx, ket_batch_template, ket_param_binding, lib
+from ._lib import RangeError, check, default_ctx, ket_batch_template, ket_op, ket_param_binding, lib
 
 
 def batch_qaoa(instances: Sequence[Tuple[int, Sequence[Tuple[int, int]], Sequence[float], Sequence[float]]],
@@ -76,51 +76,49 @@ def batch_vqe(templates, instances, use_graph: bool = True) -> np.ndarray:
     from .adjoint import _terms
     if not instances:
         return np.zeros(0)
-    nparams = max(len(p) for _, p in instances)
-    first = {}
-    for t, p in instances:
-        if not 0 <= t < len(templates):
-            raise RangeError(f"instance template index {t} out of range")
-        first.setdefault(t, p)
+    which, params = zip(*instances)
+    it = np.ascontiguousarray(which, dtype=np.int32)
+    if it.min() < 0 or it.max() >= len(templates):
+        bad = it[(it < 0) | (it >= len(templates))][0]
+        raise RangeError(f"instance template index {bad} out of range")
+    lens = np.fromiter(map(len, params), dtype=np.int64, count=len(params))
+    nparams = int(lens.max())
+    used, at = np.unique(it, return_index=True)
+    first = {int(t): params[i] for t, i in zip(used, at)}
     tmpl = (ket_batch_template * max(1, len(templates)))()
     all_ops, all_mats, all_binds, coeffs, pauli = [], [], [], [], []
+    nops = nmats = nbinds = npauli = 0
     for j, (ansatz, ham) in enumerate(templates):
         p0 = first.get(j)
         if p0 is None:
             p0 = [0.3] * getattr(ansatz, "paramCount", nparams)
-        n, arr, m, k, binds = _traced(ansatz, p0)
+        n, ops, mats, binds = _traced(ansatz, p0)
         terms = _terms(ham, n)
-        moff = len(all_mats)
-        tmpl[j].nqubits, tmpl[j].nops, tmpl[j].nbinds, tmpl[j].nterms = n, k, len(binds), len(terms)
-        tmpl[j].op_first, tmpl[j].bind_first = len(all_ops), len(all_binds)
-        tmpl[j].term_first, tmpl[j].pauli_first = len(coeffs), sum(len(x) for x in pauli)
-        for i in range(k):
-            if arr[i].mat >= 0:
-                arr[i].mat += moff
-            all_ops.append(arr[i])
-        all_mats.extend(m.tolist())
-        all_binds.extend(binds)
+        tmpl[j].nqubits, tmpl[j].nops, tmpl[j].nbinds, tmpl[j].nterms = n, len(ops), len(binds), len(terms)
+        tmpl[j].op_first, tmpl[j].bind_first = nops, nbinds
+        tmpl[j].term_first, tmpl[j].pauli_first = len(coeffs), npauli
+        ops = ops.copy()
+        ops["mat"][ops["mat"] >= 0] += nmats
+        all_ops.append(ops)
+        all_mats.append(mats)
+        all_binds.append(binds)
+        nops, nmats, nbinds = nops + len(ops), nmats + len(mats), nbinds + len(binds)
         for c, o in terms:
             coeffs.append(c)
             pauli.append(o)
-    ops_a = (type(all_ops[0]) * max(1, len(all_ops)))(*all_ops) if all_ops else None
-    mats = np.ascontiguousarray(np.asarray(all_mats or [0j], dtype=np.complex128)).view(np.float64)
-    barr = (ket_param_binding * max(1, len(all_binds)))()
-    for i, (op, gate, prm, scale, shift) in enumerate(all_binds):
-        barr[i].op, barr[i].gate, barr[i].param, barr[i].scale, barr[i].shift = op, gate, prm, scale, shift
+            npauli += len(o)
+    ops_a = np.concatenate(all_ops) if nops else np.zeros(1, dtype=_OP)
+    binds_a = np.concatenate(all_binds) if nbinds else np.zeros(1, dtype=_BIND)
+    mats = np.concatenate(all_mats + [np.zeros(1, dtype=np.complex128)]).view(np.float64)
     cf = np.ascontiguousarray(coeffs or [0.0], dtype=np.float64)
     ps = "".join(pauli).encode()
-    it = np.ascontiguousarray([t for t, _ in instances], dtype=np.int32)
-    if all(len(p) == nparams for _, p in instances):
-        th = np.ascontiguousarray(np.asarray([p for _, p in instances], dtype=np.float64).reshape(-1))
-    else:
-        th = np.zeros((len(instances), max(nparams, 1)))
-        for i, (_, p) in enumerate(instances):
-            th[i, : len(p)] = p
-        th = np.ascontiguousarray(th.reshape(-1))
+    th = np.zeros((len(instances), max(nparams, 1)))
+    if nparams:  # every instance's parameters at the start of its row
+        th[np.arange(th.shape[1]) < lens[:, None]] = np.concatenate(params, dtype=np.float64, casting="unsafe")
     out = np.zeros(len(instances))
     dp = lambda a: a.ctypes.data_as(C.POINTER(C.c_double))
-    check(lib().ket_batch_vqe(default_ctx(), len(templates), tmpl, ops_a, dp(mats), mats.size // 2, barr, dp(cf), ps,
+    check(lib().ket_batch_vqe(default_ctx(), len(templates), tmpl, ops_a.ctypes.data_as(C.POINTER(ket_op)), dp(mats),
+                              mats.size // 2, binds_a.ctypes.data_as(C.POINTER(ket_param_binding)), dp(cf), ps,
                               len(instances), it.ctypes.data_as(C.POINTER(C.c_int)), dp(th), max(nparams, 1),
                               1 if use_graph else 0, dp(out)))
     return out
@@ -128,12 +126,16 @@ def batch_vqe(templates, instances, use_graph: bool = True) -> np.ndarray:
 
 # Traced templates, kept per ansatz function while it lives: a parameter sweep
 # calls batch_vqe again and again with the same ansatze, and tracing (two
-# builds of the circuit) costs more host time than the batch's kernel.
+# builds of the circuit) costs more host time than the batch's kernel.  They are
+# kept as arrays of the ABI's structures, so that a call joins them with a few
+# array operations.
 _TRACE_CACHE = weakref.WeakKeyDictionary()
+_OP = np.dtype(ket_op)
+_BIND = np.dtype(ket_param_binding)
 
 
 def _traced(ansatz, p0):
-    """(n, ket_op array, matrices, count, bindings) of an ansatz, traced once."""
+    """(n, ket_op array, matrices, bindings) of an ansatz, traced once."""
     from .adjoint import trace
     from .circuit import ops_to_abi
     key = len(p0)
@@ -144,12 +146,12 @@ def _traced(ansatz, p0):
     if hit is None:
         n, ops, binds = trace(ansatz, [float(v) for v in p0])
         arr, m, k = ops_to_abi(ops)
-        hit = (n, arr, m, k, binds)
+        b = np.zeros(len(binds), dtype=_BIND)
+        for i, v in enumerate(binds):
+            b[i]["op"], b[i]["gate"], b[i]["param"], b[i]["scale"], b[i]["shift"] = v
+        hit = (n, np.frombuffer(arr, dtype=_OP, count=k).copy(), m, b)
         try:
             _TRACE_CACHE.setdefault(ansatz, {})[key] = hit
         except TypeError:
             pass
-    n, arr, m, k, binds = hit
-    arr2 = (type(arr[0]) * max(1, k))()
-    C.memmove(arr2, arr, C.sizeof(arr2))  # the caller shifts matrix offsets in its copy
-    return n, arr2, m, k, binds
+    return hit

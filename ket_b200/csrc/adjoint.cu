@@ -396,30 +396,82 @@ int ket_adjoint_gradient(ket_ctx* ctx, int n, uint64_t init, const ket_op* ops, 
   const int nseg = std::max(1, (int)((nops + C - 1) / C));
   const size_t half = size_t(16) << n;
 
+  // lambda = H psi by tiles; the terms that do not fit a tile go first
+  PauliGroups wide;
+  const std::vector<PauliTilePass> tiled = plan_pauli_tiles(n, terms, false, wide);
+  std::vector<DevTerm> dterms;
+  for (const auto& kv : wide)
+    for (const PauliTerm* t : kv.second) {
+      zc ph = std::pow(zc(0, 1), t->ny & 3) * t->coeff;
+      dterms.push_back(DevTerm{t->flip, t->zm, ph.real(), ph.imag()});
+    }
+  std::vector<PauliTileGroup> tgroups;
+  std::vector<PauliTileTerm> tterms;
+  for (const PauliTilePass& P : tiled) {
+    tgroups.insert(tgroups.end(), P.groups.begin(), P.groups.end());
+    tterms.insert(tterms.end(), P.terms.begin(), P.terms.end());
+  }
+  const int hblocks = 1024;
+  const size_t nslot = std::max<size_t>(nbinds, 1);
   AdjWork w;
+  w.gpart_cap = (size_t)2 * num_sms() * 8 * KET_JIT_MAX_PROBES;  // CTAs x warps x probes of one pass
+  const size_t tt_off = (sizeof(PauliTileGroup) * tgroups.size() + 255) & ~size_t(255);
+  const size_t b_slots = sizeof(double) * nslot * std::max(batch, 1), b_gpart = sizeof(double) * w.gpart_cap,
+               b_terms = sizeof(DevTerm) * std::max<size_t>(dterms.size(), 1),
+               b_tiles = tt_off + sizeof(PauliTileTerm) * tterms.size() + 1,
+               b_epart = sizeof(double) * (hblocks + 8 + std::max(batch, 1));
+  // Small calls take their buffers, checkpoints included, from one workspace that
+  // the context keeps (at most kPooled bytes); larger ones allocate for the call.
+  // (Seven allocations and frees and a query of free memory were a third of a
+  // 14-qubit gradient.)
+  constexpr size_t kPooled = size_t(64) << 20;
+  auto al = [](size_t b) { return (b + 255) & ~size_t(255); };
+  const size_t need = (size_t)(nseg + 1) * al(half) + al(b_slots) + al(b_gpart) + al(b_terms) + al(b_tiles) + al(b_epart);
+  bool pooled = need <= kPooled && g_ckpt_device_budget < 0;
+  if (pooled && ctx->adj_work_bytes < need) {
+    rc = ctx_wait(ctx);
+    if (rc) return rc;
+    if (ctx->adj_work) cudaFree(ctx->adj_work);
+    ctx->adj_work = nullptr;
+    ctx->adj_work_bytes = 0;
+    pooled = dev_alloc(&ctx->adj_work, need) == KET_OK;
+    if (pooled) ctx->adj_work_bytes = need;
+    else g_err.clear();
+  }
+  size_t used = 0;
+  std::vector<void*> own;  // allocated for this call
+  auto get = [&](void** p, size_t bytes) {
+    if (pooled) {
+      *p = (char*)ctx->adj_work + used;
+      used += al(bytes);
+      return (int)KET_OK;
+    }
+    const int r = dev_alloc(p, bytes);
+    if (r == KET_OK) own.push_back(*p);
+    return r;
+  };
   void* buf = nullptr;
-  rc = dev_alloc(&buf, 2 * half);
+  rc = get(&buf, 2 * half);
   if (rc) return rc;
   w.full.ctx = ctx; w.full.n = n + 1; w.full.precision = KET_C128; w.full.amp = buf; w.full.bytes = 2 * half;
   w.psi.ctx = ctx; w.psi.n = n; w.psi.precision = KET_C128; w.psi.amp = buf; w.psi.bytes = half;
   auto cleanup = [&]() {
     ctx_wait(ctx);
-    for (const Ckpt& k : w.ckpt) {
+    for (const Ckpt& k : w.ckpt)
       if (k.host) cudaFreeHost(k.p);
-      else cudaFree(k.p);
-    }
-    if (w.slot_out) cudaFree(w.slot_out);
-    if (w.gpart) cudaFree(w.gpart);
-    if (w.terms) cudaFree(w.terms);
-    if (w.tiles) cudaFree(w.tiles);
-    if (w.epart) cudaFree(w.epart);
-    cudaFree(buf);
+    for (void* p : own) cudaFree(p);
   };
   // Checkpoints for segments 1..nseg-1: in device memory while it holds
   // them (2 GiB spare, or the debug budget), then in pinned host memory, so a
   // state too large to keep more than one device copy still restores psi at
   // every segment boundary.
-  {
+  if (pooled) {
+    for (int sgi = 1; sgi < nseg; sgi++) {
+      Ckpt k;
+      get(&k.p, half);
+      w.ckpt.push_back(k);
+    }
+  } else {
     size_t freeb = 0, totb = 0;
     cudaMemGetInfo(&freeb, &totb);
     const size_t spare = size_t(2) << 30;
@@ -428,7 +480,7 @@ int ket_adjoint_gradient(ket_ctx* ctx, int n, uint64_t init, const ket_op* ops, 
     for (int sgi = 1; sgi < nseg; sgi++) {
       Ckpt k;
       if (dev_room >= half) {
-        if (dev_alloc(&k.p, half) == KET_OK) {
+        if (get(&k.p, half) == KET_OK) {
           dev_room -= half;
           w.ckpt.push_back(k);
           continue;
@@ -453,32 +505,11 @@ int ket_adjoint_gradient(ket_ctx* ctx, int n, uint64_t init, const ket_op* ops, 
     const Ckpt& k = w.ckpt[sg - 1];
     return cudaMemcpyAsync(buf, k.p, half, k.host ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice, ctx->stream);
   };
-  // lambda = H psi by tiles; the terms that do not fit a tile go first
-  PauliGroups wide;
-  const std::vector<PauliTilePass> tiled = plan_pauli_tiles(n, terms, false, wide);
-  std::vector<DevTerm> dterms;
-  for (const auto& kv : wide)
-    for (const PauliTerm* t : kv.second) {
-      zc ph = std::pow(zc(0, 1), t->ny & 3) * t->coeff;
-      dterms.push_back(DevTerm{t->flip, t->zm, ph.real(), ph.imag()});
-    }
-  std::vector<PauliTileGroup> tgroups;
-  std::vector<PauliTileTerm> tterms;
-  for (const PauliTilePass& P : tiled) {
-    tgroups.insert(tgroups.end(), P.groups.begin(), P.groups.end());
-    tterms.insert(tterms.end(), P.terms.begin(), P.terms.end());
-  }
-  const int hblocks = 1024;
-  const size_t nslot = std::max<size_t>(nbinds, 1);
-  rc = dev_alloc((void**)&w.slot_out, sizeof(double) * nslot * std::max(batch, 1));
-  if (!rc) {
-    w.gpart_cap = (size_t)2 * num_sms() * 8 * KET_JIT_MAX_PROBES;  // CTAs x warps x probes of one pass
-    rc = dev_alloc((void**)&w.gpart, sizeof(double) * w.gpart_cap);
-  }
-  if (!rc) rc = dev_alloc((void**)&w.terms, sizeof(DevTerm) * std::max<size_t>(dterms.size(), 1));
-  const size_t tt_off = (sizeof(PauliTileGroup) * tgroups.size() + 255) & ~size_t(255);
-  if (!rc && !tiled.empty()) rc = dev_alloc((void**)&w.tiles, tt_off + sizeof(PauliTileTerm) * tterms.size());
-  if (!rc) rc = dev_alloc((void**)&w.epart, sizeof(double) * (hblocks + 8 + std::max(batch, 1)));
+  rc = get((void**)&w.slot_out, b_slots);
+  if (!rc) rc = get((void**)&w.gpart, b_gpart);
+  if (!rc) rc = get((void**)&w.terms, b_terms);
+  if (!rc) rc = get((void**)&w.tiles, b_tiles);
+  if (!rc) rc = get((void**)&w.epart, b_epart);
   if (rc) { cleanup(); return rc; }
   if (!dterms.empty())
     cudaMemcpyAsync(w.terms, dterms.data(), sizeof(DevTerm) * dterms.size(), cudaMemcpyHostToDevice, ctx->stream);
@@ -646,8 +677,7 @@ int ket_adjoint_gradient(ket_ctx* ctx, int n, uint64_t init, const ket_op* ops, 
     ctx->d2h_bytes += 8 * (size_t)batch * (nslot + 1);
   }
   const auto t_queued = std::chrono::steady_clock::now();
-  rc = ctx_wait(ctx);
-  if (!rc) rc = check_status(ctx);
+  rc = ctx_finish(ctx);
   if (timing) {
     const auto t_done = std::chrono::steady_clock::now();
     fprintf(stderr, "ket_adjoint_gradient: %d vectors, %d segments: queued in %.3f s, then waited %.3f s\n", batch,

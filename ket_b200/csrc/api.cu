@@ -123,14 +123,30 @@ int ctx_wait(ket_ctx* ctx) {
   if (e != cudaSuccess) return cuda_fail(e, "cudaEventRecord");
   auto t0 = std::chrono::steady_clock::now();
   const double limit = wait_deadline_s();
-  int spins = 0;
+  // Polled without a pause for as long as a small call takes (a 50 us sleep was a
+  // sixth of a 10-qubit simulation), then with one.
+  constexpr double kSpin = 2e-3;
   for (;;) {
     e = cudaEventQuery(ctx->done);
     if (e == cudaSuccess) break;
     if (e != cudaErrorNotReady) return cuda_fail(e, "device execution");
-    if (++spins > 64) std::this_thread::sleep_for(std::chrono::microseconds(50));
-    double el = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
+    const double el = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
     if (el > limit) return fail(KET_ERR_TIMEOUT, "device work did not finish within the wait deadline");
+    if (el > kSpin) std::this_thread::sleep_for(std::chrono::microseconds(50));
+  }
+  return KET_OK;
+}
+
+int ctx_finish(ket_ctx* c) {
+  // (a copy in stream order: a synchronous one after the wait is another round trip)
+  cudaError_t e = cudaMemcpyAsync(c->h_status, c->d_status, sizeof(int), cudaMemcpyDeviceToHost, c->stream);
+  if (e != cudaSuccess) return cuda_fail(e, "status read");
+  const int rc = ctx_wait(c);
+  if (rc) return rc;
+  const int st = *c->h_status;
+  if (st != 0) {
+    cudaMemsetAsync(c->d_status, 0, sizeof(int), c->stream);
+    return fail(st, "a device-side bounded wait ran out (status " + std::to_string(st) + ")");
   }
   return KET_OK;
 }
@@ -200,6 +216,16 @@ int ket_ctx_create(int device, ket_ctx** out) {
   int rc = dev_alloc(&st, 256);
   if (rc) { cudaEventDestroy(c->done); cudaStreamDestroy(c->stream); delete c; return rc; }
   c->d_status = (int*)st;
+  void* hst = nullptr;
+  e = cudaHostAlloc(&hst, sizeof(int), cudaHostAllocDefault);
+  if (e != cudaSuccess) {
+    cudaFree(st);
+    cudaEventDestroy(c->done);
+    cudaStreamDestroy(c->stream);
+    delete c;
+    return cuda_fail(e, "cudaHostAlloc(status)");
+  }
+  c->h_status = (int*)hst;
   cudaMemsetAsync(c->d_status, 0, 256, c->stream);
   *out = c;
   return KET_OK;
@@ -211,7 +237,9 @@ int ket_ctx_destroy(ket_ctx* c) {
   ctx_wait(c);
   if (c->scratch) cudaFree(c->scratch);
   if (c->scratch2) cudaFree(c->scratch2);
+  if (c->adj_work) cudaFree(c->adj_work);
   if (c->d_status) cudaFree(c->d_status);
+  if (c->h_status) cudaFreeHost(c->h_status);
   if (c->graph_exec) cudaGraphExecDestroy(c->graph_exec);
   if (c->vqe_graph_exec) cudaGraphExecDestroy(c->vqe_graph_exec);
   if (c->vqe_work) cudaFree(c->vqe_work);
@@ -228,7 +256,7 @@ int ket_ctx_destroy(ket_ctx* c) {
 
 int ket_ctx_scratch_bytes(const ket_ctx* c, uint64_t* out) {
   if (!c || !out) return fail(KET_ERR_TYPE, "null argument");
-  *out = c->scratch_bytes + c->scratch2_bytes;
+  *out = c->scratch_bytes + c->scratch2_bytes + c->adj_work_bytes;
   return KET_OK;
 }
 
@@ -320,16 +348,8 @@ int ket_state_set_basis(ket_state* s, uint64_t idx) {
   cudaSetDevice(s->ctx->device);
   cudaError_t e = cudaMemsetAsync(s->amp, 0, s->bytes, s->ctx->stream);
   if (e != cudaSuccess) return cuda_fail(e, "cudaMemsetAsync");
-  s->ctx->h2d_bytes += s->precision == KET_C64 ? 8 : 16;
-  if (s->precision == KET_C64) {
-    float one[2] = {1.0f, 0.0f};
-    e = cudaMemcpyAsync((char*)s->amp + 8 * idx, one, 8, cudaMemcpyHostToDevice, s->ctx->stream);
-  } else {
-    double one[2] = {1.0, 0.0};
-    e = cudaMemcpyAsync((char*)s->amp + 16 * idx, one, 16, cudaMemcpyHostToDevice, s->ctx->stream);
-  }
-  if (e != cudaSuccess) return cuda_fail(e, "cudaMemcpyAsync");
-  return ctx_wait(s->ctx);
+  e = launch_set_one(s->amp, s->precision, idx, s->ctx->stream);  // (queued: nothing to wait for)
+  return e == cudaSuccess ? KET_OK : cuda_fail(e, "set_basis launch");
 }
 
 int ket_state_set_amplitudes(ket_state* s, uint64_t off, uint64_t cnt, const double* re_im) {
@@ -645,22 +665,7 @@ int run_plan(ket_state* s, const Plan& plan, const ket_exec_opts& o, bool wait, 
     prof_end(c, kind);
     if (e != cudaSuccess) return cuda_fail(e, "kernel launch");
   }
-  if (!wait) return KET_OK;
-  int rc = ctx_wait(c);
-  if (rc) return rc;
-  return check_status(c);
-}
-
-// Read and clear the device status word (set by kernels whose bounded waits ran out).
-int check_status(ket_ctx* c) {
-  int st = 0;
-  cudaError_t e = cudaMemcpy(&st, c->d_status, sizeof(int), cudaMemcpyDeviceToHost);
-  if (e != cudaSuccess) return cuda_fail(e, "status read");
-  if (st != 0) {
-    cudaMemset(c->d_status, 0, sizeof(int));
-    return fail(st, "a device-side bounded wait ran out (status " + std::to_string(st) + ")");
-  }
-  return KET_OK;
+  return wait ? ctx_finish(c) : KET_OK;
 }
 
 }  // namespace ket

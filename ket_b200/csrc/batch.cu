@@ -692,7 +692,5 @@ extern "C" int ket_batch_qaoa(ket_ctx* c, int ninst, const int* n, const int* ne
   e = cudaMemcpyAsync(out, dout, 8 * (size_t)ninst, cudaMemcpyDeviceToHost, c->stream);
   if (e != cudaSuccess) return cuda_fail(e, "cudaMemcpyAsync(out)");
   c->d2h_bytes += 8 * (size_t)ninst;
-  int rc = ctx_wait(c);
-  if (rc) return rc;
-  return check_status(c);
+  return ctx_finish(c);
 }

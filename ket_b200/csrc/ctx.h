@@ -27,6 +27,9 @@ struct ket_ctx {
   uint64_t vqe_graph_key = 0;
   // launch accounting and optional per-launch CUDA-event timing
   int* d_status = nullptr;        // device status word written by kernels (bounded waits)
+  int* h_status = nullptr;        // its copy in pinned memory (ctx_finish)
+  void* adj_work = nullptr;       // ket_adjoint_gradient's buffers while they are small
+  size_t adj_work_bytes = 0;
   uint64_t launches = 0;
   uint64_t h2d_bytes = 0, d2h_bytes = 0;  // host<->device copies made by the context
   bool prof = false;
@@ -74,7 +77,8 @@ int ctx_upload(ket_ctx* ctx, void* dst, const void* src, size_t bytes);
 // one another.  first, last: run only passes [first, last) of the plan.
 int run_plan(ket_state* s, const Plan& plan, const ket_exec_opts& o, bool wait = true, size_t first = 0,
              size_t last = SIZE_MAX);
-int check_status(ket_ctx* c);
+// ctx_wait, then the status word the kernels so far may have set (read and cleared).
+int ctx_finish(ket_ctx* c);
 // ket_sample with the sequential CDF up to seq_qubits qubits (see read.h).
 int sample_indices(const ket_state* s, const double* r, size_t shots, double thr, uint64_t* out);
 

@@ -138,6 +138,14 @@ __global__ void k_mat2(typename Vec2<R>::T* a, uint64_t nq, int ta, int tb, uint
   }
 }
 
+template <typename V>
+__global__ void k_set_one(V* a) {
+  V v;
+  v.x = 1;
+  v.y = 0;
+  *a = v;
+}
+
 // Dense k-qubit unitaries.  Row r of a group of D = 2^k amplitudes is
 // sum_c m[r][c] x[c], the terms added in ascending c in FP64 whatever the state's
 // precision (the order of applyUnitary, statevector.ts:240-270).
@@ -511,6 +519,12 @@ DevOp encode_devop(const Gate& g, const Pass& p, bool prune) {
 cudaError_t launch_gate(const Gate& g, int precision, void* amp, int n, const void* dev_matk, cudaStream_t s) {
   return precision == KET_C64 ? launch_gate_t<float>(g, amp, n, dev_matk, s)
                               : launch_gate_t<double>(g, amp, n, dev_matk, s);
+}
+
+cudaError_t launch_set_one(void* amp, int precision, uint64_t idx, cudaStream_t s) {
+  if (precision == KET_C64) k_set_one<<<1, 1, 0, s>>>((float2*)amp + idx);
+  else k_set_one<<<1, 1, 0, s>>>((double2*)amp + idx);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_fused(const PassArgs& a, int precision, cudaStream_t s) {

@@ -60,6 +60,8 @@ struct Ctx;
 DevOp encode_devop(const Gate& g, const Pass& p, bool prune);
 // Single-gate pass over the whole state.
 cudaError_t launch_gate(const Gate& g, int precision, void* amp, int n, const void* dev_matk, cudaStream_t s);
+// amp[idx] = 1.
+cudaError_t launch_set_one(void* amp, int precision, uint64_t idx, cudaStream_t s);
 // Fused tile pass.
 cudaError_t launch_fused(const PassArgs& a, int precision, cudaStream_t s);
 
