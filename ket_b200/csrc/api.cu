@@ -5,6 +5,7 @@
 // deadline by polling an event (never an unbounded synchronize), and report
 // CUDA failures as status codes with a thread-local message.
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <cmath>
 #include <cstdlib>
@@ -12,6 +13,7 @@
 #include <mutex>
 #include <string>
 #include <thread>
+#include <unordered_set>
 #include <vector>
 
 #include "common.cuh"
@@ -150,6 +152,37 @@ int ctx_finish(ket_ctx* c) {
   }
   return KET_OK;
 }
+
+// Circuits of up to kSmallQubits qubits whose kernels were compiled ahead
+// (ket_jit_compile): they run on those kernels, as the default policy promises.
+// Known by a hash of their ops' kinds and qubits; like the kernels, kept until the
+// process ends.
+namespace {
+std::mutex g_ahead_mu;
+std::unordered_set<uint64_t> g_ahead;
+std::atomic<bool> g_any_ahead{false};
+uint64_t circuit_hash(int n, int precision, bool prune, const ket_op* ops, size_t nops) {
+  uint64_t h = 1469598103934665603ull;
+  auto mix = [&](uint64_t v) { h = (h ^ v) * 1099511628211ull; };
+  mix((uint64_t)n << 8 | (uint64_t)precision << 1 | prune);
+  for (size_t i = 0; i < nops; i++) {
+    mix((uint64_t)ops[i].kind << 8 | (uint64_t)ops[i].nq);
+    for (int j = 0; j < ops[i].nq && j < KET_MAX_OP_QUBITS; j++) mix((uint64_t)ops[i].q[j]);
+  }
+  return h;
+}
+void note_ahead(uint64_t h) {
+  std::lock_guard<std::mutex> lk(g_ahead_mu);
+  g_ahead.insert(h);
+  g_any_ahead.store(true);
+}
+bool compiled_ahead(int n, int precision, bool prune, const ket_op* ops, size_t nops) {
+  if (!g_any_ahead.load()) return false;
+  const uint64_t h = circuit_hash(n, precision, prune, ops, nops);
+  std::lock_guard<std::mutex> lk(g_ahead_mu);
+  return g_ahead.count(h) != 0;
+}
+}  // namespace
 
 static size_t amp_bytes(int precision) { return precision == KET_C64 ? 8 : 16; }
 
@@ -495,6 +528,7 @@ int ket_jit_compile(int n, int precision, const ket_op* ops, size_t nops, const 
                          use_staged(n, o.stage)});
   std::string clog;
   rc = jit_compile(jp, precision, kernels, clog);
+  if (!rc && n <= kSmallQubits && !jp.empty()) note_ahead(circuit_hash(n, precision, o.prune != 0, ops, nops));
   if (log && logcap) {
     strncpy(log, clog.c_str(), logcap - 1);
     log[logcap - 1] = 0;
@@ -515,6 +549,14 @@ int ket_apply_ops(ket_state* s, const ket_op* ops, size_t nops, const double* ma
   if (rc) return fail(rc, err);
   if (o.fusion != 0) fold_single_qubit(plan.gates, o.prune != 0);
   if (plan.gates.empty()) return KET_OK;
+  // Small complex128 states, with everything automatic, run in one launch.
+  if (s->precision == KET_C128 && s->n <= kSmallQubits && o.fusion < 0 && o.specialize == 0 && o.reg_bits == 0 && o.stage == 0 &&
+      !compiled_ahead(s->n, s->precision, o.prune != 0, ops, nops)) {
+    bool ran = false;
+    rc = run_small(s, plan.gates, o.prune != 0, &ran);
+    if (rc) return rc;
+    if (ran) return ctx_finish(s->ctx);
+  }
   plan_passes(s->n, s->precision, o.fusion, o.prune != 0, plan);
   return run_plan(s, plan, o);
 }

@@ -77,6 +77,9 @@ int ctx_upload(ket_ctx* ctx, void* dst, const void* src, size_t bytes);
 // one another.  first, last: run only passes [first, last) of the plan.
 int run_plan(ket_state* s, const Plan& plan, const ket_exec_opts& o, bool wait = true, size_t first = 0,
              size_t last = SIZE_MAX);
+// A circuit on a complex128 state of up to kSmallQubits qubits in one launch (small.cu).
+constexpr int kSmallQubits = 20;
+int run_small(ket_state* s, const std::vector<Gate>& gates, bool prune, bool* ran);
 // ctx_wait, then the status word the kernels so far may have set (read and cleared).
 int ctx_finish(ket_ctx* c);
 // ket_sample with the sequential CDF up to seq_qubits qubits (see read.h).

@@ -23,7 +23,7 @@
 
 namespace ket {
 
-constexpr int kRoundBits = 4;        // dimension of a round's span
+constexpr int kRoundBits = 4;        // dimension of a round's span, at most
 constexpr int kRoundGates = 16;      // gates in a round, at most
 constexpr int kRoundQubits = 13;
 
@@ -55,17 +55,19 @@ struct RoundSlots {
 
 struct RoundGate {
   uint8_t x;         // 1: X under its controls, 0: a 2x2 under its controls
+  uint8_t diag;      // 1: diagonal on the functional r, 2: on (r, r2); it has no mask
   uint8_t bit;       // the gate's mask = basis mask `bit` of the round
   uint8_t nc;        // controls
   uint8_t cj[3];     // per control: the basis masks that flip it
-  uint16_t r;        // row functional of the target
+  uint8_t rj[2];     // diagonal: the basis masks that flip r, r2
+  uint16_t r, r2;    // row functional of the target
   uint16_t m;        // pair mask of the target
   uint16_t rc[3];    // row functionals of the controls
   int32_t op;        // the caller's op
 };
 
 struct Round {
-  uint8_t k;                     // dimension: kRoundBits, or that of a dense round
+  uint8_t k;                     // dimension: the builder's, or that of a dense round
   uint8_t dense;                 // 1: one 2^k x 2^k, local index bit i on mask i
   uint8_t piv[kRoundBits];       // pivot bits of the span, ascending
   uint16_t m[kRoundBits];        // basis masks
@@ -74,46 +76,52 @@ struct Round {
   int32_t gate0, ngates;
 };
 
-// The relabelling and the round under construction.
-class RoundPlan {
+// Rounds from gates given by their masks and functionals.
+class RoundBuilder {
  public:
   std::vector<Round> rounds;
   std::vector<RoundGate> gates;
-  uint16_t row[kRoundQubits], col[kRoundQubits];
 
-  // n: the state's qubits, at least kRoundBits.
-  explicit RoundPlan(int n) : n_(n) {
-    for (int q = 0; q < kRoundQubits; q++) row[q] = col[q] = (uint16_t)(1u << q);
-  }
-  void cnot(int c, int t) { row[t] ^= row[c]; col[c] ^= col[t]; }
-  void swap(int a, int b) { std::swap(row[a], row[b]); std::swap(col[a], col[b]); }
+  // n: bits of an index, at least `bits`; bits: the dimension of the rounds.
+  explicit RoundBuilder(int n, int bits = kRoundBits) : n_(n), bits_(bits) {}
 
-  // A one-qubit gate (or X) on q under controls cs.
-  void gate(int q, const int* cs, int nc, bool x, int op) {
+  // A one-qubit gate (or X) on the target (m, r) under controls rc.
+  void add(uint16_t m, uint16_t r, const uint16_t* rc, int nc, bool x, int op) {
     RoundGate g = {};
     g.x = x;
     g.nc = (uint8_t)nc;
-    g.r = row[q];
-    g.m = col[q];
-    for (int i = 0; i < nc; i++) g.rc[i] = row[cs[i]];
+    g.r = r;
+    g.m = m;
+    std::copy(rc, rc + nc, g.rc);
     g.op = op;
     if (!join(g)) {
       close();
       join(g);
     }
   }
-  // A 2^k x 2^k on qs (qs[0] = MSB) under controls cs: a round of its own.
-  void dense(const int* qs, int k, const int* cs, int nc, int op) {
+  // A diagonal on the functional r, or with two set on (r, r2): it pairs nothing, so
+  // it takes no dimension of the round.
+  void add_diag(uint16_t r, uint16_t r2, bool two, const uint16_t* rc, int nc, int op) {
+    if ((int)cur_.size() >= kRoundGates) close();
+    RoundGate g = {};
+    g.diag = two ? 2 : 1;
+    g.nc = (uint8_t)nc;
+    g.r = r;
+    g.r2 = r2;
+    std::copy(rc, rc + nc, g.rc);
+    g.op = op;
+    cur_.push_back(g);
+  }
+  // A 2^k x 2^k, local index bit i on (ms[i], rs[i]), under controls: a round of its own.
+  void add_dense(const uint16_t* ms, const uint16_t* rs, int k, const uint16_t* rc, int nc, int op) {
     close();
     RoundGate g = {};
     g.nc = (uint8_t)nc;
-    for (int i = 0; i < nc; i++) g.rc[i] = row[cs[i]];
+    std::copy(rc, rc + nc, g.rc);
     g.op = op;
     cur_ = {g};
-    for (int i = 0; i < k; i++) {
-      basis_.push_back(col[qs[k - 1 - i]]);
-      rd_[i] = row[qs[k - 1 - i]];
-    }
+    basis_.assign(ms, ms + k);
+    std::copy(rs, rs + k, rd_);
     dense_ = true;
     close();
   }
@@ -143,11 +151,9 @@ class RoundPlan {
       R.gate0 = (int32_t)gates.size();
       R.ngates = (int32_t)cur_.size();
       for (RoundGate& g : cur_) {
-        for (int c = 0; c < g.nc; c++) {
-          g.cj[c] = 0;
-          for (int i = 0; i < R.k; i++)
-            if (odd(basis_[i] & g.rc[c])) g.cj[c] |= (uint8_t)(1u << i);
-        }
+        for (int c = 0; c < g.nc; c++) g.cj[c] = flipped_by(g.rc[c]);
+        g.rj[0] = flipped_by(g.r);
+        g.rj[1] = flipped_by(g.r2);
         gates.push_back(g);
       }
       rounds.push_back(R);
@@ -159,12 +165,18 @@ class RoundPlan {
   }
 
  private:
-  int n_;
+  int n_, bits_;
   std::vector<RoundGate> cur_;
   std::vector<uint16_t> basis_, brow_;  // masks, and the targets' row functionals: brow_[i] . basis_[j] = (i == j)
   uint16_t rd_[kRoundBits] = {};
   bool dense_ = false;
 
+  uint8_t flipped_by(uint16_t r) const {
+    uint8_t f = 0;
+    for (size_t i = 0; i < basis_.size(); i++)
+      if (odd(basis_[i] & r)) f |= (uint8_t)(1u << i);
+    return f;
+  }
   static bool odd(uint32_t x) { return __builtin_popcount(x) & 1; }
   bool independent(uint16_t m) const {
     uint32_t x = m;
@@ -186,7 +198,7 @@ class RoundPlan {
     if (at < basis_.size()) {
       if (brow_[at] != g.r) return false;
     } else {
-      if ((int)at >= kRoundBits || !independent(g.m)) return false;
+      if ((int)at >= bits_ || !independent(g.m)) return false;
       for (size_t i = 0; i < at; i++)
         if (odd(basis_[i] & g.r) || odd(g.m & brow_[i])) return false;
       basis_.push_back(g.m);
@@ -200,12 +212,40 @@ class RoundPlan {
   // vectors, each made orthogonal to the targets' functionals.
   void fill() {
     const size_t k = brow_.size();
-    for (int b = n_ - 1; b >= 0 && (int)basis_.size() < kRoundBits; b--) {
+    for (int b = n_ - 1; b >= 0 && (int)basis_.size() < bits_; b--) {
       uint16_t m = (uint16_t)(1u << b);
       for (size_t i = 0; i < k; i++)
         if (odd(m & brow_[i])) m ^= basis_[i];
       if (m && independent(m)) basis_.push_back(m);
     }
+  }
+};
+
+// Rounds of gates on logical qubits, with the relabelling.
+class RoundPlan : public RoundBuilder {
+ public:
+  uint16_t row[kRoundQubits], col[kRoundQubits];
+
+  explicit RoundPlan(int n) : RoundBuilder(n) {
+    for (int q = 0; q < kRoundQubits; q++) row[q] = col[q] = (uint16_t)(1u << q);
+  }
+  void cnot(int c, int t) { row[t] ^= row[c]; col[c] ^= col[t]; }
+  void swap(int a, int b) { std::swap(row[a], row[b]); std::swap(col[a], col[b]); }
+  // A one-qubit gate (or X) on q under controls cs.
+  void gate(int q, const int* cs, int nc, bool x, int op) {
+    uint16_t rc[3];
+    for (int i = 0; i < nc; i++) rc[i] = row[cs[i]];
+    add(col[q], row[q], rc, nc, x, op);
+  }
+  // A 2^k x 2^k on qs (qs[0] = MSB) under controls cs.
+  void dense(const int* qs, int k, const int* cs, int nc, int op) {
+    uint16_t rc[3], ms[kRoundBits], rs[kRoundBits];
+    for (int i = 0; i < nc; i++) rc[i] = row[cs[i]];
+    for (int i = 0; i < k; i++) {
+      ms[i] = col[qs[k - 1 - i]];
+      rs[i] = row[qs[k - 1 - i]];
+    }
+    add_dense(ms, rs, k, rc, nc, op);
   }
 };
 
