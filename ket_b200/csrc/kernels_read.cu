@@ -384,15 +384,16 @@ __global__ void __launch_bounds__(32 * kColRows) k_marginal_dist_combine(const d
 // Only blocks holding a binade crossing, a tie or the first kept entry run
 // entry by entry: a crossing happens about once per doubling of s.
 constexpr int kCdfThreads = 1024;
-constexpr int kCdfPer = 4;                          // entries per thread per chunk
-constexpr int kCdfChunk = kCdfThreads * kCdfPer;    // 4096
+constexpr int kWalkThreads = 1024;                  // the walker's
+constexpr int kCdfPer = 4;                          // entries of a block per walker thread
+constexpr int kCdfHead = 128;                       // entries after the first kept one, added one by one
 constexpr int kCdfBlock = 4096;                     // entries per block
 constexpr int kCdfSub = 32;                         // entries per checkpoint
 constexpr int kCdfSubPerBlock = kCdfBlock / kCdfSub;
 constexpr int kCdfWalkPer = 4;                      // blocks per walker thread per window
 constexpr long long kTwo52 = 4503599627370496ll;
 constexpr long long kTwo53 = 9007199254740992ll;
-static_assert(kCdfChunk == kCdfBlock, "an entry-by-entry block is one chunk");
+static_assert(kWalkThreads * kCdfPer == kCdfBlock, "a thread's share of a block");
 
 enum : int { kBlkUnclean = 0, kBlkClean = 1, kBlkEmpty = 2, kBlkExact = 3 };
 
@@ -526,6 +527,8 @@ __global__ void __launch_bounds__(256) k_cdf_block_d(const typename Vec2<R>::T* 
   int e = 0;
   if (A > 0.0) frexp(A, &e);
   const bool guess = A > 0.0;
+  const bool tiny = e < -900;  // (1 / u leaves the normal numbers)
+  const double inv_u = __longlong_as_double((long long)(1023 + 53 - (tiny ? 0 : e)) << 52);
   bool pos = false, bad = false;
   long long mine = 0;  // lane k < 16: the d-sum of sub-chunk 16w + k
 #pragma unroll 4
@@ -535,10 +538,12 @@ __global__ void __launch_bounds__(256) k_cdf_block_d(const typename Vec2<R>::T* 
     pos |= p > 0.0;
     long long d = 0;
     if (guess) {
-      const double q = ldexp(p, 53 - e);  // p / u, exact
-      if (q >= 4503599627370496.0) bad = true;  // 2^52: S + d would leave the binade
-      else if (q - floor(q) == 0.5) bad = true;   // a tie: the rounding depends on S
-      else d = (long long)rint(q);
+      const double q = tiny ? ldexp(p, 53 - e) : p * inv_u;  // p / u, exact
+      // rounded to an integer (ties to even) by the 2^52 that it is added to
+      const double y = q + 4503599627370496.0, r = y - 4503599627370496.0;
+      if (q >= 4503599627370496.0) bad = true;   // 2^52: S + d would leave the binade
+      else if (fabs(q - r) == 0.5) bad = true;    // a tie: the rounding depends on S
+      else d = __double_as_longlong(y) - 0x4330000000000000ll;
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
@@ -566,50 +571,102 @@ __global__ void __launch_bounds__(256) k_cdf_block_d(const typename Vec2<R>::T* 
   }
 }
 
-// The running sum over entries [lo, hi) (hi - lo <= kCdfChunk) in the
-// reference's rounding, from the exact sum *s_io before lo.  Writes the
-// checkpoints ck[(i + 1) / 32] for entries i with (i + 1) % 32 == 0 and
-// i + 1 < hi, and leaves the sum after entry hi - 1 in *s_io.  Called by the
-// whole CTA of kCdfThreads threads.
+// p 2^k, exact where the result is a normal number (k as frexp of a sum gives it).
+__device__ __forceinline__ double scaled(double p, int k) {
+  return k >= -1000 && k <= 1000 ? p * __longlong_as_double((long long)(1023 + k) << 52) : ldexp(p, k);
+}
+
+// Exclusive prefix of v and block minimum over the walker's threads, each with one
+// barrier: every warp reduces the 32 warps' values for itself.  `buf` holds values
+// that no thread reads any more (callers alternate between two).
+__device__ __forceinline__ long long walk_scan(long long v, long long* buf) {
+  static_assert(kWalkThreads == 1024, "one value a lane");
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  long long x = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const long long y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
+  }
+  if (lane == 31) buf[w] = x;
+  __syncthreads();
+  long long z = buf[lane];
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const long long y = __shfl_up_sync(0xffffffffu, z, o);
+    if (lane >= o) z += y;
+  }
+  const long long before = __shfl_sync(0xffffffffu, z, w > 0 ? w - 1 : 0);
+  return (w > 0 ? before : 0) + x - v;
+}
+__device__ __forceinline__ uint32_t walk_min(uint32_t v, uint32_t* buf) {
+  v = __reduce_min_sync(0xffffffffu, v);
+  if ((threadIdx.x & 31) == 0) buf[threadIdx.x >> 5] = v;
+  __syncthreads();
+  return __reduce_min_sync(0xffffffffu, buf[threadIdx.x & 31]);
+}
+
+// What the walker's threads share.  s: the exact running sum before position c.
+struct WalkShared {
+  long long scan[2][32];
+  uint32_t red[2][32];
+  double head[kCdfHead];
+  double s;
+  uint32_t c;
+};
+
+// The running sum over a block's entries [lo, hi) in the reference's rounding,
+// from the exact sum sh.s before lo.  Writes the checkpoints ck[(i + 1) / 32]
+// for entries i with (i + 1) % 32 == 0 and i + 1 < hi, and leaves the sum after
+// entry hi - 1 in sh.s.  Called by the whole CTA of kWalkThreads threads.
+//
+// A thread's entries lo + kCdfPer t + k stay in its registers; a step runs from
+// position c to the next tie or crossing, with three barriers (reloading the
+// entries of each step and twelve barriers took 5 us a step, a dozen steps a
+// block).
 template <typename R>
 __device__ void cdf_exact_range(const typename Vec2<R>::T* a, uint64_t lo, uint64_t hi, double thr, double* ck,
-                                double* s_io, unsigned long long* c_io, long long* wsum, unsigned long long* wred) {
-  const int tid = threadIdx.x;
-  const unsigned long long NONE = ~0ull;
-  if (tid == 0) *c_io = lo;
+                                WalkShared& sh, int& turn) {
+  const uint32_t tid = threadIdx.x, len = (uint32_t)(hi - lo), NONE = ~0u, i0 = kCdfPer * tid;
+  double pv[kCdfPer];
+#pragma unroll
+  for (int k = 0; k < kCdfPer; k++) pv[k] = i0 + k < len ? kept_p<R>(a, lo + i0 + k, thr) : 0.0;
+  auto checkpoint = [&](uint32_t i, double v) {  // the sum after entry i
+    if (((lo + i + 1) & (kCdfSub - 1)) == 0 && i + 1 < len) ck[(lo + i + 1) / kCdfSub] = v;
+  };
+  if (tid == 0) sh.c = 0;
   __syncthreads();
   for (;;) {
-    const uint64_t c = *c_io;
-    const double s = *s_io;
-    if (c >= hi) break;
-    // this thread's entries c + kCdfPer*tid + k
-    const uint64_t i0 = c + (uint64_t)kCdfPer * tid;
-    double pv[kCdfPer];
-#pragma unroll
-    for (int k = 0; k < kCdfPer; k++) pv[k] = i0 + k < hi ? kept_p<R>(a, i0 + k, thr) : 0.0;
+    const uint32_t c = sh.c;
+    const double s = sh.s;
+    if (c >= len) break;
+    turn ^= 1;
     if (s == 0.0) {
       // before the first positive kept entry the sum is +0.0; that entry sets
       // it exactly
-      unsigned long long f = NONE;
+      uint32_t f = NONE;
 #pragma unroll
-      for (int k = 0; k < kCdfPer; k++)
-        if (f == NONE && pv[k] > 0.0) f = i0 + k;
-      f = block_min_u64<kCdfThreads>(f, wred);
-      const uint64_t z = f == NONE ? hi : f;
+      for (int k = kCdfPer - 1; k >= 0; k--)
+        if (i0 + k >= c && pv[k] > 0.0) f = i0 + k;
+      const uint32_t z = min(walk_min(f, sh.red[turn]), len);
 #pragma unroll
       for (int k = 0; k < kCdfPer; k++) {
-        const uint64_t i = i0 + k;
-        if (i < z && ((i + 1) & (kCdfSub - 1)) == 0 && i + 1 < hi) ck[(i + 1) / kCdfSub] = 0.0;
+        const uint32_t i = i0 + k;
+        if (i >= c && i < z) checkpoint(i, 0.0);
+        if (i >= z && i < len && i - z < (uint32_t)kCdfHead) sh.head[i - z] = pv[k];
       }
+      __syncthreads();
+      // from there the sum doubles every few entries, and a step ends at each
+      // doubling: one thread adds the first entries as the reference does
       if (tid == 0) {
-        if (f != NONE) {
-          const double sn = 0.0 + kept_p<R>(a, f, thr);
-          if (((f + 1) & (kCdfSub - 1)) == 0 && f + 1 < hi) ck[(f + 1) / kCdfSub] = sn;
-          *s_io = sn;
-          *c_io = f + 1;
-        } else {
-          *c_io = hi;
+        const uint32_t cnt = min(len - z, (uint32_t)kCdfHead);
+        double t = 0.0;
+        for (uint32_t i = 0; i < cnt; i++) {
+          t += sh.head[i];
+          checkpoint(z + i, t);
         }
+        sh.s = t;
+        sh.c = z + cnt;
       }
       __syncthreads();
       continue;
@@ -617,165 +674,156 @@ __device__ void cdf_exact_range(const typename Vec2<R>::T* a, uint64_t lo, uint6
     // s in [2^(e-1), 2^e): u = 2^(e-53), S = s / u
     int e;
     frexp(s, &e);
-    const long long S0 = (long long)ldexp(s, 53 - e);
-    unsigned long long special = NONE;  // first entry that is a tie or crosses for sure
+    const long long S0 = (long long)scaled(s, 53 - e);
+    uint32_t stop = NONE;  // this thread's first entry that is a tie or crosses
     long long d[kCdfPer];
     long long tsum = 0;
 #pragma unroll
     for (int k = 0; k < kCdfPer; k++) {
-      const uint64_t i = i0 + k;
+      const uint32_t i = i0 + k;
       d[k] = 0;
-      if (i >= hi) continue;
-      const double q = ldexp(pv[k], 53 - e);  // p / u, exact
-      if (q >= 9007199254740992.0) {          // 2^53: the sum leaves the binade
-        if (special == NONE) special = i;
+      if (i < c || i >= len || stop != NONE) continue;
+      const double q = scaled(pv[k], 53 - e);  // p / u, exact
+      // 2^53: the sum leaves the binade; half: a tie, the rounding depends on S
+      if (q >= 9007199254740992.0 || q - floor(q) == 0.5) {
+        stop = i;
         continue;
       }
-      if (q - floor(q) == 0.5) {              // a tie: the rounding depends on S
-        if (special == NONE) special = i;
-        continue;
-      }
-      if (special == NONE) {
-        d[k] = (long long)rint(q);
-        tsum += d[k];
-      }
+      d[k] = (long long)rint(q);
+      tsum += d[k];
     }
-    special = block_min_u64<kCdfThreads>(special, wred);
-    // entries at or after the first special one do not count in the scan
-    if (special != NONE) {
-      tsum = 0;
-#pragma unroll
-      for (int k = 0; k < kCdfPer; k++)
-        if (i0 + k < special) tsum += d[k];
-    }
-    const long long incl = block_scan_incl<kCdfThreads>(tsum, wsum);
-    long long Sr = S0 + incl - tsum;  // S before this thread's first entry
-    unsigned long long cross = NONE;  // first entry whose sum reaches 2^53 u
+    // (past the first such entry of the block the prefix is of no use, but then
+    // neither is a crossing found there: the earliest position counts)
+    const long long S1 = S0 + walk_scan(tsum, sh.scan[turn]);
+    long long Sr = S1;  // S before this thread's first entry
 #pragma unroll
     for (int k = 0; k < kCdfPer; k++) {
-      const uint64_t i = i0 + k;
-      if (i >= hi || i >= special) break;
-      const long long Sn = Sr + d[k];
-      if (Sn >= kTwo53) { cross = i; break; }
-      Sr = Sn;
-    }
-    cross = block_min_u64<kCdfThreads>(cross, wred);
-    const uint64_t lim = c + (uint64_t)kCdfChunk < hi ? c + (uint64_t)kCdfChunk : hi;
-    uint64_t stop = special < cross ? (uint64_t)special : (uint64_t)cross;
-    if (stop > lim) stop = lim;
-    // the exact sums of the entries before `stop`
-    Sr = S0 + incl - tsum;
-#pragma unroll
-    for (int k = 0; k < kCdfPer; k++) {
-      const uint64_t i = i0 + k;
-      if (i >= stop) break;
+      const uint32_t i = i0 + k;
+      if (i < c || i >= len || i >= stop) continue;
+      if (Sr + d[k] >= kTwo53) { stop = i; continue; }
       Sr += d[k];
-      const double v = ldexp((double)Sr, e - 53);
-      if (((i + 1) & (kCdfSub - 1)) == 0 && i + 1 < hi) ck[(i + 1) / kCdfSub] = v;
-      if (i + 1 == stop) *s_io = v;
     }
-    __syncthreads();
-    if (tid == 0) {
-      double sp = *s_io;  // the sum before `stop` (s itself when stop == c)
-      if (stop < lim) {
+    stop = min(walk_min(stop, sh.red[turn]), len);
+    // the exact sums of the entries before `stop`
+    Sr = S1;
+#pragma unroll
+    for (int k = 0; k < kCdfPer; k++) {
+      const uint32_t i = i0 + k;
+      if (i < c || i > stop || i >= len) continue;
+      if (i == stop) {
         // the special entry, by the reference's own FP64 addition
-        sp = sp + kept_p<R>(a, stop, thr);
-        if (((stop + 1) & (kCdfSub - 1)) == 0 && stop + 1 < hi) ck[(stop + 1) / kCdfSub] = sp;
-        *s_io = sp;
-        *c_io = stop + 1;
-      } else {
-        *c_io = stop;
+        const double sp = scaled((double)Sr, e - 53) + pv[k];
+        checkpoint(i, sp);
+        sh.s = sp;
+        continue;
       }
+      Sr += d[k];
+      const double v = scaled((double)Sr, e - 53);
+      checkpoint(i, v);
+      if (i + 1 == len) sh.s = v;  // (stop == len)
     }
+    if (tid == 0) sh.c = stop < len ? stop + 1 : len;
     __syncthreads();
   }
 }
 
+// Windows of kCdfWalkPer blocks a thread: their states are read once, and the walk
+// steps through them as cdf_exact_range steps through entries.  27 qubits (32768
+// blocks, 27 doublings of the sum): 337 -> 222 us; 16 qubits 139 -> 71.
 template <typename R>
-__global__ void __launch_bounds__(kCdfThreads) k_cdf_walk(const typename Vec2<R>::T* a, uint64_t N, double thr,
+__global__ void __launch_bounds__(kWalkThreads) k_cdf_walk(const typename Vec2<R>::T* a, uint64_t N, double thr,
                                                           uint64_t nb, uint64_t nk, double* ck, const long long* bd,
                                                           int* bst, const int* be, double* bstart) {
-  __shared__ long long wsum[32];
-  __shared__ unsigned long long wred[33];
-  __shared__ double s_sh;              // the exact running sum before block c
-  __shared__ unsigned long long c_sh;  // the next block
-  __shared__ unsigned long long x_sh;  // cdf_exact_range's position
-  const int tid = threadIdx.x;
-  const unsigned long long NONE = ~0ull;
-  if (tid == 0) { s_sh = 0.0; c_sh = 0; }
-  __syncthreads();
-  for (;;) {
-    const uint64_t c = c_sh;
-    const double s = s_sh;
-    if (c >= nb) break;
-    int e = 0;
-    long long S0 = 0;
-    if (s > 0.0) {
-      frexp(s, &e);
-      S0 = (long long)ldexp(s, 53 - e);
-    }
-    // this thread's blocks c + kCdfWalkPer*tid + k
-    const uint64_t b0 = c + (uint64_t)kCdfWalkPer * tid;
-    long long dv[kCdfWalkPer];
-    unsigned long long fail = NONE;  // first block that is not taken whole
+  __shared__ WalkShared sh;
+  __shared__ uint32_t at_sh;           // the next block, in the window
+  __shared__ double sum_sh;            // the exact running sum before it
+  const uint32_t tid = threadIdx.x, NONE = ~0u, j0 = kCdfWalkPer * tid;
+  int turn = 0;
+  if (tid == 0) sum_sh = 0.0;
+  for (uint64_t win = 0; win < nb; win += kCdfWalkPer * kWalkThreads) {
+    const uint32_t len = (uint32_t)(nb - win < kCdfWalkPer * kWalkThreads ? nb - win : kCdfWalkPer * kWalkThreads);
+    int st[kCdfWalkPer], eb[kCdfWalkPer];
+    long long D[kCdfWalkPer];
 #pragma unroll
     for (int k = 0; k < kCdfWalkPer; k++) {
-      const uint64_t b = b0 + k;
-      dv[k] = 0;
-      if (b >= nb || fail != NONE) continue;
-      const int st = bst[b];
-      if (st == kBlkEmpty) continue;
-      if (st == kBlkClean && s > 0.0 && be[b] == e) dv[k] = bd[b];
-      else fail = b;
-    }
-    fail = block_min_u64<kCdfThreads>(fail, wred);
-    long long tsum = 0;
-#pragma unroll
-    for (int k = 0; k < kCdfWalkPer; k++)
-      if (b0 + k < fail) tsum += dv[k];
-    const long long incl = block_scan_incl<kCdfThreads>(tsum, wsum);  // each D < 2^53: no overflow
-    long long Sr = S0 + incl - tsum;
-    unsigned long long cross = NONE;  // first block whose sum reaches 2^53 u
-#pragma unroll
-    for (int k = 0; k < kCdfWalkPer; k++) {
-      const uint64_t b = b0 + k;
-      if (b >= nb || b >= fail) break;
-      if (Sr + dv[k] >= kTwo53) { cross = b; break; }
-      Sr += dv[k];
-    }
-    cross = block_min_u64<kCdfThreads>(cross, wred);
-    const uint64_t lim = c + (uint64_t)kCdfWalkPer * kCdfThreads < nb ? c + (uint64_t)kCdfWalkPer * kCdfThreads : nb;
-    uint64_t stop = fail < cross ? (uint64_t)fail : (uint64_t)cross;
-    if (stop > lim) stop = lim;
-    // blocks before `stop` are taken whole
-    Sr = S0 + incl - tsum;
-#pragma unroll
-    for (int k = 0; k < kCdfWalkPer; k++) {
-      const uint64_t b = b0 + k;
-      if (b >= stop) break;
-      bstart[b] = s > 0.0 ? ldexp((double)Sr, e - 53) : 0.0;
-      Sr += dv[k];
-      if (b + 1 == stop) s_sh = s > 0.0 ? ldexp((double)Sr, e - 53) : 0.0;
-    }
-    __syncthreads();
-    if (stop < lim) {
-      // block `stop` entry by entry
-      if (tid == 0) {
-        const double sb = s_sh;
-        bstart[stop] = sb;
-        bst[stop] = kBlkExact;
-        ck[stop * kCdfSubPerBlock] = sb;
+      st[k] = kBlkEmpty;
+      eb[k] = 0;
+      D[k] = 0;
+      if (j0 + k < len) {
+        st[k] = bst[win + j0 + k];
+        eb[k] = be[win + j0 + k];
+        D[k] = bd[win + j0 + k];
       }
-      const uint64_t lo = stop * kCdfBlock;
-      const uint64_t hi = lo + kCdfBlock < N ? lo + kCdfBlock : N;
-      cdf_exact_range<R>(a, lo, hi, thr, ck, &s_sh, &x_sh, wsum, wred);
-      if (tid == 0) c_sh = stop + 1;
-    } else if (tid == 0) {
-      c_sh = stop;
     }
+    if (tid == 0) at_sh = 0;
     __syncthreads();
+    for (;;) {
+      const uint32_t c = at_sh;
+      const double s = sum_sh;
+      if (c >= len) break;
+      turn ^= 1;
+      int e = 0;
+      long long S0 = 0;
+      if (s > 0.0) {
+        frexp(s, &e);
+        S0 = (long long)scaled(s, 53 - e);
+      }
+      uint32_t stop = NONE;  // this thread's first block that is not taken whole
+      long long dv[kCdfWalkPer];
+      long long tsum = 0;
+#pragma unroll
+      for (int k = 0; k < kCdfWalkPer; k++) {
+        const uint32_t j = j0 + k;
+        dv[k] = 0;
+        if (j < c || j >= len || stop != NONE || st[k] == kBlkEmpty) continue;
+        if (st[k] == kBlkClean && s > 0.0 && eb[k] == e) dv[k] = D[k];
+        else stop = j;
+        tsum += dv[k];
+      }
+      const long long S1 = S0 + walk_scan(tsum, sh.scan[turn]);  // (blocks of one binade: no overflow)
+      long long Sr = S1;
+#pragma unroll
+      for (int k = 0; k < kCdfWalkPer; k++) {
+        const uint32_t j = j0 + k;
+        if (j < c || j >= len || j >= stop) continue;
+        if (Sr + dv[k] >= kTwo53) { stop = j; continue; }  // the sum reaches 2^53 u
+        Sr += dv[k];
+      }
+      stop = min(walk_min(stop, sh.red[turn]), len);
+      // blocks before `stop` are taken whole
+      Sr = S1;
+#pragma unroll
+      for (int k = 0; k < kCdfWalkPer; k++) {
+        const uint32_t j = j0 + k;
+        if (j < c || j > stop || j >= len) continue;
+        const double before = s > 0.0 ? scaled((double)Sr, e - 53) : 0.0;
+        bstart[win + j] = before;
+        if (j == stop) {
+          bst[win + j] = kBlkExact;
+          ck[(win + j) * kCdfSubPerBlock] = before;
+          sh.s = before;
+          continue;
+        }
+        Sr += dv[k];
+        if (j + 1 == len) sum_sh = s > 0.0 ? scaled((double)Sr, e - 53) : 0.0;  // (stop == len)
+      }
+      __syncthreads();
+      if (stop < len) {
+        // block `stop` entry by entry
+        const uint64_t lo = (win + stop) * kCdfBlock;
+        cdf_exact_range<R>(a, lo, lo + kCdfBlock < N ? lo + kCdfBlock : N, thr, ck, sh, turn);
+        if (tid == 0) {
+          sum_sh = sh.s;
+          at_sh = stop + 1;
+        }
+      } else if (tid == 0) {
+        at_sh = len;
+      }
+      __syncthreads();
+    }
+    __syncthreads();  // (at_sh is reset for the next window)
   }
-  if (tid == 0) ck[nk] = s_sh;
+  if (tid == 0) ck[nk] = sum_sh;
 }
 
 // Checkpoints of the blocks taken whole: the exact start plus the sub-chunk's
@@ -1239,7 +1287,7 @@ static cudaError_t sample_t(const void* amp, int n, double thr, const double* r,
   k_cdf_block_sums<R><<<(unsigned)nb, 256, 0, s>>>(a, N, thr, c.bsum, c.bfirst, c.blast);
   k_cdf_block_prefix<<<1, kCdfThreads, 0, s>>>(c.bsum, c.bfirst, c.blast, nb, c.fl);
   k_cdf_block_d<R><<<(unsigned)nb, 256, 0, s>>>(a, N, thr, c.bsum, (long long*)c.ck, c.bd, c.bst, c.be);
-  k_cdf_walk<R><<<1, kCdfThreads, 0, s>>>(a, N, thr, nb, nk, c.ck, c.bd, c.bst, c.be, c.bstart);
+  k_cdf_walk<R><<<1, kWalkThreads, 0, s>>>(a, N, thr, nb, nk, c.ck, c.bd, c.bst, c.be, c.bstart);
   k_cdf_fill<<<gridn(nk, 256), 256, 0, s>>>(c.ck, nk, c.bst, c.be, c.bstart);
   k_sample_ck<R><<<gridn(shots, 128), 128, 0, s>>>(a, N, thr, c.ck, nk, r, shots, c.fl, out);
   return cudaGetLastError();
