@@ -183,6 +183,19 @@ void daggerize(const ket_op& op, const double* mats, std::vector<double>& out_ma
 
 }  // namespace
 
+// The probes of the rotation families, marked for the compiled kernels: FOF_REAL
+// on D = [[0, -y], [y, 0]], FOF_RXFORM on D = [[0, i y], [i y, 0]] and on an
+// imaginary diagonal.  The interpreter takes any D in its general form.
+static void mark_probe_form(FOp& f) {
+  const double* m = f.m;  // re, im of the entries, row by row
+  if (f.type == FO_GRADD) {
+    if (m[0] == 0 && m[2] == 0) f.flags |= FOF_RXFORM;
+  } else if (f.type == FO_GRADM && m[0] == 0 && m[1] == 0 && m[6] == 0 && m[7] == 0) {
+    if (m[3] == 0 && m[5] == 0 && m[2] == -m[4]) f.flags |= FOF_REAL;
+    else if (m[2] == 0 && m[4] == 0 && m[3] == m[5]) f.flags |= FOF_RXFORM;
+  }
+}
+
 // Reverse-sweep runner: like run_plan, with gradient probes reduced per pass
 // into slot_out (device, indexed by the probes' global slot).
 // Nothing waits: the probe partials (gpart) and the op images are reused by
@@ -226,7 +239,10 @@ static int run_plan_grad(ket_state* s, Plan& plan, double* slot_out, double* gpa
     plan_program(plan, p, s->precision, false, 4, prog, a.load_pos, a.store_pos);
     // the probes of this pass write slots 0..nprobe-1 (they are consecutive)
     for (FOp& f : prog)
-      if (f.type == FO_GRADM || f.type == FO_GRADD || f.type == FO_GRADM2) f.slot = (int16_t)(f.slot - slot_lo);
+      if (f.type == FO_GRADM || f.type == FO_GRADD || f.type == FO_GRADM2) {
+        f.slot = (int16_t)(f.slot - slot_lo);
+        mark_probe_form(f);
+      }
     a.nreg = 4;  // probes: 256 threads, ancilla on register bit 3
     void* dev;
     size_t fb = sizeof(FOp) * prog.size();

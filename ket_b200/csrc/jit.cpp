@@ -180,20 +180,35 @@ Driver& driver() {
 const char* real_name(int precision) { return precision == KET_C64 ? "float" : "double"; }
 
 // The lane or thread-id bit that lane ops and thread diagonals take as a
-// template argument (0 for other ops).
+// template argument, and a diagonal probe's target (0 for other ops).
 int static_lane(const FOp& f) {
-  return (f.opc >= OC_MAT1L && f.opc < OC_MAT1L + 3) || f.opc == OC_X1L || f.opc == OC_DIAGT ? f.a : 0;
+  return (f.opc >= OC_MAT1L && f.opc < OC_MAT1L + 3) || f.opc == OC_X1L || f.opc == OC_DIAGT || f.opc == OC_GRADD ? f.a : 0;
 }
 
 // Stages of the staged form: one per tile group and one in flight (64 KB
 // each at complex128, 32 KB at complex64).
 int stage_count(int) { return 3; }
 
-// A program with adjoint probes: its kernel keeps per-CTA probe sums.
-bool has_probes(const FOp* prog, int nops) {
-  for (int k = 0; k < nops; k++)
-    if (prog[k].type != FO_CONT && prog[k].opc >= OC_GRADM && prog[k].opc <= OC_GRADM2) return true;
-  return false;
+// The adjoint probes of a program: its kernel keeps their sums per CTA.
+bool is_probe(const FOp& f) { return f.type != FO_CONT && f.opc >= OC_GRADM && f.opc <= OC_GRADM2; }
+int count_probes(const FOp* prog, int nops) {
+  int c = 0;
+  for (int k = 0; k < nops; k++) c += is_probe(prog[k]);
+  return c;
+}
+
+// Up to this many probes a pass keep a sum for each of the CTA's 256 threads
+// (48 KB; with the exchange buffer two CTAs fill an SM's shared memory).
+constexpr int kProbeThreadSlots = 24, kProbeThreads = 256;
+// Sums a probe: one for each thread, or one for each warp.
+int probe_stride(int probes) { return probes <= kProbeThreadSlots ? kProbeThreads : 8; }
+constexpr int kProbeBytesMax = (int)sizeof(double) * (kProbeThreadSlots * kProbeThreads > KET_JIT_MAX_PROBES * 8
+                                                          ? kProbeThreadSlots * kProbeThreads
+                                                          : KET_JIT_MAX_PROBES * 8);
+
+// The flags that select an op's code.
+unsigned code_flags(const FOp& f) {
+  return f.flags & (is_probe(f) ? FOF_REAL | FOF_RXFORM | FOF_TGT_THR | FOF_TGT_CTX : FOF_PRUNE | FOF_D0ONE | FOF_SW);
 }
 
 std::string make_source(const FOp* prog, int nops, int precision, int NR, bool staged) {
@@ -202,6 +217,8 @@ std::string make_source(const FOp* prog, int nops, int precision, int NR, bool s
   std::string s;
   s.reserve(300 + 96 * (size_t)nops);
   if (staged) s += "#define KET_STAGED_THREADS " + std::to_string(NT) + "\n";
+  const int probes = count_probes(prog, nops);
+  if (probes > 0 && probe_stride(probes) == kProbeThreads) s += "#define KET_PROBE_PER_THREAD " + std::to_string(NT) + "\n";
   s += "#include \"jit_ops.cuh\"\n";
   s += "__constant__ ket::jit::COp c_ops[" + std::to_string(nops > 0 ? nops : 1) + "];\n";
   if (staged) {
@@ -209,7 +226,7 @@ std::string make_source(const FOp* prog, int nops, int precision, int NR, bool s
          ", 1) ket_pass(const ket::Pass2Args a, const __grid_constant__ ket::jit::TMap tm) {\n";
   } else {
     s += "extern \"C\" __global__ void __launch_bounds__(" + std::to_string(NT) +
-         (has_probes(prog, nops) ? ", 2) ket_probe_pass(const ket::Pass2Args a) {\n"
+         (probes > 0 ? ", 2) ket_probe_pass(const ket::Pass2Args a) {\n"
                                  : ", 2) ket_pass(const ket::Pass2Args a) {\n");
   }
   s += "  using namespace ket;\n";
@@ -220,12 +237,12 @@ std::string make_source(const FOp* prog, int nops, int precision, int NR, bool s
          "], SLay<" + std::to_string(NR) + ">& sl, jit::Tile& t) {\n";
   else
     s += std::string("  jit::run_tiles<") + R + ", " + std::to_string(NR) +
-         (has_probes(prog, nops) ? ", true" : ", false") + ">(a, [&](cpx<" + R + "> (&x)[" + std::to_string(1 << NR) +
+         (probes > 0 ? ", true" : ", false") + ">(a, [&](cpx<" + R + "> (&x)[" + std::to_string(1 << NR) +
          "], SLay<" + std::to_string(NR) + ">& sl, jit::Tile& t) {\n";
   for (int k = 0; k < nops; k++) {
     const FOp& f = prog[k];
     if (f.type == FO_CONT || f.opc == OC_NOP) continue;
-    const unsigned fl = f.flags & (FOF_PRUNE | FOF_D0ONE | FOF_SW);
+    const unsigned fl = code_flags(f);
     s += std::string("    jit::step<") + R + ", " + std::to_string(NR) + ", " + std::to_string((int)f.opc) + ", " +
          std::to_string(fl) + ", " + std::to_string((int)f.creg) + ", " + std::to_string((unsigned)f.cthr) + "u, " +
          (f.cctx ? "true" : "false") + ", " + std::to_string(static_lane(f)) + ">(x, sl, c_ops[" + std::to_string(k) +
@@ -245,7 +262,7 @@ std::string shape_key(const FOp* prog, int nops, int precision, int nreg, bool s
       k += '.';
       continue;
     }
-    const unsigned fl = f.flags & (FOF_PRUNE | FOF_D0ONE | FOF_SW);
+    const unsigned fl = code_flags(f);
     char buf[32];
     snprintf(buf, sizeof buf, "%x,%x,%x,%x,%d,%d;", (unsigned)f.opc, fl, (unsigned)f.creg, (unsigned)f.cthr,
              f.cctx ? 1 : 0, static_lane(f));
@@ -259,7 +276,7 @@ std::string shape_key(const FOp* prog, int nops, int precision, int nreg, bool s
 struct Entry {
   enum { QUEUED, BUSY, READY, FAILED } st = QUEUED;
   bool staged = false;
-  bool grad = false;  // adjoint probe pass (per-CTA probe sums after the exchange buffer)
+  int probes = 0;     // adjoint probe pass: its probes (their sums follow the exchange buffer)
   std::string src, log;
   std::vector<char> cubin;
   // (device, stream) -> the kernel loaded for it: each stream owns a module
@@ -365,7 +382,7 @@ std::vector<std::string> enqueue(Cache& C, const std::vector<JitPass>& passes, i
       Entry& e = C.map[keys[i]];
       e.src = make_source(p.prog, p.nops, precision, p.nreg, p.staged);
       e.staged = p.staged;
-      e.grad = !p.staged && has_probes(p.prog, p.nops);
+      e.probes = p.staged ? 0 : count_probes(p.prog, p.nops);
       if (const char* dir = getenv("KET_JIT_DUMP")) {  // kernel sources, for inspection
         const std::string path = std::string(dir) + "/ket_pass_" + std::to_string(C.map.size()) + ".cu";
         if (FILE* fp = fopen(path.c_str(), "w")) {
@@ -455,19 +472,19 @@ int jit_prepare(const std::vector<JitPass>& passes, int precision, int mode, cud
       CUfunction fn;
       CUdeviceptr cops = 0;
       size_t cbytes = 0;
-      if (D.load(&mod, e.cubin.data()) != CUDA_SUCCESS || D.get(&fn, mod, e.grad ? "ket_probe_pass" : "ket_pass") != CUDA_SUCCESS ||
+      if (D.load(&mod, e.cubin.data()) != CUDA_SUCCESS || D.get(&fn, mod, e.probes ? "ket_probe_pass" : "ket_pass") != CUDA_SUCCESS ||
           D.global(&cops, &cbytes, mod, "c_ops") != CUDA_SUCCESS) {
         if (mode == 1) return err = "loading a run-time compiled pass kernel failed", KET_ERR_CUDA;
         continue;
       }
-      const int smem = pass_smem(precision, e.staged) + (e.grad ? 64 * KET_JIT_MAX_PROBES : 0);
+      const int smem = pass_smem(precision, e.staged) + (e.probes ? kProbeBytesMax : 0);
       if (D.attr(fn, CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES, smem) != CUDA_SUCCESS) {
         if (mode == 1) return err = "setting the shared memory of a pass kernel failed", KET_ERR_CUDA;
         continue;
       }
       JitFn j;
       j.staged = e.staged;
-      j.grad = e.grad;
+      j.probes = e.probes;
       j.fn = (void*)fn;
       j.cops = (unsigned long long)cops;
       j.cops_bytes = cbytes;
@@ -562,11 +579,13 @@ cudaError_t jit_launch(const JitFn& f, const Pass2Args& in, int precision, cudaS
                         nullptr);
   } else {
     // two CTAs per SM at either register-bit count (__launch_bounds__(NT, 2));
-    // probe passes add their per-(slot, warp) sums after the exchange buffer
-    if (f.grad && (a.nslots < 1 || a.nslots > KET_JIT_MAX_PROBES)) return cudaErrorInvalidValue;
+    // probe passes keep their sums after the exchange buffer
+    if (f.probes && (a.nslots < f.probes || a.nslots > KET_JIT_MAX_PROBES)) return cudaErrorInvalidValue;
+    const int psums = f.probes ? (int)sizeof(double) * a.nslots * probe_stride(f.probes) : 0;
+    if (psums > kProbeBytesMax) return cudaErrorInvalidValue;
     const unsigned blocks = jit_grid(a.n);
     void* params[1] = {&a};
-    r = driver().launch((CUfunction)f.fn, blocks, 1, 1, 32 << (7 - a.nreg), 1, 1, smem + (f.grad ? 64 * a.nslots : 0),
+    r = driver().launch((CUfunction)f.fn, blocks, 1, 1, 32 << (7 - a.nreg), 1, 1, smem + psums,
                         (CUstream)s, params, nullptr);
   }
   {

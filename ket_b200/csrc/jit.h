@@ -43,7 +43,7 @@ int tiled_nreg(int nqubits, int reg_bits = 0);
 
 struct JitFn {
   bool staged = false;              // the staged form (one CTA per SM, two tile groups, TMA copies)
-  bool grad = false;                // an adjoint probe pass
+  int probes = 0;              // adjoint probe pass: its probes
   void* fn = nullptr;               // CUfunction, null = run the interpreter
   unsigned long long cops = 0;      // device address of the kernel's constant op array
   size_t cops_bytes = 0;

@@ -119,7 +119,7 @@ struct Tile {
   int tid, lane, warp;
   int ltid;       // logical thread id: tid with the lane bits moved by deferred lane X gates (FOF_SW on FO_X1L)
   uint64_t ctx0;  // global index bits of the tile outside its 12 bits
-  double* sgrad;  // adjoint probe passes: the CTA's partial sums [slot][warp] in shared memory
+  double* sgrad;  // adjoint probe passes: partial sums in shared memory, [slot][thread] or [slot][warp] (probe_add)
   uint32_t sw;    // deferred register swaps (FOF_SW): physical slot j holds logical slot j ^ sw
   uint32_t bar;   // staged form: the named barrier of the tile's thread group
   uint32_t xbar;  // register form: mbarrier on which the warps announce their reads of the exchange buffer
@@ -198,6 +198,65 @@ __device__ __forceinline__ void realize_swaps(cpx<R> (&x)[1 << NR], Tile& t) {
   t.sw &= ~(uint32_t)M;
 }
 
+// Add a thread's share of an adjoint probe to its partial sum.  With up to
+// KET_PROBE_THREAD_SLOTS probes (KET_PROBE_PER_THREAD) every thread keeps its own
+// sum a probe in shared memory, one read and one write nothing waits for, and the
+// threads' sums meet once, after the last tile; a warp sum a probe and tile was a
+// chain of five shuffles and additions that four warps a scheduler did not hide.
+// More probes (two CTAs' sums no longer fit an SM) take the warp sums.  With the
+// forms below, a 24-qubit probe pass (25 qubits with the ancilla, 10 to 21 probes):
+// 458 -> 349 us.  Bound now: latency at 16 warps an SM (FP64 pipe 41%, HBM 36%).
+__device__ __forceinline__ void probe_add(const Tile& t, int slot, double v) {
+#ifdef KET_PROBE_PER_THREAD
+  t.sgrad[slot * KET_PROBE_PER_THREAD + t.tid] += v;
+#else
+  grad_accum(t.sgrad, slot, t.warp, t.lane, v);
+#endif
+}
+
+// Probes of the rotation families (D known up to its scale), 4 FMAs a pair of psi
+// and the pair of lambda where the general 2x2 takes 20 operations:
+// D = [[0, -y], [y, 0]] (Ry) sums conj(l1) x0 - conj(l0) x1, real part;
+// D = [[0, i y], [i y, 0]] (Rx) sums the real part of i (conj(l0) x1 + conj(l1) x0).
+// Two chains each.
+template <int A, bool RX>
+__device__ __forceinline__ double probe_rot(const cpx<double>* x, double y, uint32_t smask) {
+  double a = 0.0, b = 0.0;
+#pragma unroll
+  for (int j = 0; j < 8; j++) {
+    if ((j >> A) & 1) continue;
+    if (!((smask >> j) & 1)) continue;
+    const cpx<double>&x0 = x[j], &x1 = x[j | (1 << A)], &l0 = x[j + 8], &l1 = x[(j | (1 << A)) + 8];
+    if constexpr (RX) {
+      a = fma(l0.im, x1.re, a);
+      b = fma(l0.re, -x1.im, b);
+      a = fma(l1.im, x0.re, a);
+      b = fma(l1.re, -x0.im, b);
+    } else {
+      a = fma(l1.re, x0.re, a);
+      b = fma(l0.re, -x1.re, b);
+      a = fma(l1.im, x0.im, a);
+      b = fma(l0.im, -x1.im, b);
+    }
+  }
+  return y * (a + b);
+}
+// D = diag(i y0, i y1) (Rz, U1): the real part of i conj(l) x by target bit, 2 FMAs
+// an amplitude of psi and of lambda (6 operations with a general diagonal).  A < 0: one
+// value of the target bit for the thread, in y0.
+template <int A>
+__device__ __forceinline__ double probe_phase(const cpx<double>* x, double y0, double y1, uint32_t smask) {
+  double s[2] = {0.0, 0.0};
+#pragma unroll
+  for (int j = 0; j < 8; j++) {
+    if (!((smask >> j) & 1)) continue;
+    const int k = A >= 0 ? (j >> (A < 0 ? 0 : A)) & 1 : j & 1;  // (two chains in either case)
+    s[k] = fma(x[j + 8].im, x[j].re, s[k]);
+    s[k] = fma(x[j + 8].re, -x[j].im, s[k]);
+  }
+  return A >= 0 ? y0 * s[0] + y1 * s[1] : y0 * (s[0] + s[1]);
+}
+
 // Rare ops on the shared-memory copy of the tile, as in k_fused2.
 template <typename R, int NR, int OPC, int FL>
 __device__ __forceinline__ void smem_op(cpx<R> (&x)[1 << NR], const SLay<NR>& sl, const FOp* op, Tile& t) {
@@ -245,7 +304,7 @@ __device__ __forceinline__ void smem_op(cpx<R> (&x)[1 << NR], const SLay<NR>& sl
         acc += (double)lam.re * (s0.re + s1.re) + (double)lam.im * (s0.im + s1.im);
       }
     }
-    grad_accum(t.sgrad, slot, t.warp, t.lane, acc);
+    probe_add(t, slot, acc);
     xbuf_release(t);
     return;
   } else if constexpr (OPC == OC_X1S) {
@@ -358,21 +417,23 @@ __device__ __forceinline__ void step(cpx<R> (&x)[1 << NR], SLay<NR>& sl, const C
     double acc;
     if constexpr (OPC == OC_GRADD) {
       const R d0r = (R)c.m[0], d0i = (R)c.m[1], d1r = (R)c.m[2], d1i = (R)c.m[3];
-      if (c.flags & (FOF_TGT_THR | FOF_TGT_CTX)) {
-        const bool one = (c.flags & FOF_TGT_CTX) ? (t.ctx0 & c.dg0) != 0 : (bool)((t.ltid >> c.a) & 1);
-        acc = grad_d<R, -1>(x, one ? d1r : d0r, one ? d1i : d0i, one ? d1r : d0r, one ? d1i : d0i, smask);
-      } else if (c.a == 0) {
-        acc = grad_d<R, 0>(x, d0r, d0i, d1r, d1i, smask);
-      } else if (c.a == 1) {
-        acc = grad_d<R, 1>(x, d0r, d0i, d1r, d1i, smask);
+      constexpr bool PH = (FL & FOF_RXFORM) != 0;  // an imaginary diagonal
+      if constexpr ((FL & (FOF_TGT_THR | FOF_TGT_CTX)) != 0) {
+        const bool one = (FL & FOF_TGT_CTX) ? (t.ctx0 & c.dg0) != 0 : (bool)((t.ltid >> LA) & 1);
+        if constexpr (PH) acc = probe_phase<-1>(x, one ? d1i : d0i, 0.0, smask);
+        else acc = grad_d<R, -1>(x, one ? d1r : d0r, one ? d1i : d0i, one ? d1r : d0r, one ? d1i : d0i, smask);
+      } else if constexpr (PH) {
+        acc = probe_phase<LA>(x, d0i, d1i, smask);
       } else {
-        acc = grad_d<R, 2>(x, d0r, d0i, d1r, d1i, smask);
+        acc = grad_d<R, LA>(x, d0r, d0i, d1r, d1i, smask);
       }
+    } else if constexpr ((FL & (FOF_REAL | FOF_RXFORM)) != 0) {
+      acc = probe_rot<OPC - OC_GRADM, (FL & FOF_RXFORM) != 0>(x, (FL & FOF_RXFORM) ? c.m[3] : c.m[4], smask);
     } else {
       const R d[8] = {(R)c.m[0], (R)c.m[1], (R)c.m[2], (R)c.m[3], (R)c.m[4], (R)c.m[5], (R)c.m[6], (R)c.m[7]};
       acc = grad_m<R, OPC - OC_GRADM>(x, d, smask);
     }
-    grad_accum(t.sgrad, c.slot, t.warp, t.lane, acc);
+    probe_add(t, c.slot, acc);
     return;
   }
   if constexpr (CTHR != 0) {
@@ -512,8 +573,8 @@ __device__ __forceinline__ void store_tile(char* p, const uint64_t* rb, uint32_t
 
 // The tile loop around a program: load each tile in the load layout, run the
 // ops, store it in the store layout -- the same addressing as k_fused2.
-// GRAD: an adjoint probe pass; its probes add into per-(slot, warp) partial
-// sums in shared memory after the exchange buffer, written to a.gpart per CTA
+// GRAD: an adjoint probe pass; its probes add into partial sums in shared memory
+// after the exchange buffer (probe_add), written to a.gpart per CTA, slot and warp
 // at the end (k_grad_reduce adds them in a fixed order).
 template <typename R, int NR, bool GRAD = false, typename Body>
 __device__ __forceinline__ void run_tiles(const Pass2Args& a, Body body) {
@@ -534,8 +595,14 @@ __device__ __forceinline__ void run_tiles(const Pass2Args& a, Body body) {
     mbar_init(t.xbar, NT / 32);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+#ifdef KET_PROBE_PER_THREAD
+  static_assert(!GRAD || NT == KET_PROBE_PER_THREAD, "one sum a thread and slot");
+  constexpr int GW = NT;
+#else
+  constexpr int GW = 8;
+#endif
   if constexpr (GRAD)
-    for (int i = t.tid; i < a.nslots * 8; i += NT) t.sgrad[i] = 0.0;
+    for (int i = t.tid; i < a.nslots * GW; i += NT) t.sgrad[i] = 0.0;
   __syncthreads();
   char* const amp = reinterpret_cast<char*>(a.amp);
   const uint64_t ntiles = uint64_t(1) << (a.n - KET_T2_BITS);
@@ -552,6 +619,19 @@ __device__ __forceinline__ void run_tiles(const Pass2Args& a, Body body) {
       gl += a.lgb[5 + r];
       gs += a.sgb[5 + r];
     }
+  // Probe passes prefetch the next tile into L2, each thread its 128-byte lines: at
+  // 4 register bits there are registers left for the addresses (24 qubits 349 -> 339
+  // us; the ordinary pass at 5 register bits got slower, 285 -> 306).
+  constexpr int kLineAmps = 128 / (int)sizeof(V), kLines = GRAD ? (1 << KET_T2_BITS) / kLineAmps / NT : 0;
+  uint64_t line[GRAD ? kLines : 1];
+#pragma unroll
+  for (int i = 0; i < kLines; i++) {
+    const uint32_t k = (uint32_t)(t.tid * kLines + i) * kLineAmps;
+    uint64_t idx = k & ((1u << a.L) - 1);
+    for (int e = 0; e < a.nh; e++)
+      if ((k >> (a.L + e)) & 1) idx |= uint64_t(1) << a.hbits[e];
+    line[i] = idx * sizeof(V);
+  }
   cpx<R> x[NS];
   for (uint64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
     t.ctx0 = ctx_of(a, tile);
@@ -566,6 +646,11 @@ __device__ __forceinline__ void run_tiles(const Pass2Args& a, Body body) {
         x[j] = ld_amp<R>(reinterpret_cast<const V*>(p + o));
       }
     }
+    if (GRAD && tile + gridDim.x < ntiles) {
+      const char* p = amp + ctx_of(a, tile + gridDim.x) * sizeof(V);
+#pragma unroll
+      for (int i = 0; i < kLines; i++) asm volatile("prefetch.global.L2 [%0];" ::"l"(p + line[i]));
+    }
     SLay<NR> sl = make_slay<NR>(a.lbx, t.lane, t.warp);
     t.sw = 0;
     t.ltid = t.tid;
@@ -573,8 +658,15 @@ __device__ __forceinline__ void run_tiles(const Pass2Args& a, Body body) {
     store_tile<R, NR>(amp + t.ctx0 * sizeof(V) + logical_base(gs, a.sgb, t), a.sgb + 5 + NW, t.sw, x);
   }
   if constexpr (GRAD) {
+#ifdef KET_PROBE_PER_THREAD
+    for (int s = 0; s < a.nslots; s++) {
+      const double v = warp_sum(t.sgrad[s * GW + t.tid]);
+      if (t.lane == 0) a.gpart[((size_t)blockIdx.x * a.nslots + s) * 8 + t.warp] = v;
+    }
+#else
     __syncthreads();
     for (int i = t.tid; i < a.nslots * 8; i += NT) a.gpart[(size_t)blockIdx.x * a.nslots * 8 + i] = t.sgrad[i];
+#endif
   }
 }
 
