@@ -583,6 +583,7 @@ int ket_adjoint_gradient(ket_ctx* ctx, int n, uint64_t init, const ket_op* ops, 
       if (rc) { cleanup(); return fail(rc, err); }
       if (fp.gates.empty()) continue;
       plan_passes(n, KET_C128, -1, false, fp);
+      if (specialize == 1) split_long_passes(n, KET_C128, false, tiled_nreg(n, 0), fp);
       tick(1);
       rc = run_plan(&w.psi, fp, fo, false);
       if (rc) { cleanup(); return rc; }
@@ -678,6 +679,7 @@ int ket_adjoint_gradient(ket_ctx* ctx, int n, uint64_t init, const ket_op* ops, 
       if (bp.gates.empty()) continue;
       tick(4);
       plan_passes(n + 1, KET_C128, -1, false, bp);
+      if (specialize == 1) split_long_passes(n + 1, KET_C128, false, 4, bp);
       tick(5);
       // probes must stay in order within each pass: slots are consecutive per pass by construction
       rc = run_plan_grad(&w.full, bp, slots_b, w.gpart, w.gpart_cap, specialize);

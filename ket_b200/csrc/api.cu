@@ -153,7 +153,7 @@ int ctx_finish(ket_ctx* c) {
   return KET_OK;
 }
 
-// Circuits of up to kSmallQubits qubits whose kernels were compiled ahead
+// Circuits below KET_JIT_AUTO_QUBITS qubits whose kernels were compiled ahead
 // (ket_jit_compile): they run on those kernels, as the default policy promises.
 // Known by a hash of their ops' kinds and qubits; like the kernels, kept until the
 // process ends.
@@ -513,6 +513,7 @@ int ket_jit_compile(int n, int precision, const ket_op* ops, size_t nops, const 
   if (rc) return fail(rc, err);
   if (o.fusion != 0) fold_single_qubit(plan.gates, o.prune != 0);
   plan_passes(n, precision, o.fusion, o.prune != 0, plan);
+  split_long_passes(n, precision, o.prune != 0, tiled_nreg(n, o.reg_bits), plan);
   std::vector<std::vector<FOp>> progs;
   std::vector<std::vector<uint8_t>> lps;
   for (auto& p : plan.passes) {
@@ -528,7 +529,7 @@ int ket_jit_compile(int n, int precision, const ket_op* ops, size_t nops, const 
                          use_staged(n, o.stage)});
   std::string clog;
   rc = jit_compile(jp, precision, kernels, clog);
-  if (!rc && n <= kSmallQubits && !jp.empty()) note_ahead(circuit_hash(n, precision, o.prune != 0, ops, nops));
+  if (!rc && n < KET_JIT_AUTO_QUBITS && !jp.empty()) note_ahead(circuit_hash(n, precision, o.prune != 0, ops, nops));
   if (log && logcap) {
     strncpy(log, clog.c_str(), logcap - 1);
     log[logcap - 1] = 0;
@@ -549,15 +550,20 @@ int ket_apply_ops(ket_state* s, const ket_op* ops, size_t nops, const double* ma
   if (rc) return fail(rc, err);
   if (o.fusion != 0) fold_single_qubit(plan.gates, o.prune != 0);
   if (plan.gates.empty()) return KET_OK;
+  const bool ahead = o.specialize == 0 && s->n < KET_JIT_AUTO_QUBITS &&
+                     compiled_ahead(s->n, s->precision, o.prune != 0, ops, nops);
   // Small complex128 states, with everything automatic, run in one launch.
   if (s->precision == KET_C128 && s->n <= kSmallQubits && o.fusion < 0 && o.specialize == 0 && o.reg_bits == 0 && o.stage == 0 &&
-      !compiled_ahead(s->n, s->precision, o.prune != 0, ops, nops)) {
+      !ahead) {
     bool ran = false;
     rc = run_small(s, plan.gates, o.prune != 0, &ran);
     if (rc) return rc;
     if (ran) return ctx_finish(s->ctx);
   }
   plan_passes(s->n, s->precision, o.fusion, o.prune != 0, plan);
+  // (the interpreter's code does not grow with the pass: it takes whole passes)
+  if (o.specialize == 1 || ahead || (o.specialize == 0 && s->n >= KET_JIT_AUTO_QUBITS))
+    split_long_passes(s->n, s->precision, o.prune != 0, tiled_nreg(s->n, o.reg_bits), plan);
   return run_plan(s, plan, o);
 }
 

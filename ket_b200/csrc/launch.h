@@ -49,6 +49,10 @@ void fill_pass2_offsets(Pass2Args& a, int precision);
 // reads as a control or a diagonal target, or -1.
 int choose_pairbit(const std::vector<FOp>& prog, const Pass2Args& a);
 
+// Cut the passes whose compiled kernels would be longer than the instruction
+// cache holds (program.cpp) at gate boundaries, each part a pass of the same tile.
+void split_long_passes(int n, int precision, bool prune, int nreg, Plan& plan);
+
 // Lower one fused pass to a register-tiled program (segments + exchanges).
 void plan_program(const Plan& plan, const Pass& p, int precision, bool prune, int nreg, std::vector<FOp>& prog,
                   uint8_t load_pos[KET_T2_BITS], uint8_t store_pos[KET_T2_BITS]);

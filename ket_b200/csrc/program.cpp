@@ -972,4 +972,90 @@ void plan_program(const Plan& plan, const Pass& p, int precision, bool prune, in
   for (FOp& o : prog) assign_opcode(o);
 }
 
+
+// ---------------------------------------------------------------- code size
+namespace {
+
+// Machine instructions of an op in a compiled kernel, roughly: what it does to
+// each of the thread's 2^nreg amplitudes, unrolled.
+int code_estimate(const FOp& f, int nreg, int precision) {
+  const int ns = 1 << nreg, words = precision == KET_C64 ? 2 : 4;  // 32-bit words an amplitude (shuffles, selects)
+  const bool plain = f.flags & (FOF_REAL | FOF_RXFORM);
+  const int prune = f.flags & FOF_PRUNE ? 6 * ns : 0;
+  switch (f.type) {
+    case FO_CONT: case FO_X1R: case FO_RELAY: case FO_SYNC: return 8;
+    case FO_EXCH: return 2 * ns + 100;
+    case FO_MAT1R: return (plain ? 4 : 8) * ns + prune;
+    case FO_MAT1L: return (plain ? 4 : 8) * ns + words * ns + prune;
+    case FO_X1L: return f.flags & FOF_SW ? 8 : words * ns;
+    case FO_DIAGR: return (f.flags & FOF_D0ONE ? 2 : 4) * ns;
+    case FO_DIAGT: case FO_DIAGX: return 4 * ns + 8;
+    case FO_REAL: return words * ns;
+    case FO_CPHASE: case FO_PPOLY: return 4 * ns + 200;
+    case FO_GRADM: return plain ? 24 : 96;
+    case FO_GRADD: return plain ? 24 : 56;
+    default: return 4 * ns + 150;  // through shared memory
+  }
+}
+
+// A gate's share of its pass's code.
+double code_weight(const Gate& g) {
+  switch (g.type) {
+    case G_X1: case G_SWAP: return 0.5;
+    case G_GRADM: case G_GRADD: return 0.5;
+    case G_DIAG1: case G_DIAG2: return 4;
+    default: return 6;
+  }
+}
+
+}  // namespace
+
+// A compiled kernel is straight-line code run once a tile; one longer than the
+// instruction cache is fetched again for every tile.  A 24-qubit pass of 99 ops (11
+// exchanges) spent half its issue slots without an instruction, 990 us where two
+// passes of half its ops take 304 and 280; an extra pass costs a read and a write of
+// the state, 82 us.  So passes are cut into equal parts of at most kCodeLimit
+// instructions of 16 bytes, 128 KB; limits of 6000 to 9000 measured alike, 5000 and
+// less slower.  The gradient of 8 parameter vectors at 24 qubits: 127 -> 121 ms on
+// the device; a 25-qubit complex64 circuit of mixed gates 3.82 -> 3.67 ms.
+void split_long_passes(int n, int precision, bool prune, int nreg, Plan& plan) {
+  constexpr int kCodeLimit = 8000;
+  std::vector<Pass> out;
+  std::vector<FOp> prog;
+  uint8_t lp[KET_T2_BITS], sp[KET_T2_BITS];
+  for (Pass& p : plan.passes) {
+    double w = 0;
+    for (int gi : p.gates) w += code_weight(plan.gates[gi]);
+    // (a gate's code with its share of the exchanges is below 4 weights a slot)
+    if (!(p.fused && p.m == KET_T2_BITS && n >= KET_T2_BITS) || 4 * w * (1 << nreg) < kCodeLimit) {
+      out.push_back(std::move(p));
+      continue;
+    }
+    plan_program(plan, p, precision, prune, nreg, prog, lp, sp);
+    int code = 0;
+    bool merged = false;
+    for (const FOp& f : prog) {
+      code += code_estimate(f, nreg, precision);
+      merged = merged || f.type == FO_CPHASE || f.type == FO_PPOLY;
+    }
+    // (a cut between phases that merge into one op would change their rounding)
+    const int parts = merged ? 1 : (code + kCodeLimit - 1) / kCodeLimit;
+    double at = 0;
+    int part = 0;
+    Pass q = p;
+    q.gates.clear();
+    for (int gi : p.gates) {
+      if (part + 1 < parts && at >= w * (part + 1) / parts && !q.gates.empty()) {
+        out.push_back(q);
+        q.gates.clear();
+        part++;
+      }
+      q.gates.push_back(gi);
+      at += code_weight(plan.gates[gi]);
+    }
+    out.push_back(std::move(q));
+  }
+  plan.passes.swap(out);
+}
+
 }  // namespace ket
