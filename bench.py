@@ -572,13 +572,14 @@ def vqe24_measure():
 def qaoa_flops_bytes(n, p, tile=12):
     """FP64 flops and HBM bytes of one batch QAOA instance as k_batch_qaoa runs
     it: per layer the cost phase (a complex multiply, 6 flops per amplitude)
-    and Rx on every qubit (6 flops per amplitude each), then the <C>
-    reduction (3 flops per amplitude).  Instances of up to `tile` qubits live
-    in shared memory (no HBM bytes); wider ones run 2p passes over HBM, the
-    first writing and the last reading the state once, the others both."""
+    and Rx on every qubit (without its scalar factor, two FMAs or 4 flops per
+    amplitude each), then the <C> reduction (3 flops per amplitude).  Instances
+    of up to `tile` qubits live in shared memory (no HBM bytes); wider ones run
+    p + 1 passes over HBM, the first writing and the last reading the state
+    once, the others both."""
     N = 2.0 ** n
-    flops = p * N * (6 + 6 * n) + 3 * N
-    hbm = 0.0 if n <= tile else (2 * p - 1) * 2 * 16 * N
+    flops = p * N * (6 + 4 * n) + 3 * N
+    hbm = 0.0 if n <= tile else 2 * p * 16 * N
     return flops, hbm
 
 

@@ -96,7 +96,10 @@ typedef struct ket_exec_opts {
                           the interpreter otherwise, compiling on background threads for states of
                           26+ qubits; 1 = compile what is
                           missing first, then use compiled kernels only; -1 = interpreter only.
-                          Results are identical either way.  No counterpart in the reference. */
+                          Results are identical either way.  With every option automatic, a
+                          complex128 circuit of up to 20 qubits whose kernels were not compiled
+                          ahead runs in one launch instead, equal to these to rounding.  No
+                          counterpart in the reference. */
   int32_t reg_bits;    /* register bits of the compiled kernels' programs: 0 = automatic (default:
                           5 below 26 qubits, 4 from there on), 4 or 5 = that count at any size, so
                           that the programs large states run can be checked on small ones.  The
@@ -215,7 +218,9 @@ KET_API int ket_apply_ops(ket_state* st, const ket_op* ops, size_t nops, const d
 
 /* Planner statistics for an op list on an n-qubit state without launching
  * anything (no GPU needed): passes[0] = fused tile passes, passes[1] = single-
- * gate passes, passes[2] = gates absorbed.  Used by host-side tests. */
+ * gate passes, passes[2] = gates absorbed.  Compiled kernels run a pass too long for
+ * the instruction cache in several parts, which count as one here.  Used by
+ * host-side tests. */
 KET_API int ket_plan_stats(int nqubits, int precision, const ket_op* ops, size_t nops, const double* mats, size_t nmat,
                    const ket_exec_opts* opts, int64_t passes[3]);
 
@@ -433,7 +438,8 @@ typedef struct ket_batch_template {
  * energy[i] = sum_t coeff_t <psi_i|P_t|psi_i>, as a parameter sweep of
  * vqe(ansatz(params), H) would, one call per instance.  Templates may differ in
  * qubit count, gates and Hamiltonian.  All instances run in one persistent
- * launch (one CTA per instance with its state in shared memory, widest first);
+ * launch (one CTA per instance, or per pack of narrow instances of one template,
+ * with its state in shared memory, widest first);
  * with use_graph = 1 the launch is captured in a CUDA graph that later calls of
  * the same shape replay.  Ops: single, controlled, two, unitary of 1-2 qubits,
  * cnot, swap, toffoli, cswap, csrswap, barrier. */

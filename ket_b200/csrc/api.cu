@@ -156,7 +156,7 @@ int ctx_finish(ket_ctx* c) {
 // Circuits below KET_JIT_AUTO_QUBITS qubits whose kernels were compiled ahead
 // (ket_jit_compile): they run on those kernels, as the default policy promises.
 // Known by a hash of their ops' kinds and qubits; like the kernels, kept until the
-// process ends.
+// process ends, and bounded (a circuit past the bound takes the other route).
 namespace {
 std::mutex g_ahead_mu;
 std::unordered_set<uint64_t> g_ahead;
@@ -173,7 +173,7 @@ uint64_t circuit_hash(int n, int precision, bool prune, const ket_op* ops, size_
 }
 void note_ahead(uint64_t h) {
   std::lock_guard<std::mutex> lk(g_ahead_mu);
-  g_ahead.insert(h);
+  if (g_ahead.size() < 65536) g_ahead.insert(h);
   g_any_ahead.store(true);
 }
 bool compiled_ahead(int n, int precision, bool prune, const ket_op* ops, size_t nops) {
