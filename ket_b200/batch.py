@@ -81,10 +81,18 @@ def batch_vqe(templates, instances, use_graph: bool = True) -> np.ndarray:
     if it.min() < 0 or it.max() >= len(templates):
         bad = it[(it < 0) | (it >= len(templates))][0]
         raise RangeError(f"instance template index {bad} out of range")
-    lens = np.fromiter(map(len, params), dtype=np.int64, count=len(params))
-    nparams = int(lens.max())
-    used, at = np.unique(it, return_index=True)
-    first = {int(t): params[i] for t, i in zip(used, at)}
+    few = len(instances) <= 64  # (where an array operation costs more than a loop)
+    if few:
+        lens = [len(v) for v in params]
+        nparams = max(lens)
+        first = {}
+        for t, v in instances:
+            first.setdefault(int(t), v)
+    else:
+        lens = np.fromiter(map(len, params), dtype=np.int64, count=len(params))
+        nparams = int(lens.max())
+        used, at = np.unique(it, return_index=True)
+        first = {int(t): params[i] for t, i in zip(used, at)}
     tmpl = (ket_batch_template * max(1, len(templates)))()
     all_ops, all_mats, all_binds, coeffs, pauli = [], [], [], [], []
     nops = nmats = nbinds = npauli = 0
@@ -97,8 +105,9 @@ def batch_vqe(templates, instances, use_graph: bool = True) -> np.ndarray:
         tmpl[j].nqubits, tmpl[j].nops, tmpl[j].nbinds, tmpl[j].nterms = n, len(ops), len(binds), len(terms)
         tmpl[j].op_first, tmpl[j].bind_first = nops, nbinds
         tmpl[j].term_first, tmpl[j].pauli_first = len(coeffs), npauli
-        ops = ops.copy()
-        ops["mat"][ops["mat"] >= 0] += nmats
+        if nmats:
+            ops = ops.copy()
+            ops["mat"][ops["mat"] >= 0] += nmats
         all_ops.append(ops)
         all_mats.append(mats)
         all_binds.append(binds)
@@ -113,7 +122,10 @@ def batch_vqe(templates, instances, use_graph: bool = True) -> np.ndarray:
     cf = np.ascontiguousarray(coeffs or [0.0], dtype=np.float64)
     ps = "".join(pauli).encode()
     th = np.zeros((len(instances), max(nparams, 1)))
-    if nparams:  # every instance's parameters at the start of its row
+    if nparams and few:  # every instance's parameters at the start of its row
+        for row, v in zip(th, params):
+            row[:len(v)] = v
+    elif nparams:
         th[np.arange(th.shape[1]) < lens[:, None]] = np.concatenate(params, dtype=np.float64, casting="unsafe")
     out = np.zeros(len(instances))
     dp = lambda a: a.ctypes.data_as(C.POINTER(C.c_double))

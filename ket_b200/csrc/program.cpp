@@ -1018,8 +1018,13 @@ double code_weight(const Gate& g) {
 // instructions of 16 bytes, 128 KB; limits of 6000 to 9000 measured alike, 5000 and
 // less slower.  The gradient of 8 parameter vectors at 24 qubits: 127 -> 121 ms on
 // the device; a 25-qubit complex64 circuit of mixed gates 3.82 -> 3.67 ms.
+// Below kCutQubits a pass is shorter than the launch and the second lowering that a
+// cut costs: with cuts a compiled complex64 circuit of 16 qubits took 1100 us against
+// 888, of 19 qubits 1300 against 1138; 21 qubits are even (1634 and 1508 against 1566
+// and 1620), 22 gain (1815 against 2056).
 void split_long_passes(int n, int precision, bool prune, int nreg, Plan& plan) {
-  constexpr int kCodeLimit = 8000;
+  constexpr int kCodeLimit = 8000, kCutQubits = 22;
+  if (n < kCutQubits) return;
   std::vector<Pass> out;
   std::vector<FOp> prog;
   uint8_t lp[KET_T2_BITS], sp[KET_T2_BITS];
@@ -1027,7 +1032,7 @@ void split_long_passes(int n, int precision, bool prune, int nreg, Plan& plan) {
     double w = 0;
     for (int gi : p.gates) w += code_weight(plan.gates[gi]);
     // (a gate's code with its share of the exchanges is below 4 weights a slot)
-    if (!(p.fused && p.m == KET_T2_BITS && n >= KET_T2_BITS) || 4 * w * (1 << nreg) < kCodeLimit) {
+    if (!(p.fused && p.m == KET_T2_BITS) || 4 * w * (1 << nreg) < kCodeLimit) {
       out.push_back(std::move(p));
       continue;
     }

@@ -1,9 +1,9 @@
 """Passes whose compiled kernels would outgrow the instruction cache are cut into
 several: the state is the interpreter's, which takes them whole, bit for bit (the
 cut stores and reloads the amplitudes unchanged; the circuits hold no controlled
-phases, which merge by pass).  Deep circuits on the 12 qubits of one tile, one of
-them of 2000 gates to cut in many places, and single gates that leave
-nothing to cut."""
+phases, which merge by pass).  Deep circuits on the 12 qubits of one tile, at the
+smallest size that is cut and on both sides of it, one of 1000 gates to cut in
+many places, and a single gate that leaves nothing to cut."""
 import random
 
 import numpy as np
@@ -34,7 +34,7 @@ def _circuit(n, gates, seed):
 
 
 @pytest.mark.parametrize("n,gates,precision,prune", [
-    (12, 1, 0, True), (13, 60, 0, True), (13, 400, 0, False), (14, 300, 1, True), (12, 2000, 0, True), (21, 250, 0, True),
+    (21, 250, 0, True), (22, 1, 0, True), (22, 60, 0, False), (22, 250, 0, True), (22, 300, 1, True), (23, 1000, 0, False),
 ])
 def test_cut_passes_equal_the_interpreter(n, gates, precision, prune):
     from ket_b200.circuit import DeviceState, flatten_ops, ops_to_abi
