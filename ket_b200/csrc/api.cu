@@ -427,7 +427,15 @@ int ket_state_copy(ket_state* dst, const ket_state* src) {
   if (!dst || !src) return fail(KET_ERR_TYPE, "null state");
   if (dst->n != src->n || dst->precision != src->precision) return fail(KET_ERR_TYPE, "state shape mismatch");
   cudaSetDevice(dst->ctx->device);
-  cudaError_t e = cudaMemcpyAsync(dst->amp, src->amp, src->bytes, cudaMemcpyDeviceToDevice, dst->ctx->stream);
+  cudaError_t e = cudaSuccess;
+  if (src->ctx != dst->ctx) {
+    // a call on the source may have left its work queued (ket_state_set_basis): the
+    // copy, on the destination's stream, follows it
+    e = cudaEventRecord(src->ctx->done, src->ctx->stream);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(dst->ctx->stream, src->ctx->done, 0);
+    if (e != cudaSuccess) return cuda_fail(e, "ordering a copy behind its source");
+  }
+  e = cudaMemcpyAsync(dst->amp, src->amp, src->bytes, cudaMemcpyDeviceToDevice, dst->ctx->stream);
   if (e != cudaSuccess) return cuda_fail(e, "cudaMemcpyAsync");
   return ctx_wait(dst->ctx);
 }
