@@ -76,23 +76,15 @@ def batch_vqe(templates, instances, use_graph: bool = True) -> np.ndarray:
     from .adjoint import _terms
     if not instances:
         return np.zeros(0)
-    which, params = zip(*instances)
-    it = np.ascontiguousarray(which, dtype=np.int32)
-    if it.min() < 0 or it.max() >= len(templates):
-        bad = it[(it < 0) | (it >= len(templates))][0]
+    which = [t for t, _ in instances]
+    params = [v for _, v in instances]
+    if not (0 <= min(which) and max(which) < len(templates)):
+        bad = next(t for t in which if not 0 <= t < len(templates))
         raise RangeError(f"instance template index {bad} out of range")
-    few = len(instances) <= 64  # (where an array operation costs more than a loop)
-    if few:
-        lens = [len(v) for v in params]
-        nparams = max(lens)
-        first = {}
-        for t, v in instances:
-            first.setdefault(int(t), v)
-    else:
-        lens = np.fromiter(map(len, params), dtype=np.int64, count=len(params))
-        nparams = int(lens.max())
-        used, at = np.unique(it, return_index=True)
-        first = {int(t): params[i] for t, i in zip(used, at)}
+    it = np.ascontiguousarray(which, dtype=np.int32)
+    lens = list(map(len, params))
+    nparams = max(lens)
+    first = dict(zip(reversed(which), reversed(params)))  # (the first instance of a template stays)
     tmpl = (ket_batch_template * max(1, len(templates)))()
     all_ops, all_mats, all_binds, coeffs, pauli = [], [], [], [], []
     nops = nmats = nbinds = npauli = 0
@@ -116,17 +108,13 @@ def batch_vqe(templates, instances, use_graph: bool = True) -> np.ndarray:
             coeffs.append(c)
             pauli.append(o)
             npauli += len(o)
-    ops_a = np.concatenate(all_ops) if nops else np.zeros(1, dtype=_OP)
-    binds_a = np.concatenate(all_binds) if nbinds else np.zeros(1, dtype=_BIND)
+    join = lambda a: a[0] if len(a) == 1 else np.concatenate(a)
+    ops_a = join(all_ops) if nops else np.zeros(1, dtype=_OP)
+    binds_a = join(all_binds) if nbinds else np.zeros(1, dtype=_BIND)
     mats = np.concatenate(all_mats + [np.zeros(1, dtype=np.complex128)]).view(np.float64)
     cf = np.ascontiguousarray(coeffs or [0.0], dtype=np.float64)
     ps = "".join(pauli).encode()
-    th = np.zeros((len(instances), max(nparams, 1)))
-    if nparams and few:  # every instance's parameters at the start of its row
-        for row, v in zip(th, params):
-            row[:len(v)] = v
-    elif nparams:
-        th[np.arange(th.shape[1]) < lens[:, None]] = np.concatenate(params, dtype=np.float64, casting="unsafe")
+    th = _theta(params, lens, nparams)
     out = np.zeros(len(instances))
     dp = lambda a: a.ctypes.data_as(C.POINTER(C.c_double))
     check(lib().ket_batch_vqe(default_ctx(), len(templates), tmpl, ops_a.ctypes.data_as(C.POINTER(ket_op)), dp(mats),
@@ -134,6 +122,26 @@ def batch_vqe(templates, instances, use_graph: bool = True) -> np.ndarray:
                               len(instances), it.ctypes.data_as(C.POINTER(C.c_int)), dp(th), max(nparams, 1),
                               1 if use_graph else 0, dp(out)))
     return out
+
+
+def _theta(params, lens, nparams):
+    """Every instance's parameters at the start of its row of max(nparams, 1)."""
+    n = len(params)
+    if nparams and min(lens) == nparams:
+        return np.ascontiguousarray(np.asarray(params, dtype=np.float64).reshape(-1))
+    th = np.zeros((n, max(nparams, 1)))
+    if n > 64 and isinstance(params[0], np.ndarray):  # (arrays join faster than a loop copies them; lists do not)
+        try:
+            flat = np.concatenate(params)
+        except ValueError:  # (of shapes that do not join)
+            flat = None
+        # plain numbers only: what else an assignment converts or refuses is left to it
+        if flat is not None and flat.ndim == 1 and flat.dtype.kind in "biuf":
+            th[np.arange(th.shape[1]) < np.asarray(lens)[:, None]] = flat
+            return th
+    for row, v in zip(th, params):
+        row[:len(v)] = v
+    return th
 
 
 # Traced templates, kept per ansatz function while it lives: a parameter sweep
