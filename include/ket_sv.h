@@ -173,6 +173,12 @@ KET_API int ket_debug_adjoint_budget(int64_t device_bytes);
  * two seconds) and the call returns KET_ERR_TIMEOUT with the context still
  * usable; -1 disables.  No counterpart in the reference. */
 KET_API int ket_debug_stage_drop(int64_t tile);
+/* Test hook for the one-launch path of small complex128 states: max_ctas > 0 stands in
+ * for the number of CTAs the device holds at once (a launch that needs more is left to
+ * the passes), spin_limit sets how many polls its grid barrier makes before it
+ * gives up and the call returns KET_ERR_TIMEOUT (0 = the default, 2^22); 0, 0
+ * disables.  No counterpart in the reference (which has no device waits). */
+KET_API int ket_debug_rounds_hook(int max_ctas, uint32_t spin_limit);
 
 /* Dense state of 2^nqubits amplitudes, resident in device memory, set to |0..0>
  * (zero(n), statevector.ts:16).  precision: KET_C128 or KET_C64. */

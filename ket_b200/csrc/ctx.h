@@ -30,6 +30,7 @@ struct ket_ctx {
   int* h_status = nullptr;        // its copy in pinned memory (ctx_finish)
   void* adj_work = nullptr;       // ket_adjoint_gradient's buffers while they are small
   size_t adj_work_bytes = 0;
+  int rounds_ctas[3] = {0, 0, 0};  // co-resident CTAs of small.cu's kernels by tile bits 10..12 (0: not asked yet)
   uint64_t launches = 0;
   uint64_t h2d_bytes = 0, d2h_bytes = 0;  // host<->device copies made by the context
   bool prof = false;

@@ -35,7 +35,12 @@ namespace {
 
 constexpr int kTileBits = 12;
 constexpr int kMaxRounds = 64, kMaxGates = 64, kMaxSlots = 128;  // of one pass, in shared memory
-constexpr uint32_t kSpinLimit = 1u << 22;  // seconds
+constexpr uint32_t kSpinLimit = 1u << 22;  // polls of the barrier: seconds
+
+// Test hook (ket_debug_rounds_hook): the co-resident CTAs a launch may count on (0:
+// what the device holds) and the barrier's polls.
+int g_max_ctas = 0;
+uint32_t g_spin_limit = kSpinLimit;
 
 enum : uint8_t { FM_GEN = 0, FM_REAL = 1, FM_RX = 2, FM_DIAG = 3, FM_DIAG2 = 4, FM_X = 5, FM_PHASE = 6 };
 enum : uint8_t { GF_PRUNE = 1, GF_CHAIN = 2 };  // CHAIN: the next gate is a phase of the same target, too
@@ -91,6 +96,7 @@ struct RArgs {
   int* status;
   int npasses, n, d;           // d: tile bits
   int permute;                 // the relabelling is not the identity
+  uint32_t spin_limit;
   uint32_t beta;               // physical index of logical index l: A l ^ beta
   uint32_t acol[20];
 };
@@ -262,7 +268,7 @@ __device__ __forceinline__ bool grid_barrier(const RArgs& a, unsigned int target
     uint32_t spins = 0;
     int bad = 0;
     while (*p < target) {
-      if (++spins > kSpinLimit) {
+      if (++spins > a.spin_limit) {
         atomicExch(a.status, (int)KET_ERR_TIMEOUT);
         bad = 1;
         break;
@@ -671,10 +677,27 @@ struct SPlan {
   }
 };
 
+// Dynamic shared memory and threads of a launch on tiles of 2^d amplitudes.
+size_t rounds_smem(int d) { return (sizeof(double2) << d) + 2 * sizeof(Records); }
+template <int K>
+unsigned rounds_threads(int d) { return std::max(32u, 1u << (d - K)); }
+
+// CTAs that are resident together.
+template <int K>
+cudaError_t rounds_resident(int device, int d, int* ctas) {
+  const int smem = (int)rounds_smem(d);
+  int per_sm = 0, sms = 0;
+  cudaError_t e = cudaFuncSetAttribute(k_rounds<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_rounds<K>, rounds_threads<K>(d), smem);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+  *ctas = per_sm * sms;
+  return e;
+}
+
 template <int K>
 cudaError_t launch_rounds(const RArgs& a, unsigned grid, cudaStream_t s) {
-  const size_t smem = (sizeof(double2) << a.d) + 2 * sizeof(Records);
-  const unsigned nt = std::max(32u, 1u << (a.d - K));
+  const size_t smem = rounds_smem(a.d);
+  const unsigned nt = rounds_threads<K>(a.d);
   cudaError_t e = cudaFuncSetAttribute(k_rounds<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   if (grid == 1) {
@@ -688,13 +711,24 @@ cudaError_t launch_rounds(const RArgs& a, unsigned grid, cudaStream_t s) {
 }  // namespace
 
 // The circuit in one launch (not waited for); *ran = false when it holds something
-// this path does not take (unitaries of more than four qubits).
+// this path does not take (unitaries of more than four qubits), or the device has no
+// room for all its CTAs at once (a share of a GPU): the passes run it then.
 int run_small(ket_state* s, const std::vector<Gate>& gates, bool prune, bool* ran) {
   *ran = false;
   SPlan P(s->n);
-  if (!P.lower(gates, prune)) return KET_OK;
   ket_ctx* c = s->ctx;
   cudaSetDevice(c->device);
+  const unsigned grid = s->n > P.d ? 1u << (s->n - P.d) : 1u;
+  if (grid > 1) {
+    int& fit = c->rounds_ctas[P.d - 10];  // (tiles of a grid are of 2^10 to 2^12)
+    if (fit == 0) {
+      const cudaError_t e =
+          P.rb_ == 4 ? rounds_resident<4>(c->device, P.d, &fit) : rounds_resident<3>(c->device, P.d, &fit);
+      if (e != cudaSuccess) return cuda_fail(e, "rounds occupancy");
+    }
+    if (grid > (unsigned)(g_max_ctas > 0 ? g_max_ctas : fit)) return KET_OK;
+  }
+  if (!P.lower(gates, prune)) return KET_OK;
   size_t total = 256;  // the barrier's counter
   auto place = [&](size_t bytes) {
     const size_t at = total;
@@ -727,6 +761,7 @@ int run_small(ket_state* s, const std::vector<Gate>& gates, bool prune, bool* ra
   a.npasses = (int)P.passes.size();
   a.n = s->n;
   a.d = P.d;
+  a.spin_limit = g_spin_limit;
   a.beta = P.beta;
   a.permute = P.beta != 0;
   for (int q = 0; q < 20; q++) {
@@ -734,7 +769,6 @@ int run_small(ket_state* s, const std::vector<Gate>& gates, bool prune, bool* ra
     if (q < s->n && P.col[q] != 1u << q) a.permute = 1;
   }
   prof_begin(c);
-  const unsigned grid = s->n > P.d ? 1u << (s->n - P.d) : 1u;
   const cudaError_t e = P.rb_ == 4 ? launch_rounds<4>(a, grid, c->stream) : launch_rounds<3>(a, grid, c->stream);
   prof_end(c, PK_FUSED1);
   if (e != cudaSuccess) return cuda_fail(e, "rounds launch");
@@ -743,3 +777,10 @@ int run_small(ket_state* s, const std::vector<Gate>& gates, bool prune, bool* ra
 }
 
 }  // namespace ket
+
+extern "C" int ket_debug_rounds_hook(int max_ctas, uint32_t spin_limit) {
+  if (max_ctas < 0) return ket::fail(KET_ERR_TYPE, "negative CTA count");
+  ket::g_max_ctas = max_ctas;
+  ket::g_spin_limit = spin_limit ? spin_limit : ket::kSpinLimit;
+  return KET_OK;
+}
