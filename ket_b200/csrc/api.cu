@@ -153,32 +153,42 @@ int ctx_finish(ket_ctx* c) {
   return KET_OK;
 }
 
-// Circuits below KET_JIT_AUTO_QUBITS qubits whose kernels were compiled ahead
-// (ket_jit_compile): they run on those kernels, as the default policy promises.
-// Known by a hash of their ops' kinds and qubits; like the kernels, kept until the
-// process ends, and bounded (a circuit past the bound takes the other route).
+// Circuits below KET_JIT_AUTO_QUBITS qubits whose kernels the default options find in the
+// cache: compiled ahead (ket_jit_compile), or by a specialize = 1 run.  They are planned
+// as they were then.  Known by a hash of their lowered gates -- qubits, and which matrix
+// entries are zero or one, the only values that select code; like the kernels, kept
+// until the process ends, and bounded (a circuit past the bound takes the other route).
 namespace {
 std::mutex g_ahead_mu;
 std::unordered_set<uint64_t> g_ahead;
 std::atomic<bool> g_any_ahead{false};
-uint64_t circuit_hash(int n, int precision, bool prune, const ket_op* ops, size_t nops) {
+uint64_t circuit_hash(int n, int precision, bool prune, const std::vector<Gate>& gates) {
   uint64_t h = 1469598103934665603ull;
   auto mix = [&](uint64_t v) { h = (h ^ v) * 1099511628211ull; };
   mix((uint64_t)n << 8 | (uint64_t)precision << 1 | prune);
-  for (size_t i = 0; i < nops; i++) {
-    mix((uint64_t)ops[i].kind << 8 | (uint64_t)ops[i].nq);
-    for (int j = 0; j < ops[i].nq && j < KET_MAX_OP_QUBITS; j++) mix((uint64_t)ops[i].q[j]);
+  for (const Gate& g : gates) {
+    mix((uint64_t)g.type << 32 | (uint64_t)(g.t0 + 1) << 16 | (uint64_t)(g.t1 + 1) << 8 | g.prune);
+    mix(g.cmask);
+    uint64_t form = 0;
+    if (g.type != G_X1 && g.type != G_SWAP)  // (which have no matrix)
+      for (const cd& z : g.m) form = form << 3 | (uint64_t)(z.re == 0) | (uint64_t)(z.im == 0) << 1 | (uint64_t)(z.re == 1) << 2;
+    mix(form);
+    for (int q : g.tk) mix((uint64_t)q + 1);
   }
   return h;
+}
+// Whether a run with the default options would look for kernels of these options' programs.
+bool default_programs(int n, const ket_exec_opts& o) {
+  return o.fusion < 0 && tiled_nreg(n, o.reg_bits) == tiled_nreg(n) && use_staged(n, o.stage) == use_staged(n, 0);
 }
 void note_ahead(uint64_t h) {
   std::lock_guard<std::mutex> lk(g_ahead_mu);
   if (g_ahead.size() < 65536) g_ahead.insert(h);
   g_any_ahead.store(true);
 }
-bool compiled_ahead(int n, int precision, bool prune, const ket_op* ops, size_t nops) {
+bool compiled_ahead(int n, int precision, bool prune, const std::vector<Gate>& gates) {
   if (!g_any_ahead.load()) return false;
-  const uint64_t h = circuit_hash(n, precision, prune, ops, nops);
+  const uint64_t h = circuit_hash(n, precision, prune, gates);
   std::lock_guard<std::mutex> lk(g_ahead_mu);
   return g_ahead.count(h) != 0;
 }
@@ -537,7 +547,8 @@ int ket_jit_compile(int n, int precision, const ket_op* ops, size_t nops, const 
                          use_staged(n, o.stage)});
   std::string clog;
   rc = jit_compile(jp, precision, kernels, clog);
-  if (!rc && n < KET_JIT_AUTO_QUBITS && !jp.empty()) note_ahead(circuit_hash(n, precision, o.prune != 0, ops, nops));
+  if (!rc && n < KET_JIT_AUTO_QUBITS && !jp.empty() && default_programs(n, o))
+    note_ahead(circuit_hash(n, precision, o.prune != 0, plan.gates));
   if (log && logcap) {
     strncpy(log, clog.c_str(), logcap - 1);
     log[logcap - 1] = 0;
@@ -558,8 +569,8 @@ int ket_apply_ops(ket_state* s, const ket_op* ops, size_t nops, const double* ma
   if (rc) return fail(rc, err);
   if (o.fusion != 0) fold_single_qubit(plan.gates, o.prune != 0);
   if (plan.gates.empty()) return KET_OK;
-  const bool ahead = o.specialize == 0 && s->n < KET_JIT_AUTO_QUBITS &&
-                     compiled_ahead(s->n, s->precision, o.prune != 0, ops, nops);
+  const bool automatic = o.specialize == 0 && s->n < KET_JIT_AUTO_QUBITS && default_programs(s->n, o);
+  const bool ahead = automatic && compiled_ahead(s->n, s->precision, o.prune != 0, plan.gates);
   // Small complex128 states, with everything automatic, run in one launch.
   if (s->precision == KET_C128 && s->n <= kSmallQubits && o.fusion < 0 && o.specialize == 0 && o.reg_bits == 0 && o.stage == 0 &&
       !ahead) {
@@ -569,9 +580,18 @@ int ket_apply_ops(ket_state* s, const ket_op* ops, size_t nops, const double* ma
     if (ran) return ctx_finish(s->ctx);
   }
   plan_passes(s->n, s->precision, o.fusion, o.prune != 0, plan);
-  // (the interpreter's code does not grow with the pass: it takes whole passes)
-  if (o.specialize == 1 || ahead || (o.specialize == 0 && s->n >= KET_JIT_AUTO_QUBITS))
+  // Below KET_JIT_AUTO_QUBITS qubits the interpreter, whose code does not grow with the
+  // pass, takes whole passes; from there on it runs what is being compiled.
+  if (o.specialize == 1 || ahead || (o.specialize == 0 && s->n >= KET_JIT_AUTO_QUBITS)) {
+    const size_t whole = plan.passes.size();
     split_long_passes(s->n, s->precision, o.prune != 0, tiled_nreg(s->n, o.reg_bits), plan);
+    // (a later call with the default options has to cut alike to find these kernels)
+    if (o.specialize == 1 && plan.passes.size() != whole && s->n < KET_JIT_AUTO_QUBITS && default_programs(s->n, o)) {
+      rc = run_plan(s, plan, o);
+      if (!rc) note_ahead(circuit_hash(s->n, s->precision, o.prune != 0, plan.gates));
+      return rc;
+    }
+  }
   return run_plan(s, plan, o);
 }
 
