@@ -7,10 +7,11 @@
 // (algorithms.ts:260-276: cnot . rz . cnot per edge) and measures it with
 // vqe(., maxCutHamiltonian(n, E)) (algorithms.ts:231-241, 301-336).
 //
-// Work items are pulled from a global queue by a persistent grid:
-//   * an instance of n <= TILE qubits is one item, simulated on the chip (all
-//     layers and the <C> reduction);
-//   * a wider instance is split into p + 1 passes of tiles of 2^TILE amplitudes.
+// Work items are pulled from global queues by persistent grids:
+//   * an instance of n <= TILE qubits is one item of k_qaoa_chip, its whole state in
+//     shared memory (all layers and the <C> reduction);
+//   * a wider instance is split into p + 1 passes of tiles of 2^TILE amplitudes
+//     (k_batch_qaoa).
 //     A tile holds either the low TILE qubits (even passes) or the qubits above
 //     them with the lowest qubits (odd passes).  Rx gates commute and the cost
 //     phase is diagonal, so pass k finishes layer k - 1 on its qubits, applies
@@ -20,7 +21,7 @@
 //     of pass k-1 of its instance has been written back; the queue hands items
 //     out in an order where everything a tile waits on was handed out earlier, so
 //     the fully resident grid cannot deadlock.
-// A tile lives in registers, 2^K consecutive values of K of its bits a thread; Rx on
+// A tile of a wide instance lives in registers, 2^K consecutive values of K of its bits a thread; Rx on
 // those bits needs no exchange, and the other bits come round through shared memory.
 // Rx(2 beta) = cos(beta) (1 - i tan(beta) X) is applied without its scalar, so an
 // amplitude takes two FMAs a gate; <C> is divided by the norm that is left.  Where
@@ -50,7 +51,7 @@ namespace {
 #define KQ_MAX_P 16
 
 struct QInst {
-  int n, ne, p, ntiles;     // ntiles = 2^(n - tile) for split instances, 1 otherwise
+  int n, ne, p, ntiles;     // ntiles = 2^(n - tile) for split instances, 0 on the chip
   int multi, pad;           // an edge occurs twice: cut(x) is counted for every amplitude
   int64_t state;            // offset (amplitudes) of the instance's state in the workspace (split only)
   int64_t edge_off;         // first edge in the edge array
@@ -59,16 +60,15 @@ struct QInst {
 };
 
 // The queue's items in order: run r holds items [first, the next run's first), the
-// tiles of one pass of an instance (or one whole instance).
+// tiles of one pass (0..p) of a wide instance.
 struct QRun {
-  int first, inst;
-  int pass;   // -1: whole instance on the chip; else pass index 0..p
-  int pad;
+  int first, inst, pass, pad;
 };
 
 struct QArgs {
   const QInst* inst;
   const QRun* runs;         // and an end mark
+  const int* chip;          // the instances that fit the chip, widest first
   const uint32_t* emask;    // edge masks (1<<u | 1<<v)
   const double* gamma;      // [inst * p + l]
   const double* beta;
@@ -76,11 +76,13 @@ struct QArgs {
   double2* tab;             // phases by instance, layer and cut
   double2* work;            // split-instance states
   double2* part;            // (<C>, norm) partials
-  unsigned int* next;       // queue head
+  double* out;              // <C> by instance
+  unsigned int* next;       // queue heads: tiles of wide instances, chip instances
   unsigned int* done;       // per instance: tiles finished (pass-major)
   int* status;
   uint32_t spin_limit;      // polls before a wait gives up (status KET_ERR_TIMEOUT)
   int nitems;
+  int nchip, chip_bits;     // instances on the chip, qubits of the widest
   int drop;                 // test hook: an item that is left out (-1: none)
 };
 
@@ -88,6 +90,7 @@ struct QArgs {
 __global__ void k_qaoa_tables(QArgs a, int p) {
   const int i = blockIdx.x / p, l = blockIdx.x % p;
   const QInst I = a.inst[i];
+  if (I.ntiles == 0) return;
   const double gamma = a.gamma[blockIdx.x];
   for (int c = threadIdx.x; c <= I.ne; c += blockDim.x) {
     double s, co;
@@ -330,7 +333,7 @@ __global__ void __launch_bounds__(NT, QLay<NT, T>::CTAS) k_batch_qaoa(QArgs a) {
       }
       if (t < 32) sh.nbr[t] = 0;
       __syncthreads();
-      ready = w.pass <= 0;
+      ready = w.pass == 0;
       for (int e = t; e < I.ne; e += NT) sh.em[e] = a.emask[I.edge_off + e];
       __syncthreads();
       for (int e = t; e < I.ne; e += NT) {
@@ -349,38 +352,6 @@ __global__ void __launch_bounds__(NT, QLay<NT, T>::CTAS) k_batch_qaoa(QArgs a) {
       for (int c = t; c <= I.ne; c += NT) sh.tab[c] = a.tab[I.tab_off + (int64_t)l * (I.ne + 1) + c];
     };
     double2 v[NS];
-    if (w.pass < 0) {
-      // ---- whole instance on the chip (p = 0: <C> of the uniform state, whatever n)
-      const QMap m = {0u, T, T};
-      if (I.p == 0) {
-        if (t == 0) a.part[I.part_off] = make_double2(0.5 * I.ne, 1.0);
-        __syncthreads();
-        continue;
-      }
-      const double amp0 = 1.0 / sqrt((double)(1u << n));
-#pragma unroll
-      for (int j = 0; j < NS; j++)
-        v[j] = make_double2((tile_index<NT, T, 0>(t) | reg_index<NT, T, 0>(j)) < (1u << n) ? amp0 : 0.0, 0.0);
-      const uint32_t bits = (1u << n) - 1u;
-      for (int l = 0; l < I.p; l++) {
-        __syncthreads();  // the last layer's reads of the table
-        load_table(l);
-        __syncthreads();
-        const double r = a.tan[(int64_t)w.inst * I.p + l];
-        if (l & 1) {
-          phase_regs<NT, T, TOP>(v, m, t, sh, I);
-          rx_down<NT, T, TOP>(v, s, t, bits, r);
-        } else {
-          phase_regs<NT, T, 0>(v, m, t, sh, I);
-          rx_up<NT, T, 0>(v, s, t, bits, r);
-        }
-      }
-      if (I.p & 1) tile_cut<NT, T, TOP>(v, m, t, sh, I, a.part + I.part_off);
-      else tile_cut<NT, T, 0>(v, m, t, sh, I, a.part + I.part_off);
-      __syncthreads();
-      continue;
-    }
-    // ---- one tile of one pass of a wide instance
     if (fresh && w.pass < I.p) load_table(w.pass);
     if (!ready) {
       // wait until every tile of the previous pass has been written back; a
@@ -447,11 +418,12 @@ __global__ void __launch_bounds__(NT, QLay<NT, T>::CTAS) k_batch_qaoa(QArgs a) {
   }
 }
 
-// <C> of an instance: its partials added by a warp (strided runs, then a tree).
+// <C> of a wide instance: its partials added by a warp (strided runs, then a tree).
 __global__ void k_qaoa_reduce(const QInst* inst, int ninst, const double2* part, double* out) {
   const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (i >= ninst) return;
   const QInst I = inst[i];
+  if (I.ntiles == 0) return;
   double acc = 0.0, nrm = 0.0;
   for (int t = lane; t < I.ntiles; t += 32) {
     const double2 p = part[I.part_off + t];
@@ -461,6 +433,158 @@ __global__ void k_qaoa_reduce(const QInst* inst, int ninst, const double2* part,
   acc = warp_sum(acc);
   nrm = warp_sum(nrm);
   if (lane == 0) out[i] = acc / nrm;
+}
+
+// ---------------------------------------------------------------- instances on the chip
+// Shared-memory position of amplitude i: the three low index bits are XORed with
+// bits 3-5.  For every group of rotated bits below, the eight threads of a quarter
+// warp then touch eight distinct 16-byte slots of a 128-byte row (conflict-free),
+// whichever bits the group holds.
+__device__ __forceinline__ uint32_t sw(uint32_t i) { return i ^ ((i >> 3) & 7u); }
+
+// Rx(2 beta) = [[c, -i s], [-i s, c]] on one pair, in registers.
+__device__ __forceinline__ void rx_pair(double2& a, double2& b, double cb, double sb) {
+  const double2 x = a, y = b;
+  a = make_double2(fma(cb, x.x, sb * y.y), fma(cb, x.y, -sb * y.x));
+  b = make_double2(fma(cb, y.x, sb * x.y), fma(cb, y.y, -sb * x.x));
+}
+
+// Rx(2 beta) on the K bits g[0] < ... < g[K-1] of a block of 2^m amplitudes: each
+// thread loads the 2^K amplitudes of a subcube into registers, rotates every bit of
+// the group there (lowest first), and stores them back -- one shared-memory round
+// trip per group instead of one per bit.
+template <int NT, int K>
+__device__ void rx_group(double2* s, int m, uint32_t gp, double cb, double sb) {
+  int g[K];  // the group's bits, packed one per byte of gp (kept in registers)
+#pragma unroll
+  for (int q = 0; q < K; q++) g[q] = (int)((gp >> (8 * q)) & 0xffu);
+  const uint32_t nsub = 1u << (m - K);
+  for (uint32_t u = threadIdx.x; u < nsub; u += NT) {
+    uint32_t b = u;
+#pragma unroll
+    for (int q = 0; q < K; q++) b = insert0_32(b, g[q]);
+    double2 v[1 << K];
+#pragma unroll
+    for (int j = 0; j < (1 << K); j++) {
+      uint32_t o = b;
+#pragma unroll
+      for (int q = 0; q < K; q++)
+        if ((j >> q) & 1) o |= 1u << g[q];
+      v[j] = s[sw(o)];
+    }
+#pragma unroll
+    for (int q = 0; q < K; q++)
+#pragma unroll
+      for (int j = 0; j < (1 << K); j++)
+        if (!((j >> q) & 1)) rx_pair(v[j], v[j | (1 << q)], cb, sb);
+#pragma unroll
+    for (int j = 0; j < (1 << K); j++) {
+      uint32_t o = b;
+#pragma unroll
+      for (int q = 0; q < K; q++)
+        if ((j >> q) & 1) o |= 1u << g[q];
+      s[sw(o)] = v[j];
+    }
+  }
+}
+
+// Bits per group: three at 256 threads per CTA, so that the registers of three
+// resident CTAs (what 12 qubits of shared memory allow) hold a group's 8 amplitudes
+// without spills; four at 128 and 512 threads.
+template <int NT>
+constexpr int rx_group_bits() { return NT == 256 ? 3 : 4; }
+template <int NT>
+constexpr int chip_min_blocks() { return NT == 512 ? 1 : 3; }
+
+// Rx(2 beta) on all m bits, in ascending order, a group of bits per shared-memory
+// round trip.
+template <int NT>
+__device__ void rx_bits(double2* s, int m, double cb, double sb) {
+  constexpr int KM = rx_group_bits<NT>();
+  for (int b = 0; b < m; b += KM) {
+    const uint32_t gp = 0x03020100u + 0x01010101u * (uint32_t)b;
+    const int k = min(KM, m - b);
+    __syncthreads();
+    if constexpr (KM == 4) {
+      if (k == 4) { rx_group<NT, 4>(s, m, gp, cb, sb); continue; }
+    }
+    switch (k) {
+      case 3: rx_group<NT, 3>(s, m, gp, cb, sb); break;
+      case 2: rx_group<NT, 2>(s, m, gp, cb, sb); break;
+      default: rx_group<NT, 1>(s, m, gp, cb, sb); break;
+    }
+  }
+}
+
+// Shared memory of a CTA: state, phase table, edge masks, sums, cut(x) per amplitude.
+constexpr size_t kChipFixed = 16 * (KQ_MAX_EDGES + 1) + 4 * KQ_MAX_EDGES + 8 * 32;
+static_assert(kChipFixed % 16 == 0, "cut bytes 16-byte aligned");
+size_t chip_smem(int bits) { return kChipFixed + (size_t(17) << bits) + 16; }
+
+// One instance a CTA at a time, 2^n amplitudes in shared memory.  Bound: latency -- a
+// layer is n / 3 round trips and as many barriers.  The wide kernel's tiles take every
+// layout move of 12 bits and a launch for their tables, whatever the instance's
+// width: 2000 instances of 2 qubits and 6 layers 365 us on them, 48 here; 500 of 12
+// qubits and 3 layers, which fill a tile, 93 and 69.
+template <int NT>
+__global__ void __launch_bounds__(NT, chip_min_blocks<NT>()) k_qaoa_chip(QArgs a) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  double2* s = reinterpret_cast<double2*>(smraw);
+  double2* tab = s + (1u << a.chip_bits);
+  uint32_t* em = reinterpret_cast<uint32_t*>(tab + KQ_MAX_EDGES + 1);
+  double* red = reinterpret_cast<double*>(em + KQ_MAX_EDGES);
+  uint8_t* cutb = reinterpret_cast<uint8_t*>(red + 32);
+  __shared__ int item_sh;
+  for (;;) {
+    if (threadIdx.x == 0) item_sh = (int)atomicAdd(a.next + 1, 1u);
+    __syncthreads();
+    const int it = item_sh;
+    __syncthreads();
+    if (it >= a.nchip) break;
+    const int i = a.chip[it];
+    const QInst I = a.inst[i];
+    if (I.p == 0) {  // <C> of the uniform state, whatever n
+      if (threadIdx.x == 0) a.out[i] = 0.5 * I.ne;
+      continue;
+    }
+    for (int e = threadIdx.x; e < I.ne; e += NT) em[e] = a.emask[I.edge_off + e];
+    const int n = I.n;
+    const uint32_t N = 1u << n;
+    const double amp0 = 1.0 / sqrt((double)N);
+    __syncthreads();  // edge masks in
+    // cut(x) depends on x only: computed once, read by every layer and <C>
+    for (uint32_t x = threadIdx.x; x < N; x += NT) {
+      s[sw(x)] = make_double2(amp0, 0.0);
+      cutb[x] = (uint8_t)cut_of(x, em, I.ne);
+    }
+    for (int l = 0; l < I.p; l++) {
+      const double gamma = a.gamma[(int64_t)i * I.p + l];
+      __syncthreads();
+      for (int c = threadIdx.x; c <= I.ne; c += NT) {
+        double sn, co;
+        sincos(-gamma * (double)(I.ne - 2 * c), &sn, &co);
+        tab[c] = make_double2(co, sn);
+      }
+      __syncthreads();
+      for (uint32_t x = threadIdx.x; x < N; x += NT) {
+        const double2 ph = tab[cutb[x]];
+        const double2 v = s[sw(x)];
+        s[sw(x)] = make_double2(fma(ph.x, v.x, -ph.y * v.y), fma(ph.x, v.y, ph.y * v.x));
+      }
+      double sb, cb;
+      sincos(a.beta[(int64_t)i * I.p + l], &sb, &cb);
+      rx_bits<NT>(s, n, cb, sb);
+    }
+    __syncthreads();
+    double acc = 0.0;
+    for (uint32_t x = threadIdx.x; x < N; x += NT) {
+      const double2 v = s[sw(x)];
+      acc += (v.x * v.x + v.y * v.y) * (double)cutb[x];
+    }
+    acc = block_sum<NT>(acc, red);
+    if (threadIdx.x == 0) a.out[i] = acc;
+    __syncthreads();
+  }
 }
 
 // Test hook (ket_debug_batch_hook): leave one work item out and
@@ -473,29 +597,39 @@ uint32_t g_spin_limit = 1u << 24;
 
 using namespace ket;
 
-// Launch the tables, the persistent batch kernel (NT threads per CTA, every CTA
-// resident at once) and its fixed-order reduction, captured in a CUDA graph when
-// use_graph is set.
+// Launch the wide instances' tables, their persistent kernel (NT threads per CTA, every
+// CTA resident at once) and its fixed-order reduction, then the instances that fit
+// the chip, captured in a CUDA graph when use_graph is set.
 template <int NT, int T>
-static cudaError_t run_batch(ket_ctx* c, const QArgs& a, int p, int ninst, double* dout, int use_graph) {
-  const size_t smem = (sizeof(double2) << T) + sizeof(QShared);
-  // the shared-memory limit is a per-device attribute of the kernel
+static cudaError_t run_batch(ket_ctx* c, const QArgs& a, int p, int ninst, int use_graph) {
+  const size_t smem = (sizeof(double2) << T) + sizeof(QShared), smem_chip = chip_smem(a.chip_bits);
+  // the shared-memory limit is a per-device attribute of the kernels
   static std::atomic<uint64_t> attr_set{0};
   const uint64_t bit = uint64_t(1) << (c->device & 63);
   if (!(attr_set.load() & bit)) {
     cudaError_t e = cudaFuncSetAttribute(k_batch_qaoa<NT, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(k_qaoa_chip<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)chip_smem(12));
     if (e != cudaSuccess) return e;
     attr_set.fetch_or(bit);
   }
-  int per_sm = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch_qaoa<NT, T>, NT, smem);
-  per_sm = std::max(1, per_sm);
-  const int grid = num_sms() * per_sm;
+  int per_sm = 0, grid = 0, grid_chip = 0;
+  if (a.nitems) {
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch_qaoa<NT, T>, NT, smem);
+    grid = num_sms() * std::max(1, per_sm);
+  }
+  if (a.nchip) {
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_qaoa_chip<NT>, NT, smem_chip);
+    grid_chip = std::min(a.nchip, num_sms() * std::max(1, per_sm));
+  }
   auto record = [&]() -> cudaError_t {
-    cudaMemsetAsync(a.next, 0, 4 * ((size_t)ninst + 2), c->stream);
-    if (p > 0) k_qaoa_tables<<<(unsigned)ninst * p, 64, 0, c->stream>>>(a, p);
-    k_batch_qaoa<NT, T><<<grid, NT, smem, c->stream>>>(a);
-    k_qaoa_reduce<<<(ninst + 3) / 4, 128, 0, c->stream>>>(a.inst, ninst, a.part, dout);
+    cudaMemsetAsync(a.next, 0, 4 * (a.nitems ? (size_t)ninst + 2 : 2), c->stream);
+    if (a.nitems) {
+      k_qaoa_tables<<<(unsigned)ninst * p, 64, 0, c->stream>>>(a, p);
+      k_batch_qaoa<NT, T><<<grid, NT, smem, c->stream>>>(a);
+      k_qaoa_reduce<<<(ninst + 3) / 4, 128, 0, c->stream>>>(a.inst, ninst, a.part, a.out);
+    }
+    if (a.nchip) k_qaoa_chip<NT><<<grid_chip, NT, smem_chip, c->stream>>>(a);
     return cudaGetLastError();
   };
   if (!use_graph) return record();
@@ -511,9 +645,9 @@ static cudaError_t run_batch(ket_ctx* c, const QArgs& a, int p, int ninst, doubl
   mix(&tile, sizeof(tile));
   mix(&p, sizeof(p));
   mix(&ninst, sizeof(ninst));
-  mix(&dout, sizeof(dout));
   mix(&nt, sizeof(nt));
   mix(&grid, sizeof(grid));
+  mix(&grid_chip, sizeof(grid_chip));
   if (c->graph_exec && c->graph_key == key) return cudaGraphLaunch(c->graph_exec, c->stream);
   cudaGraph_t graph;
   cudaError_t e = cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal);
@@ -558,9 +692,10 @@ extern "C" int ket_batch_qaoa(ket_ctx* c, int ninst, const int* n, const int* ne
   if (ninst == 0) return KET_OK;
   cudaSetDevice(c->device);
   const int T = c->batch_tile;
-  std::vector<QInst> inst(ninst);
+  std::vector<QInst> inst(ninst, QInst{});
   std::vector<uint32_t> masks;
   int64_t work = 0, parts = 0, phases = 0;
+  int chip_bits = 0;
   for (int i = 0; i < ninst; i++) {
     if (n[i] < 1 || n[i] > 30) return fail(KET_ERR_RANGE, "instance qubit count out of range (1..30)");
     if (ne[i] < 0 || ne[i] > KQ_MAX_EDGES) return fail(KET_ERR_TYPE, "instance edge count out of range (0..64)");
@@ -577,15 +712,18 @@ extern "C" int ket_batch_qaoa(ket_ctx* c, int ninst, const int* n, const int* ne
       if (u == v) return fail(KET_ERR_TYPE, "self-loop edge");
       masks.push_back((uint32_t(1) << u) | (uint32_t(1) << v));
     }
+    if (I.n <= T || p == 0) {
+      chip_bits = std::max(chip_bits, p > 0 ? I.n : 0);
+      continue;
+    }
     std::vector<uint32_t> em(masks.begin() + I.edge_off, masks.end());
     std::sort(em.begin(), em.end());
     I.multi = std::adjacent_find(em.begin(), em.end()) != em.end();
     I.tab_off = phases;
     phases += (int64_t)p * (ne[i] + 1);
-    const bool split = I.n > T && p > 0;
-    I.ntiles = split ? (1 << (I.n - T)) : 1;
-    I.state = split ? work : 0;
-    if (split) work += int64_t(1) << I.n;
+    I.ntiles = 1 << (I.n - T);
+    I.state = work;
+    work += int64_t(1) << I.n;
     I.part_off = parts;
     parts += I.ntiles;
   }
@@ -597,16 +735,15 @@ extern "C" int ket_batch_qaoa(ket_ctx* c, int ninst, const int* n, const int* ne
   int64_t nitems = 0;
   auto add = [&](int i, int pass) {
     runs.push_back(QRun{(int)nitems, i, pass, 0});
-    nitems += pass < 0 ? 1 : inst[i].ntiles;
+    nitems += inst[i].ntiles;
   };
   // Wide instances go in sets whose states share the 126 MB L2, all passes of a set
   // before the next, the set's instances in turn so that a tile rarely waits (512
   // instances of up to 64 MB: 15.9 ms in one set, 15.3 in sets of 80 MB, 15.5 and
   // 15.7 of 70 and 112 MB).
   constexpr int64_t kSetBytes = int64_t(80) << 20;
-  std::vector<int> wide;
-  for (int i : order)
-    if (inst[i].n > T && p > 0) wide.push_back(i);
+  std::vector<int> wide, chip;
+  for (int i : order) (inst[i].ntiles ? wide : chip).push_back(i);
   while (!wide.empty()) {
     std::vector<int> set, rest;
     int64_t bytes = 0;
@@ -619,20 +756,19 @@ extern "C" int ket_batch_qaoa(ket_ctx* c, int ninst, const int* n, const int* ne
       for (int i : set) add(i, k);
     wide.swap(rest);
   }
-  for (int i : order)
-    if (!(inst[i].n > T && p > 0)) add(i, -1);
   if (nitems > INT32_MAX / 2) return fail(KET_ERR_UNSUPPORTED, "too many tiles in a batch");
   runs.push_back(QRun{INT32_MAX, 0, 0, 0});  // end marks
   runs.push_back(QRun{INT32_MAX, 0, 0, 0});
   // device buffers in the second scratch pool
   auto al = [](size_t b) { return (b + 255) & ~size_t(255); };
   size_t off_inst = 0, off_runs = al(sizeof(QInst) * ninst), off_mask = off_runs + al(sizeof(QRun) * runs.size());
-  size_t off_g = off_mask + al(4 * std::max<size_t>(masks.size(), 1));
+  size_t off_chip = off_mask + al(4 * std::max<size_t>(masks.size(), 1));
+  size_t off_g = off_chip + al(4 * chip.size());
   size_t off_b = off_g + al(8 * (size_t)ninst * p + 8);
   size_t off_tan = off_b + al(8 * (size_t)ninst * p + 8);
   size_t off_tab = off_tan + al(8 * std::max<size_t>((size_t)ninst * p, 1));
   size_t off_part = off_tab + al(16 * std::max<size_t>((size_t)phases, 1));
-  size_t off_out = off_part + al(16 * (size_t)parts);
+  size_t off_out = off_part + al(16 * std::max<size_t>((size_t)parts, 1));
   size_t off_cnt = off_out + al(8 * (size_t)ninst);
   size_t off_work = off_cnt + al(4 * ((size_t)ninst + 2));
   size_t total = off_work + al(16 * (size_t)work) + 256;
@@ -651,45 +787,52 @@ extern "C" int ket_batch_qaoa(ket_ctx* c, int ninst, const int* n, const int* ne
   char* base = (char*)c->scratch2;
   std::vector<double> gv(gamma, gamma + (size_t)ninst * p), bv(beta, beta + (size_t)ninst * p);
   cudaMemcpyAsync(base + off_inst, inst.data(), sizeof(QInst) * ninst, cudaMemcpyHostToDevice, c->stream);
-  cudaMemcpyAsync(base + off_runs, runs.data(), sizeof(QRun) * runs.size(), cudaMemcpyHostToDevice, c->stream);
+  if (nitems)
+    cudaMemcpyAsync(base + off_runs, runs.data(), sizeof(QRun) * runs.size(), cudaMemcpyHostToDevice, c->stream);
+  if (!chip.empty())
+    cudaMemcpyAsync(base + off_chip, chip.data(), 4 * chip.size(), cudaMemcpyHostToDevice, c->stream);
   if (!masks.empty()) cudaMemcpyAsync(base + off_mask, masks.data(), 4 * masks.size(), cudaMemcpyHostToDevice, c->stream);
   if (p > 0) {
     cudaMemcpyAsync(base + off_g, gv.data(), 8 * gv.size(), cudaMemcpyHostToDevice, c->stream);
     cudaMemcpyAsync(base + off_b, bv.data(), 8 * bv.size(), cudaMemcpyHostToDevice, c->stream);
   }
-  c->h2d_bytes += sizeof(QInst) * ninst + sizeof(QRun) * runs.size() + 4 * masks.size() + 16 * gv.size();
+  c->h2d_bytes += sizeof(QInst) * ninst + (nitems ? sizeof(QRun) * runs.size() : 0) + 4 * chip.size() + 4 * masks.size() +
+                  16 * gv.size();
   QArgs a;
   memset(&a, 0, sizeof(a));  // its bytes are the graph's key
   a.inst = (const QInst*)(base + off_inst);
   a.runs = (const QRun*)(base + off_runs);
+  a.chip = (const int*)(base + off_chip);
   a.emask = (const uint32_t*)(base + off_mask);
   a.gamma = (const double*)(base + off_g);
   a.beta = (const double*)(base + off_b);
   a.tan = (double*)(base + off_tan);
   a.tab = (double2*)(base + off_tab);
   a.part = (double2*)(base + off_part);
+  a.out = (double*)(base + off_out);
   a.next = (unsigned int*)(base + off_cnt);
   a.done = a.next + 2;
   a.status = c->d_status;
   a.spin_limit = g_spin_limit;
   a.work = (double2*)(base + off_work);
   a.nitems = (int)nitems;
+  a.nchip = (int)chip.size();
+  a.chip_bits = chip_bits;
   a.drop = g_drop_item;
-  double* dout = (double*)(base + off_out);
   prof_begin(c);
   cudaError_t e;
   switch (c->batch_threads + T) {
-    case 128 + 11: e = run_batch<128, 11>(c, a, p, ninst, dout, use_graph); break;
-    case 256 + 11: e = run_batch<256, 11>(c, a, p, ninst, dout, use_graph); break;
-    case 512 + 11: e = run_batch<512, 11>(c, a, p, ninst, dout, use_graph); break;
-    case 128 + 12: e = run_batch<128, 12>(c, a, p, ninst, dout, use_graph); break;
-    case 512 + 12: e = run_batch<512, 12>(c, a, p, ninst, dout, use_graph); break;
-    default: e = run_batch<256, 12>(c, a, p, ninst, dout, use_graph); break;
+    case 128 + 11: e = run_batch<128, 11>(c, a, p, ninst, use_graph); break;
+    case 256 + 11: e = run_batch<256, 11>(c, a, p, ninst, use_graph); break;
+    case 512 + 11: e = run_batch<512, 11>(c, a, p, ninst, use_graph); break;
+    case 128 + 12: e = run_batch<128, 12>(c, a, p, ninst, use_graph); break;
+    case 512 + 12: e = run_batch<512, 12>(c, a, p, ninst, use_graph); break;
+    default: e = run_batch<256, 12>(c, a, p, ninst, use_graph); break;
   }
   prof_end(c, PK_BATCH);
-  c->launches += 1 + (p > 0);  // the reduction and the tables (prof_end counted the batch kernel)
+  c->launches += (nitems ? 3 : 0) + (chip.empty() ? 0 : 1) - 1;  // (prof_end counted one)
   if (e != cudaSuccess) return cuda_fail(e, "batch launch");
-  e = cudaMemcpyAsync(out, dout, 8 * (size_t)ninst, cudaMemcpyDeviceToHost, c->stream);
+  e = cudaMemcpyAsync(out, a.out, 8 * (size_t)ninst, cudaMemcpyDeviceToHost, c->stream);
   if (e != cudaSuccess) return cuda_fail(e, "cudaMemcpyAsync(out)");
   c->d2h_bytes += 8 * (size_t)ninst;
   return ctx_finish(c);
