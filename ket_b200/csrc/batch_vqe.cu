@@ -42,7 +42,13 @@ namespace {
 
 constexpr int kVqeMaxQubits = 13;
 constexpr int kVqeMinQubits = 4;    // narrower templates get idle qubits: a coset of a round lies in one instance
-constexpr int kVqeThreads = 512;    // 16 amplitudes a thread of 2^13
+constexpr int kVqeMaxThreads = 512;
+// Threads of a CTA that holds 2^tile amplitudes: 16 amplitudes each, and at least 128 to
+// form the matrices.  At 128 registers a thread an SM then has one CTA of 2^13
+// amplitudes, two of 2^12 or up to four narrower ones; with 512 threads whatever the tile, an
+// SM had one, and 150 instances of 8 qubits ran in two turns (34 us; 24 now).
+constexpr int vqe_threads(int tile) { return tile <= 11 ? 128 : 1 << (tile - 4); }
+static_assert(vqe_threads(kVqeMaxQubits) == kVqeMaxThreads, "the widest tile");
 constexpr int kVqePackBits = 5;     // instances in a pack, at most 32
 // What shared memory holds of a template at a time (a chunk): 2x2 matrices (a 4x4
 // takes 4), rounds and their gates.
@@ -68,7 +74,7 @@ struct BMat {
 
 // Rounds whose matrices are in shared memory together.
 struct BChunk {
-  int32_t round0, nrounds, gate0, ngates, mat0, nmats, slot0;
+  int32_t round0, nrounds, gate0, ngates, mat0, nmats, slot0, nslots;
 };
 
 struct BRoundGate {
@@ -120,6 +126,7 @@ struct BArgs {
   double* energy;
   unsigned int* next;
   int nitems, nparams, tile;  // tile: log2 of the amplitudes a CTA holds
+  int slots, rounds_max;      // matrix slots and rounds of the largest chunk
 };
 
 // G_fam(a) into m (row-major, 2x2 or 4x4), the formulas of gates.ts.
@@ -195,7 +202,7 @@ __device__ __forceinline__ void factor_matrix(const BArgs& a, const BFactor& f, 
 }
 
 __device__ __forceinline__ void copy_words(void* dst, const void* src, int bytes) {
-  for (int i = threadIdx.x; i < bytes / 4; i += kVqeThreads)
+  for (int i = threadIdx.x; i < bytes / 4; i += blockDim.x)
     static_cast<uint32_t*>(dst)[i] = static_cast<const uint32_t*>(src)[i];
 }
 
@@ -239,7 +246,7 @@ __device__ __forceinline__ void run_round(double2* s, const BRound& R, const BRo
                                           int n, int lgpack) {
   constexpr int K = kRoundBits;
   const uint32_t nsub = 1u << (n + lgpack - K);
-  for (uint32_t u = threadIdx.x; u < nsub; u += kVqeThreads) {
+  for (uint32_t u = threadIdx.x; u < nsub; u += blockDim.x) {
     uint32_t base = u;
 #pragma unroll
     for (int i = 0; i < K; i++) base = insert0_32(base, R.piv[i]);
@@ -279,7 +286,7 @@ __device__ __forceinline__ void run_round(double2* s, const BRound& R, const BRo
 __device__ __forceinline__ void run_two(double2* s, const BRound& R, const BRoundGate& g, const double2* mats, int n,
                                         int lgpack) {
   const uint32_t nsub = 1u << (n + lgpack - 2);
-  for (uint32_t u = threadIdx.x; u < nsub; u += kVqeThreads) {
+  for (uint32_t u = threadIdx.x; u < nsub; u += blockDim.x) {
     const uint32_t base = insert0_32(insert0_32(u, R.piv[0]), R.piv[1]);
     if (g.nc && !(controls_ok(g, base) & 1)) continue;
     const uint32_t sb = round_slot(base), l0 = 2 * (__popc(base & R.r2[1]) & 1) + (__popc(base & R.r2[0]) & 1);
@@ -345,13 +352,13 @@ __device__ __forceinline__ double thread_energy(const BArgs& a, const double2* s
 // instance's width: 2048 instances of 8 to 13 qubits and 4 layers 2.16 -> 0.46 ms
 // (FP64 pipe 36% busy; the rest is latency at 16 warps an SM, which 128 KB of state
 // allow).
-__global__ void __launch_bounds__(kVqeThreads) k_batch_vqe(BArgs a) {
+__global__ void __launch_bounds__(kVqeMaxThreads) k_batch_vqe(BArgs a) {
   extern __shared__ __align__(16) unsigned char smraw[];
   double2* s = reinterpret_cast<double2*>(smraw);
   double2* mats = s + (1u << a.tile);
-  BRound* rounds = reinterpret_cast<BRound*>(mats + 4 * kVqeSlots);
-  BRoundGate* gates = reinterpret_cast<BRoundGate*>(rounds + kVqeRounds);
-  __shared__ double red[kVqeThreads / 32];
+  BRound* rounds = reinterpret_cast<BRound*>(mats + 4 * a.slots);
+  BRoundGate* gates = reinterpret_cast<BRoundGate*>(rounds + a.rounds_max);
+  __shared__ double red[kVqeMaxThreads / 32];
   __shared__ int item_sh;
   const int tid = threadIdx.x;
   for (;;) {
@@ -364,14 +371,14 @@ __global__ void __launch_bounds__(kVqeThreads) k_batch_vqe(BArgs a) {
     const int n = T.n, pack = 1 << T.lgpack;
     // a short pack repeats its last instance
     auto instance = [&](int i) { return a.order[item.first + min(i, item.count - 1)]; };
-    for (uint32_t i = tid; i < 1u << (n + T.lgpack); i += kVqeThreads)
+    for (uint32_t i = tid; i < 1u << (n + T.lgpack); i += blockDim.x)
       s[round_slot(i)] = make_double2((i & ((1u << n) - 1)) == 0 ? 1.0 : 0.0, 0.0);
     for (int c = 0; c < T.nchunks; c++) {
       const BChunk C = a.chunks[T.chunk_first + c];
       static_assert(sizeof(BRound) % 4 == 0 && sizeof(BRoundGate) % 4 == 0, "copied as words");
       copy_words(rounds, a.rounds + C.round0, C.nrounds * sizeof(BRound));
       copy_words(gates, a.gates + C.gate0, C.ngates * sizeof(BRoundGate));
-      for (int e = tid; e < C.nmats << T.lgpack; e += kVqeThreads) {
+      for (int e = tid; e < C.nmats << T.lgpack; e += blockDim.x) {
         const BMat B = a.matv[C.mat0 + (e >> T.lgpack)];
         const int i = e & (pack - 1);
         const double* th = a.theta + (size_t)instance(i) * a.nparams;
@@ -514,9 +521,10 @@ int64_t lower_template(std::vector<HOp>& ops, const std::vector<PauliTerm>& term
   int slot = 0;
   BChunk C;
   auto new_chunk = [&]() {
-    C = BChunk{(int32_t)im.rounds.size(), 0, (int32_t)im.gates.size(), 0, (int32_t)im.matv.size(), 0, slot};
+    C = BChunk{(int32_t)im.rounds.size(), 0, (int32_t)im.gates.size(), 0, (int32_t)im.matv.size(), 0, slot, 0};
   };
   auto end_chunk = [&]() {
+    C.nslots = slot - C.slot0;
     if (C.nrounds) im.chunks.push_back(C);
     new_chunk();
   };
@@ -734,18 +742,27 @@ extern "C" int ket_batch_vqe(ket_ctx* c, int ntmpl, const ket_batch_template* tp
     blk[0] = 1; blk[2 * 5] = h; blk[2 * 6 + 1] = h; blk[2 * 9 + 1] = h; blk[2 * 10] = h; blk[2 * 15] = 1;
     dm.insert(dm.end(), blk, blk + 32);
   }
-  // ---- packs: instances by template, as many to a pack as leaves every SM one
+  // ---- packs: instances by template, as few to a pack as lets all packs run at once, and
+  // where no size does, as many as a pack takes
   std::vector<int64_t> count(ntmpl, 0);
   for (int i = 0; i < ninst; i++) {
     if (inst_tmpl[i] < 0 || inst_tmpl[i] >= ntmpl) return fail(KET_ERR_RANGE, "instance template index out of range");
     count[inst_tmpl[i]]++;
   }
   auto pack_bits = [&](int j, int cap) { return std::min(cap, kVqeMaxQubits - im.tmpl[j].n); };
-  int cap = kVqePackBits;
-  for (; cap > 0; cap--) {
+  constexpr size_t kVqeFixed = 64 * kVqeSlots + sizeof(BRound) * kVqeRounds + sizeof(BRoundGate) * kVqeGates;
+  int cap = 0;
+  for (; cap < kVqePackBits; cap++) {
     int64_t packs = 0;
-    for (int j = 0; j < ntmpl; j++) packs += (count[j] + (1 << pack_bits(j, cap)) - 1) >> pack_bits(j, cap);
-    if (packs >= num_sms()) break;
+    int widest = kVqeMinQubits;
+    for (int j = 0; j < ntmpl; j++) {
+      if (count[j] == 0) continue;
+      packs += (count[j] + (1 << pack_bits(j, cap)) - 1) >> pack_bits(j, cap);
+      widest = std::max(widest, im.tmpl[j].n + pack_bits(j, cap));
+    }
+    const int by_regs = kVqeMaxThreads / vqe_threads(widest);
+    const int by_smem = (int)(size_t(227 * 1024) / ((size_t(16) << widest) + kVqeFixed + 1024));
+    if (packs <= (int64_t)num_sms() * std::max(1, std::min(by_regs, by_smem))) break;
   }
   std::vector<int> order(ninst);
   std::vector<BItem> items;
@@ -807,14 +824,17 @@ extern "C" int ket_batch_vqe(ket_ctx* c, int ntmpl, const ket_batch_template* tp
     c->vqe_work_bytes = total;
   }
   char* base = (char*)c->vqe_work;
-  std::vector<unsigned char> img(image, 0);  // everything before the parameters, one copy
+  // One copy for everything before the parameters, and for those where they are few
+  const size_t theta_bytes = 8 * (size_t)ninst * nparams, with = theta_bytes <= (64 << 10) ? theta_bytes : 0;
+  std::vector<unsigned char> img(image + with, 0);
   for (const Part& p : parts)
     if (p.bytes) memcpy(img.data() + p.at, p.src, p.bytes);
+  if (with) memcpy(img.data() + o_theta, theta, with);
   cudaError_t e = cudaMemcpyAsync(base, img.data(), img.size(), cudaMemcpyHostToDevice, c->stream);
-  if (e == cudaSuccess && nparams > 0)
-    e = cudaMemcpyAsync(base + o_theta, theta, 8 * (size_t)ninst * nparams, cudaMemcpyHostToDevice, c->stream);
+  if (e == cudaSuccess && with != theta_bytes)
+    e = cudaMemcpyAsync(base + o_theta, theta, theta_bytes, cudaMemcpyHostToDevice, c->stream);
   if (e != cudaSuccess) return cuda_fail(e, "cudaMemcpyAsync(batch)");
-  c->h2d_bytes += img.size() + 8 * (size_t)ninst * nparams;
+  c->h2d_bytes += image + theta_bytes;
   BArgs a;
   memset(&a, 0, sizeof(a));  // its bytes are the graph's key
   a.tmpl = (const BTmpl*)(base + o_tmpl);
@@ -834,9 +854,19 @@ extern "C" int ket_batch_vqe(ket_ctx* c, int ntmpl, const ket_batch_template* tp
   a.nitems = (int)items.size();
   a.nparams = nparams;
   a.tile = tile;
-  // ---- launch: a resident grid sized for the widest pack's shared memory
-  constexpr size_t kVqeFixed = 64 * kVqeSlots + sizeof(BRound) * kVqeRounds + sizeof(BRoundGate) * kVqeGates;
-  const size_t smem = (size_t(16) << tile) + kVqeFixed;
+  // ---- launch: a resident grid sized for the widest pack's shared memory and the
+  // largest chunk
+  int gates_max = 1;
+  a.slots = a.rounds_max = 1;
+  for (const BTmpl& T : im.tmpl)
+    for (int k = 0; k < T.nchunks; k++) {
+      const BChunk& C = im.chunks[T.chunk_first + k];
+      a.slots = std::max(a.slots, C.nslots << T.lgpack);
+      a.rounds_max = std::max(a.rounds_max, (int)C.nrounds);
+      gates_max = std::max(gates_max, (int)C.ngates);
+    }
+  const int threads = vqe_threads(tile);
+  const size_t smem = (size_t(16) << tile) + 64 * (size_t)a.slots + sizeof(BRound) * a.rounds_max + sizeof(BRoundGate) * gates_max;
   static std::atomic<uint64_t> attr_set{0};
   const uint64_t bit = uint64_t(1) << (c->device & 63);
   if (!(attr_set.load() & bit)) {
@@ -846,11 +876,11 @@ extern "C" int ket_batch_vqe(ket_ctx* c, int ntmpl, const ket_batch_template* tp
     attr_set.fetch_or(bit);
   }
   int per_sm = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch_vqe, kVqeThreads, smem);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch_vqe, threads, smem);
   const int grid = std::max(1, std::min(num_sms() * std::max(1, per_sm), a.nitems));
   auto record = [&]() -> cudaError_t {
     cudaMemsetAsync(a.next, 0, 4, c->stream);
-    k_batch_vqe<<<grid, kVqeThreads, smem, c->stream>>>(a);
+    k_batch_vqe<<<grid, threads, smem, c->stream>>>(a);
     return cudaGetLastError();
   };
   prof_begin(c);
@@ -864,6 +894,7 @@ extern "C" int ket_batch_vqe(ket_ctx* c, int ntmpl, const ket_batch_template* tp
     mix(&a, sizeof(a));
     mix(&smem, sizeof(smem));
     mix(&grid, sizeof(grid));
+    mix(&threads, sizeof(threads));
     if (c->vqe_graph_exec && c->vqe_graph_key == key) {
       e = cudaGraphLaunch(c->vqe_graph_exec, c->stream);
     } else {
