@@ -100,9 +100,9 @@ def batch_vqe(templates, instances, use_graph: bool = True) -> np.ndarray:
         if nmats:
             ops = ops.copy()
             ops["mat"][ops["mat"] >= 0] += nmats
-        all_ops.append(ops)
+        all_ops.append(ops.view(np.uint8))  # (plain bytes join faster than structures)
         all_mats.append(mats)
-        all_binds.append(binds)
+        all_binds.append(binds.view(np.uint8))
         nops, nmats, nbinds = nops + len(ops), nmats + len(mats), nbinds + len(binds)
         for c, o in terms:
             coeffs.append(c)
