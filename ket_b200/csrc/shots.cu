@@ -669,6 +669,11 @@ Jump jump_power(uint64_t d) {
     step.col[k] = Jump::step(1u << k);
     acc.col[k] = 1u << k;
   }
+  if (d <= 64) {  // (few steps are cheaper than their squares)
+    for (; d; d--)
+      for (int k = 0; k < 32; k++) acc.col[k] = Jump::step(acc.col[k]);
+    return acc;
+  }
   while (d) {
     if (d & 1) {
       Jump t;
@@ -953,11 +958,14 @@ template <typename R, int NT>
 cudaError_t launch_shots_t(const SArgs& a, size_t smem, cudaStream_t s) {
   cudaError_t e = cudaFuncSetAttribute(k_shots<R, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  int per_sm = 0;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_shots<R, NT>, NT, smem);
-  if (e != cudaSuccess) return e;
-  if (per_sm < 1) return cudaErrorInvalidConfiguration;
-  const uint64_t grid = std::min<uint64_t>(a.shots, (uint64_t)per_sm * num_sms());
+  uint64_t grid = a.shots;
+  if (grid > (uint64_t)num_sms()) {
+    int per_sm = 0;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_shots<R, NT>, NT, smem);
+    if (e != cudaSuccess) return e;
+    if (per_sm < 1) return cudaErrorInvalidConfiguration;
+    grid = std::min<uint64_t>(grid, (uint64_t)per_sm * num_sms());
+  }
   k_shots<R, NT><<<(unsigned)grid, NT, smem, s>>>(a);
   return cudaGetLastError();
 }
@@ -1007,16 +1015,19 @@ int run_batched(ket_state* st, const std::vector<TOp>& tops, int64_t draws, cons
       std::copy(J.col, J.col + 32, jump.begin() + 32 * i);
     }
   }
-  // the shots' start states, a byte of the state at a time
+  // the shots' start states, a byte of the state at a time (an entry is the XOR of two
+  // filled before it: a jump an entry took 30 us, more than a small call's kernel)
   const Jump J = jump_power((uint64_t)draws);
-  std::vector<uint32_t> byte_img(4 * 256);
-  for (int b = 0; b < 4; b++)
-    for (uint32_t v = 0; v < 256; v++) byte_img[256 * b + v] = J.apply(v << (8 * b));
+  uint32_t byte_img[4][256];
+  for (int b = 0; b < 4; b++) {
+    byte_img[b][0] = 0;
+    for (int v = 1; v < 256; v++) byte_img[b][v] = byte_img[b][v & (v - 1)] ^ J.col[8 * b + __builtin_ctz(v)];
+  }
   std::vector<uint32_t> start(shots);
   uint32_t s = *prng ? *prng : 1u;
   for (size_t i = 0; i < shots; i++) {
     start[i] = s;
-    s = byte_img[s & 255] ^ byte_img[256 + ((s >> 8) & 255)] ^ byte_img[512 + ((s >> 16) & 255)] ^ byte_img[768 + (s >> 24)];
+    s = byte_img[0][s & 255] ^ byte_img[1][(s >> 8) & 255] ^ byte_img[2][(s >> 16) & 255] ^ byte_img[3][s >> 24];
   }
   size_t total = 0;
   struct Part { const void* src; size_t bytes, at; };
