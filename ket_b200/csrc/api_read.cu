@@ -235,26 +235,33 @@ int pauli_terms_expect(const ket_state* s, const std::vector<PauliTerm>& terms, 
   }
   const size_t nres = gl.size() + (tiled.empty() ? 0 : 1);
   if (nres == 0) { *out = 0.0; return KET_OK; }
-  std::vector<PauliTileGroup> hg;
-  std::vector<PauliTileTerm> ht;
+  // the passes' groups, then their terms
+  size_t ng = 0, nt = 0;
   for (const PauliTilePass& P : tiled) {
-    hg.insert(hg.end(), P.groups.begin(), P.groups.end());
-    ht.insert(ht.end(), P.terms.begin(), P.terms.end());
+    ng += P.groups.size();
+    nt += P.terms.size();
+  }
+  const size_t t_at = (sizeof(PauliTileGroup) * ng + 15) & ~size_t(15);
+  std::vector<unsigned char> tables(t_at + sizeof(PauliTileTerm) * nt);
+  unsigned char *gp = tables.data(), *tp = tables.data() + t_at;
+  for (const PauliTilePass& P : tiled) {
+    memcpy(gp, P.groups.data(), sizeof(PauliTileGroup) * P.groups.size());
+    memcpy(tp, P.terms.data(), sizeof(PauliTileTerm) * P.terms.size());
+    gp += sizeof(PauliTileGroup) * P.groups.size();
+    tp += sizeof(PauliTileTerm) * P.terms.size();
   }
   const unsigned grid = tiled.empty() ? 0 : pauli_tile_grid(s->n);
   const size_t part_bytes = std::max<size_t>(gl.empty() ? 0 : pauli_scratch(s->n), 8 * (size_t)grid * tiled.size());
   void* scr;
-  TRY(ctx_scratch(s->ctx, 8 * nres + part_bytes + sizeof(PauliTileGroup) * hg.size() + sizeof(PauliTileTerm) * ht.size() +
-                              2048, &scr));
+  TRY(ctx_scratch(s->ctx, 8 * nres + part_bytes + tables.size() + 1024, &scr));
   double* res = (double*)scr;
   double* partial = (double*)align_up((char*)(res + nres), 256);
   PauliTileGroup* dg = (PauliTileGroup*)align_up((char*)partial + part_bytes, 256);
-  PauliTileTerm* dt = (PauliTileTerm*)align_up((char*)(dg + hg.size()), 256);
+  PauliTileTerm* dt = (PauliTileTerm*)((char*)dg + t_at);
   for (size_t i = 0; i < gl.size(); i++)
     TRY(LAUNCH_READ2(s->ctx, launch_pauli_group(s->amp, s->n, s->precision, gl[i], partial, res + i, s->ctx->stream)));
   if (!tiled.empty()) {
-    TRY(h2d(s->ctx, dg, hg.data(), sizeof(PauliTileGroup) * hg.size()));
-    TRY(h2d(s->ctx, dt, ht.data(), sizeof(PauliTileTerm) * ht.size()));
+    TRY(h2d(s->ctx, dg, tables.data(), tables.size()));
     for (size_t i = 0; i < tiled.size(); i++) {
       TRY(LAUNCH_READ(s->ctx, launch_pauli_tile(s->amp, s->n, s->precision, tiled[i].args, dg, dt, partial + i * grid,
                                                 s->ctx->stream)));
