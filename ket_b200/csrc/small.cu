@@ -8,7 +8,7 @@
 // Here the whole circuit is one cooperative launch over a state that stays in
 // the L2:
 //   * CNOTs, swaps and X gates are relabellings over GF(2) of the whole state
-//     (rounds.h) and move nothing; the last step puts the amplitudes back in order;
+//     (rounds.h) and move nothing; the last pass stores the amplitudes in order;
 //   * a pass takes the next gates, in program order, while their pair masks span at
 //     most 10 to 12 dimensions with the two lowest index bits (so that memory is read in
 //     runs of four).  A CTA holds one coset of the span in shared memory and runs
@@ -99,6 +99,8 @@ struct RArgs {
   uint32_t spin_limit;
   uint32_t beta;               // physical index of logical index l: A l ^ beta
   uint32_t acol[20];
+  uint32_t lbeta;              // logical index of physical index p: B p ^ lbeta
+  uint32_t bcol[20];
 };
 
 __device__ __forceinline__ uint32_t par(uint32_t x) { return (uint32_t)__popc(x) & 1u; }
@@ -256,14 +258,22 @@ __device__ __forceinline__ void copy_words(void* dst, const void* src, int bytes
     static_cast<uint4*>(dst)[i] = __ldg(static_cast<const uint4*>(src) + i);
 }
 
-// Every CTA of the (co-resident) grid has written what it wrote before.  False:
-// the wait ran out (status set).
-__device__ __forceinline__ bool grid_barrier(const RArgs& a, unsigned int target, int* failed) {
+// The grid's barrier in two halves: a CTA's loads and stores before arrive() are done
+// for every CTA after wait().  (The grid is co-resident.)
+__device__ __forceinline__ void arrive(const RArgs& a) {
   __syncthreads();
-  if (gridDim.x == 1) return true;
-  if (threadIdx.x == 0) {
+  if (threadIdx.x == 0 && gridDim.x > 1) {
     __threadfence();
     atomicAdd(a.arrived, 1u);
+  }
+}
+// False: the wait ran out (status set).
+__device__ __forceinline__ bool wait(const RArgs& a, unsigned int target, int* failed) {
+  if (gridDim.x == 1) {
+    __syncthreads();
+    return true;
+  }
+  if (threadIdx.x == 0) {
     volatile unsigned int* p = a.arrived;
     uint32_t spins = 0;
     int bad = 0;
@@ -348,6 +358,8 @@ __global__ void __launch_bounds__(K == 4 ? 256 : 512, K == 4 ? 2 : 1) k_rounds(c
 #pragma unroll
     for (int j = 0; j < (1 << K); j++)
       if (t + nt * j < T) s[round_slot(t + nt * j)] = v[j];
+    const bool last = pass + 1 == a.npasses, scatter = last && a.permute && gridDim.x > 1;
+    if (scatter) arrive(a);  // (this CTA's tile is read)
     for (int r = 0; r < P.nrounds; r++) {
       __syncthreads();
       const RRound& Q = W.rounds[r];
@@ -363,7 +375,7 @@ __global__ void __launch_bounds__(K == 4 ? 256 : 512, K == 4 ? 2 : 1) k_rounds(c
       }
     }
     __syncthreads();
-    if (pass + 1 == a.npasses && gridDim.x == 1) {
+    if (last && gridDim.x == 1) {
       // one tile, whose index is the physical index: written in logical order
       for (uint32_t l = t; l < N; l += nt) {
         uint32_t p = a.beta;
@@ -373,31 +385,41 @@ __global__ void __launch_bounds__(K == 4 ? 256 : 512, K == 4 ? 2 : 1) k_rounds(c
       }
       return;
     }
+    if (scatter) {
+      // in logical order, over other CTAs' tiles: once every CTA has read its own
+      met += gridDim.x;
+      if (!wait(a, met, &failed)) return;
+      auto logical = [&](uint32_t p) {
+        uint32_t l = 0;
+        for (int b = 0; b < a.n; b++)
+          if ((p >> b) & 1) l ^= a.bcol[b];
+        return l;
+      };
+      const uint32_t l0 = logical(cbase ^ tl) ^ a.lbeta;
+      uint32_t lhi[K];
+#pragma unroll
+      for (int b = 0; b < K; b++) lhi[b] = logical(hi[b]);
+#pragma unroll
+      for (int j = 0; j < (1 << K); j++) {
+        uint32_t l = l0;
+#pragma unroll
+        for (int b = 0; b < K; b++)
+          if ((j >> b) & 1) l ^= lhi[b];
+        if (t + nt * j < T) amp[l] = s[round_slot(t + nt * j)];
+      }
+      return;
+    }
 #pragma unroll
     for (int j = 0; j < (1 << K); j++) {
       const uint32_t p = index(j);
       if (t + nt * j < T && p < N) amp[p] = s[round_slot(t + nt * j)];
     }
-    if (pass + 1 < a.npasses) fetch(pass + 1);
+    if (last) return;
+    arrive(a);
+    fetch(pass + 1);
     met += gridDim.x;
-    if (!grid_barrier(a, met, &failed)) return;
+    if (!wait(a, met, &failed)) return;
   }
-  if (!a.permute) return;
-  // every logical index's amplitude into registers, then, once all are, into place
-  double2 v[1 << K];
-  const uint32_t l0 = blockIdx.x * T + t;
-#pragma unroll
-  for (int j = 0; j < (1 << K); j++) {
-    const uint32_t l = l0 + nt * j;
-    uint32_t p = a.beta;
-    for (int b = 0; b < a.n; b++)
-      if ((l >> b) & 1) p ^= a.acol[b];
-    v[j] = __ldcg(amp + p);
-  }
-  met += gridDim.x;
-  if (!grid_barrier(a, met, &failed)) return;
-#pragma unroll
-  for (int j = 0; j < (1 << K); j++) amp[l0 + nt * j] = v[j];
 }
 
 // ---------------------------------------------------------------- planning
@@ -681,6 +703,12 @@ struct SPlan {
 size_t rounds_smem(int d) { return (sizeof(double2) << d) + 2 * sizeof(Records); }
 template <int K>
 unsigned rounds_threads(int d) { return std::max(32u, 1u << (d - K)); }
+// A launch of one CTA has four warps from 8 qubits on: those beyond a round's cosets share
+// the loads and the ordered store (an H on 8 qubits by one warp: 39.5 us a call, 32.8 by
+// four; on 10 qubits sixteen in place of four make every round's barrier dearer,
+// 112 us a circuit and 118).
+template <int K>
+unsigned rounds_threads_alone(int d) { return std::max(d >= 8 ? 128u : 32u, 1u << (d - K)); }
 
 // CTAs that are resident together.
 template <int K>
@@ -697,7 +725,7 @@ cudaError_t rounds_resident(int device, int d, int* ctas) {
 template <int K>
 cudaError_t launch_rounds(const RArgs& a, unsigned grid, cudaStream_t s) {
   const size_t smem = rounds_smem(a.d);
-  const unsigned nt = rounds_threads<K>(a.d);
+  const unsigned nt = grid == 1 ? rounds_threads_alone<K>(a.d) : rounds_threads<K>(a.d);
   cudaError_t e = cudaFuncSetAttribute(k_rounds<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   if (grid == 1) {
@@ -768,6 +796,11 @@ int run_small(ket_state* s, const std::vector<Gate>& gates, bool prune, bool* ra
     a.acol[q] = P.col[q];
     if (q < s->n && P.col[q] != 1u << q) a.permute = 1;
   }
+  if (a.permute && grid > 1)
+    for (int q = 0; q < s->n; q++) {
+      for (uint32_t r = P.row[q]; r; r &= r - 1) a.bcol[__builtin_ctz(r)] |= 1u << q;
+      a.lbeta |= ((uint32_t)__builtin_popcount(P.beta & P.row[q]) & 1u) << q;
+    }
   prof_begin(c);
   const cudaError_t e = P.rb_ == 4 ? launch_rounds<4>(a, grid, c->stream) : launch_rounds<3>(a, grid, c->stream);
   prof_end(c, PK_FUSED1);
