@@ -196,6 +196,55 @@ __global__ void __launch_bounds__(128) k_matk_reg(typename Vec2<R>::T* a, uint64
   }
 }
 
+// k >= 5, few groups: a CTA a group, staged in shared memory (inputs xs, outputs ys,
+// global indices idx), a thread a row.  The tiles of k_matk below work off 2^12
+// amplitudes a CTA however few there are.  Up to these many groups this is the faster
+// (us, this / tiles, c128, at the line and at twice as many groups): 5 qubits 31 / 33 and
+// 48 / 33, 6 qubits 26 / 54 and 61 / 54, 7 qubits 79 / 87 and 210 / 87, 8 qubits 150 / 164
+// and 291 / 164, 10 qubits 1194 / 1420 and 2940 / 1418; one group of 5 qubits 12 / 28.
+constexpr uint64_t kMatkGroups[KET_MAX_OP_QUBITS - 4] = {2048, 512, 512, 256, 128, 128};
+template <typename R>
+__global__ void k_matk_group(typename Vec2<R>::T* a, uint64_t ngroups, int k, const int* tq, const double* mat, int prune,
+                             double thr, double qthr) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  const uint32_t D = 1u << k;
+  cpx<R>* xs = reinterpret_cast<cpx<R>*>(smraw);
+  cpx<R>* ys = xs + D;
+  uint64_t* idx = reinterpret_cast<uint64_t*>(ys + D);
+  int sorted[KET_MAX_OP_QUBITS];
+  for (int j = 0; j < k; j++) sorted[j] = tq[j];
+  for (int x = 1; x < k; x++)
+    for (int y = x; y > 0 && sorted[y - 1] > sorted[y]; y--) { int t = sorted[y]; sorted[y] = sorted[y - 1]; sorted[y - 1] = t; }
+  for (uint64_t g = blockIdx.x; g < ngroups; g += gridDim.x) {
+    uint64_t ctx = g;
+    for (int j = 0; j < k; j++) ctx = insert0(ctx, sorted[j]);
+    for (uint32_t i = threadIdx.x; i < D; i += blockDim.x) {
+      uint64_t b = ctx;
+      for (int bit = 0; bit < k; bit++)
+        if ((i >> (k - 1 - bit)) & 1) b |= uint64_t(1) << tq[bit];
+      idx[i] = b;
+      xs[i] = ld_amp<R>(a + b);
+    }
+    __syncthreads();
+    for (uint32_t r = threadIdx.x; r < D; r += blockDim.x) {
+      double sr = 0, si = 0;
+      const double* row = mat + 2 * (size_t)r * D;
+      for (uint32_t c = 0; c < D; c++) {
+        const double mr = row[2 * c], mi = row[2 * c + 1];
+        const double xr = xs[c].re, xi = xs[c].im;
+        sr = fma(mr, xr, fma(-mi, xi, sr));
+        si = fma(mr, xi, fma(mi, xr, si));
+      }
+      cpx<R> o{(R)sr, (R)si};
+      if (prune) prune_amp(o, thr, qthr);
+      ys[r] = o;
+    }
+    __syncthreads();
+    for (uint32_t r = threadIdx.x; r < D; r += blockDim.x) st_amp<R>(a + idx[r], ys[r]);
+    __syncthreads();
+  }
+}
+
 // k >= 5: a CTA multiplies the matrix by the 2^12 amplitudes of GB = 2^(12-k)
 // groups, held in shared memory as FP64; each thread accumulates 4 rows x 4
 // groups in registers, so 8 shared-memory reads feed 64 FMAs, and the matrix
@@ -459,6 +508,12 @@ cudaError_t launch_gate_t(const Gate& g, void* ampv, int n, const void* dev_matk
       if (k == 4) { launch_matk_reg<R, 4>(a, ngroups, g, pr, thr, qthr, s); break; }
       const int* dq = reinterpret_cast<const int*>(dev_matk);
       const double2* dm = reinterpret_cast<const double2*>(reinterpret_cast<const char*>(dev_matk) + 64);
+      if (ngroups <= kMatkGroups[k - 5]) {
+        const size_t smem = (2 * sizeof(cpx<R>) + sizeof(uint64_t)) << k;  // (at most 40 KB)
+        k_matk_group<R><<<(unsigned)std::min<uint64_t>(ngroups, (uint64_t)num_sms() * 8), 256, smem, s>>>(
+            a, ngroups, k, dq, reinterpret_cast<const double*>(dm), pr, thr, qthr);
+        break;
+      }
       cudaFuncSetAttribute(k_matk<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMatkSmem);
       const uint64_t ctas = (ngroups + (uint64_t(1) << (12 - k)) - 1) >> (12 - k);
       k_matk<R><<<(unsigned)std::min<uint64_t>(ctas, (uint64_t)num_sms() * 2), kMatkThreads, kMatkSmem, s>>>(
