@@ -576,13 +576,19 @@ __global__ void __launch_bounds__(NT, chip_min_blocks<NT>()) k_qaoa_chip(QArgs a
       rx_bits<NT>(s, n, cb, sb);
     }
     __syncthreads();
-    double acc = 0.0;
+    // over the norm: n p rotations with one rounded cosine and sine let it drift (9
+    // qubits, 4 layers: <C> off by 1.9e-14, over the norm by 1.6e-15)
+    double acc = 0.0, nrm = 0.0;
     for (uint32_t x = threadIdx.x; x < N; x += NT) {
       const double2 v = s[sw(x)];
-      acc += (v.x * v.x + v.y * v.y) * (double)cutb[x];
+      const double q = v.x * v.x + v.y * v.y;
+      nrm += q;
+      acc = fma(q, (double)cutb[x], acc);
     }
     acc = block_sum<NT>(acc, red);
-    if (threadIdx.x == 0) a.out[i] = acc;
+    __syncthreads();
+    nrm = block_sum<NT>(nrm, red);
+    if (threadIdx.x == 0) a.out[i] = acc / nrm;
     __syncthreads();
   }
 }
