@@ -364,8 +364,8 @@ std::vector<std::string> enqueue(Cache& C, const std::vector<JitPass>& passes, i
   bool queued = false;
   for (size_t i = 0; i < passes.size(); i++) {
     const JitPass& p = passes[i];
-    // the constant op array holds at most 64 KB (512 records)
-    if (!p.prog || (size_t)p.nops * sizeof(jit::COp) > 60000) continue;
+    static_assert(KET_JIT_MAX_OPS * sizeof(jit::COp) <= 60000, "the constant op array");
+    if (!p.prog || p.nops > KET_JIT_MAX_OPS) continue;
     keys[i] = shape_key(p.prog, p.nops, precision, p.nreg, p.staged);
     if (C.map.find(keys[i]) == C.map.end()) {
       // below min_qubits a ready kernel is used but none is compiled

@@ -17,6 +17,7 @@ namespace ket {
 // Distinct program shapes a process compiles at most (their modules stay
 // loaded for the life of the process).
 #define KET_JIT_MAX_KERNELS 4096
+#define KET_JIT_MAX_OPS 468 // ops of a compiled pass: its constant array holds at most 64 KB
 
 struct JitPass {
   const FOp* prog = nullptr;  // host copy of the pass's program; null = not a register-tiled pass

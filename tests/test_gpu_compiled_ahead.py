@@ -98,3 +98,14 @@ def test_compiled_ahead_with_default_options_still_serves():
     got, ran = run(14, abi)
     want, _ = run(14, abi, specialize=-1)
     assert ran > 0 and np.array_equal(got, want)
+
+
+@pytest.mark.parametrize("precision,prune,cut", [(0, True, False), (0, False, True), (1, True, True)])
+def test_passes_beyond_a_kernel(precision, prune, cut):
+    """More ops than a compiled kernel holds: cut for kernels, or one pass of the interpreter
+    where that is the faster (complex128 with pruning)."""
+    n = 22
+    abi = long_circuit(n, 27, 5).to_abi()
+    want, _ = run(n, abi, precision, prune=prune, specialize=-1)
+    got, ran = run(n, abi, precision, prune=prune, specialize=1)
+    assert (ran > 1 if cut else ran == 0) and np.array_equal(got, want)
