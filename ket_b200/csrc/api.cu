@@ -585,15 +585,15 @@ int ket_apply_ops(ket_state* s, const ket_op* ops, size_t nops, const double* ma
     if (ran) return ctx_finish(s->ctx);
   }
   plan_passes(s->n, s->precision, o.fusion, o.prune != 0, plan);
-  // Below KET_JIT_AUTO_QUBITS qubits the interpreter, whose code does not grow with the
-  // pass, takes whole passes; from there on it runs what is being compiled.
+  // (the interpreter's code does not grow with the pass: it takes whole passes)
   if (o.specialize == 1 || ahead || (o.specialize == 0 && s->n >= KET_JIT_AUTO_QUBITS)) {
-    const size_t whole = plan.passes.size();
+    const std::vector<Pass> whole = plan.passes;
     split_long_passes(s->n, s->precision, o.prune != 0, tiled_nreg(s->n, o.reg_bits), plan);
-    // (a later call with the default options has to cut alike to find these kernels)
-    if (o.specialize == 1 && plan.passes.size() != whole && s->n < KET_JIT_AUTO_QUBITS && default_programs(s->n, o)) {
-      rc = run_plan(s, plan, o);
-      if (!rc) note_ahead(circuit_hash(s->n, s->precision, o.prune != 0, plan.gates));
+    if (plan.passes.size() != whole.size()) {
+      rc = run_plan(s, plan, o, true, 0, SIZE_MAX, o.specialize == 0 ? &whole : nullptr);
+      // (a later call with the default options has to cut alike to find these kernels)
+      if (!rc && o.specialize == 1 && s->n < KET_JIT_AUTO_QUBITS && default_programs(s->n, o))
+        note_ahead(circuit_hash(s->n, s->precision, o.prune != 0, plan.gates));
       return rc;
     }
   }
@@ -604,7 +604,8 @@ int ket_apply_ops(ket_state* s, const ket_op* ops, size_t nops, const double* ma
 
 namespace ket {
 
-int run_plan(ket_state* s, const Plan& plan, const ket_exec_opts& o, bool wait, size_t first, size_t last) {
+int run_plan(ket_state* s, const Plan& plan, const ket_exec_opts& o, bool wait, size_t first, size_t last,
+             const std::vector<Pass>* whole) {
   ket_ctx* c = s->ctx;
   cudaSetDevice(c->device);
   const bool prune = o.prune != 0;
@@ -647,6 +648,18 @@ int run_plan(ket_state* s, const Plan& plan, const ket_exec_opts& o, bool wait, 
     std::string err;
     int rc = jit_prepare(jp, s->precision, o.specialize, c->stream, jf, err);
     if (rc) return fail(rc, err);
+    if (whole) {
+      for (size_t i = 0; i < np; i++) {
+        if (!use2[i] || jf[i].fn) continue;
+        Plan p;
+        p.gates = plan.gates;
+        p.passes = *whole;
+        p.anc = plan.anc;
+        ket_exec_opts oi = o;
+        oi.specialize = -1;
+        return run_plan(s, p, oi, wait);
+      }
+    }
     for (size_t i = 0; i < np; i++)
       if (use2[i] && !jf[i].fn && jit_nr != KET_FUSED_NREG) lower_pass(i, KET_FUSED_NREG);
   }

@@ -76,8 +76,10 @@ int ctx_upload(ket_ctx* ctx, void* dst, const void* src, size_t bytes);
 // launches are queued (the caller waits and reads the status word later);
 // every buffer the passes read is stream-ordered, so queued plans may follow
 // one another.  first, last: run only passes [first, last) of the plan.
+// whole: the plan's passes before they were cut for compiled kernels; they run on the
+// interpreter instead where a kernel of the cut ones is not ready (specialize = 0).
 int run_plan(ket_state* s, const Plan& plan, const ket_exec_opts& o, bool wait = true, size_t first = 0,
-             size_t last = SIZE_MAX);
+             size_t last = SIZE_MAX, const std::vector<Pass>* whole = nullptr);
 // A circuit on a complex128 state of up to kSmallQubits qubits in one launch (small.cu).
 constexpr int kSmallQubits = 20;
 int run_small(ket_state* s, const std::vector<Gate>& gates, bool prune, bool* ran);

@@ -100,6 +100,20 @@ def test_compiled_ahead_with_default_options_still_serves():
     assert ran > 0 and np.array_equal(got, want)
 
 
+def test_whole_passes_until_kernels_are_ready():
+    """From 26 qubits on a default call whose cut passes still wait for their kernels takes
+    the whole passes on the interpreter; once the kernels are ready it runs those."""
+    n = 26
+    abi = long_circuit(n, 10, 77).to_abi()
+    want, ran = run(n, abi, specialize=-1)
+    assert ran == 0
+    first, ran = run(n, abi)
+    assert ran == 0 and np.array_equal(first, want)
+    _lib.check(_lib.lib().ket_jit_wait())
+    got, ran = run(n, abi)
+    assert ran > 1 and np.array_equal(got, want)
+
+
 @pytest.mark.parametrize("precision,prune,cut", [(0, True, False), (0, False, True), (1, True, True)])
 def test_passes_beyond_a_kernel(precision, prune, cut):
     """More ops than a compiled kernel holds: cut for kernels, or one pass of the interpreter
