@@ -978,12 +978,14 @@ void plan_program(const Plan& plan, const Pass& p, int precision, bool prune, in
 namespace {
 
 // Machine instructions of an op in a compiled kernel, roughly: what it does to
-// each of the thread's 2^nreg amplitudes, unrolled.  (Pruning a gate's amplitudes is 10 a
-// complex128 one and 17 a complex64 one by the sizes of kernels that differ by it.)
-int code_estimate(const FOp& f, int nreg, int precision) {
+// each of the thread's 2^nreg amplitudes, unrolled.  `rare`: with the flush of pruned
+// amplitudes, which most tiles jump over (by the sizes of kernels that differ by
+// pruning, its screen and flush are 10 instructions an amplitude at complex128 and 17 at
+// complex64).
+int code_estimate(const FOp& f, int nreg, int precision, bool rare) {
   const int ns = 1 << nreg, words = precision == KET_C64 ? 2 : 4;  // 32-bit words an amplitude (shuffles, selects)
   const bool plain = f.flags & (FOF_REAL | FOF_RXFORM);
-  const int prune = f.flags & FOF_PRUNE ? (precision == KET_C64 ? 17 : 10) * ns : 0;
+  const int prune = f.flags & FOF_PRUNE ? (!rare ? 6 : precision == KET_C64 ? 17 : 10) * ns : 0;
   switch (f.type) {
     case FO_CONT: case FO_X1R: case FO_RELAY: case FO_SYNC: return 8;
     case FO_EXCH: return 2 * ns + 100;
@@ -1016,17 +1018,20 @@ double code_weight(const Gate& g) {
 // instruction cache is fetched again for every tile.  A 24-qubit pass of 99 ops (11
 // exchanges) spent half its issue slots without an instruction, 990 us where two
 // passes of half its ops take 304 and 280; an extra pass costs a read and a write of
-// the state, 82 us.  So passes are cut into equal parts of at most kCodeLimit
-// instructions of 16 bytes, 104 KB.  Limits of 5000 / 6500 / 8000 / 10000: 24 qubits, 240
-// pruned one-qubit gates on ten of them 4.92 / 5.04 / 5.08 / 6.45 ms (whole 22.5), at
-// complex64 8.29 / 7.91 / 7.90 / 8.69, 26 qubits at complex64 unpruned 7.40 / 7.95 / 9.30 /
-// 9.12, the gradient of 8 parameter vectors at 24 qubits 131.7 / 130.5 / 131.0 / 134.3.
+// the state, 82 us.  So passes of more than kCodeLimit instructions of 16 bytes, 128 KB,
+// are cut into equal parts of at most kCodePart, 104 KB.  What is rarely run counts for
+// the parts but not for the decision: counted there too, the passes of pruned ansatz
+// and brickwork circuits are cut that gain nothing (25 qubits, 3.92 -> 4.35 ms and at
+// complex64 4.76 -> 5.13).  Parts of 5000 / 6500 / 8000 / 10000: 24 qubits, 240 pruned
+// one-qubit gates on ten of them 4.92 / 5.04 / 5.08 / 6.45 ms (whole 22.5), at complex64
+// 8.29 / 7.91 / 7.90 / 8.69, 26 qubits at complex64 unpruned 7.40 / 7.95 / 9.30 / 9.12, the
+// gradient of 8 parameter vectors at 24 qubits 131.7 / 130.5 / 131.0 / 134.3.
 // Below kCutQubits a pass is shorter than the launch and the second lowering that a
 // cut costs: with cuts a compiled complex64 circuit of 16 qubits took 1100 us against
 // 888, of 19 qubits 1300 against 1138; 21 qubits are even (1634 and 1508 against 1566
 // and 1620), 22 gain (1815 against 2056).
 void split_long_passes(int n, int precision, bool prune, int nreg, Plan& plan) {
-  constexpr int kCodeLimit = 6500, kCutQubits = 22;
+  constexpr int kCodeLimit = 8000, kCodePart = 6500, kCutQubits = 22;
   if (n < kCutQubits) return;
   std::vector<Pass> out;
   std::vector<FOp> prog;
@@ -1034,16 +1039,17 @@ void split_long_passes(int n, int precision, bool prune, int nreg, Plan& plan) {
   for (Pass& p : plan.passes) {
     double w = 0;
     for (int gi : p.gates) w += code_weight(plan.gates[gi]);
-    // (a gate's code with its share of the exchanges is below 6 weights a slot)
-    if (!(p.fused && p.m == KET_T2_BITS) || 6 * w * (1 << nreg) < kCodeLimit) {
+    // (a gate's code with its share of the exchanges is below 4 weights a slot)
+    if (!(p.fused && p.m == KET_T2_BITS) || 4 * w * (1 << nreg) < kCodeLimit) {
       out.push_back(std::move(p));
       continue;
     }
     plan_program(plan, p, precision, prune, nreg, prog, lp, sp);
-    int code = 0;
+    int code = 0, all = 0;
     bool merged = false;
     for (const FOp& f : prog) {
-      code += code_estimate(f, nreg, precision);
+      code += code_estimate(f, nreg, precision, false);
+      all += code_estimate(f, nreg, precision, true);
       merged = merged || f.type == FO_CPHASE || f.type == FO_PPOLY;
     }
     // What a kernel cannot hold whole runs on the interpreter, which beats the parts
@@ -1051,7 +1057,7 @@ void split_long_passes(int n, int precision, bool prune, int nreg, Plan& plan) {
     // one pass, 16.8 in 60; on 26, where a thread holds 16 amplitudes, 63.4 and 51.9).
     const bool interpreted = (int)prog.size() > KET_JIT_MAX_OPS && precision == KET_C128 && prune && nreg == KET_FUSED_NREG;
     // (a cut between phases that merge into one op would change their rounding)
-    const int parts = merged || interpreted ? 1 : (code + kCodeLimit - 1) / kCodeLimit;
+    const int parts = merged || interpreted || code <= kCodeLimit ? 1 : (all + kCodePart - 1) / kCodePart;
     double at = 0;
     int part = 0;
     Pass q = p;
