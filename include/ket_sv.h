@@ -95,10 +95,14 @@ typedef struct ket_exec_opts {
                           pass's program where one is ready (from earlier runs or ket_jit_compile),
                           the interpreter otherwise, compiling on background threads for states of
                           26+ qubits; 1 = compile what is
-                          missing first, then use compiled kernels only; -1 = interpreter only.
+                          missing first, then use compiled kernels only (a pass of more than 468
+                          ops that is not cut stays with the interpreter); -1 = interpreter only.
                           Results are identical either way.  With every option automatic, a
-                          complex128 circuit of up to 20 qubits whose kernels were not compiled
-                          ahead runs in one launch instead, equal to these to rounding.  No
+                          complex128 circuit of up to 20 qubits that ket_jit_compile was not
+                          given runs in one launch instead, equal to these to rounding
+                          (where the device holds that launch's grid).  complex64
+                          circuits take the passes at every size: in the launch's order their
+                          roundings would show in what is read from them.  No
                           counterpart in the reference. */
   int32_t reg_bits;    /* register bits of the compiled kernels' programs: 0 = automatic (default:
                           5 below 26 qubits, 4 from there on), 4 or 5 = that count at any size, so

@@ -301,8 +301,8 @@ __device__ __forceinline__ void tile_cut(const double2* v, const QMap& m, int t,
 // Bound: for wide instances the state's traffic (2 p reads and writes) and shared
 // memory's (a tile moves through it four times a pass), then the FP64 pipe (two
 // FMAs an amplitude and Rx).  512 instances of 10 to 22 qubits, p = 4:
-// 35.9 ms as 2 p passes of three-bit rounds, 15.3 now (FP64 pipe 28% busy, HBM a
-// fifth; two CTAs of 8 warps wait for barriers and loads).
+// 35.9 ms as 2 p passes of three-bit rounds, 15.3 now (96 of 13 to 20 qubits: FP64 pipe 27%
+// busy, HBM 20%; two CTAs of 8 warps wait for barriers and loads).
 template <int NT, int T>
 __global__ void __launch_bounds__(NT, QLay<NT, T>::CTAS) k_batch_qaoa(QArgs a) {
   typedef QLay<NT, T> L;

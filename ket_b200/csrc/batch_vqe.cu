@@ -6,9 +6,10 @@
 // per parameter vector.  Here a batch names circuit templates (an op list whose
 // parametric ops are bound to parameters, the same bindings as the adjoint
 // gradient) and instances (a template and a parameter vector).  A persistent
-// grid pulls work from a queue, largest first; one CTA runs one instance
-// with its whole state in shared memory (up to 13 qubits, 128 KB), or a pack of up
-// to 32 instances of one template of fewer qubits:
+// grid pulls work from a queue, largest first; one CTA, of 128 to 512 threads by the
+// amplitudes it holds, runs one instance with its whole state in shared memory (up to 13
+// qubits, 128 KB), or, where not all would run at once, a pack of up to 32 instances of
+// one template of fewer qubits:
 //   * |0...0>, then the ops in order, with the reference's per-gate pruning
 //     (accumulate(), statevector.ts:19-27) after each matrix op.  CNOTs and
 //     swaps are relabellings, and one-qubit gates run in rounds of up to 16 on
@@ -349,9 +350,9 @@ __device__ __forceinline__ double thread_energy(const BArgs& a, const double2* s
 
 // Bound: the FP64 pipe (8 FMAs an amplitude and gate).  In place of one pass over
 // shared memory and one barrier per op, with one CTA of 8 warps an SM whatever the
-// instance's width: 2048 instances of 8 to 13 qubits and 4 layers 2.16 -> 0.46 ms
-// (FP64 pipe 36% busy; the rest is latency at 16 warps an SM, which 128 KB of state
-// allow).
+// instance's width: 2048 instances of 8 to 13 qubits and 4 layers 2.16 -> 0.41 ms
+// (FP64 pipe 31% busy, issue slots 41%; the rest is latency at 16 warps an SM, which
+// 128 KB of state allow).
 __global__ void __launch_bounds__(kVqeMaxThreads) k_batch_vqe(BArgs a) {
   extern __shared__ __align__(16) unsigned char smraw[];
   double2* s = reinterpret_cast<double2*>(smraw);

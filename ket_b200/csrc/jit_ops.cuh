@@ -199,13 +199,14 @@ __device__ __forceinline__ void realize_swaps(cpx<R> (&x)[1 << NR], Tile& t) {
 }
 
 // Add a thread's share of an adjoint probe to its partial sum.  With up to
-// KET_PROBE_THREAD_SLOTS probes (KET_PROBE_PER_THREAD) every thread keeps its own
+// kProbeThreadSlots probes (jit.cpp; KET_PROBE_PER_THREAD) every thread keeps its own
 // sum a probe in shared memory, one read and one write nothing waits for, and the
 // threads' sums meet once, after the last tile; a warp sum a probe and tile was a
 // chain of five shuffles and additions that four warps a scheduler did not hide.
 // More probes (two CTAs' sums no longer fit an SM) take the warp sums.  With the
 // forms below, a 24-qubit probe pass (25 qubits with the ancilla, 10 to 21 probes):
-// 458 -> 349 us.  Bound now: latency at 16 warps an SM (FP64 pipe 41%, HBM 36%).
+// 458 -> 349 us.  Bound now: latency at 16 warps an SM, at most half of whose issue slots are
+// taken (passes of 200, 271 and 349 us: FP64 pipe 39, 65 and 43%, HBM 64, 47 and 36%).
 __device__ __forceinline__ void probe_add(const Tile& t, int slot, double v) {
 #ifdef KET_PROBE_PER_THREAD
   t.sgrad[slot * KET_PROBE_PER_THREAD + t.tid] += v;

@@ -154,8 +154,8 @@ __global__ void k_set_one(V* a) {
 // kernel parameter, so every product reads its entry from the constant bank
 // and nothing is staged or synchronised.  Bound: HBM at k = 3 (32 FP64 FMAs an
 // amplitude), about even with the FP64 pipe at k = 4 (64).  In place of one CTA
-// per group: 3 qubits on 2^25 c64 amplitudes 5.9 -> 0.08 ms, 4 qubits on 2^22
-// c128 amplitudes 0.91 -> 0.05 ms.
+// per group: 3 qubits on 2^25 c64 amplitudes 5.9 -> 0.09 ms, 4 qubits on 2^22
+// c128 amplitudes 0.91 -> 0.026 ms.
 template <int K>
 struct MatKArgs {
   uint64_t off[1 << K];   // amplitude offset of local index i

@@ -245,7 +245,8 @@ __global__ void __launch_bounds__(256) k_marginals(const typename Vec2<R>::T* a,
 // outside the mask are folded, and the warps' sums added in shared memory.  Every
 // load is of consecutive amplitudes and every block runs 16 of them a thread, where
 // a thread a bin over 2^20 indices left most of the chip idle (20 qubits, 10 low
-// qubits: one block, 489 -> 8 us; 27 qubits: 2.86 -> 0.30 ms).
+// qubits: one block, 489 -> 16 us, half of them k_marginal_dist_combine's; 27 qubits: 2.86 ->
+// 0.31 ms).
 template <typename R>
 __global__ void __launch_bounds__(256) k_marginal_dist(const typename Vec2<R>::T* a, int n, int c, uint64_t mask,
                                                        double* partial) {

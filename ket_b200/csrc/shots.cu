@@ -619,7 +619,7 @@ __global__ void __launch_bounds__(NT, NT <= 64 ? 8 : 512 / NT) k_shots(const __g
       double before = carry;
       for (int w = 0; w < (t >> 5); w++) before = __dadd_rn(before, red[w]);
       for (int w = 0; w < NW; w++) carry = __dadd_rn(carry, red[w]);
-      // the sum before the thread's own entries (rounded, so kept from going below 0)
+      // the sum before the thread's own entries
       const double y = __shfl_up_sync(0xffffffffu, incl, 1);
       if (t & 31) before = __dadd_rn(before, y);
       double w = before;

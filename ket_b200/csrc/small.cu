@@ -295,9 +295,9 @@ __device__ __forceinline__ bool wait(const RArgs& a, unsigned int target, int* f
 // have to be resident two an SM.  (16 at 16 qubits: 290 us against 221; a gate's
 // straight-line code is half as long and twice the warps hide its latency.)
 // Bound: latency -- of a gate (about 0.4 us of dependent reads, FP64 chain and
-// pruning screen) and of a pass (about 3 us of barrier, loads and stores).  20
-// brickwork layers of 16 qubits: 487 us in 20 launches and 770 of planning before,
-// 210 and 90 now; QFT of 20 qubits 142 and 220, 130 and 75 now.
+// pruning screen) and of a pass (about 3 us of barrier, loads and stores); issue slots
+// are 13 to 24% taken.  20 brickwork layers of 16 qubits: 487 us in 20 launches and 770 of
+// planning before, 210 and 90 now; QFT of 20 qubits 142 and 220, 127 and 75 now.
 template <int K>
 __global__ void __launch_bounds__(K == 4 ? 256 : 512, K == 4 ? 2 : 1) k_rounds(const __grid_constant__ RArgs a) {
   extern __shared__ __align__(16) unsigned char smraw[];
