@@ -79,3 +79,22 @@ def test_against_the_oracle(sizes, ninst, depth):
         want = energy(oracle(inst[i][1]).simulate(mode=O.DENSE_PRUNE).dense(), terms)
         # FP64 rounding of `depth` gates and their terms, and of merged diagonal factors
         assert abs(got[i] - want) <= 1e-14 * depth * sum(abs(c) for c, _ in terms), i
+
+
+@pytest.mark.parametrize("n", [1, 3, 5, 6, 8, 9, 10, 11, 12, 13])
+@pytest.mark.parametrize("ninst,strings", [(1, 1), (3, 37), (160, 90), (700, 20)])
+def test_shares_of_the_hamiltonian(n, ninst, strings):
+    """Threads beyond an instance's amplitudes take a share of its flip groups: fewer groups
+    than shares, more, and packs."""
+    from oracle import oracle as O
+    ansatz, _, oracle = template(n, 20, 7 * n)
+    r = np.random.default_rng(n + ninst)
+    terms = [(float(r.normal()), "".join(r.choice(list("IXYZ"), n))) for _ in range(strings)]
+    inst = [(0, r.uniform(0, 2 * math.pi, 5)) for _ in range(ninst)]
+    got = batch_vqe([(ansatz, terms)], inst)
+    ident = sum(c for c, o in terms if set(o) == {"I"})
+    rest = [(c, o) for c, o in terms if set(o) != {"I"}]
+    for i in {0, ninst - 1, ninst // 2}:
+        want = ident + energy(oracle(inst[i][1]).simulate(mode=O.DENSE_PRUNE).dense(), rest)
+        # FP64 rounding of 20 gates and the terms
+        assert abs(got[i] - want) <= 2e-13 * sum(abs(c) for c, _ in terms)
