@@ -171,21 +171,32 @@ struct SNoise {
   uint16_t ma, ra, mb, rb;
   int32_t two;
 };
-// Gates between measurements, resets and ifs, as many as shared memory holds.
+// Gates between measurements, resets and ifs, as many as shared memory holds: round0,
+// gate0 and slot0 are places in the segment's chunk.
 struct SSeg {
-  int32_t round0, nrounds, gate0, ngates, slot0, nslots;
+  int32_t chunk, round0, nrounds, gate0, ngates, slot0;
   int32_t noise0, ndraws, per, jump0;  // draws, draws a thread, first jump row
+};
+// Segments whose records are in shared memory together (a program that fits is read
+// once a CTA; one that measures after every gate is not read again for each: with draws
+// stepped from the draw before, 200 measurements of 4 qubits, 100 shots, 1260 us before
+// and 990 now, 100 of 10 qubits, 1000 shots, 1400 and 1270, 50 of 12, 2000, 3440 and 3120).
+struct SChunk {
+  int32_t round0, nrounds, gate0, ngates, slot0, nslots;
 };
 enum { ST_SEG = 0, ST_MEASURE = 1, ST_RESET = 2, ST_IF = 3 };
 struct SStep {
   int32_t kind;
-  int32_t a, b, c, d;  // SEG: index; MEASURE: cbit, jump row; RESET: -, jump row; IF: first, size, value, steps to skip
+  // SEG: index; MEASURE: cbit, jump row, steps from the draw of the one before (0: jump);
+  // RESET: -, jump row, steps; IF: first, size, value, steps to skip
+  int32_t a, b, c, d;
   uint16_t r, m;       // MEASURE, RESET: the qubit's functional and mask (r = 0: a qubit outside the state)
 };
 
 struct SArgs {
   const SStep* steps;
   const SSeg* segs;
+  const SChunk* chunks;
   const SRound* rounds;
   const SGate* gates;
   const double2* mats;   // by 64-byte slots
@@ -197,7 +208,7 @@ struct SArgs {
   uint64_t shots, init;
   ket_noise nz;
   int nsteps, n, ne, ncbits;  // ne: qubits with idle ones
-  int last_row;               // jump row of the sampling draw
+  int last_row, last_gap;     // jump row of the sampling draw, or its steps
   // shared-memory layout (bytes)
   int off_mats, off_rounds, off_gates, off_events, off_red, off_bits;
   uint16_t acol[kRoundQubits];  // the final relabelling: physical mask of each logical bit
@@ -502,6 +513,15 @@ __global__ void __launch_bounds__(NT, NT <= 64 ? 8 : 512 / NT) k_shots(const __g
   for (uint64_t shot = blockIdx.x; shot < a.shots; shot += gridDim.x) {
     const uint32_t s0 = a.start[shot];
     uint32_t beta = 0, zeta = 0;
+    uint32_t xd = s0;  // the stream at the last measurement's or reset's draw
+    auto draw = [&](int gap, int row) {
+      if (gap > 0) {
+        for (int k = 0; k < gap; k++) xd = xs_step(xd);
+      } else {
+        xd = xs_jump(a.jump + 32 * row, s0);
+      }
+      return xd;
+    };
     for (uint32_t i = t; i < 1u << n; i += NT) stc(st, round_slot(i), cd{i == a.init ? 1.0 : 0.0, 0.0});
     for (int b = t; b < a.ncbits; b += NT) bits[b] = 0;
     __syncthreads();
@@ -510,12 +530,15 @@ __global__ void __launch_bounds__(NT, NT <= 64 ? 8 : 512 / NT) k_shots(const __g
       const int kind = o.kind;
       if (kind == ST_SEG) {
         const SSeg S = a.segs[o.a];
-        if (loaded != o.a) {
-          copy_words(rounds, a.rounds + S.round0, S.nrounds * sizeof(SRound), NT);
-          copy_words(gates, a.gates + S.gate0, S.ngates * sizeof(SGate), NT);
-          copy_words(mats, a.mats + 4 * S.slot0, S.nslots * 64, NT);
-          loaded = o.a;
+        if (loaded != S.chunk) {
+          const SChunk C = a.chunks[S.chunk];
+          copy_words(rounds, a.rounds + C.round0, C.nrounds * sizeof(SRound), NT);
+          copy_words(gates, a.gates + C.gate0, C.ngates * sizeof(SGate), NT);
+          copy_words(mats, a.mats + 4 * C.slot0, C.nslots * 64, NT);
+          loaded = S.chunk;
         }
+        SGate* sgates = gates + S.gate0;
+        const double2* smats = mats + 4 * S.slot0;
         if (t == 0) nev = 0;
         __syncthreads();
         const int d0 = t * S.per, d1 = min(d0 + S.per, S.ndraws);
@@ -546,8 +569,8 @@ __global__ void __launch_bounds__(NT, NT <= 64 ? 8 : 512 / NT) k_shots(const __g
         for (int g = t; g < S.ngates; g += NT) {
           uint32_t f = beta | zeta << 16;
           for (int e = 0; e < ne; e++)
-            if (events[e].d < gates[g].dpos) f ^= events[e].bz;
-          gates[g].frame = f;
+            if (events[e].d < sgates[g].dpos) f ^= events[e].bz;
+          sgates[g].frame = f;
         }
         for (int e = 0; e < ne; e++) {
           beta ^= events[e].bz & 0xffffu;
@@ -555,20 +578,20 @@ __global__ void __launch_bounds__(NT, NT <= 64 ? 8 : 512 / NT) k_shots(const __g
         }
         for (int q = 0; q < S.nrounds; q++) {
           __syncthreads();
-          const SRound& Q = rounds[q];
-          const SGate* G = gates + Q.gate0;
+          const SRound& Q = rounds[S.round0 + q];
+          const SGate* G = sgates + Q.gate0;
           if (Q.dense) {
             switch (Q.k) {
-              case 2: shot_dense<R, NT, 2>(st, Q, *G, mats, n); break;
-              case 3: shot_dense<R, NT, 3>(st, Q, *G, mats, n); break;
-              default: shot_dense<R, NT, 4>(st, Q, *G, mats, n); break;
+              case 2: shot_dense<R, NT, 2>(st, Q, *G, smats, n); break;
+              case 3: shot_dense<R, NT, 3>(st, Q, *G, smats, n); break;
+              default: shot_dense<R, NT, 4>(st, Q, *G, smats, n); break;
             }
           } else {
-            shot_round<R, NT>(st, Q, G, mats, n);
+            shot_round<R, NT>(st, Q, G, smats, n);
           }
         }
       } else if (kind == ST_MEASURE || kind == ST_RESET) {
-        uint32_t x = xs_jump(a.jump + 32 * o.b, s0);
+        uint32_t x = draw(o.c, o.b);
         const int outcome = shot_collapse<R, NT>(st, n, o.r, beta, xs_value(x), red);
         if (kind == ST_RESET) {
           if (outcome == 1) beta ^= o.m;
@@ -588,7 +611,7 @@ __global__ void __launch_bounds__(NT, NT <= 64 ? 8 : 512 / NT) k_shots(const __g
     // sampleSV (circuit.ts:75-83): the first logical index whose running sum of
     // |a|^2 reaches the draw, else the last nonzero entry.  Thread t holds logical
     // indices 16 t .. 16 t + 15; a scan gives it the sum before them.
-    uint32_t x = xs_jump(a.jump + 32 * a.last_row, s0);
+    uint32_t x = draw(a.last_gap, a.last_row);
     const double r = xs_value(x);
     if (t == 0) { pick = 0xffffffffu; last = 0; }
     const uint32_t N = 1u << a.n;
@@ -750,12 +773,14 @@ struct ShotPlan {
   int ne = 0, nt = 0;
   std::vector<SStep> steps;
   std::vector<SSeg> segs;
+  std::vector<SChunk> chunks;
   std::vector<SRound> rounds;
   std::vector<SGate> gates;
   std::vector<double> mats;    // 8 doubles a slot
   std::vector<SNoise> noise;
   std::vector<int64_t> rows;   // draw index (0-based) of each jump row
   SCaps used = {0, 0, 0, 0};
+  int last_gap = 0;
   uint16_t acol[kRoundQubits];
 };
 
@@ -808,8 +833,9 @@ class ShotPlanner {
           SStep s = {};
           s.kind = o.kind == KET_OP_MEASURE ? ST_MEASURE : ST_RESET;
           s.a = o.kind == KET_OP_MEASURE ? q[1] : -1;
+          s.c = gap();
           s.b = (int)P.rows.size();
-          P.rows.push_back(draw_);
+          if (!s.c) P.rows.push_back(draw_);
           draw_ += o.kind == KET_OP_MEASURE && flips_ ? 2 : 1;
           if (q[0] >= 0 && q[0] < n_) { s.r = rp_.row[q[0]]; s.m = rp_.col[q[0]]; }
           P.steps.push_back(s);
@@ -832,7 +858,8 @@ class ShotPlanner {
   void finish() {
     end_segment();
     std::copy(rp_.col, rp_.col + kRoundQubits, P.acol);
-    P.rows.push_back(draw_);
+    P.last_gap = gap();
+    if (!P.last_gap) P.rows.push_back(draw_);
   }
   void set_flips(bool f) { flips_ = f; }
 
@@ -847,8 +874,16 @@ class ShotPlanner {
   std::vector<int> dpos_;              // per gate of it, in program order
   int ndraws_ = 0;
   int64_t draw_ = 0;                   // first draw of the segment
+  int64_t last_draw_ = -1;             // of the last measurement or reset
   bool flips_ = false;
 
+  // Steps from there to the next draw, which becomes the last; 0 where a jump is the
+  // shorter way (a row from memory, 32 columns: as long as some 30 steps).
+  int gap() {
+    const int64_t g = draw_ - last_draw_;
+    last_draw_ = draw_;
+    return g <= 24 ? (int)g : 0;
+  }
   void x1(int c, int t, int op) { gate(t, &c, 1, true, op); }
   static int slots_of(int k) { return k <= 1 ? 1 : 1 << (2 * k - 2); }
   void room(int slots) {
@@ -872,11 +907,23 @@ class ShotPlanner {
     rp_.close();
     if (rp_.rounds.empty() && ndraws_ == 0) return;
     SSeg S = {};
-    S.round0 = (int)P.rounds.size();
+    const int slot0 = (int)(P.mats.size() / 8);
     S.nrounds = (int)rp_.rounds.size();
-    S.gate0 = (int)P.gates.size();
     S.ngates = (int)rp_.gates.size();
-    S.slot0 = (int)(P.mats.size() / 8);
+    int nslots = 0;
+    for (const Round& r : rp_.rounds)
+      for (int g = r.gate0; g < r.gate0 + r.ngates; g++) nslots += rp_.gates[g].x ? 0 : r.dense ? slots_of(r.k) : 1;
+    if (P.chunks.empty() || P.chunks.back().nrounds + S.nrounds > caps_.rounds ||
+        P.chunks.back().ngates + S.ngates > caps_.gates || P.chunks.back().nslots + nslots > caps_.slots)
+      P.chunks.push_back(SChunk{(int)P.rounds.size(), 0, (int)P.gates.size(), 0, slot0, 0});
+    SChunk& C = P.chunks.back();
+    S.chunk = (int)P.chunks.size() - 1;
+    S.round0 = C.nrounds;
+    S.gate0 = C.ngates;
+    S.slot0 = C.nslots;
+    C.nrounds += S.nrounds;
+    C.ngates += S.ngates;
+    C.nslots += nslots;
     int slot = 0;
     for (const Round& r : rp_.rounds) {
       SRound Q = {};
@@ -913,7 +960,6 @@ class ShotPlanner {
         P.gates.push_back(G);
       }
     }
-    S.nslots = slot;
     S.noise0 = (int)P.noise.size();
     S.ndraws = ndraws_;
     P.noise.insert(P.noise.end(), noise_.begin(), noise_.end());
@@ -921,9 +967,9 @@ class ShotPlanner {
     S.jump0 = (int)P.rows.size();
     for (int d = 0; d < ndraws_; d += std::max(S.per, 1)) P.rows.push_back(draw_ + d);
     draw_ += ndraws_;
-    P.used.rounds = std::max(P.used.rounds, S.nrounds);
-    P.used.gates = std::max(P.used.gates, S.ngates);
-    P.used.slots = std::max(P.used.slots, S.nslots);
+    P.used.rounds = std::max(P.used.rounds, C.nrounds);
+    P.used.gates = std::max(P.used.gates, C.ngates);
+    P.used.slots = std::max(P.used.slots, C.nslots);
     P.used.draws = std::max(P.used.draws, S.ndraws);
     SStep st = {};
     st.kind = ST_SEG;
@@ -1041,7 +1087,7 @@ int run_batched(ket_state* st, const std::vector<TOp>& tops, int64_t draws, cons
     parts.push_back(Part{v.data(), v.size() * sizeof(v[0]), place(v.size() * sizeof(v[0]))});
     return parts.back().at;
   };
-  const size_t o_steps = part(P.steps), o_segs = part(P.segs), o_rounds = part(P.rounds), o_gates = part(P.gates),
+  const size_t o_steps = part(P.steps), o_segs = part(P.segs), o_chunks = part(P.chunks), o_rounds = part(P.rounds), o_gates = part(P.gates),
                o_mats = part(P.mats), o_noise = part(P.noise), o_jump = part(jump), o_start = part(start);
   const size_t image = total, o_idx = place(8 * shots), o_bits = place(shots * ncbits);
   void* scr;
@@ -1057,6 +1103,7 @@ int run_batched(ket_state* st, const std::vector<TOp>& tops, int64_t draws, cons
   memset(&a, 0, sizeof(a));
   a.steps = (const SStep*)(base + o_steps);
   a.segs = (const SSeg*)(base + o_segs);
+  a.chunks = (const SChunk*)(base + o_chunks);
   a.rounds = (const SRound*)(base + o_rounds);
   a.gates = (const SGate*)(base + o_gates);
   a.mats = (const double2*)(base + o_mats);
@@ -1073,6 +1120,7 @@ int run_batched(ket_state* st, const std::vector<TOp>& tops, int64_t draws, cons
   a.ne = P.ne;
   a.ncbits = ncbits;
   a.last_row = (int)P.rows.size() - 1;
+  a.last_gap = P.last_gap;
   std::copy(P.acol, P.acol + kRoundQubits, a.acol);
   size_t smem = (st->precision == KET_C64 ? sizeof(float2) : sizeof(double2)) << P.ne;
   auto area = [&](size_t bytes) {
