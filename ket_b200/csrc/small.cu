@@ -99,8 +99,8 @@ struct RArgs {
   uint32_t spin_limit;
   uint32_t beta;               // physical index of logical index l: A l ^ beta
   uint32_t acol[20];
-  uint32_t lbeta;              // logical index of physical index p: B p ^ lbeta
-  uint32_t bcol[20];
+  // (in memory: a launch carries what each of its blocks reads)
+  const uint32_t* inverse;     // logical index of physical index p: B p ^ lbeta; lbeta, then B's columns
 };
 
 __device__ __forceinline__ uint32_t par(uint32_t x) { return (uint32_t)__popc(x) & 1u; }
@@ -262,17 +262,13 @@ __device__ __forceinline__ void copy_words(void* dst, const void* src, int bytes
 // for every CTA after wait().  (The grid is co-resident.)
 __device__ __forceinline__ void arrive(const RArgs& a) {
   __syncthreads();
-  if (threadIdx.x == 0 && gridDim.x > 1) {
+  if (threadIdx.x == 0) {
     __threadfence();
     atomicAdd(a.arrived, 1u);
   }
 }
 // False: the wait ran out (status set).
 __device__ __forceinline__ bool wait(const RArgs& a, unsigned int target, int* failed) {
-  if (gridDim.x == 1) {
-    __syncthreads();
-    return true;
-  }
   if (threadIdx.x == 0) {
     volatile unsigned int* p = a.arrived;
     uint32_t spins = 0;
@@ -298,7 +294,8 @@ __device__ __forceinline__ bool wait(const RArgs& a, unsigned int target, int* f
 // pruning screen) and of a pass (about 3 us of barrier, loads and stores); issue slots
 // are 13 to 24% taken.  20 brickwork layers of 16 qubits: 487 us in 20 launches and 770 of
 // planning before, 210 and 90 now; QFT of 20 qubits 142 and 220, 127 and 75 now.
-template <int K>
+// ALONE: one CTA, without the grid's code (10 qubits 48.3 -> 46.6 us).
+template <int K, bool ALONE>
 __global__ void __launch_bounds__(K == 4 ? 256 : 512, K == 4 ? 2 : 1) k_rounds(const __grid_constant__ RArgs a) {
   extern __shared__ __align__(16) unsigned char smraw[];
   double2* s = reinterpret_cast<double2*>(smraw);
@@ -358,7 +355,7 @@ __global__ void __launch_bounds__(K == 4 ? 256 : 512, K == 4 ? 2 : 1) k_rounds(c
 #pragma unroll
     for (int j = 0; j < (1 << K); j++)
       if (t + nt * j < T) s[round_slot(t + nt * j)] = v[j];
-    const bool last = pass + 1 == a.npasses, scatter = last && a.permute && gridDim.x > 1;
+    const bool last = pass + 1 == a.npasses, scatter = !ALONE && last && a.permute;
     if (scatter) arrive(a);  // (this CTA's tile is read)
     for (int r = 0; r < P.nrounds; r++) {
       __syncthreads();
@@ -375,7 +372,7 @@ __global__ void __launch_bounds__(K == 4 ? 256 : 512, K == 4 ? 2 : 1) k_rounds(c
       }
     }
     __syncthreads();
-    if (last && gridDim.x == 1) {
+    if (ALONE && last) {
       // one tile, whose index is the physical index: written in logical order
       for (uint32_t l = t; l < N; l += nt) {
         uint32_t p = a.beta;
@@ -392,10 +389,10 @@ __global__ void __launch_bounds__(K == 4 ? 256 : 512, K == 4 ? 2 : 1) k_rounds(c
       auto logical = [&](uint32_t p) {
         uint32_t l = 0;
         for (int b = 0; b < a.n; b++)
-          if ((p >> b) & 1) l ^= a.bcol[b];
+          if ((p >> b) & 1) l ^= __ldg(a.inverse + 1 + b);
         return l;
       };
-      const uint32_t l0 = logical(cbase ^ tl) ^ a.lbeta;
+      const uint32_t l0 = logical(cbase ^ tl) ^ __ldg(a.inverse);
       uint32_t lhi[K];
 #pragma unroll
       for (int b = 0; b < K; b++) lhi[b] = logical(hi[b]);
@@ -415,6 +412,11 @@ __global__ void __launch_bounds__(K == 4 ? 256 : 512, K == 4 ? 2 : 1) k_rounds(c
       if (t + nt * j < T && p < N) amp[p] = s[round_slot(t + nt * j)];
     }
     if (last) return;
+    if constexpr (ALONE) {
+      fetch(pass + 1);
+      __syncthreads();
+      continue;
+    }
     arrive(a);
     fetch(pass + 1);
     met += gridDim.x;
@@ -715,8 +717,9 @@ template <int K>
 cudaError_t rounds_resident(int device, int d, int* ctas) {
   const int smem = (int)rounds_smem(d);
   int per_sm = 0, sms = 0;
-  cudaError_t e = cudaFuncSetAttribute(k_rounds<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_rounds<K>, rounds_threads<K>(d), smem);
+  cudaError_t e = cudaFuncSetAttribute(k_rounds<K, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e == cudaSuccess)
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_rounds<K, false>, rounds_threads<K>(d), smem);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
   *ctas = per_sm * sms;
   return e;
@@ -725,15 +728,19 @@ cudaError_t rounds_resident(int device, int d, int* ctas) {
 template <int K>
 cudaError_t launch_rounds(const RArgs& a, unsigned grid, cudaStream_t s) {
   const size_t smem = rounds_smem(a.d);
-  const unsigned nt = grid == 1 ? rounds_threads_alone<K>(a.d) : rounds_threads<K>(a.d);
-  cudaError_t e = cudaFuncSetAttribute(k_rounds<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
-  if (grid == 1) {
-    k_rounds<K><<<1, nt, smem, s>>>(a);
-    return cudaGetLastError();
+  if constexpr (K == 3) {  // (tiles of fewer than 2^10 amplitudes are never part of a grid)
+    if (grid == 1) {
+      const cudaError_t e =
+          cudaFuncSetAttribute(k_rounds<K, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      if (e != cudaSuccess) return e;
+      k_rounds<K, true><<<1, rounds_threads_alone<K>(a.d), smem, s>>>(a);
+      return cudaGetLastError();
+    }
   }
+  const cudaError_t e = cudaFuncSetAttribute(k_rounds<K, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
   void* args[] = {const_cast<RArgs*>(&a)};
-  return cudaLaunchCooperativeKernel((const void*)k_rounds<K>, dim3(grid), dim3(nt), args, smem, s);
+  return cudaLaunchCooperativeKernel((const void*)k_rounds<K, false>, dim3(grid), dim3(rounds_threads<K>(a.d)), args, smem, s);
 }
 
 }  // namespace
@@ -757,7 +764,8 @@ int run_small(ket_state* s, const std::vector<Gate>& gates, bool prune, bool* ra
     if (grid > (unsigned)(g_max_ctas > 0 ? g_max_ctas : fit)) return KET_OK;
   }
   if (!P.lower(gates, prune)) return KET_OK;
-  size_t total = 256;  // the barrier's counter
+  constexpr size_t kInverse = 128;
+  size_t total = 256;  // the barrier's counter, then the relabelling's inverse
   auto place = [&](size_t bytes) {
     const size_t at = total;
     total += (bytes + 255) & ~size_t(255);
@@ -773,6 +781,20 @@ int run_small(ket_state* s, const std::vector<Gate>& gates, bool prune, bool* ra
   if (!P.rounds.empty()) memcpy(img.data() + o_round, P.rounds.data(), sizeof(RRound) * P.rounds.size());
   if (!P.gates.empty()) memcpy(img.data() + o_gate, P.gates.data(), sizeof(RGate) * P.gates.size());
   if (!P.mats.empty()) memcpy(img.data() + o_mat, P.mats.data(), 8 * P.mats.size());
+  const bool permute = [&] {
+    for (int q = 0; q < s->n; q++)
+      if (P.col[q] != 1u << q) return true;
+    return P.beta != 0;
+  }();
+  if (permute && grid > 1) {
+    uint32_t inv[21] = {};
+    for (int q = 0; q < s->n; q++) {
+      for (uint32_t r = P.row[q]; r; r &= r - 1) inv[1 + __builtin_ctz(r)] |= 1u << q;
+      inv[0] |= ((uint32_t)__builtin_popcount(P.beta & P.row[q]) & 1u) << q;
+    }
+    static_assert(kInverse + sizeof(inv) <= 256, "before the passes");
+    memcpy(img.data() + kInverse, inv, sizeof(inv));
+  }
   c->h2d_bytes += total;
   rc = ctx_upload(c, dev, img.data(), total);
   if (rc) return rc;
@@ -791,16 +813,9 @@ int run_small(ket_state* s, const std::vector<Gate>& gates, bool prune, bool* ra
   a.d = P.d;
   a.spin_limit = g_spin_limit;
   a.beta = P.beta;
-  a.permute = P.beta != 0;
-  for (int q = 0; q < 20; q++) {
-    a.acol[q] = P.col[q];
-    if (q < s->n && P.col[q] != 1u << q) a.permute = 1;
-  }
-  if (a.permute && grid > 1)
-    for (int q = 0; q < s->n; q++) {
-      for (uint32_t r = P.row[q]; r; r &= r - 1) a.bcol[__builtin_ctz(r)] |= 1u << q;
-      a.lbeta |= ((uint32_t)__builtin_popcount(P.beta & P.row[q]) & 1u) << q;
-    }
+  a.permute = permute;
+  a.inverse = (const uint32_t*)(base + kInverse);
+  std::copy(P.col, P.col + 20, a.acol);
   prof_begin(c);
   const cudaError_t e = P.rb_ == 4 ? launch_rounds<4>(a, grid, c->stream) : launch_rounds<3>(a, grid, c->stream);
   prof_end(c, PK_FUSED1);
