@@ -174,9 +174,10 @@ uint64_t circuit_hash(int n, int precision, bool prune, const std::vector<Gate>&
   for (const Gate& g : gates) {
     mix((uint64_t)g.type << 32 | (uint64_t)(g.t0 + 1) << 16 | (uint64_t)(g.t1 + 1) << 8 | g.prune);
     mix(g.cmask);
+    const int entries = g.type == G_MAT2 ? 16 : g.type == G_MAT1 || g.type == G_DIAG2 ? 4 : g.type == G_DIAG1 ? 2 : 0;
     uint64_t form = 0;
-    if (g.type != G_X1 && g.type != G_SWAP)  // (which have no matrix)
-      for (const cd& z : g.m) form = form << 3 | (uint64_t)(z.re == 0) | (uint64_t)(z.im == 0) << 1 | (uint64_t)(z.re == 1) << 2;
+    for (int e = 0; e < entries; e++)
+      form = form << 3 | (uint64_t)(g.m[e].re == 0) | (uint64_t)(g.m[e].im == 0) << 1 | (uint64_t)(g.m[e].re == 1) << 2;
     mix(form);
     for (int q : g.tk) mix((uint64_t)q + 1);
   }
